@@ -306,6 +306,11 @@ int lm_debug_inject_wait(lm_ctx* ctx, double seconds);
  * 1 <= bins <= 256. */
 int lm_distance_histogram(lm_ctx* ctx, const float* lat, const float* lon, int64_t n, const int64_t* seg, int n_seg,
                           int bins, double radius_m, uint64_t* counts);
+/* The same with one histogram per species (sandbox/pairwise_distance_histogram_distributed.jl:130-147):
+ * the points of species 1, 2, 3 (host int8 [n]; other values are in no histogram and may be
+ * non-finite) are the three segments, in index order. counts: host uint64 [3][bins + 1]. */
+int lm_species_histogram(lm_ctx* ctx, const float* lat, const float* lon, const int8_t* species, int64_t n, int bins,
+                         double radius_m, uint64_t* counts);
 
 #ifdef __cplusplus
 }

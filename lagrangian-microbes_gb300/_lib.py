@@ -145,6 +145,7 @@ SIGNATURES = {
     "lm_adjoint_cell_signature": [P, P],
     "lm_adjoint_final_positions": [P, P, P],
     "lm_distance_histogram": [P, P, P, I64, P, I32, I32, F64, P],
+    "lm_species_histogram": [P, P, P, P, I64, I32, F64, P],
     "lm_debug_inject_wait": [P, F64],
 }
 

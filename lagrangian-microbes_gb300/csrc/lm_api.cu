@@ -105,6 +105,10 @@ struct lm_ctx {
   uint32_t snap_slots = 0;
   int64_t snap_step = -1;
 
+  // working arrays of the synchronous calls (ctx_scratch)
+  unsigned char* scratch = nullptr;
+  size_t scratch_n = 0;
+
   // pair log
   uint32_t* plog = nullptr;
   uint32_t plog_cap = 0;
@@ -834,7 +838,7 @@ int lm_ctx_destroy(lm_ctx* c) {
                    c->rank,   c->sid,   c->skey,   c->sens,   c->deg,    c->slab,    c->longv,
                    c->wstate, c->level,  c->act,    c->spos,
                    c->map_d,  c->block_ens, c->ens_d, c->grids, c->eord, c->ebox, c->census,  c->ccount, c->cstart,
-                   c->csum,   c->ovf,   c->oprio,  c->ctrl,   c->plog,  c->snap_xo, c->snap_yo, c->snap_sp,
+                   c->csum,   c->ovf,   c->oprio,  c->ctrl,   c->plog,  c->scratch, c->snap_xo, c->snap_yo, c->snap_sp,
                    c->snap_st};
   for (void* p : bufs_)
     if (p) cudaFree(p);
@@ -1545,6 +1549,23 @@ int ctx_device(const lm_ctx* c) { return c->device; }
 int ctx_sms(const lm_ctx* c) { return c->sms; }
 cudaStream_t ctx_stream(const lm_ctx* c) { return c->st; }
 void ctx_set_error(lm_ctx* c, const char* msg) { c->err = msg ? msg : ""; }
+int ctx_scratch(lm_ctx* c, size_t bytes, void** p) {
+  if (bytes > c->scratch_n) {
+    CK(cudaSetDevice(c->device));
+    if (c->scratch) cudaFree(c->scratch);
+    c->scratch = nullptr;
+    c->scratch_n = 0;
+    const cudaError_t e = cudaMalloc((void**)&c->scratch, bytes);
+    if (e != cudaSuccess) {
+      c->scratch = nullptr;
+      cudaGetLastError();
+      return fail(c, LM_ERR_OOM, "cudaMalloc of %zu bytes of scratch failed: %s", bytes, cudaGetErrorString(e));
+    }
+    c->scratch_n = bytes;
+  }
+  *p = c->scratch;
+  return LM_OK;
+}
 
 bool uniform_axis(const double* a, int n, double* d) {
   if (n < 2) return false;

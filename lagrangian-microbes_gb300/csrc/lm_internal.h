@@ -406,6 +406,9 @@ int ctx_device(const lm_ctx* c);
 int ctx_sms(const lm_ctx* c);
 cudaStream_t ctx_stream(const lm_ctx* c);
 void ctx_set_error(lm_ctx* c, const char* msg);
+// A device buffer of at least `bytes` owned by the context (grown, never shrunk, freed with it), for
+// the working arrays of one synchronous call; its contents do not outlive the call.
+int ctx_scratch(lm_ctx* c, size_t bytes, void** p);
 
 // Ordered-int encoding of floats for atomicMin/atomicMax.
 __host__ __device__ inline uint32_t enc_f(float f) {

@@ -71,8 +71,20 @@ def species_distance_histograms(lons, lats, species, bins: int = 70, radius: flo
     if not (lons.size == lats.size == species.size):
         raise ValueError("lons, lats and species differ in length")
     kinds = (ROCK, PAPER, SCISSORS)
-    order = np.concatenate([np.flatnonzero(species == k) for k in kinds])
-    sizes = [int(np.count_nonzero(species == k)) for k in kinds]
-    seg = np.concatenate([[0], np.cumsum(sizes)])
-    c = _histograms(lats[order], lons[order], seg, bins, radius, device, ctx)
+    if species.dtype != np.int8:  # codes of any other type, compared before they are narrowed
+        codes = np.zeros(species.size, np.int8)
+        for k in kinds:
+            codes[species == k] = k
+        species = codes
+    counts = np.zeros((len(kinds), bins + 1), np.uint64)
+    lats, lons, species = (np.ascontiguousarray(a) for a in (lats, lons, species))
+    own = ctx is None
+    ctx = ctx or _lib.Context(device)
+    try:
+        ctx.call("lm_species_histogram", _lib.ptr(lats), _lib.ptr(lons), _lib.ptr(species), lats.size, int(bins),
+                 float(radius), _lib.ptr(counts))
+    finally:
+        if own:
+            ctx.close()
+    c = counts.astype(np.int64)
     return {k: (c[s, :bins], int(c[s, bins])) for s, k in enumerate(kinds)}

@@ -139,3 +139,52 @@ def test_short_route_gives_the_reference_chain_bins(pdh, monkeypatch):
         monkeypatch.delenv("LM_HIST_EXACT")
         np.testing.assert_array_equal(fast[0], exact[0])
         assert fast[1] == exact[1]
+
+
+def _layout(rng, name, n):
+    if name == "patch":
+        return _points(rng, n, box=(25.0, 30.0, 200.0, 205.0))
+    if name == "globe":
+        lat, lon = rng.uniform(-90, 90, n), rng.uniform(-180, 180, n)
+        lat[: n // 8] *= -1
+        return lat.astype(np.float32), lon.astype(np.float32)
+    # metre-scale clumps with outliers across the domain: tiles much wider than their leaves
+    lat, lon = _points(rng, n, box=(20.0, 40.0, 20.0, 40.0))
+    k = n - n // 16
+    lat[:k] = (30 + 1e-4 * rng.random(k)).astype(np.float32)
+    lon[:k] = (25 + 1e-3 * rng.random(k)).astype(np.float32)
+    lat[: n // 4] = lat[0]
+    return lat, lon
+
+
+@pytest.mark.parametrize("layout", ["patch", "globe", "clumps"])
+@pytest.mark.parametrize("n", [2, 7, 8, 9, 31, 33, 255, 256, 257, 264, 513, 3001])
+def test_counts_by_groups_of_points_equal_the_reference_chain(pdh, monkeypatch, layout, n):
+    """Whole groups of pairs counted from their boxes, leaf pairs against one threshold, ragged leaves
+    and tiles: the bins are the chain's for every pair (integers, so exactly)."""
+    rng = np.random.default_rng(1000 + n)
+    lat, lon = _layout(rng, layout, n)
+    for bins in (1, 66, 256):
+        fast = pdh.pairwise_distance_histogram(lat, lon, bins)
+        monkeypatch.setenv("LM_HIST_EXACT", "1")
+        exact = pdh.pairwise_distance_histogram(lat, lon, bins)
+        monkeypatch.delenv("LM_HIST_EXACT")
+        np.testing.assert_array_equal(fast[0], exact[0])
+        assert fast[1] == exact[1] and fast[0].sum() + fast[1] == n * (n - 1) // 2
+
+
+@pytest.mark.parametrize("dtype", [np.int8, np.uint8, np.int64, np.float64])
+def test_species_of_any_type_select_the_same_points(pdh, dtype):
+    rng = np.random.default_rng(17)
+    lat, lon = _points(rng, 1000, box=(25.0, 30.0, 200.0, 205.0))
+    species = rng.integers(0, 6, 1000)
+    species[:20] = 3  # an uneven split
+    codes = species.astype(dtype)
+    if np.dtype(dtype).itemsize > 1:
+        codes[species == 5] = 257  # not a species, although its low byte is one
+    lat[species == 0] = np.nan  # in no histogram
+    got = pdh.species_distance_histograms(lon, lat, codes, 70)
+    for k in (1, 2, 3):
+        want = pdh.pairwise_distance_histogram(lat[species == k], lon[species == k], 70)
+        np.testing.assert_array_equal(got[k][0], want[0])
+        assert got[k][1] == want[1]
