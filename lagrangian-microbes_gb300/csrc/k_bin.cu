@@ -426,23 +426,24 @@ void launch_cell_scan(const Bufs& b, Ctrl* ctrl, cudaStream_t st) {
 }
 
 // Particles into cell order: id, key, ensemble, position.
-__global__ void __launch_bounds__(SLOT_BLOCK) k_scatter(Bufs b, Ctrl* ctrl) {
+__global__ void __launch_bounds__(SLOT_BLOCK) k_scatter(Bufs b, Ctrl* ctrl, int dense) {
   pdl_wait();
   if (ctrl->halt) return;
   const uint32_t p = blockIdx.x * SLOT_BLOCK + threadIdx.x;
   if (p >= b.nslots) return;
   const uint32_t key = b.key[p];
   if (key == NONE) return;
-  const uint32_t s = b.cstart[key] + b.rank[p];
+  const uint32_t rank = b.rank[p], s = b.cstart[key] + rank;
+  if (dense && rank == COUNT_DENSE - 1) b.act[atomicAdd(&ctrl->act_n, 1u)] = key;  // once per dense cell
   b.sid[s] = p;
   b.skey[s] = key;
   b.sens[s] = b.block_ens[blockIdx.x];
   b.spos[s] = make_float2(b.plon[p], b.plat[p]);
 }
 
-void launch_scatter(const Bufs& b, Ctrl* ctrl, cudaStream_t st) {
+void launch_scatter(const Bufs& b, Ctrl* ctrl, bool dense, cudaStream_t st) {
   if (b.nslots == 0) return;
-  launch_dep(k_scatter, dim3((b.nslots + SLOT_BLOCK - 1) / SLOT_BLOCK), dim3(SLOT_BLOCK), st, b, ctrl);
+  launch_dep(k_scatter, dim3((b.nslots + SLOT_BLOCK - 1) / SLOT_BLOCK), dim3(SLOT_BLOCK), st, b, ctrl, dense ? 1 : 0);
 }
 
 }  // namespace lm

@@ -325,14 +325,23 @@ void launch_sweep(const Bufs& b, const PairParams& pp, const StepArgs& a, Ctrl* 
 
 // Count-only pair search (the clustered stress workload, whose 1e11+ pairs per step cannot be
 // listed): every unordered pair within the radius is counted once, with the same cell grid and
-// the same distance test as the sweep. Microbe a (cell order) tests the members of its own cell
+// the same distance test as the sweep. Microbe a (cell order) takes the members of its own cell
 // with a higher cell-order index and every member of its four "forward" cells: (cx+1, cy) and the
-// three cells of row cy+1 (cx-1 .. cx+1, one contiguous run). A block whose 256 microbes all lie
-// in one cell (cluster cores, thousands per cell) walks those runs through shared-memory tiles;
-// any other block lets each thread walk its own runs. Counts are summed per block and added to
-// the step's directed-entry counter (2 per pair) with one atomic.
+// three cells of row cy+1 (cx-1 .. cx+1, one contiguous run).
+//
+// Where cells hold thousands of microbes (cluster cores), most candidates are far inside the radius
+// or far outside it together with their neighbours. k_count_order sorts the members of every cell
+// of at least COUNT_DENSE along a Hilbert curve, k_count_boxes takes the bounding box of every 32
+// consecutive microbes (a leaf), and k_count_pairs, one warp per leaf, compares boxes first: a leaf
+// whose farthest corner lies inside the radius is counted at once, one whose nearest point lies
+// outside is skipped, and only the others (12 % of the candidates at 13k microbes a cell) are tested
+// microbe by microbe. A warp whose microbes have few candidates lets each lane walk its own runs.
+// Bound by instruction issue. 3M microbes in 400 clusters (1.3e10 pairs): 13.2 ms with every
+// candidate tested, 1.7 ms by leaves (ordering 0.06 ms and boxes 0.02 ms beside it).
 constexpr uint32_t COUNT_THREADS = 256;
 constexpr int COUNT_RUNS = 4;
+constexpr uint32_t COUNT_FEW = 256;  // candidates up to which a lane walks its runs alone: box tests, a
+                                     // shared tile and a few shuffles per leaf cost about as much
 
 __device__ __forceinline__ void count_runs(const Vertex& v, const Bufs& b, uint32_t* r0, uint32_t* r1) {
   // r[0] = the rest of the own cell, r[1] = (cx+1, cy), r[2..3] = row cy+1 from cx-1 to cx+1 (one
@@ -357,97 +366,246 @@ __device__ __forceinline__ void count_runs(const Vertex& v, const Bufs& b, uint3
   }
 }
 
+// Place of sub-cell (x, y) of a 32 x 32 grid along Hilbert's curve.
+__device__ __forceinline__ uint32_t hilbert32(uint32_t x, uint32_t y) {
+  uint32_t d = 0;
+#pragma unroll
+  for (int k = 4; k >= 0; --k) {
+    const uint32_t rx = (x >> k) & 1u, ry = (y >> k) & 1u;
+    d = (d << 2) | ((3u * rx) ^ ry);
+    if (!ry) {  // into the quadrant's own frame: mirrored when it is the last one, and transposed
+      const uint32_t m = rx ? (2u << k) - 1u : 0u, t = x ^ m;
+      x = y ^ m;
+      y = t;
+    }
+  }
+  return d;
+}
+
+// The members of every dense cell (listed in act by k_scatter) in the order of their 32 x 32 sub-cells
+// along the curve: a counting sort through shared memory, one block per cell, by way of `tmp` (the
+// state words, unused here). Only the positions move: counting needs no ids.
+constexpr int ORDER_THREADS = 512;
+constexpr uint32_t ORDER_BINS = 1024;
+__global__ void __launch_bounds__(ORDER_THREADS) k_count_order(Bufs b, Ctrl* ctrl) {
+  pdl_wait();
+  if (ctrl->halt) return;
+  __shared__ uint32_t cnt[ORDER_BINS];
+  float2* tmp = reinterpret_cast<float2*>(b.wstate);
+  const uint32_t n = ctrl->act_n;
+  for (uint32_t q = blockIdx.x; q < n; q += gridDim.x) {
+    const uint32_t key = b.act[q], c0 = b.cstart[key], c1 = b.cstart[key + 1];
+    const EnsGrid g = b.grids[b.sens[c0]];
+    uint32_t cx, cy;
+    cell_coords(g, key - g.cell_base, &cx, &cy);
+    const float ox = g.x0 + (float)cx * g.c, oy = g.y0 + (float)cy * g.c, scale = 32.f * g.inv_c;
+    auto sub = [&](float2 p) {  // any assignment is valid, so the clamps only keep it in range
+      const uint32_t x = (uint32_t)fminf(fmaxf((p.x - ox) * scale, 0.f), 31.f);
+      const uint32_t y = (uint32_t)fminf(fmaxf((p.y - oy) * scale, 0.f), 31.f);
+      return hilbert32(x, y);
+    };
+    for (uint32_t i = threadIdx.x; i < ORDER_BINS; i += ORDER_THREADS) cnt[i] = 0;
+    __syncthreads();
+    for (uint32_t i = c0 + threadIdx.x; i < c1; i += ORDER_THREADS) atomicAdd(&cnt[sub(b.spos[i])], 1u);
+    __syncthreads();
+    if (threadIdx.x < 32) {  // exclusive scan, a row of 32 counts at a time
+      uint32_t run = 0;
+      for (uint32_t k = threadIdx.x; k < ORDER_BINS; k += 32) {
+        const uint32_t c = cnt[k];
+        uint32_t incl = c;
+        for (int o = 1; o < 32; o <<= 1) {
+          const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+          if (threadIdx.x >= (uint32_t)o) incl += y;
+        }
+        cnt[k] = run + incl - c;
+        run += __shfl_sync(0xffffffffu, incl, 31);
+      }
+    }
+    __syncthreads();
+    for (uint32_t i = c0 + threadIdx.x; i < c1; i += ORDER_THREADS) {
+      const float2 p = b.spos[i];
+      tmp[c0 + atomicAdd(&cnt[sub(p)], 1u)] = p;
+    }
+    __syncthreads();
+    for (uint32_t i = c0 + threadIdx.x; i < c1; i += ORDER_THREADS) b.spos[i] = tmp[i];
+    __syncthreads();
+  }
+}
+
+// Bounding box (x0, y0, x1, y1) of every leaf, kept in the slab rows (unused here).
+__global__ void __launch_bounds__(COUNT_THREADS) k_count_boxes(Bufs b, Ctrl* ctrl) {
+  pdl_wait();
+  if (ctrl->halt || ctrl->act_n == 0) return;
+  const uint32_t s = blockIdx.x * COUNT_THREADS + threadIdx.x, n = ctrl->n_valid;
+  if ((s & ~31u) >= n) return;  // warp-uniform
+  const float2 p = s < n ? b.spos[s] : make_float2(NAN, NAN);  // fminf and fmaxf ignore NaN
+  float4 v = make_float4(p.x, p.y, p.x, p.y);
+  for (int o = 16; o > 0; o >>= 1) {
+    v.x = fminf(v.x, __shfl_xor_sync(0xffffffffu, v.x, o));
+    v.y = fminf(v.y, __shfl_xor_sync(0xffffffffu, v.y, o));
+    v.z = fmaxf(v.z, __shfl_xor_sync(0xffffffffu, v.z, o));
+    v.w = fmaxf(v.w, __shfl_xor_sync(0xffffffffu, v.w, o));
+  }
+  if ((s & 31u) == 0) reinterpret_cast<float4*>(b.slab)[s >> 5] = v;
+}
+
+// The float32 value that the pair test of each norm compares (r^2 for p = 2, else r).
+__device__ __forceinline__ float norm_value(int norm, float dx, float dy) {
+  if (norm == 2) return fmaf(dx, dx, dy * dy);
+  if (norm == 1) return fabsf(dx) + fabsf(dy);
+  return fmaxf(fabsf(dx), fabsf(dy));
+}
+
+// Members of `tile` (32 of them, shared memory) within the radius of `me`. A value's place in the
+// float32 band around the radius is a number f clamped to [0, 1]: 1 below the band, 0 above; where
+// the sum of f differs from the sum of f^2, a candidate lies inside the band and the tile is
+// recounted with the exact test (the same decision as within(); one fused multiply-add in d^2 is far
+// inside the band). All of it runs in the FMA pipe: two compares and two adds a candidate would
+// cost more issue slots.
+template <int NORM>
+__device__ __forceinline__ uint32_t count_tile(const PairParams& pp, float scale, float shift, float2 me,
+                                               const float2* tile) {
+  const float4* t4 = reinterpret_cast<const float4*>(tile);
+  float f1 = 0.f, f2 = 0.f;
+#pragma unroll 8
+  for (int k = 0; k < 16; ++k) {
+    const float4 q = t4[k];
+    const float fa = __saturatef(fmaf(norm_value(NORM, me.x - q.x, me.y - q.y), scale, shift));
+    const float fb = __saturatef(fmaf(norm_value(NORM, me.x - q.z, me.y - q.w), scale, shift));
+    f1 += fa + fb;
+    f2 = fmaf(fa, fa, fmaf(fb, fb, f2));
+  }
+  uint32_t c = (uint32_t)f1;
+  if (f1 != f2) {
+    c = 0;
+    for (int k = 0; k < 32; ++k) c += within(pp, me, tile[k]) ? 1u : 0u;
+  }
+  return c;
+}
+
+// Pairs of the warp's microbes of one cell (lanes `grp`, consecutive) with the candidates of its runs.
+template <int NORM>
+__device__ __forceinline__ unsigned long long count_group(const Bufs& b, const PairParams& pp, float lo, float hi,
+                                                          float2 me, uint32_t grp, uint32_t s_last, const uint32_t* r0,
+                                                          const uint32_t* r1, float2* tile) {
+  const uint32_t lane = threadIdx.x & 31u;
+  const bool in = (grp >> lane) & 1u;
+  const uint32_t members = __popc(grp);
+  const float scale = -1.f / (hi - lo), shift = hi / (hi - lo);
+  const float4* boxes = reinterpret_cast<const float4*>(b.slab);
+  unsigned long long cnt = 0;
+  // pairs inside the group
+  for (uint32_t rest = grp; rest; rest &= rest - 1) {
+    const int j = __ffs(rest) - 1;
+    const float2 p = make_float2(__shfl_sync(0xffffffffu, me.x, j), __shfl_sync(0xffffffffu, me.y, j));
+    if (in && lane < (uint32_t)j && within(pp, me, p)) ++cnt;
+  }
+  float4 box = in ? make_float4(me.x, me.y, me.x, me.y) : make_float4(NAN, NAN, NAN, NAN);
+  for (int o = 16; o > 0; o >>= 1) {
+    box.x = fminf(box.x, __shfl_xor_sync(0xffffffffu, box.x, o));
+    box.y = fminf(box.y, __shfl_xor_sync(0xffffffffu, box.y, o));
+    box.z = fmaxf(box.z, __shfl_xor_sync(0xffffffffu, box.z, o));
+    box.w = fmaxf(box.w, __shfl_xor_sync(0xffffffffu, box.w, o));
+  }
+  auto points = [&](uint32_t at, uint32_t n) {  // n <= 32 candidates from `at`; the others far away
+    __syncwarp();
+    tile[lane] = lane < n ? b.spos[at + lane] : make_float2(INFINITY, INFINITY);
+    __syncwarp();
+    if (in) cnt += count_tile<NORM>(pp, scale, shift, me, tile);
+  };
+#pragma unroll 1
+  for (int q = 0; q < COUNT_RUNS; ++q) {
+    const uint32_t a = q == 0 ? s_last + 1u : r0[q], e = r1[q];
+    if (a >= e) continue;  // warp-uniform
+    const uint32_t head = min(e, (a + 31u) & ~31u), tail = max(head, e & ~31u);  // whole leaves in [head, tail)
+    if (head > a) points(a, head - a);
+    for (uint32_t l0 = head >> 5; l0 < tail >> 5; l0 += 32) {
+      const uint32_t l = l0 + lane;
+      bool partial = false;
+      if (l < tail >> 5) {
+        const float4 v = boxes[l];
+        const float nx = fmaxf(0.f, fmaxf(v.x - box.z, box.x - v.z)), ny = fmaxf(0.f, fmaxf(v.y - box.w, box.y - v.w));
+        const float fx = fmaxf(v.z - box.x, box.z - v.x), fy = fmaxf(v.w - box.y, box.w - v.y);
+        if (norm_value(NORM, fx, fy) < lo) cnt += 32u * members;
+        else partial = !(norm_value(NORM, nx, ny) > hi);
+      }
+      uint32_t m = __ballot_sync(0xffffffffu, partial);
+      if (m) {  // the next leaf is on its way while this one is tested
+        float2 next = b.spos[((l0 + __ffs(m) - 1) << 5) + lane];
+        while (m) {
+          __syncwarp();
+          tile[lane] = next;
+          __syncwarp();
+          m &= m - 1;
+          if (m) next = b.spos[((l0 + __ffs(m) - 1) << 5) + lane];
+          if (in) cnt += count_tile<NORM>(pp, scale, shift, me, tile);
+        }
+      }
+    }
+    if (e > tail) points(tail, e - tail);
+  }
+  return cnt;
+}
+
 __global__ void __launch_bounds__(COUNT_THREADS) k_count_pairs(Bufs b, PairParams pp, Ctrl* ctrl) {
   pdl_wait();
   if (ctrl->halt) return;
-  __shared__ __align__(16) float2 tile[COUNT_THREADS];
-  __shared__ uint32_t first_key, last_key;
+  __shared__ __align__(16) float2 tiles[COUNT_THREADS / 32][32];
   __shared__ unsigned long long tot;
   const uint32_t n_valid = ctrl->n_valid;
   const uint32_t blk0 = blockIdx.x * COUNT_THREADS;
   if (blk0 >= n_valid) return;  // block-uniform
-  const uint32_t s = blk0 + threadIdx.x;
-  const uint32_t last = min(n_valid, blk0 + COUNT_THREADS) - 1;
-  if (threadIdx.x == 0) {
-    first_key = b.skey[blk0];
-    last_key = b.skey[last];
-    tot = 0;
-  }
+  if (threadIdx.x == 0) tot = 0;
   __syncthreads();
+  const uint32_t s = blk0 + threadIdx.x, lane = threadIdx.x & 31u;
+  const bool valid = s < n_valid;
+  // the float32 band of the norm's value around the radius; radii that float32 cannot resolve have none
+  const float lo = pp.norm == 2 ? pp.r2f_lo : pp.rf_lo, hi = pp.norm == 2 ? pp.r2f_hi : pp.rf_hi;
+  const bool leaves = ctrl->act_n != 0 && lo > 0.f && hi < INFINITY;
   unsigned long long cnt = 0;
-  const bool dense = first_key == last_key && last - blk0 + 1 == COUNT_THREADS;
-  if (dense) {
-    // all 256 microbes share one cell and hence the same forward runs; the own-cell run starts
-    // after the block's first microbe, each thread keeps only partners with a higher index
-    const Vertex v = load_vertex(b, blk0);
-    uint32_t r0[COUNT_RUNS], r1[COUNT_RUNS];
+  Vertex v{};
+  uint32_t r0[COUNT_RUNS] = {0, 0, 0, 0}, r1[COUNT_RUNS] = {0, 0, 0, 0}, key = NONE;
+  if (valid) {
+    v = load_vertex(b, s);
+    key = b.skey[s];
     count_runs(v, b, r0, r1);
-    const float2 me = b.spos[s];
-    for (int q = 0; q < COUNT_RUNS; ++q) {
-      for (uint32_t tb = r0[q]; tb < r1[q]; tb += COUNT_THREADS) {
-        const uint32_t n_t = min(COUNT_THREADS, r1[q] - tb);
-        if (threadIdx.x < n_t) tile[threadIdx.x] = b.spos[tb + threadIdx.x];
-        __syncthreads();
-        // own cell: partner index tb + k must exceed s
-        const uint32_t k0 = q == 0 ? (s + 1 > tb ? min(s + 1 - tb, n_t) : 0u) : 0u;
-        if (pp.norm == 2) {
-          // branch-free float32 decision, two candidates per 16-byte shared load: clo counts the
-          // candidates below the float32 band around r^2, chi those not above it; a tile where they
-          // differ holds a candidate inside the band and is recounted with the exact test (the same
-          // decision as within()). d2 is one fused multiply-add: its error is far inside the band.
-          uint32_t clo = 0, chi = 0;
-          const float lo = pp.r2f_lo, hi = pp.r2f_hi;
-          uint32_t k = k0;
-          if ((k & 1u) && k < n_t) {
-            const float dx = me.x - tile[k].x, dy = me.y - tile[k].y;
-            const float d2 = fmaf(dx, dx, dy * dy);
-            clo += d2 < lo ? 1u : 0u;
-            chi += d2 <= hi ? 1u : 0u;
-            ++k;
-          }
-          const float4* t4 = reinterpret_cast<const float4*>(tile);
-#pragma unroll 4
-          for (; k + 1 < n_t; k += 2) {
-            const float4 q = t4[k >> 1];
-            const float ax = me.x - q.x, ay = me.y - q.y, bx = me.x - q.z, by = me.y - q.w;
-            const float da = fmaf(ax, ax, ay * ay), db = fmaf(bx, bx, by * by);
-            clo += (da < lo ? 1u : 0u) + (db < lo ? 1u : 0u);
-            chi += (da <= hi ? 1u : 0u) + (db <= hi ? 1u : 0u);
-          }
-          if (k < n_t) {
-            const float dx = me.x - tile[k].x, dy = me.y - tile[k].y;
-            const float d2 = fmaf(dx, dx, dy * dy);
-            clo += d2 < lo ? 1u : 0u;
-            chi += d2 <= hi ? 1u : 0u;
-          }
-          if (clo != chi) {
-            clo = 0;
-            for (uint32_t kk = k0; kk < n_t; ++kk) clo += within(pp, me, tile[kk]) ? 1u : 0u;
-          }
-          cnt += clo;
-        } else {
-          for (uint32_t k = k0; k < n_t; ++k) cnt += within(pp, me, tile[k]) ? 1u : 0u;
-        }
-        __syncthreads();
-      }
-    }
-  } else if (s < n_valid) {
-    const Vertex v = load_vertex(b, s);
-    uint32_t r0[COUNT_RUNS], r1[COUNT_RUNS];
-    count_runs(v, b, r0, r1);
+  }
+  uint32_t most = 0;
+  for (int q = 0; q < COUNT_RUNS; ++q) most += r1[q] - r0[q];
+  most = __reduce_max_sync(0xffffffffu, most);
+  if (!leaves || most <= COUNT_FEW) {
     for (int q = 0; q < COUNT_RUNS; ++q)
       for (uint32_t t = r0[q]; t < r1[q]; ++t) cnt += within(pp, v.ps, b.spos[t]) ? 1u : 0u;
+  } else {
+    for (uint32_t rest = __ballot_sync(0xffffffffu, valid); rest;) {  // the warp's cells in turn
+      const int first = __ffs(rest) - 1;
+      const uint32_t grp = __ballot_sync(0xffffffffu, valid && key == __shfl_sync(0xffffffffu, key, first));
+      uint32_t a[COUNT_RUNS], e[COUNT_RUNS];
+#pragma unroll
+      for (int q = 0; q < COUNT_RUNS; ++q) {
+        a[q] = __shfl_sync(0xffffffffu, r0[q], first);
+        e[q] = __shfl_sync(0xffffffffu, r1[q], first);
+      }
+      const uint32_t s_last = (s - lane) + 31u - __clz(grp);
+      float2* tile = tiles[threadIdx.x >> 5];
+      if (pp.norm == 2) cnt += count_group<2>(b, pp, lo, hi, v.ps, grp, s_last, a, e, tile);
+      else if (pp.norm == 1) cnt += count_group<1>(b, pp, lo, hi, v.ps, grp, s_last, a, e, tile);
+      else cnt += count_group<0>(b, pp, lo, hi, v.ps, grp, s_last, a, e, tile);
+      rest &= ~grp;
+    }
   }
   for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-  if ((threadIdx.x & 31) == 0 && cnt) atomicAdd(&tot, cnt);
+  if (lane == 0 && cnt) atomicAdd(&tot, cnt);
   __syncthreads();
   if (threadIdx.x == 0 && tot) atomicAdd(&ctrl->n_dir, 2ull * tot);
 }
 
-void launch_count_pairs(const Bufs& b, const PairParams& pp, Ctrl* ctrl, cudaStream_t st) {
+void launch_count_pairs(const Bufs& b, const PairParams& pp, Ctrl* ctrl, int sms, cudaStream_t st) {
   if (b.nslots == 0) return;
-  launch_dep(k_count_pairs, dim3((b.nslots + COUNT_THREADS - 1) / COUNT_THREADS), dim3(COUNT_THREADS), st, b, pp,
-             ctrl);
+  const unsigned blocks = (b.nslots + COUNT_THREADS - 1) / COUNT_THREADS;
+  launch_dep(k_count_order, dim3(sms * 4), dim3(ORDER_THREADS), st, b, ctrl);
+  launch_dep(k_count_boxes, dim3(blocks), dim3(COUNT_THREADS), st, b, ctrl);
+  launch_dep(k_count_pairs, dim3(blocks), dim3(COUNT_THREADS), st, b, pp, ctrl);
 }
 
 // In-place sort of one long list (priorities pr, list entries nb) into `before` order.

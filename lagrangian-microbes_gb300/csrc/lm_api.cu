@@ -500,9 +500,10 @@ cudaError_t enqueue_interaction(lm_ctx* c, const StepArgs& a, uint32_t flags, bo
   if (!own_grid) PROF(c, P_GRID, launch_grid(b, c->pp, c->ctrl, st));
   PROF(c, P_KEYS, launch_keys(b, c->pp, c->ctrl, use_status, own_grid, st));
   PROF(c, P_CELL_SCAN, launch_cell_scan(b, c->ctrl, st));
-  PROF(c, P_SCATTER, launch_scatter(b, c->ctrl, st));
-  if (flags & LM_STEP_COUNT_PAIRS) {  // count-only: no lists, no interaction
-    PROF(c, P_COUNT, launch_count_pairs(b, c->pp, c->ctrl, st));
+  const bool count = (flags & LM_STEP_COUNT_PAIRS) != 0;
+  PROF(c, P_SCATTER, launch_scatter(b, c->ctrl, count, st));
+  if (count) {  // count-only: no lists, no interaction
+    PROF(c, P_COUNT, launch_count_pairs(b, c->pp, c->ctrl, c->sms, st));
     return cudaGetLastError();
   }
   PROF(c, P_SWEEP, launch_sweep(b, c->pp, a, c->ctrl, st));

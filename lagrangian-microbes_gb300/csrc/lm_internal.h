@@ -306,11 +306,13 @@ void launch_grid(const Bufs& b, const PairParams& pp, Ctrl* ctrl, cudaStream_t s
 // own_grid (one ensemble): k_keys computes the grid itself (no launch_grid before it).
 void launch_keys(const Bufs& b, const PairParams& pp, Ctrl* ctrl, bool use_status, bool own_grid, cudaStream_t st);
 void launch_cell_scan(const Bufs& b, Ctrl* ctrl, cudaStream_t st);
-void launch_scatter(const Bufs& b, Ctrl* ctrl, cudaStream_t st);
+// dense: list the cells of at least COUNT_DENSE microbes in act (count-only steps).
+constexpr uint32_t COUNT_DENSE = 64;
+void launch_scatter(const Bufs& b, Ctrl* ctrl, bool dense, cudaStream_t st);
 
 // K3 neighbour lists.
 void launch_sweep(const Bufs& b, const PairParams& pp, const StepArgs& a, Ctrl* ctrl, cudaStream_t st);
-void launch_count_pairs(const Bufs& b, const PairParams& pp, Ctrl* ctrl, cudaStream_t st);
+void launch_count_pairs(const Bufs& b, const PairParams& pp, Ctrl* ctrl, int sms, cudaStream_t st);
 // blocks_per_sm: grid of sms x blocks_per_sm blocks of LONG_WARPS warps (tuning)
 void launch_sweep_long(const Bufs& b, const PairParams& pp, const StepArgs& a, Ctrl* ctrl, int sms,
                        int blocks_per_sm, cudaStream_t st);

@@ -85,3 +85,38 @@ def test_fused_count_step_counts_the_advected_positions(engine, lm, orc, small_f
     _, _, sp, _ = sim.state()
     assert (sp == 1).all()  # counting leaves the species alone
     sim.close()
+
+
+@pytest.mark.parametrize("p", [2, 1, np.inf])
+@pytest.mark.parametrize("per_cell", [40, 63, 64, 65, 300, 2500])
+def test_count_over_leaves_of_dense_cells_matches_oracle(engine, orc, per_cell, p):
+    """Cells around the size from which their members are counted by leaves of 32, with coincident
+    microbes, pairs exactly one radius apart and sparse neighbours beside dense cells."""
+    rng = np.random.default_rng(45 + per_cell)
+    r = 0.01
+    n = min(per_cell * 16, 12000)
+    side = r * np.sqrt(n / per_cell)
+    lon, lat = 200.0 + side * rng.random(n), 25.0 + side * rng.random(n)
+    lon[:70], lat[:70] = lon[0], lat[0]  # one point, 70 times
+    grid = np.arange(100)
+    lon[100:200], lat[100:200] = 200.25 + 0.0078125 * (grid % 10), 25.25 + 0.0078125 * (grid // 10)
+    lon[200:260] += 3 * side * rng.random(60)  # stragglers around the dense patch
+    lon, lat = lon.astype(np.float32), lat.astype(np.float32)
+    for radius in (r, 0.0078125, 0.0):
+        q = engine.PairQuery(radius, p)
+        assert q.count(lon, lat) == orc.count_pairs(lon, lat, radius, p), radius
+        q.ctx.close()
+
+
+def test_count_step_keeps_dense_ensembles_apart(engine, lm, orc, small_field):
+    rng = np.random.default_rng(46)
+    members, want = [], 0
+    for n in (1, 3000, 33, 9000):
+        lon, lat = 200.0 + 0.03 * rng.random(n), 25.0 + 0.03 * rng.random(n)
+        members.append((lon, lat, np.ones(n, np.int8)))
+    sim = engine.EnsembleSimulation(small_field, members, radius=0.01)
+    rec = sim.step(float(small_field.times[0]), 3600.0, 1, record=True, count_pairs=True)
+    for lon, lat in zip(sim.split(rec["lon"][0]), sim.split(rec["lat"][0])):
+        want += orc.count_pairs(lon, lat, 0.01, 2)
+    assert sim.stats()["pairs"] == want
+    sim.close()
