@@ -1161,6 +1161,14 @@ void launch_adj_signature(const FieldView& f, int prec, const AdjStep* table, in
                                                              (const float*)y, status, sig);
 }
 
+void launch_scan(const uint32_t* in, uint32_t* out, size_t n, uint32_t* bsum, cudaStream_t st) {
+  if (!n) return;
+  const size_t chunk = (n + SCAN_BLOCKS - 1) / SCAN_BLOCKS;
+  const unsigned nb = grid_for(n, chunk);
+  k_scan_sums<<<nb, 256, 0, st>>>(in, n, chunk, bsum);
+  k_scan_chunks<<<nb, 256, 0, st>>>(in, out, n, chunk, bsum);
+}
+
 size_t adj_sort_hist_len(uint32_t m) { return (size_t)RS_RADIX_MAX * grid_for(m, RS_TILE); }
 
 void adj_sort(const AdjSortBufs& sb, uint32_t m, int key_bits, cudaStream_t st, const uint32_t** skey,
@@ -1176,11 +1184,7 @@ void adj_sort(const AdjSortBufs& sb, uint32_t m, int key_bits, cudaStream_t st, 
     const int shift = p * width;
     const int bits = key_bits - shift < width ? key_bits - shift : width;
     k_rs_hist<<<tiles, RS_THREADS, 0, st>>>(kin, m, shift, bits, sb.hist, tiles);
-    const size_t len = ((size_t)1 << bits) * tiles;
-    const size_t chunk = (len + SCAN_BLOCKS - 1) / SCAN_BLOCKS;
-    const unsigned nb = grid_for(len, chunk);
-    k_scan_sums<<<nb, 256, 0, st>>>(sb.hist, len, chunk, sb.bsum);
-    k_scan_chunks<<<nb, 256, 0, st>>>(sb.hist, sb.hscan, len, chunk, sb.bsum);
+    launch_scan(sb.hist, sb.hscan, ((size_t)1 << bits) * tiles, sb.bsum, st);
     k_rs_scatter<<<tiles, RS_THREADS, 0, st>>>(kin, vin, kout, vout, m, shift, bits, sb.hscan, tiles);
     kin = kout;
     vin = vout;

@@ -1277,33 +1277,30 @@ int lm_query_pairs(lm_ctx* c, int64_t n, const float* lon, const float* lat, int
     break;
   }
   if ((r = clear_err_bits(c, ERRB_NAN))) return r;  // non-finite query points are never paired
-  const uint32_t nv = c->hctrl->n_valid;
-  const size_t novf = (size_t)c->hctrl->ovf_used;
-  std::vector<uint32_t> deg(nv), ids(nv), slab((size_t)nv * SLAB), ovf(novf);
-  if (nv) {
-    CK(cudaMemcpyAsync(deg.data(), c->deg, nv * 4, cudaMemcpyDeviceToHost, c->st));
-    CK(cudaMemcpyAsync(ids.data(), c->sid, nv * 4, cudaMemcpyDeviceToHost, c->st));
-    CK(cudaMemcpyAsync(slab.data(), c->slab, (size_t)nv * SLAB * 4, cudaMemcpyDeviceToHost, c->st));
-  }
-  if (novf) CK(cudaMemcpyAsync(ovf.data(), c->ovf, novf * 4, cudaMemcpyDeviceToHost, c->st));
+  const uint64_t m = c->hctrl->n_dir / 2;
+  *n_pairs = (int64_t)m;
+  if (!pi || !pj || m == 0) return LM_OK;  // count query
+  if ((int64_t)m > cap)
+    return fail(c, LM_ERR_CAPACITY, "pair buffer holds %lld pairs, %llu needed", (long long)cap, (unsigned long long)m);
+  if (m > 0xffffffffull) return fail(c, LM_ERR_OOM, "too many pairs for one query (%llu)", (unsigned long long)m);
+  // the pairs i < j in (i, j) order, written on the device: counts per i, their prefix sums, the rows
+  const size_t nn = ((size_t)n + 63) / 64 * 64, mm = ((size_t)m + 63) / 64 * 64;
+  void* mem = nullptr;
+  if ((r = ctx_scratch(c, (2 * nn + SCAN_BLOCKS + 2 * mm) * sizeof(uint32_t), &mem))) return r;
+  uint32_t* cnt = static_cast<uint32_t*>(mem);
+  uint32_t* off = cnt + nn;
+  int32_t* di = reinterpret_cast<int32_t*>(off + nn);
+  int32_t* dj = di + mm;
+  uint32_t* bsum = reinterpret_cast<uint32_t*>(dj + mm);
+  CK(cudaMemsetAsync(cnt, 0, (size_t)n * sizeof(uint32_t), c->st));
+  const Bufs b = bufs(c, false);
+  launch_pair_counts(b, c->hctrl->n_valid, c->hctrl->n_long, cnt, c->sms, c->st);
+  launch_scan(cnt, off, (size_t)n, bsum, c->st);
+  launch_pair_rows(b, c->hctrl->n_valid, c->hctrl->n_long, off, di, dj, c->sms, c->st);
+  CK(cudaGetLastError());
+  CK(cudaMemcpyAsync(pi, di, m * sizeof(int32_t), cudaMemcpyDeviceToHost, c->st));
+  CK(cudaMemcpyAsync(pj, dj, m * sizeof(int32_t), cudaMemcpyDeviceToHost, c->st));
   CK(cudaStreamSynchronize(c->st));
-  std::vector<uint64_t> pairs;
-  pairs.reserve((size_t)c->hctrl->n_dir / 2);
-  for (uint32_t s = 0; s < nv; ++s)
-    for (uint32_t h = 0; h < deg[s]; ++h) {
-      const uint32_t t = entry_id(deg[s] <= SLAB ? slab[(size_t)s * SLAB + h] : ovf[(size_t)slab[(size_t)s * SLAB] + h]);
-      const uint32_t a_ = ids[s], b_ = ids[t];
-      if (a_ < b_) pairs.push_back(((uint64_t)a_ << 32) | b_);
-    }
-  std::sort(pairs.begin(), pairs.end());
-  *n_pairs = (int64_t)pairs.size();
-  if (!pi || !pj) return LM_OK;  // count query
-  if ((int64_t)pairs.size() > cap)
-    return fail(c, LM_ERR_CAPACITY, "pair buffer holds %lld pairs, %zu needed", (long long)cap, pairs.size());
-  for (size_t k = 0; k < pairs.size(); ++k) {
-    pi[k] = (int32_t)(pairs[k] >> 32);
-    pj[k] = (int32_t)(pairs[k] & 0xffffffffu);
-  }
   return LM_OK;
 }
 

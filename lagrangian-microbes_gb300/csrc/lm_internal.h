@@ -317,6 +317,14 @@ void launch_count_pairs(const Bufs& b, const PairParams& pp, Ctrl* ctrl, int sms
 void launch_sweep_long(const Bufs& b, const PairParams& pp, const StepArgs& a, Ctrl* ctrl, int sms,
                        int blocks_per_sm, cudaStream_t st);
 
+// The pairs of a query (one ensemble) by caller index: cnt[i] = partners of i above it; with their
+// exclusive prefix sums off, the pairs (i, j), i < j, in (i, j) order.
+void launch_pair_counts(const Bufs& b, uint32_t n_valid, uint32_t n_long, uint32_t* cnt, int sms, cudaStream_t st);
+void launch_pair_rows(const Bufs& b, uint32_t n_valid, uint32_t n_long, const uint32_t* off, int32_t* pi, int32_t* pj,
+                      int sms, cudaStream_t st);
+// Exclusive scan of n values (bsum: SCAN_BLOCKS words of working memory).
+void launch_scan(const uint32_t* in, uint32_t* out, size_t n, uint32_t* bsum, cudaStream_t st);
+
 // K4/K5 interaction dataflow (cooperative persistent kernel).
 // Grid of the cooperative launch with `threads` (512 or 1,024) per block; *block receives the block size.
 int rounds_grid(int device, int threads, int* block);

@@ -120,3 +120,22 @@ def test_count_step_keeps_dense_ensembles_apart(engine, lm, orc, small_field):
         want += orc.count_pairs(lon, lat, 0.01, 2)
     assert sim.stats()["pairs"] == want
     sim.close()
+
+
+@pytest.mark.parametrize("size", [1, 2, 8, 9, 10, 33, 512, 513, 514, 1500])
+def test_query_rows_of_every_list_length_are_in_order(engine, orc, size):
+    """Clumps of `size` microbes that all pair with one another (lists of size - 1 partners: none, a
+    slab row, a warp's shared row, beyond it) among scattered ones, in shuffled order."""
+    rng = np.random.default_rng(47 + size)
+    lon = np.concatenate([200.1 + 0.004 * rng.random(size), 200.5 + 0.004 * rng.random(size), 200 + rng.random(3000)])
+    lat = np.concatenate([25.1 + 0.004 * rng.random(size), 25.5 + 0.004 * rng.random(size), 25 + rng.random(3000)])
+    order = rng.permutation(lon.size)
+    lon, lat = lon[order].astype(np.float32), lat[order].astype(np.float32)
+    lon[0] = np.nan
+    q = engine.PairQuery(0.01, 2)
+    pi, pj = q.pairs(lon, lat)
+    assert q.count(lon, lat) == pi.size
+    q.ctx.close()
+    oi, oj = orc.pairs(lon, lat, 0.01, 2)
+    np.testing.assert_array_equal(pi, oi)
+    np.testing.assert_array_equal(pj, oj)
