@@ -7,22 +7,35 @@
 // their Jacobians backward:
 //   x' = x + dt/6 (k1 + 2 k2 + 2 k3 + k4),  k_s = f(t_s, x_s),  f = (U / (M cos lat), V / M),
 //   with U, V bilinear in (lon, lat), linear in time, M = 1852 * 60 m per degree.
-// For every stage it emits a record (a, b, dL/dU_s, dL/dV_s) keyed by (field cell, stage time):
-// the stage's bilinear fractions inside its cell and its adjoint in field units.
+// For every stage it emits a record (a, b, dL/dU_s, dL/dV_s) for the field cell it sampled: the
+// stage's bilinear fractions inside its cell and its adjoint in field units.
 //
-// K7, the deterministic segmented reduction: the 4 N records of a step are put in (cell, stage
-// time, record id) order by a stable LSD radix sort (block-local ranks from warp match masks, no
-// atomics on positions); one warp per cell then sums each (cell, stage time) segment into the four
-// corner weights (fixed lane order, Neumaier-compensated float32 lane sums, fixed-shape warp tree);
-// a node pass adds, for every grid node, the four cells around it in a fixed order and spreads the
-// three stage times onto the field's frames with the linear-in-time weights. No float atomics: the
-// gradient is bit-identical from run to run.
+// K7, the deterministic reduction of the records onto the grid. Sums are taken in integers (scaled by
+// a power of two from the cell's largest adjoint, at least 38 bits below it), so they do not depend on
+// the order of the records and no sort is needed:
+//   k_adj_alloc    reserves room for the entries of every occupied cell (K6 counted them) and lists
+//                  the cells, in whatever order its blocks come;
+//   k_adj_scatter  puts an entry (microbe, which of its stages) into each cell a microbe sampled;
+//   k_adj_gather   one warp per listed cell: its records into the four corner sums of each stage time;
+//   k_adj_nodes    adds, for every grid node, the four cells around it in a fixed order and spreads the
+//                  three stage times onto the field's frames with the linear-in-time weights.
+// The gradient is bit-identical from run to run and for every checkpoint interval. A sort of the
+// microbes by cell (two radix passes of four launches) with compensated float sums in a fixed order
+// took 13 launches a step; here several steps share one set of launches when their records fit L2
+// together (a microbe's steps only depend on its own adjoint), and a batch is reduced on a stream of its
+// own beside the next one's steps. Forward and backward with the benchmark's loss: 5,000 microbes x 24
+// steps in f64 5.96 -> 2.87 ms, 100k x 48 in f32 6.62 -> 2.30 ms, 1M x 24 in ds 7.02 -> 4.54 ms.
 #include <algorithm>
 
 #include "lm_field.cuh"
 #include "lm_internal.h"
 
 namespace lm {
+
+// Threads per block of the stepping kernels (at most). With 128, the backward step keeps seven blocks an
+// SM at 72 registers (a few spills): 1M microbes in double-float, forward and backward of 24 steps, take
+// 4.49 ms against 4.75 at its 95 registers (five blocks) and 4.93 with two blocks of 256.
+constexpr unsigned ADJ_THREADS = 128;
 
 // ---------------------------------------------------------------- stage table, recompute
 
@@ -168,15 +181,24 @@ __device__ __forceinline__ void vel_jac_at(const FieldView& f, int k, T w, int i
     va = va + w * (((T(1) - b) * ((T)q01.y - (T)q00.y) + b * ((T)q11.y - (T)q10.y)) - va);
     vb = vb + w * (((T(1) - a) * ((T)q10.y - (T)q00.y) + a * ((T)q11.y - (T)q01.y)) - vb);
   }
-  const T c = cospi_t(lat * (T(1) / T(180)));
-  const T sn = sinpi_t(lat * (T(1) / T(180)));
   const T M = (T)M_PER_DEG;
-  r.flon = u / (M * c);
+  T c, tan_lat;
+  if constexpr (sizeof(T) == 8) {  // one argument reduction, one division
+    T sn;
+    sincospi(lat * (T(1) / T(180)), &sn, &c);
+    r.inv_mc = T(1) / (M * c);
+    r.flon = u * r.inv_mc;
+    tan_lat = sn * M * r.inv_mc;
+  } else {  // the forward's operations
+    c = cospi_t(lat * (T(1) / T(180)));
+    r.flon = u / (M * c);
+    r.inv_mc = T(1) / (M * c);
+    tan_lat = sinpi_t(lat * (T(1) / T(180))) / c;
+  }
   r.flat = v * (T(1) / M);
-  r.inv_mc = T(1) / (M * c);
   // d/dlat (1 / cos(lat)) = tan(lat) / cos(lat) * pi / 180 per degree
   r.dlon_dx = ua * inv_dx * r.inv_mc;
-  r.dlon_dy = ub * inv_dy * r.inv_mc + r.flon * (sn / c) * (T)0.017453292519943295;
+  r.dlon_dy = ub * inv_dy * r.inv_mc + r.flon * tan_lat * (T)0.017453292519943295;
   r.dlat_dx = va * inv_dx * (T(1) / M);
   r.dlat_dy = vb * inv_dy * (T(1) / M);
   r.cell = (uint32_t)j * (uint32_t)(f.nx - 1) + (uint32_t)i;
@@ -222,7 +244,7 @@ __device__ __forceinline__ bool rk4_t<double>(const FieldView& f, const Geo<doub
 // Steps [m0, m1) of every microbe in registers, the forward's freezing rules. With rec_* set, the
 // state before every step is stored ([m - m0][n]) for the backward sweep.
 template <class T>
-__global__ void __launch_bounds__(256) k_adj_forward(FieldView f, const AdjStep* __restrict__ table, int m0, int m1,
+__global__ void __launch_bounds__(ADJ_THREADS) k_adj_forward(FieldView f, const AdjStep* __restrict__ table, int m0, int m1,
                                                      T dt, uint32_t n, T* __restrict__ xs, T* __restrict__ ys,
                                                      uint8_t* __restrict__ sts, T* __restrict__ rec_x,
                                                      T* __restrict__ rec_y, uint8_t* __restrict__ rec_st,
@@ -263,91 +285,113 @@ __global__ void __launch_bounds__(256) k_adj_forward(FieldView f, const AdjStep*
 }
 
 // The backward of one RK4 step of microbe p from its four stage Jacobians (every precision):
-// lambda_{m+1} -> lambda_m in lx, ly, plus its 4 records and their keys. `ok` false: the step was
-// frozen (a stage left the grid or the step was non-finite), x_{m+1} = x_m and the adjoint passes
-// through.
+// lambda_{m+1} -> lambda_m in gx, gy, plus its 4 records. Returns the float bits of the records' largest
+// |dL/dU|, |dL/dV| (NaN above infinity above every number).
 template <class T>
-__device__ __forceinline__ void adj_tail(const FieldView& f, uint32_t p, bool ok, const VelJac<T>& J1,
-                                         const VelJac<T>& J2, const VelJac<T>& J3, const VelJac<T>& J4, T dt,
-                                         T* __restrict__ lx, T* __restrict__ ly, float4* __restrict__ rec,
-                                         uint32_t* __restrict__ key, uint32_t sent, uint32_t* __restrict__ mkey,
-                                         uint32_t* __restrict__ mcode, uint32_t msent, uint32_t* err) {
-  if (!ok) {  // frozen this step: x_{m+1} = x_m, the adjoint passes through
-    if (mkey)
-      mkey[p] = msent;
-    else
-      reinterpret_cast<uint4*>(key)[p] = make_uint4(sent, sent, sent, sent);
-    return;
-  }
-  if (mkey) {
-    // gather form: every stage is coded by the slot (dj + 1) * 3 + (di + 1) of its cell around the
-    // cell where the step starts (stage 1), 4 bits a stage; the microbe is keyed by that cell * 2 +
-    // (1 when a stage leaves the cell). A stage outside the 3 x 3 cells sets ADJ_WIDE and the
-    // backward is redone with the record sort.
-    const uint32_t cw = (uint32_t)(f.nx - 1);
-    const int bi = (int)(J1.cell % cw), bj = (int)(J1.cell / cw);
-    const uint32_t cs[3] = {J2.cell, J3.cell, J4.cell};
-    uint32_t code = 4u;
-    bool wide = false;
-#pragma unroll
-    for (int q = 0; q < 3; ++q) {
-      const int di = (int)(cs[q] % cw) - bi, dj = (int)(cs[q] / cw) - bj;
-      wide |= abs(di) > 1 || abs(dj) > 1;
-      code |= (uint32_t)((dj + 1) * 3 + (di + 1)) << (4 * (q + 1));
-    }
-    mcode[p] = code;
-    mkey[p] = 2u * J1.cell + (code != 0x4444u ? 1u : 0u);
-    if (wide) atomicOr(err, ADJ_WIDE);
-  }
-  const T gx = lx[p], gy = ly[p];
+__device__ __forceinline__ uint32_t adj_tail(const VelJac<T>* J, T dt, T& gx, T& gy, float4* __restrict__ rec) {
   const T h6 = dt * (T(1) / T(6)), h3 = dt * (T(1) / T(3)), h2 = T(0.5) * dt;
   // dL/dk4, then back through x3 = x + dt k3, x2 = x + dt/2 k2, x1 = x + dt/2 k1
   const T g4x = h6 * gx, g4y = h6 * gy;
-  const T x3x = J4.dlon_dx * g4x + J4.dlat_dx * g4y, x3y = J4.dlon_dy * g4x + J4.dlat_dy * g4y;
+  const T x3x = J[3].dlon_dx * g4x + J[3].dlat_dx * g4y, x3y = J[3].dlon_dy * g4x + J[3].dlat_dy * g4y;
   const T g3x = h3 * gx + dt * x3x, g3y = h3 * gy + dt * x3y;
-  const T x2x = J3.dlon_dx * g3x + J3.dlat_dx * g3y, x2y = J3.dlon_dy * g3x + J3.dlat_dy * g3y;
+  const T x2x = J[2].dlon_dx * g3x + J[2].dlat_dx * g3y, x2y = J[2].dlon_dy * g3x + J[2].dlat_dy * g3y;
   const T g2x = h3 * gx + h2 * x2x, g2y = h3 * gy + h2 * x2y;
-  const T x1x = J2.dlon_dx * g2x + J2.dlat_dx * g2y, x1y = J2.dlon_dy * g2x + J2.dlat_dy * g2y;
+  const T x1x = J[1].dlon_dx * g2x + J[1].dlat_dx * g2y, x1y = J[1].dlon_dy * g2x + J[1].dlat_dy * g2y;
   const T g1x = h6 * gx + h2 * x1x, g1y = h6 * gy + h2 * x1y;
-  const T x0x = J1.dlon_dx * g1x + J1.dlat_dx * g1y, x0y = J1.dlon_dy * g1x + J1.dlat_dy * g1y;
-  lx[p] = gx + ((x0x + x1x) + (x2x + x3x));
-  ly[p] = gy + ((x0y + x1y) + (x2y + x3y));
+  const T x0x = J[0].dlon_dx * g1x + J[0].dlat_dx * g1y, x0y = J[0].dlon_dy * g1x + J[0].dlat_dy * g1y;
+  gx = gx + ((x0x + x1x) + (x2x + x3x));
+  gy = gy + ((x0y + x1y) + (x2y + x3y));
   // records: dL/dU_s = dL/dk_s,lon / (M cos lat_s), dL/dV_s = dL/dk_s,lat / M (float32 for the reduction)
   const T invM = T(1) / (T)M_PER_DEG;
-  float4* rq = rec + 4 * (size_t)p;
-  rq[0] = make_float4((float)J1.a, (float)J1.b, (float)(g1x * J1.inv_mc), (float)(g1y * invM));
-  rq[1] = make_float4((float)J2.a, (float)J2.b, (float)(g2x * J2.inv_mc), (float)(g2y * invM));
-  rq[2] = make_float4((float)J3.a, (float)J3.b, (float)(g3x * J3.inv_mc), (float)(g3y * invM));
-  rq[3] = make_float4((float)J4.a, (float)J4.b, (float)(g4x * J4.inv_mc), (float)(g4y * invM));
-  if (!mkey)
-    reinterpret_cast<uint4*>(key)[p] =
-        make_uint4(4u * J1.cell + 0u, 4u * J2.cell + 1u, 4u * J3.cell + 1u, 4u * J4.cell + 2u);
+  const float4 r[4] = {
+      make_float4((float)J[0].a, (float)J[0].b, (float)(g1x * J[0].inv_mc), (float)(g1y * invM)),
+      make_float4((float)J[1].a, (float)J[1].b, (float)(g2x * J[1].inv_mc), (float)(g2y * invM)),
+      make_float4((float)J[2].a, (float)J[2].b, (float)(g3x * J[2].inv_mc), (float)(g3y * invM)),
+      make_float4((float)J[3].a, (float)J[3].b, (float)(g4x * J[3].inv_mc), (float)(g4y * invM))};
+  uint32_t top = 0;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    rec[k] = r[k];
+    top = max(top, max(__float_as_uint(r[k].z) & 0x7fffffffu, __float_as_uint(r[k].w) & 0x7fffffffu));
+  }
+  return top;
 }
 
-// lambda_{m+1} -> lambda_m, plus 4 records per microbe (key = cell * 4 + stage time, or `sent`).
-template <class T>
-__global__ void __launch_bounds__(256) k_adj_step(FieldView f, AdjStep s, T dt, uint32_t n, const T* __restrict__ xs,
-                                                  const T* __restrict__ ys, const uint8_t* __restrict__ sts,
-                                                  T* __restrict__ lx, T* __restrict__ ly, float4* __restrict__ rec,
-                                                  uint32_t* __restrict__ key, uint32_t sent, uint32_t* __restrict__ mkey,
-                                                  uint32_t* __restrict__ mcode, uint32_t msent, uint32_t* err) {
-  const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= n) return;
-  const Geo<T> g(f);
-  const T x = xs[p], y = ys[p];
-  const T w0 = stage_w<T>(s, 0), w1 = stage_w<T>(s, 1), w2 = stage_w<T>(s, 2);
-  VelJac<T> J1, J2, J3, J4;
-  bool ok = sts[p] == STATUS_OK;
-  ok = ok && vel_jac(f, g, s.k[0], w0, x, y, J1);
-  ok = ok && vel_jac(f, g, s.k[1], w1, x + T(0.5) * dt * J1.flon, y + T(0.5) * dt * J1.flat, J2);
-  ok = ok && vel_jac(f, g, s.k[1], w1, x + T(0.5) * dt * J2.flon, y + T(0.5) * dt * J2.flat, J3);
-  ok = ok && vel_jac(f, g, s.k[2], w2, x + dt * J3.flon, y + dt * J3.flat, J4);
-  if (ok) {  // a non-finite step was frozen by the forward: identity, like a stage off the grid
-    const T nx = x + (J1.flon + T(2) * J2.flon + T(2) * J3.flon + J4.flon) * (dt * (T(1) / T(6)));
-    const T ny = y + (J1.flat + T(2) * J2.flat + T(2) * J3.flat + J4.flat) * (dt * (T(1) / T(6)));
-    ok = isfinite(nx) && isfinite(ny);
+// A microbe has one entry in every cell its stages sampled: the stages of that cell as bits. The cell
+// of stage 1 comes first; which of the stages 2..4 open another entry, and its bits.
+__device__ __forceinline__ uint32_t base_mask(const uint4& c) {
+  return 1u | (c.y == c.x ? 2u : 0u) | (c.z == c.x ? 4u : 0u) | (c.w == c.x ? 8u : 0u);
+}
+template <class F>
+__device__ __forceinline__ void for_other_cells(const uint4& c, F&& f) {
+  if (c.y != c.x) f(c.y, 2u | (c.z == c.y ? 4u : 0u) | (c.w == c.y ? 8u : 0u));
+  if (c.z != c.x && c.z != c.y) f(c.z, 4u | (c.w == c.z ? 8u : 0u));
+  if (c.w != c.x && c.w != c.y && c.w != c.z) f(c.w, 8u);
+}
+
+// Count the entries of one microbe's step and raise its cells' largest adjoint to `top` (every lane of the
+// warp calls this; `ok` false: no entries). Lanes with the same first cell, the usual case, share the
+// atomics.
+__device__ __forceinline__ void count_entries(const AdjBatch& b, int q, bool ok, const uint4& c, uint32_t top) {
+  uint32_t* count = b.count + (size_t)q * b.cells;
+  uint32_t* most = b.top + (size_t)q * b.cells;
+  const uint32_t peers = __match_any_sync(0xffffffffu, ok ? c.x : NONE);
+  const uint32_t t = __reduce_max_sync(peers, top);
+  if (!ok) return;
+  if ((threadIdx.x & 31u) == (uint32_t)(__ffs(peers) - 1)) {
+    atomicAdd(count + c.x, (uint32_t)__popc(peers));
+    atomicMax(most + c.x, t);
   }
-  adj_tail<T>(f, p, ok, J1, J2, J3, J4, dt, lx, ly, rec, key, sent, mkey, mcode, msent, err);
+  for_other_cells(c, [&](uint32_t cell, uint32_t) {
+    atomicAdd(count + cell, 1u);
+    atomicMax(most + cell, top);
+  });
+}
+
+// Steps m_last, m_last - 1, ... (`steps` of them) of every microbe: lambda_{m+1} -> lambda_m, plus 4
+// records and the 4 stage cells a step. A frozen step (a stage left the grid or the step was
+// non-finite, as in the forward) passes the adjoint through and has no entries. xs, ys, sts: the
+// states before step m at offset (m - m_last) * n.
+template <class T>
+__global__ void __launch_bounds__(ADJ_THREADS, sizeof(T) == 8 ? 1 : 7) k_adj_step(FieldView f, const AdjStep* __restrict__ table, int m_last, T dt,
+                                                  AdjBatch b, const T* __restrict__ xs, const T* __restrict__ ys,
+                                                  const uint8_t* __restrict__ sts, T* __restrict__ lx,
+                                                  T* __restrict__ ly) {
+  const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool live = p < b.n;
+  const Geo<T> g(f);
+  T gx = live ? lx[p] : T(0), gy = live ? ly[p] : T(0);
+  for (int q = 0; q < b.steps; ++q) {
+    const AdjStep s = table[m_last - q];
+    const ptrdiff_t o = (ptrdiff_t)p - (ptrdiff_t)q * b.n;
+    const T w0 = stage_w<T>(s, 0), w1 = stage_w<T>(s, 1), w2 = stage_w<T>(s, 2);
+    VelJac<T> J[4];
+    bool ok = live && sts[o] == STATUS_OK;
+    uint4 c = make_uint4(NONE, NONE, NONE, NONE);
+    uint32_t top = 0;
+    if (ok) {
+      const T x = xs[o], y = ys[o];
+      ok = ok && vel_jac(f, g, s.k[0], w0, x, y, J[0]);
+      ok = ok && vel_jac(f, g, s.k[1], w1, x + T(0.5) * dt * J[0].flon, y + T(0.5) * dt * J[0].flat, J[1]);
+      ok = ok && vel_jac(f, g, s.k[1], w1, x + T(0.5) * dt * J[1].flon, y + T(0.5) * dt * J[1].flat, J[2]);
+      ok = ok && vel_jac(f, g, s.k[2], w2, x + dt * J[2].flon, y + dt * J[2].flat, J[3]);
+      if (ok) {
+        const T nx = x + (J[0].flon + T(2) * J[1].flon + T(2) * J[2].flon + J[3].flon) * (dt * (T(1) / T(6)));
+        const T ny = y + (J[0].flat + T(2) * J[1].flat + T(2) * J[2].flat + J[3].flat) * (dt * (T(1) / T(6)));
+        ok = isfinite(nx) && isfinite(ny);
+      }
+      if (ok) {
+        top = adj_tail<T>(J, dt, gx, gy, b.rec + 4 * ((size_t)q * b.n + p));
+        c = make_uint4(J[0].cell, J[1].cell, J[2].cell, J[3].cell);
+      }
+    }
+    if (live) b.cell[(size_t)q * b.n + p] = c;
+    count_entries(b, q, ok, c, top);
+  }
+  if (live) {
+    lx[p] = gx;
+    ly[p] = gy;
+  }
 }
 
 // ---------------------------------------------------------------- double-float positions
@@ -402,11 +446,14 @@ __device__ __forceinline__ DS ds_mul(DS a, DS b) {
 // The grid in double-float: fx = (x - gx0) / dx with 1/dx to double-float accuracy (a float32
 // 1/dx alone would shift the sampling point by up to ~0.1 m at the far edge of the grid).
 struct GeoDS {
+  // (split into two words on the host: twelve float64 operations a thread took a quarter of the time of
+  // a backward step)
   DS mgx0, mgy0, inv_dx, inv_dy;  // -gx0, -gy0 (grid origin minus state origin), 1/dx, 1/dy
   float max_fx, max_fy, org_lat, inv_dxf, inv_dyf;
   __device__ explicit GeoDS(const FieldView& f)
-      : mgx0(ds_of(-f.gx0d)), mgy0(ds_of(-f.gy0d)), inv_dx(ds_of(f.inv_dxd)), inv_dy(ds_of(f.inv_dyd)),
-        max_fx(f.max_fx), max_fy(f.max_fy), org_lat(f.org_lat), inv_dxf((float)f.inv_dxd), inv_dyf((float)f.inv_dyd) {}
+      : mgx0{f.ds_mgx0.x, f.ds_mgx0.y}, mgy0{f.ds_mgy0.x, f.ds_mgy0.y}, inv_dx{f.ds_inv_dx.x, f.ds_inv_dx.y},
+        inv_dy{f.ds_inv_dy.x, f.ds_inv_dy.y}, max_fx(f.max_fx), max_fy(f.max_fy), org_lat(f.org_lat),
+        inv_dxf(f.inv_dx), inv_dyf(f.inv_dy) {}
 };
 
 // Cell index and bilinear fraction of a double-float grid coordinate u in [0, max]; false outside.
@@ -484,7 +531,7 @@ __global__ void k_adj_final_ds(FieldView f, uint32_t n, const DS* __restrict__ x
   }
 }
 
-__global__ void __launch_bounds__(256) k_adj_forward_ds(FieldView f, const AdjStep* __restrict__ table, int m0, int m1,
+__global__ void __launch_bounds__(ADJ_THREADS) k_adj_forward_ds(FieldView f, const AdjStep* __restrict__ table, int m0, int m1,
                                                         float dt, uint32_t n, DS* __restrict__ xs, DS* __restrict__ ys,
                                                         uint8_t* __restrict__ sts, DS* __restrict__ rec_x,
                                                         DS* __restrict__ rec_y, uint8_t* __restrict__ rec_st,
@@ -524,21 +571,36 @@ __global__ void __launch_bounds__(256) k_adj_forward_ds(FieldView f, const AdjSt
   if (bits) atomicOr(err, bits);
 }
 
-__global__ void __launch_bounds__(256) k_adj_step_ds(FieldView f, AdjStep s, float dt, uint32_t n,
-                                                     const DS* __restrict__ xs, const DS* __restrict__ ys,
-                                                     const uint8_t* __restrict__ sts, float* __restrict__ lx,
-                                                     float* __restrict__ ly, float4* __restrict__ rec,
-                                                     uint32_t* __restrict__ key, uint32_t sent,
-                                                     uint32_t* __restrict__ mkey, uint32_t* __restrict__ mcode,
-                                                     uint32_t msent, uint32_t* err) {
+__global__ void __launch_bounds__(ADJ_THREADS, 7) k_adj_step_ds(FieldView f, const AdjStep* __restrict__ table, int m_last,
+                                                     float dt, AdjBatch b, const DS* __restrict__ xs,
+                                                     const DS* __restrict__ ys, const uint8_t* __restrict__ sts,
+                                                     float* __restrict__ lx, float* __restrict__ ly) {
   const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= n) return;
+  const bool live = p < b.n;
   const GeoDS g(f);
-  VelJac<float> J[4];
-  DS nx, ny;
-  bool ok = sts[p] == STATUS_OK && rk4_ds(f, g, s, dt, xs[p], ys[p], J, nx, ny);
-  ok = ok && ds_finite(nx) && ds_finite(ny);
-  adj_tail<float>(f, p, ok, J[0], J[1], J[2], J[3], dt, lx, ly, rec, key, sent, mkey, mcode, msent, err);
+  float gx = live ? lx[p] : 0.f, gy = live ? ly[p] : 0.f;
+  for (int q = 0; q < b.steps; ++q) {
+    const AdjStep s = table[m_last - q];
+    const ptrdiff_t o = (ptrdiff_t)p - (ptrdiff_t)q * b.n;
+    VelJac<float> J[4];
+    bool ok = live && sts[o] == STATUS_OK;
+    uint4 c = make_uint4(NONE, NONE, NONE, NONE);
+    uint32_t top = 0;
+    if (ok) {
+      DS nx, ny;
+      ok = rk4_ds(f, g, s, dt, xs[o], ys[o], J, nx, ny) && ds_finite(nx) && ds_finite(ny);
+      if (ok) {
+        top = adj_tail<float>(J, dt, gx, gy, b.rec + 4 * ((size_t)q * b.n + p));
+        c = make_uint4(J[0].cell, J[1].cell, J[2].cell, J[3].cell);
+      }
+    }
+    if (live) b.cell[(size_t)q * b.n + p] = c;
+    count_entries(b, q, ok, c, top);
+  }
+  if (live) {
+    lx[p] = gx;
+    ly[p] = gy;
+  }
 }
 
 __global__ void __launch_bounds__(256) k_adj_signature_ds(FieldView f, const AdjStep* __restrict__ table, int n_steps,
@@ -617,431 +679,313 @@ __global__ void __launch_bounds__(256) k_adj_signature(FieldView f, const AdjSte
   sig[p] = h;
 }
 
-// ---------------------------------------------------------------- K7a: stable LSD radix sort
+// ---------------------------------------------------------------- K7: reduction onto the grid
 
-constexpr int RS_THREADS = 256;
-constexpr int RS_ITEMS = 16;
-constexpr uint32_t RS_TILE = RS_THREADS * RS_ITEMS;
-constexpr int RS_WARPS = RS_THREADS / 32;
-
-// Digit histogram of one tile, written digit-major: hist[d * tiles + tile].
-__global__ void __launch_bounds__(RS_THREADS) k_rs_hist(const uint32_t* __restrict__ keys, uint32_t m, int shift,
-                                                        int bits, uint32_t* __restrict__ hist, uint32_t tiles) {
-  __shared__ uint32_t h[RS_RADIX_MAX];
-  const uint32_t R = 1u << bits, mask = R - 1u;
-  for (uint32_t d = threadIdx.x; d < R; d += RS_THREADS) h[d] = 0;
-  __syncthreads();
-  const uint32_t base = blockIdx.x * RS_TILE;
-  const uint32_t lane = threadIdx.x & 31u;
-  for (int r = 0; r < RS_ITEMS; ++r) {
-    const uint32_t i = base + (uint32_t)r * RS_THREADS + threadIdx.x;
-    const bool valid = i < m;
-    const uint32_t d = valid ? (keys[i] >> shift) & mask : R;
-    const uint32_t peers = __match_any_sync(0xffffffffu, d);
-    if (valid && (peers & ((1u << lane) - 1u)) == 0) atomicAdd(&h[d], (uint32_t)__popc(peers));
-  }
-  __syncthreads();
-  for (uint32_t d = threadIdx.x; d < R; d += RS_THREADS) hist[(size_t)d * tiles + blockIdx.x] = h[d];
-}
-
-// Stable scatter of one tile. Warp w takes the tile's w-th run of RS_ITEMS * 32 consecutive items
-// (RS_ITEMS rounds of 32) and ranks each item among the equal digits of its run with match masks and
-// a per-warp digit counter, without block barriers; the block then turns the counters into per-warp
-// digit offsets (the tile's offset of the digit plus the counts of the earlier warps), and each
-// item goes to its warp's offset plus its rank: equal keys keep their order.
-__global__ void __launch_bounds__(RS_THREADS) k_rs_scatter(const uint32_t* __restrict__ kin,
-                                                           const uint32_t* __restrict__ vin,
-                                                           uint32_t* __restrict__ kout, uint32_t* __restrict__ vout,
-                                                           uint32_t m, int shift, int bits,
-                                                           const uint32_t* __restrict__ hscan, uint32_t tiles) {
-  __shared__ uint32_t wcnt[RS_WARPS][RS_RADIX_MAX];
-  const uint32_t R = 1u << bits, mask = R - 1u;
+// Room for the entries of every occupied cell of step blockIdx.y (consecutive from place[c]) and the
+// list of items, one per ADJ_ITEM entries of a cell: one reservation of each per block.
+constexpr int ALLOC_THREADS = 512;
+__global__ void __launch_bounds__(ALLOC_THREADS) k_adj_alloc(AdjBatch b, uint32_t items_cap) {
+  pdl_wait();
+  __shared__ uint32_t we[ALLOC_THREADS / 32], wl[ALLOC_THREADS / 32], base[2];
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  for (uint32_t d = threadIdx.x; d < R; d += RS_THREADS)
-    for (int w = 0; w < RS_WARPS; ++w) wcnt[w][d] = 0;
-  __syncthreads();
-  const uint32_t base = blockIdx.x * RS_TILE + warp * (RS_ITEMS * 32u);
-  const uint32_t lt = (1u << lane) - 1u;
-  uint32_t kk[RS_ITEMS], rk[RS_ITEMS];
-#pragma unroll
-  for (int r = 0; r < RS_ITEMS; ++r) {
-    const uint32_t i = base + (uint32_t)r * 32u + lane;
-    const bool valid = i < m;
-    const uint32_t k = valid ? kin[i] : 0u;
-    const uint32_t d = valid ? (k >> shift) & mask : R;
-    const uint32_t peers = __match_any_sync(0xffffffffu, d);
-    const uint32_t below = peers & lt;
-    const uint32_t c = valid ? wcnt[warp][d] : 0u;  // every peer reads the count before the update
-    __syncwarp();
-    if (valid && below == 0) wcnt[warp][d] = c + (uint32_t)__popc(peers);
-    __syncwarp();
-    kk[r] = k;
-    rk[r] = c + (uint32_t)__popc(below);
-  }
-  __syncthreads();
-  for (uint32_t d = threadIdx.x; d < R; d += RS_THREADS) {
-    uint32_t o = hscan[(size_t)d * tiles + blockIdx.x];
-    for (int w = 0; w < RS_WARPS; ++w) {
-      const uint32_t c = wcnt[w][d];
-      wcnt[w][d] = o;
-      o += c;
+  const uint32_t c = blockIdx.x * ALLOC_THREADS + threadIdx.x;
+  const size_t o = (size_t)blockIdx.y * b.cells;
+  const uint32_t m = c < b.cells ? b.count[o + c] : 0u, items = (m + ADJ_ITEM - 1) / ADJ_ITEM;
+  uint32_t se = m, sl = items;  // inclusive sums over the warp
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint32_t x = __shfl_up_sync(0xffffffffu, se, d), y = __shfl_up_sync(0xffffffffu, sl, d);
+    if (lane >= (uint32_t)d) {
+      se += x;
+      sl += y;
     }
   }
-  __syncthreads();
-#pragma unroll
-  for (int r = 0; r < RS_ITEMS; ++r) {
-    const uint32_t i = base + (uint32_t)r * 32u + lane;
-    if (i < m) {
-      const uint32_t o = wcnt[warp][(kk[r] >> shift) & mask] + rk[r];
-      kout[o] = kk[r];
-      vout[o] = vin ? vin[i] : i;
-    }
-  }
-}
-
-// Exclusive scan of n uint32 values (in -> out), in SCAN_BLOCKS contiguous chunks: block sums, then
-// each block adds the sums of the blocks before it while scanning its chunk.
-__device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* sh, uint32_t* total) {
-  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  uint32_t x = v;
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-    if (lane >= (uint32_t)o) x += y;
-  }
-  if (lane == 31) sh[warp] = x;
-  __syncthreads();
-  if (warp == 0) {
-    uint32_t s = lane < blockDim.x / 32 ? sh[lane] : 0u;
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t y = __shfl_up_sync(0xffffffffu, s, o);
-      if (lane >= (uint32_t)o) s += y;
-    }
-    sh[lane] = s;  // inclusive warp totals
+  if (lane == 31) {
+    we[warp] = se;
+    wl[warp] = sl;
   }
   __syncthreads();
-  const uint32_t before = warp ? sh[warp - 1] : 0u;
-  *total = sh[blockDim.x / 32 - 1];
-  __syncthreads();
-  return before + x - v;
-}
-
-__global__ void __launch_bounds__(256) k_scan_sums(const uint32_t* __restrict__ in, size_t n, size_t chunk,
-                                                   uint32_t* __restrict__ bsum) {
-  __shared__ uint32_t red[8];
-  const size_t lo = (size_t)blockIdx.x * chunk, hi = min(n, lo + chunk);
-  uint32_t s = 0;
-  for (size_t i = lo + threadIdx.x; i < hi; i += blockDim.x) s += in[i];
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
-  __syncthreads();
-  if (threadIdx.x == 0) {
+  if (threadIdx.x < 2) {
+    uint32_t* w = threadIdx.x ? wl : we;
     uint32_t t = 0;
-    for (int w = 0; w < 8; ++w) t += red[w];
-    bsum[blockIdx.x] = t;
-  }
-}
-
-__global__ void __launch_bounds__(256) k_scan_chunks(const uint32_t* __restrict__ in, uint32_t* __restrict__ out,
-                                                     size_t n, size_t chunk, const uint32_t* __restrict__ bsum) {
-  __shared__ uint32_t sh[32];
-  __shared__ uint32_t carry;
-  if (threadIdx.x < 32) {
-    uint32_t s = 0;
-    for (uint32_t b = threadIdx.x; b < blockIdx.x; b += 32) s += bsum[b];
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (threadIdx.x == 0) carry = s;
+    for (int k = 0; k < ALLOC_THREADS / 32; ++k) {
+      const uint32_t x = w[k];
+      w[k] = t;
+      t += x;
+    }
+    base[threadIdx.x] = t ? atomicAdd(b.total + 2 * blockIdx.y + threadIdx.x, t) : 0u;
   }
   __syncthreads();
-  const size_t lo = (size_t)blockIdx.x * chunk, hi = min(n, lo + chunk);
-  for (size_t t = lo; t < hi; t += blockDim.x) {
-    const size_t i = t + threadIdx.x;
-    const uint32_t v = i < hi ? in[i] : 0u;
-    uint32_t total;
-    const uint32_t ex = block_exclusive_scan(v, sh, &total);
-    if (i < hi) out[i] = carry + ex;
-    __syncthreads();
-    if (threadIdx.x == 0) carry += total;
-    __syncthreads();
+  if (!m) return;
+  const uint32_t at = base[0] + we[warp] + se - m;
+  b.place[o + c] = at;
+  uint4* list = b.list + (size_t)blockIdx.y * items_cap + base[1] + wl[warp] + sl - items;
+  for (uint32_t k = 0; k < items; ++k) list[k] = make_uint4(c, at + k * ADJ_ITEM, min(ADJ_ITEM, m - k * ADJ_ITEM), m);
+  if (items > 1) {  // several warps add to the cell's sums
+    for (int k = 0; k < 24; ++k) b.csum[(o + c) * 24 + k] = 0ll;
   }
 }
 
-// ---------------------------------------------------------------- K7b: segmented reduction
-
-// Segment bounds of the sorted keys: cst[k] = first index, cen[k] = one past the last (both left at
-// 0 for absent keys; the reduction resets the entries it read).
-__global__ void k_adj_bounds(const uint32_t* __restrict__ skey, uint32_t m, uint32_t sent, uint32_t* __restrict__ cst,
-                             uint32_t* __restrict__ cen) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= m) return;
-  const uint32_t k = skey[i];
-  if (k >= sent) return;
-  if (i == 0 || skey[i - 1] != k) cst[k] = i;
-  if (i + 1 == m || skey[i + 1] != k) cen[k] = i + 1;
+// Entries of the microbes' steps into their cells, in whatever order they come.
+__global__ void __launch_bounds__(256) k_adj_scatter(AdjBatch b) {
+  pdl_wait();
+  const uint32_t p = blockIdx.x * 256 + threadIdx.x, lane = threadIdx.x & 31u;
+  const uint32_t q = blockIdx.y;
+  uint32_t* place = b.place + (size_t)q * b.cells;
+  uint2* ent = b.ent + (size_t)q * 4 * b.n;
+  const uint4 c = p < b.n ? b.cell[(size_t)q * b.n + p] : make_uint4(NONE, NONE, NONE, NONE);
+  const uint32_t peers = __match_any_sync(0xffffffffu, c.x);
+  if (c.x == NONE) return;
+  const int leader = __ffs(peers) - 1;
+  uint32_t at = 0;
+  if (lane == (uint32_t)leader) at = atomicAdd(place + c.x, (uint32_t)__popc(peers));
+  at = __shfl_sync(peers, at, leader) + __popc(peers & ((1u << lane) - 1u));
+  ent[at] = make_uint2(p, base_mask(c));
+  for_other_cells(c, [&](uint32_t cell, uint32_t mask) { ent[atomicAdd(place + cell, 1u)] = make_uint2(p, mask); });
 }
 
-__device__ __forceinline__ void neumaier(float& s, float& c, float v) {
-  const float t = s + v;
-  c += (fabsf(s) >= fabsf(v)) ? ((s - t) + v) : ((v - t) + s);
-  s = t;
+// Integer sum of products v scaled into [-2^21, 2^21]: hi takes the nearest integer, lo the remainder
+// in 2^-20. Adding 1.5 * 2^23 leaves the integer in a float's low bits; the sums run on the raw bits
+// (the constant is taken out at the end), so a term is four FMA-pipe operations and two adds.
+constexpr float FIX_MAGIC = 12582912.0f;  // 1.5 * 2^23
+struct FixSum {
+  uint32_t hi, lo;
+};
+__device__ __forceinline__ void fix_add(FixSum& a, float v, float scale) {
+  const float t = fmaf(v, scale, FIX_MAGIC);
+  const float rest = fmaf(v, scale, FIX_MAGIC - t);  // exact, in [-1/2, 1/2]
+  a.hi += __float_as_uint(t);
+  a.lo += __float_as_uint(fmaf(rest, 1048576.0f, FIX_MAGIC));
 }
 
-// One warp per field cell: for each stage time g, the records of segment (cell, g) in sorted order,
-// lane l taking entries l, l+32, ...; out csum[(cell * 3 + g) * 8 + q], q = corner (00, 01, 10, 11)
-// of dL/dU, then of dL/dV.
-__global__ void __launch_bounds__(256) k_adj_reduce(uint32_t ncells, uint32_t* __restrict__ cst,
-                                                    uint32_t* __restrict__ cen, const uint32_t* __restrict__ sval,
-                                                    const float4* __restrict__ rec, float* __restrict__ csum) {
+// v[i] summed over the warp, for i = lane & 15 (12 values, zeros above): every step but the last
+// halves the values a lane keeps, 16 exchanges in all.
+__device__ __forceinline__ uint32_t sum_by_lane(const uint32_t (&in)[12]) {
   const uint32_t lane = threadIdx.x & 31u;
-  const uint32_t wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
-  for (uint32_t c = wid; c < ncells; c += nw) {
-    for (uint32_t g = 0; g < 3; ++g) {
-      const uint32_t k = 4u * c + g;
-      const uint32_t lo = cst[k], hi = cen[k];
-      float* out = csum + ((size_t)c * 3 + g) * 8;
-      if (lo == hi) {  // warp-uniform: an empty segment
-        if (lane < 8) out[lane] = 0.f;
-        continue;
-      }
-      float s[8], e[8];
+  uint32_t v[8];
 #pragma unroll
-      for (int q = 0; q < 8; ++q) s[q] = e[q] = 0.f;
-      for (uint32_t i = lo + lane; i < hi; i += 32) {
-        const float4 r = rec[sval[i]];
-        const float a = r.x, b = r.y;
-        const float w[4] = {(1.f - a) * (1.f - b), a * (1.f - b), (1.f - a) * b, a * b};
+  for (int i = 0; i < 8; ++i) {
+    const uint32_t up = i + 8 < 12 ? in[i + 8 < 12 ? i + 8 : 0] : 0u;
+    const uint32_t send = lane & 8u ? in[i] : up, keep = lane & 8u ? up : in[i];
+    v[i] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
+  }
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          neumaier(s[q], e[q], w[q] * r.z);
-          neumaier(s[4 + q], e[4 + q], w[q] * r.w);
-        }
-      }
+  for (int h = 4; h > 0; h >>= 1) {
 #pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        float t = s[q] + e[q];
-        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-        s[q] = t;
-      }
-      if (lane == 0) {
-#pragma unroll
-        for (int q = 0; q < 8; ++q) out[q] = s[q];
-        cst[k] = 0;
-        cen[k] = 0;
-      }
+    for (int i = 0; i < h; ++i) {
+      const uint32_t send = lane & (uint32_t)h ? v[i] : v[i + h], keep = lane & (uint32_t)h ? v[i + h] : v[i];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, h);
     }
   }
+  return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 16);
 }
 
-// Gather form, after the stable sort of the microbe keys (cell * 2 + leaves-the-cell, so in index
-// order within a key): bounds of every key, the stage codes in sorted order, and the list of target
-// cells: a cell with microbes, and the 3 x 3 cells around one whose microbes leave it, each listed
-// once a step (mark[c] takes the step's stamp when c is listed; tcnt counts the list).
-__global__ void k_adj_cells(const uint32_t* __restrict__ skey, const uint32_t* __restrict__ sval, uint32_t m,
-                            uint32_t cw, uint32_t ch, const uint32_t* __restrict__ mcode,
-                            uint32_t* __restrict__ scode, uint32_t* __restrict__ cst, uint32_t* __restrict__ cen,
-                            uint32_t* __restrict__ mark, uint32_t stamp, uint32_t* __restrict__ tlist,
-                            uint32_t* __restrict__ tcnt) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= m) return;
-  const uint32_t k = skey[i];
-  if (k >= 2u * cw * ch) return;  // frozen microbes sort last
-  scode[i] = mcode[sval[i]];
-  if (i + 1 == m || skey[i + 1] != k) cen[k] = i + 1;
-  if (i != 0 && skey[i - 1] == k) return;
-  cst[k] = i;
-  const uint32_t b = k >> 1;
-  if (!(k & 1u)) {
-    if (atomicExch(&mark[b], stamp) != stamp) tlist[atomicAdd(tcnt, 1u)] = b;
-    return;
-  }
-  const int bi = (int)(b % cw), bj = (int)(b / cw);
-  const uint32_t cells = cw * ch;
-  uint32_t tc[9], old[9], fresh = 0;
-#pragma unroll
-  for (int r = 0; r < 9; ++r) {  // no branch between the exchanges: they are issued together
-    const int ti = bi + r % 3 - 1, tj = bj + r / 3 - 1;
-    const bool in = ti >= 0 && tj >= 0 && ti < (int)cw && tj < (int)ch;
-    tc[r] = in ? (uint32_t)tj * cw + (uint32_t)ti : cells;  // mark[cells]: a slot no target reads
-    old[r] = atomicExch(&mark[tc[r]], stamp);
-  }
-#pragma unroll
-  for (int r = 0; r < 9; ++r) fresh |= (tc[r] != cells && old[r] != stamp) ? 1u << r : 0u;
-  if (!fresh) return;
-  uint32_t o = atomicAdd(tcnt, (uint32_t)__popc(fresh));
-#pragma unroll
-  for (int r = 0; r < 9; ++r)
-    if (fresh & (1u << r)) tlist[o++] = tc[r];
-}
-
+// The stages `mask` of one entry's records into one component's sums, the four corners (00, 01, 10, 11)
+// of each stage time: stage 1 at t (group 0), stages 2 and 3 at t + dt/2 (group 1), stage 4 at t + dt
+// (group 2).
 template <int G>
-__device__ __forceinline__ void gather_add(const float4& rr, float (&acc)[3][8], float (&cmp)[3][8]) {
-  const float a = rr.x, b = rr.y;
+__device__ __forceinline__ void gather_add(const float4& r, bool V, float scale, FixSum (&acc)[12]) {
+  const float a = r.x, b = r.y, g = V ? r.w : r.z;
   const float w[4] = {(1.f - a) * (1.f - b), a * (1.f - b), (1.f - a) * b, a * b};
 #pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    neumaier(acc[G][q], cmp[G][q], w[q] * rr.z);
-    neumaier(acc[G][4 + q], cmp[G][4 + q], w[q] * rr.w);
+  for (int q = 0; q < 4; ++q) fix_add(acc[4 * G + q], w[q] * g, scale);
+}
+
+__device__ __forceinline__ uint32_t adjoint_bits(const float4& r) {
+  return max(__float_as_uint(r.z) & 0x7fffffffu, __float_as_uint(r.w) & 0x7fffffffu);
+}
+
+// A cell's scale is 2^adj_scale_bits: 2^(21 - e) for 2^e above its largest |dL/dU|, |dL/dV|, so a term
+// is kept to 2^(e - 42), where its own float32 rounding is 2^-25 of it (coarser by the factor that
+// keeps the 64-bit sums of more than 2^20 entries in range). m: entries of the cell.
+__device__ __forceinline__ int adj_scale_bits(uint32_t top, uint32_t m) {
+  const int big = m > (1u << 20) ? 12 - __clz(m) : 0;  // log2(m) - 20, rounded up
+  return 21 - big - (max((int)(top >> 23), 20) - 126);
+}
+constexpr uint32_t ADJ_NOT_FINITE = 0x7f800000u;  // `top` from here: some adjoint is infinite or NaN
+
+// Two warps per item, one for dL/dU and one for dL/dV, one entry per lane at a time. Cells of several
+// items add up with integer atomics. Sums that are not finite are formed in float by the first item.
+__global__ void __launch_bounds__(256, 4) k_adj_gather(AdjBatch b, uint32_t items_cap) {
+  pdl_wait();
+  const uint32_t lane = threadIdx.x & 31u, q = blockIdx.y;
+  const uint32_t nt = b.total[2 * q + 1];
+  const size_t oc = (size_t)q * b.cells;
+  const uint4* list = b.list + (size_t)q * items_cap;
+  const uint2* ent = b.ent + (size_t)q * 4 * b.n;
+  const float4* rec = b.rec + (size_t)q * 4 * b.n;
+  const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, stride = (gridDim.x * blockDim.x) >> 6;
+  const bool V = warp & 1u;
+  const uint32_t one = __float_as_uint(FIX_MAGIC);
+  uint4 next = (warp >> 1) < nt ? list[warp >> 1] : make_uint4(0u, 0u, 0u, 0u);
+  for (uint32_t t = warp >> 1; t < nt; t += stride) {
+    const uint32_t c = next.x, lo = next.y, m = next.z, all = next.w;
+    const uint32_t top = b.top[oc + c];
+    next = t + stride < nt ? list[t + stride] : make_uint4(0u, 0u, 0u, 0u);
+    long long* out = b.csum + (oc + c) * 24;  // per stage time: the corners of dL/dU, then of dL/dV
+    if (top >= ADJ_NOT_FINITE) {
+      const bool first = all <= ADJ_ITEM || lo + all - 1u == b.place[oc + c] - 1u;  // place: one past the cell
+      if (!V && first && lane < 24) {
+        float s = 0.f;
+        for (uint32_t i = 0; i < all; ++i) {
+          const uint2 x = ent[lo + i];
+          for (uint32_t k = 0; k < 4; ++k) {
+            if (!((x.y >> k) & 1u) || (k + 1) / 2 != lane / 8) continue;
+            const float4 z = rec[4 * (size_t)x.x + k];
+            s += (lane & 1u ? z.x : 1.f - z.x) * (lane & 2u ? z.y : 1.f - z.y) * (lane & 4u ? z.w : z.z);
+          }
+        }
+        out[lane] = (long long)__float_as_uint(s);
+      }
+      continue;
+    }
+    const float scale = __uint_as_float((uint32_t)(adj_scale_bits(top, all) + 127) << 23);
+    FixSum acc[12];
+#pragma unroll
+    for (int k = 0; k < 12; ++k) acc[k].hi = acc[k].lo = 0u;
+    uint32_t n0 = 0, n1 = 0, n2 = 0;  // terms a group's sums took
+    uint2 ents[ADJ_ITEM / 32];
+#pragma unroll
+    for (uint32_t k = 0; k < ADJ_ITEM / 32; ++k)
+      ents[k] = lane + 32 * k < m ? ent[lo + lane + 32 * k] : make_uint2(0u, 0u);
+#pragma unroll
+    for (uint32_t k4 = 0; k4 < ADJ_ITEM / 32; ++k4) {
+      if (32 * k4 >= m) break;  // warp-uniform
+      const uint2 e = ents[k4];
+      const float4* rp = rec + 4 * (size_t)e.x;
+      float4 r[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if ((e.y >> k) & 1u) r[k] = rp[k];
+      if (e.y & 1u) gather_add<0>(r[0], V, scale, acc);
+      if (e.y & 2u) gather_add<1>(r[1], V, scale, acc);
+      if (e.y & 4u) gather_add<1>(r[2], V, scale, acc);
+      if (e.y & 8u) gather_add<2>(r[3], V, scale, acc);
+      n0 += e.y & 1u;
+      n1 += __popc(e.y & 6u);
+      n2 += (e.y >> 3) & 1u;
+    }
+    uint32_t v[12];
+#pragma unroll
+    for (int k = 0; k < 12; ++k) v[k] = acc[k].hi - one * (k < 4 ? n0 : k < 8 ? n1 : n2);
+    const int hi = (int)sum_by_lane(v);  // at most 2 * ADJ_ITEM terms of 2^21
+#pragma unroll
+    for (int k = 0; k < 12; ++k) v[k] = acc[k].lo - one * (k < 4 ? n0 : k < 8 ? n1 : n2);
+    const long long sum = (long long)hi * 1048576ll + (int)sum_by_lane(v);
+    if (lane < 12) {
+      long long* at = out + (lane >> 2) * 8 + (lane & 3u) + (V ? 4 : 0);
+      if (all <= ADJ_ITEM)
+        *at = sum;
+      else
+        atomicAdd(reinterpret_cast<unsigned long long*>(at), (unsigned long long)sum);
+    }
   }
 }
 
-// One warp per listed target cell c. Neighbour cell r = (dj + 1) * 3 + (di + 1) in turn: its whole
-// run for r = 4 (c itself), else only its microbes that leave it; lane l takes entries l, l + 32,
-// ... of each run, and a stage of a microbe of neighbour r lands in c when its slot is 8 - r. Stage
-// times: stage 1 at t (group 0), stages 2 and 3 at t + dt/2 (group 1), stage 4 at t + dt (group 2).
-// Sums as in k_adj_reduce (Neumaier float32 per lane, fixed warp tree), so the result does not
-// depend on which warp took c.
-__global__ void __launch_bounds__(256) k_adj_gather(uint32_t cw, uint32_t ch, const uint32_t* __restrict__ tcnt,
-                                                    const uint32_t* __restrict__ tlist,
-                                                    const uint32_t* __restrict__ cst,
-                                                    const uint32_t* __restrict__ cen,
-                                                    const uint32_t* __restrict__ scode,
-                                                    const uint32_t* __restrict__ sval,
-                                                    const float4* __restrict__ rec, float* __restrict__ csum) {
-  const uint32_t lane = threadIdx.x & 31u;
-  const uint32_t nt = *tcnt;
-  const uint32_t stride = gridDim.x * (blockDim.x >> 5);
-  for (uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < nt; t += stride) {
-    const uint32_t c = tlist[t];
-    const int ci = (int)(c % cw), cj = (int)(c / cw);
-    uint32_t lo = 0, hi = 0;
-    if (lane < 9) {
-      const int bi = ci + (int)(lane % 3) - 1, bj = cj + (int)(lane / 3) - 1;
-      if (bi >= 0 && bj >= 0 && bi < (int)cw && bj < (int)ch) {
-        const uint32_t k1 = 2u * ((uint32_t)bj * cw + (uint32_t)bi) + 1u;
-        const uint32_t e1 = cen[k1];  // bounds of absent keys: cen = 0
-        if (lane == 4) {              // keys 2b and 2b + 1 are adjacent in sorted order
-          const uint32_t e0 = cen[k1 - 1];
-          lo = e0 ? cst[k1 - 1] : (e1 ? cst[k1] : 0u);
-          hi = e1 ? e1 : e0;
-        } else if (e1) {
-          lo = cst[k1];
-          hi = e1;
-        }
-      }
-    }
-    float acc[3][8], cmp[3][8];
-#pragma unroll
-    for (int g = 0; g < 3; ++g)
-#pragma unroll
-      for (int q = 0; q < 8; ++q) acc[g][q] = cmp[g][q] = 0.f;
-    {  // c's own microbes: stage 1 always lands in c, the others mostly; two entries in flight
-      const uint32_t rlo = __shfl_sync(0xffffffffu, lo, 4), rhi = __shfl_sync(0xffffffffu, hi, 4);
-      for (uint32_t s = rlo + lane; s < rhi; s += 64) {
-        const uint32_t s2 = s + 32;
-        const bool two = s2 < rhi;
-        const uint32_t code0 = scode[s], code1 = two ? scode[s2] : 0u;
-        const float4* rp0 = rec + 4 * (size_t)sval[s];
-        const float4* rp1 = rec + 4 * (size_t)(two ? sval[s2] : 0u);
-        float4 r[2][4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) r[0][q] = rp0[q];
-        if (two) {
-#pragma unroll
-          for (int q = 0; q < 4; ++q) r[1][q] = rp1[q];
-        }
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          if (h == 1 && !two) break;
-          const uint32_t code = h ? code1 : code0;
-          gather_add<0>(r[h][0], acc, cmp);
-          if (((code >> 4) & 15u) == 4u) gather_add<1>(r[h][1], acc, cmp);
-          if (((code >> 8) & 15u) == 4u) gather_add<1>(r[h][2], acc, cmp);
-          if (((code >> 12) & 15u) == 4u) gather_add<2>(r[h][3], acc, cmp);
-        }
-      }
-    }
-#pragma unroll 1
-    for (int r = 0; r < 9; ++r) {
-      if (r == 4) continue;
-      const uint32_t rlo = __shfl_sync(0xffffffffu, lo, r), rhi = __shfl_sync(0xffffffffu, hi, r);
-      const uint32_t slot = 8u - (uint32_t)r;
-      for (uint32_t s = rlo + lane; s < rhi; s += 64) {
-        const uint32_t s2 = s + 32;
-        const uint32_t c0 = scode[s];
-        const uint32_t c1 = s2 < rhi ? scode[s2] : 0xffffffffu;  // slot 15 matches nothing
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const uint32_t code = h ? c1 : c0;
-          const bool m1 = ((code >> 4) & 15u) == slot, m2 = ((code >> 8) & 15u) == slot;
-          const bool m3 = ((code >> 12) & 15u) == slot;  // stage 1 never leaves its cell
-          if (!(m1 | m2 | m3)) continue;
-          const float4* rp = rec + 4 * (size_t)sval[h ? s2 : s];
-          if (m1) gather_add<1>(rp[1], acc, cmp);
-          if (m2) gather_add<1>(rp[2], acc, cmp);
-          if (m3) gather_add<2>(rp[3], acc, cmp);
-        }
-      }
-    }
-    float* out = csum + (size_t)c * 24;
-#pragma unroll
-    for (int g = 0; g < 3; ++g)
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        float v = acc[g][q] + cmp[g][q];
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if (lane == (uint32_t)(g * 8 + q)) out[g * 8 + q] = v;
-      }
-  }
-}
-
-// One thread per grid node: the four cells around it in a fixed order, then the three stage times
-// spread onto frames k_g (weight 1 - w_g) and k_g + 1 (weight w_g), added to the gradient.
-__global__ void __launch_bounds__(256) k_adj_nodes(int nx, int ny, AdjStep s, const float* __restrict__ csum,
-                                                   const uint32_t* __restrict__ mark, uint32_t stamp,
-                                                   float* __restrict__ gu, float* __restrict__ gv) {
-  const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= (uint32_t)nx * (uint32_t)ny) return;
-  const int ni = (int)(q % (uint32_t)nx), nj = (int)(q / (uint32_t)nx);
+// The sums of a batch onto the grid: a block takes 32 consecutive nodes, its warp w step w of every
+// blockDim.y steps. The four cells around a node in a fixed order give its sums at the three stage
+// times; the first warp then spreads them onto frames k_g (weight 1 - w_g) and k_g + 1 (weight w_g) and
+// adds them to the gradient, the steps in turn.
+constexpr int NODE_STEPS = 8;
+__global__ void __launch_bounds__(32 * NODE_STEPS) k_adj_nodes(int nx, int ny, const AdjStep* __restrict__ table,
+                                                               int m_last, AdjBatch b, float* __restrict__ gu,
+                                                               float* __restrict__ gv) {
+  pdl_wait();
+  __shared__ float sums[NODE_STEPS][6][32];
+  __shared__ uint32_t busy[NODE_STEPS];  // nodes with sums at the step
+  const uint32_t lane = threadIdx.x, w = threadIdx.y;
+  const uint32_t node = blockIdx.x * 32 + lane;
+  const bool in = node < (uint32_t)nx * (uint32_t)ny;
+  const int ni = (int)(node % (uint32_t)nx), nj = (int)(node / (uint32_t)nx);
   const int cw = nx - 1;
-  float U[3] = {0.f, 0.f, 0.f}, V[3] = {0.f, 0.f, 0.f};
   // cell (ci, cj) sees this node as corner (nj - cj) * 2 + (ni - ci)
   const int ci_[4] = {ni - 1, ni, ni - 1, ni}, cj_[4] = {nj - 1, nj - 1, nj, nj}, corner[4] = {3, 2, 1, 0};
+  for (int q0 = 0; q0 < b.steps; q0 += (int)blockDim.y) {
+    const int q = q0 + (int)w;
+    float U[3] = {0.f, 0.f, 0.f}, V[3] = {0.f, 0.f, 0.f};
+    if (in && q < b.steps) {
+      uint32_t m[4];
 #pragma unroll
-  for (int t = 0; t < 4; ++t) {
-    const int ci = ci_[t], cj = cj_[t];
-    if (ci < 0 || cj < 0 || ci > nx - 2 || cj > ny - 2) continue;
-    const size_t cell = (size_t)cj * cw + ci;
-    if (mark && mark[cell] != stamp) continue;  // gather form: only listed cells were summed
-    const float* cs = csum + cell * 24;
-#pragma unroll
-    for (int g = 0; g < 3; ++g) {
-      U[g] += cs[g * 8 + corner[t]];
-      V[g] += cs[g * 8 + 4 + corner[t]];
-    }
-  }
-  if (U[0] == 0.f && U[1] == 0.f && U[2] == 0.f && V[0] == 0.f && V[1] == 0.f && V[2] == 0.f) return;
-  int kmin = s.k[0], kmax = s.k[0];
-#pragma unroll
-  for (int g = 0; g < 3; ++g) {
-    kmin = min(kmin, s.k[g]);
-    kmax = max(kmax, s.k[g] + (s.w[g] != 0.f ? 1 : 0));
-  }
-  const size_t plane = (size_t)nx * ny;
-  for (int fr = kmin; fr <= kmax; ++fr) {
-    float du = 0.f, dv = 0.f;
-    bool any = false;
-#pragma unroll
-    for (int g = 0; g < 3; ++g) {
-      if (s.k[g] == fr) {
-        du += (1.f - s.w[g]) * U[g];
-        dv += (1.f - s.w[g]) * V[g];
-        any = true;
+      for (int t = 0; t < 4; ++t) {
+        const int ci = ci_[t], cj = cj_[t];
+        const bool cell = !(ci < 0 || cj < 0 || ci > nx - 2 || cj > ny - 2);
+        m[t] = cell ? b.count[(size_t)q * b.cells + (size_t)cj * cw + ci] : 0u;
       }
-      if (s.w[g] != 0.f && s.k[g] + 1 == fr) {
-        du += s.w[g] * U[g];
-        dv += s.w[g] * V[g];
-        any = true;
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        if (m[t] == 0u) continue;  // only cells with entries were summed
+        const size_t cell = (size_t)q * b.cells + (size_t)cj_[t] * cw + ci_[t];
+        const uint32_t top = b.top[cell];
+        const int bits = adj_scale_bits(top, m[t]) + 20;
+        const long long* cs = b.csum + cell * 24 + corner[t];
+#pragma unroll
+        for (int g = 0; g < 3; ++g) {
+          const long long u = cs[g * 8], v = cs[g * 8 + 4];
+          U[g] += top < ADJ_NOT_FINITE ? ldexpf(__ll2float_rn(u), -bits) : __uint_as_float((uint32_t)u);
+          V[g] += top < ADJ_NOT_FINITE ? ldexpf(__ll2float_rn(v), -bits) : __uint_as_float((uint32_t)v);
+        }
       }
     }
+    const bool any = !(U[0] == 0.f && U[1] == 0.f && U[2] == 0.f && V[0] == 0.f && V[1] == 0.f && V[2] == 0.f);
+    const uint32_t mask = __ballot_sync(0xffffffffu, any);
+    if (lane == 0) busy[w] = mask;
     if (any) {
-      gu[(size_t)fr * plane + q] += du;
-      gv[(size_t)fr * plane + q] += dv;
+#pragma unroll
+      for (int g = 0; g < 3; ++g) {
+        sums[w][g][lane] = U[g];
+        sums[w][3 + g][lane] = V[g];
+      }
     }
+    __syncthreads();
+    if (w == 0) {
+      for (int k = 0; k < (int)blockDim.y; ++k) {
+        if (!((busy[k] >> lane) & 1u)) continue;
+        const AdjStep s = table[m_last - q0 - k];
+        int kmin = s.k[0], kmax = s.k[0];
+#pragma unroll
+        for (int g = 0; g < 3; ++g) {
+          kmin = min(kmin, s.k[g]);
+          kmax = max(kmax, s.k[g] + (s.w[g] != 0.f ? 1 : 0));
+        }
+        const size_t plane = (size_t)nx * ny;
+        for (int fr = kmin; fr <= kmax; ++fr) {
+          float du = 0.f, dv = 0.f;
+          bool hit = false;
+#pragma unroll
+          for (int g = 0; g < 3; ++g) {
+            const float u = sums[k][g][lane], v = sums[k][3 + g][lane];
+            if (s.k[g] == fr) {
+              du += (1.f - s.w[g]) * u;
+              dv += (1.f - s.w[g]) * v;
+              hit = true;
+            }
+            if (s.w[g] != 0.f && s.k[g] + 1 == fr) {
+              du += s.w[g] * u;
+              dv += s.w[g] * v;
+              hit = true;
+            }
+          }
+          if (hit) {
+            gu[(size_t)fr * plane + node] += du;
+            gv[(size_t)fr * plane + node] += dv;
+          }
+        }
+      }
+    }
+    __syncthreads();
   }
 }
 
 // ---------------------------------------------------------------- launchers
 
 static inline unsigned grid_for(size_t n, unsigned block) { return (unsigned)((n + block - 1) / block); }
+
+// ADJ_THREADS, or fewer when that leaves SMs without a block (down to a warp). In float64 it matters
+// most: an SM's two float64 lanes are shared by the warps on it (5,000 microbes: 50 -> 24 us a step).
+static inline unsigned adj_threads(uint32_t n) {
+  unsigned threads = ADJ_THREADS;
+  while (threads > 32 && grid_for(n, threads) < 152) threads /= 2;
+  return threads;
+}
 
 void launch_adj_stages(const FieldView& f, double t_start, double dt, int n_steps, AdjStep* table, uint32_t* err,
                        cudaStream_t st) {
@@ -1101,49 +1045,44 @@ void launch_adj_forward(const FieldView& f, int prec, const AdjStep* table, int 
                         void* x, void* y, uint8_t* status, void* rec_x, void* rec_y, uint8_t* rec_st, uint32_t* err,
                         cudaStream_t st) {
   if (!n || m1 <= m0) return;
+  const unsigned threads = adj_threads(n), blocks = grid_for(n, threads);
   if (prec == ADJ_F64)
-    k_adj_forward<double><<<grid_for(n, 256), 256, 0, st>>>(f, table, m0, m1, dt, n, (double*)x, (double*)y, status,
+    k_adj_forward<double><<<blocks, threads, 0, st>>>(f, table, m0, m1, dt, n, (double*)x, (double*)y, status,
                                                             (double*)rec_x, (double*)rec_y, rec_st, err);
   else if (prec == ADJ_DS)
-    k_adj_forward_ds<<<grid_for(n, 256), 256, 0, st>>>(f, table, m0, m1, (float)dt, n, (DS*)x, (DS*)y, status,
+    k_adj_forward_ds<<<blocks, threads, 0, st>>>(f, table, m0, m1, (float)dt, n, (DS*)x, (DS*)y, status,
                                                        (DS*)rec_x, (DS*)rec_y, rec_st, err);
   else
-    k_adj_forward<float><<<grid_for(n, 256), 256, 0, st>>>(f, table, m0, m1, (float)dt, n, (float*)x, (float*)y, status,
+    k_adj_forward<float><<<blocks, threads, 0, st>>>(f, table, m0, m1, (float)dt, n, (float*)x, (float*)y, status,
                                                            (float*)rec_x, (float*)rec_y, rec_st, err);
 }
 
-void launch_adj_step(const FieldView& f, int prec, const AdjStep& s, double dt, uint32_t n, const void* x,
-                     const void* y, const uint8_t* status, void* lx, void* ly, float4* rec, uint32_t* key, uint32_t sent,
-                     uint32_t* mkey, uint32_t* mcode, uint32_t msent, uint32_t* err, cudaStream_t st) {
-  if (!n) return;
+void launch_adj_step(const FieldView& f, int prec, const AdjStep* table, int m_last, double dt, const AdjBatch& b,
+                     const void* x, const void* y, const uint8_t* status, void* lx, void* ly, cudaStream_t st) {
+  if (!b.n) return;
+  const unsigned threads = adj_threads(b.n), blocks = grid_for(b.n, threads);
   if (prec == ADJ_F64)
-    k_adj_step<double><<<grid_for(n, 256), 256, 0, st>>>(f, s, dt, n, (const double*)x, (const double*)y, status,
-                                                         (double*)lx, (double*)ly, rec, key, sent, mkey, mcode, msent,
-                                                         err);
+    k_adj_step<double><<<blocks, threads, 0, st>>>(f, table, m_last, dt, b, (const double*)x, (const double*)y, status,
+                                                   (double*)lx, (double*)ly);
   else if (prec == ADJ_DS)
-    k_adj_step_ds<<<grid_for(n, 256), 256, 0, st>>>(f, s, (float)dt, n, (const DS*)x, (const DS*)y, status,
-                                                    (float*)lx, (float*)ly, rec, key, sent, mkey, mcode, msent, err);
+    k_adj_step_ds<<<blocks, threads, 0, st>>>(f, table, m_last, (float)dt, b, (const DS*)x, (const DS*)y, status,
+                                              (float*)lx, (float*)ly);
   else
-    k_adj_step<float><<<grid_for(n, 256), 256, 0, st>>>(f, s, (float)dt, n, (const float*)x, (const float*)y, status,
-                                                        (float*)lx, (float*)ly, rec, key, sent, mkey, mcode, msent,
-                                                        err);
+    k_adj_step<float><<<blocks, threads, 0, st>>>(f, table, m_last, (float)dt, b, (const float*)x, (const float*)y,
+                                                  status, (float*)lx, (float*)ly);
 }
 
-void launch_adj_cells(const uint32_t* skey, const uint32_t* sval, uint32_t m, uint32_t cw, uint32_t ch,
-                      const uint32_t* mcode, uint32_t* scode, uint32_t* cst, uint32_t* cen, uint32_t* mark,
-                      uint32_t stamp, uint32_t* tlist, uint32_t* tcnt, cudaStream_t st) {
-  if (m) k_adj_cells<<<grid_for(m, 256), 256, 0, st>>>(skey, sval, m, cw, ch, mcode, scode, cst, cen, mark, stamp,
-                                                       tlist, tcnt);
-}
-
-void launch_adj_gather(uint32_t cw, uint32_t ch, const uint32_t* tcnt, const uint32_t* tlist, const uint32_t* cst,
-                       const uint32_t* cen, const uint32_t* scode, const uint32_t* sval, const float4* rec,
-                       float* csum, int sms, cudaStream_t st) {
-  const size_t ncells = (size_t)cw * ch;
-  unsigned blocks = grid_for(ncells * 32, 256);
-  const unsigned cap = (unsigned)(sms > 0 ? sms : 152) * 8u;
-  if (blocks > cap) blocks = cap;
-  if (ncells) k_adj_gather<<<blocks, 256, 0, st>>>(cw, ch, tcnt, tlist, cst, cen, scode, sval, rec, csum);
+void launch_adj_reduce(int nx, int ny, const AdjStep* table, int m_last, const AdjBatch& b, float* gu, float* gv,
+                       int sms, cudaStream_t st) {
+  if (!b.n) return;
+  const unsigned steps = (unsigned)b.steps;
+  const uint32_t items = (uint32_t)adj_items(b.n, b.cells);
+  launch_dep(k_adj_alloc, dim3(grid_for(b.cells, ALLOC_THREADS), steps), dim3(ALLOC_THREADS), st, b, items);
+  launch_dep(k_adj_scatter, dim3(grid_for(b.n, 256), steps), dim3(256), st, b);
+  // two warps per item, at most eight blocks an SM over all steps
+  const unsigned cap = std::max(1u, (unsigned)(sms > 0 ? sms : 152) * 8u / steps);
+  launch_dep(k_adj_gather, dim3(std::min(grid_for((size_t)items * 64, 256), cap), steps), dim3(256), st, b, items);
+  launch_dep(k_adj_nodes, dim3(grid_for((size_t)nx * ny, 32)), dim3(32, std::min(b.steps, NODE_STEPS)), st, nx, ny, table, m_last, b, gu, gv);
 }
 
 void launch_adj_signature(const FieldView& f, int prec, const AdjStep* table, int n_steps, double dt, uint32_t n,
@@ -1159,56 +1098,6 @@ void launch_adj_signature(const FieldView& f, int prec, const AdjStep* table, in
   else
     k_adj_signature<float><<<grid_for(n, 256), 256, 0, st>>>(f, table, n_steps, (float)dt, n, (const float*)x,
                                                              (const float*)y, status, sig);
-}
-
-void launch_scan(const uint32_t* in, uint32_t* out, size_t n, uint32_t* bsum, cudaStream_t st) {
-  if (!n) return;
-  const size_t chunk = (n + SCAN_BLOCKS - 1) / SCAN_BLOCKS;
-  const unsigned nb = grid_for(n, chunk);
-  k_scan_sums<<<nb, 256, 0, st>>>(in, n, chunk, bsum);
-  k_scan_chunks<<<nb, 256, 0, st>>>(in, out, n, chunk, bsum);
-}
-
-size_t adj_sort_hist_len(uint32_t m) { return (size_t)RS_RADIX_MAX * grid_for(m, RS_TILE); }
-
-void adj_sort(const AdjSortBufs& sb, uint32_t m, int key_bits, cudaStream_t st, const uint32_t** skey,
-              const uint32_t** sval) {
-  const uint32_t tiles = grid_for(m, RS_TILE);
-  const int passes = key_bits <= RS_BITS_MAX ? 1 : (key_bits + RS_BITS_MAX - 1) / RS_BITS_MAX;
-  const int width = (key_bits + passes - 1) / passes;
-  const uint32_t* kin = sb.key;
-  const uint32_t* vin = nullptr;
-  for (int p = 0; p < passes; ++p) {
-    uint32_t* kout = (p & 1) ? sb.k2 : sb.k1;
-    uint32_t* vout = (p & 1) ? sb.v2 : sb.v1;
-    const int shift = p * width;
-    const int bits = key_bits - shift < width ? key_bits - shift : width;
-    k_rs_hist<<<tiles, RS_THREADS, 0, st>>>(kin, m, shift, bits, sb.hist, tiles);
-    launch_scan(sb.hist, sb.hscan, ((size_t)1 << bits) * tiles, sb.bsum, st);
-    k_rs_scatter<<<tiles, RS_THREADS, 0, st>>>(kin, vin, kout, vout, m, shift, bits, sb.hscan, tiles);
-    kin = kout;
-    vin = vout;
-  }
-  *skey = kin;
-  *sval = vin;
-}
-
-void launch_adj_bounds(const uint32_t* skey, uint32_t m, uint32_t sent, uint32_t* cst, uint32_t* cen,
-                       cudaStream_t st) {
-  if (m) k_adj_bounds<<<grid_for(m, 256), 256, 0, st>>>(skey, m, sent, cst, cen);
-}
-
-void launch_adj_reduce(uint32_t ncells, uint32_t* cst, uint32_t* cen, const uint32_t* sval, const float4* rec,
-                       float* csum, int sms, cudaStream_t st) {
-  unsigned blocks = grid_for((size_t)ncells * 32, 256);
-  const unsigned cap = (unsigned)(sms > 0 ? sms : 152) * 16u;
-  if (blocks > cap) blocks = cap;
-  if (ncells) k_adj_reduce<<<blocks, 256, 0, st>>>(ncells, cst, cen, sval, rec, csum);
-}
-
-void launch_adj_nodes(int nx, int ny, const AdjStep& s, const float* csum, const uint32_t* mark, uint32_t stamp,
-                      float* gu, float* gv, cudaStream_t st) {
-  k_adj_nodes<<<grid_for((size_t)nx * ny, 256), 256, 0, st>>>(nx, ny, s, csum, mark, stamp, gu, gv);
 }
 
 }  // namespace lm

@@ -759,7 +759,7 @@ int dh_run(lm_ctx* c, const float* lat, const float* lon, const int8_t* species,
   int seg_bits = 0;
   while (seg_bits < 31 && (n_seg >> seg_bits) != 0) ++seg_bits;
   const int mb = std::min(DH_CURVE_BITS, 32 - seg_bits) & ~1;
-  const size_t hl = adj_sort_hist_len(n);
+  const size_t hl = radix_sort_hist_len(n);
   const size_t out_n = nb * n_seg;
   DhArena ar;
   float *dlat = nullptr, *dlon = nullptr;
@@ -824,7 +824,7 @@ int dh_run(lm_ctx* c, const float* lat, const float* lon, const int8_t* species,
   if (species) k_dh_species_segs<<<1, 1, 0, st>>>(dctl, dseg);
   k_dh_key<<<blocks_n, 256, 0, st>>>(dlat, dlon, sp, n, dseg, n_seg, mb, dctl, key);
   const uint32_t *skey, *sval;
-  adj_sort(AdjSortBufs{key, k1, k2, v1, v2, hist, hscan, bsum}, n, std::max(1, mb + seg_bits), st, &skey, &sval);
+  radix_sort(SortBufs{key, k1, k2, v1, v2, hist, hscan, bsum}, n, std::max(1, mb + seg_bits), st, &skey, &sval);
   k_dh_gather<<<(unsigned)n_tiles, DH_TILE, 0, st>>>(dlat, dlon, sval, dseg, n_seg, pts, vec, tiles);
   const size_t smem = (size_t)DH_WARPS * nb * DH_COPIES * sizeof(uint32_t) + (size_t)bins * sizeof(float2);
   int per_sm = 0;

@@ -8,11 +8,8 @@
 //   ck_*    T, T, uint8 [ceil(S/K)][n]     state at steps 0, K, 2K, ... (T = float or double)
 //   seg_*   T, T, uint8 [K][n]             state before every step of the segment being reversed
 //   lx, ly  T [n]                          the adjoint dL/dx_m
-//   rec     float4 [4n], key/k1/k2/v1/v2 uint32 [4n]  stage records and the radix-sort ping-pong
-//   mkey, mcode, scode  uint32 [n]         gather form: key 2 * (cell where the step starts) + (a stage
-//                                          leaves it), slots of the stages around it (sorted: scode)
-//   mark [C + 1], tlist [C], tcnt [S]      gather form: target cells listed per step (stamped in mark)
-//   cst/cen uint32 [4C + 1], csum float [C][3][8]     segment bounds, per-cell corner sums
+//   rec, cell, count, place, list, ent, csum, total   the backward steps whose records are reduced
+//                                          together (AdjBatch), B at a time
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -55,12 +52,21 @@ struct lm_adjoint {
   std::vector<AdjStep> table_h;
   // positions of adj_state_bytes(prec) per element; adjoint state lx, ly of adj_lambda_bytes(prec)
   DBuf<unsigned char> x, y, ck_x, ck_y, seg_x, seg_y, lx, ly, fin_x, fin_y;
-  DBuf<float> csum;
+  int batch = 1;     // backward steps reduced together
+  int seg_held = -1;  // segment whose states seg_* hold
+  DBuf<long long> csum;
   DBuf<uint8_t> st, ck_st, seg_st;
   DBuf<float4> rec;
-  DBuf<uint32_t> key, k1, k2, v1, v2, hist, hscan, bsum, cst, cen, mkey, mcode, scode, mark, tlist, tcnt;
+  DBuf<uint4> cell;
+  DBuf<uint2> ent;
+  DBuf<uint4> list;
+  DBuf<uint32_t> count, place;  // count: [B][cells], top [B][cells] and the totals [B][2], zeroed together
   uint32_t* err_d = nullptr;
   uint32_t* err_h = nullptr;
+  // the reduction of a batch runs on a stream of its own beside the next batch's steps: two sets of
+  // batch buffers, `stepped` (records written) and `reduced` (records read) per set
+  cudaStream_t red_st = nullptr;
+  cudaEvent_t stepped[2] = {}, reduced[2] = {};
 };
 
 namespace {
@@ -84,7 +90,7 @@ int afail(lm_adjoint* a, int code, const char* fmt, ...) {
   } while (0)
 
 template <class T>
-int grow(lm_adjoint* a, DBuf<T>& b, size_t need, bool zero = false) {
+int grow(lm_adjoint* a, DBuf<T>& b, size_t need) {
   if (need == 0) need = 1;
   if (b.p && b.cap >= need) return LM_OK;
   if (b.p) cudaFree(b.p);
@@ -97,7 +103,6 @@ int grow(lm_adjoint* a, DBuf<T>& b, size_t need, bool zero = false) {
     return afail(a, LM_ERR_OOM, "cudaMalloc of %zu bytes failed: %s", need * sizeof(T), cudaGetErrorString(e));
   }
   b.cap = need;
-  if (zero) ACK(cudaMemset(b.p, 0, need * sizeof(T)));
   return LM_OK;
 }
 
@@ -118,9 +123,31 @@ bool on_device(const void* p) {
   return at.type == cudaMemoryTypeDevice || at.type == cudaMemoryTypeManaged;
 }
 
-int key_bits_for(uint32_t sent) {
-  int b = 1;
-  while (b < 32 && (sent >> b) != 0) ++b;
+// Backward steps reduced together: as many as keep the records and entries of a batch in L2 (96 of its
+// 129 MB) and both sets of per-cell arrays below 1 GB, at most 16 and a checkpoint interval. The
+// launches of a batch cost about 25 us however little they do: at 100k microbes eight steps share them,
+// at 1M the records of one step fill L2.
+int batch_steps(uint32_t n, uint64_t cells, int K) {
+  const double fit = std::min(96e6 / (110.0 * n + 1.0), 1e9 / (2.0 * 220.0 * cells));
+  return std::max(1, std::min({16, K, (int)std::min(fit, 16.0)}));
+}
+
+// Set `set` of the batch buffers, for `steps` steps.
+AdjBatch batch_buffers(const lm_adjoint* a, uint32_t cells, int set, int steps) {
+  const size_t k = (size_t)set * a->batch;  // steps before this set
+  AdjBatch b{};
+  b.n = a->n;
+  b.cells = cells;
+  b.steps = steps;
+  b.rec = a->rec.p + 4 * k * a->n;
+  b.cell = a->cell.p + k * a->n;
+  b.count = a->count.p + k * (2 * (size_t)cells + 2);
+  b.top = b.count + (size_t)steps * cells;
+  b.total = b.top + (size_t)steps * cells;
+  b.place = a->place.p + k * cells;
+  b.list = a->list.p + k * adj_items(a->n, cells);
+  b.ent = a->ent.p + 4 * k * a->n;
+  b.csum = a->csum.p + k * cells * 24;
   return b;
 }
 
@@ -144,7 +171,12 @@ int lm_adjoint_create(lm_ctx* ctx, lm_adjoint** out) {
   a->sms = ctx_sms(ctx);
   cudaError_t e;
   if ((e = cudaSetDevice(a->device)) != cudaSuccess || (e = cudaMalloc((void**)&a->err_d, sizeof(uint32_t))) != cudaSuccess ||
-      (e = cudaMallocHost((void**)&a->err_h, sizeof(uint32_t))) != cudaSuccess) {
+      (e = cudaMallocHost((void**)&a->err_h, sizeof(uint32_t))) != cudaSuccess ||
+      (e = cudaStreamCreateWithFlags(&a->red_st, cudaStreamNonBlocking)) != cudaSuccess ||
+      (e = cudaEventCreateWithFlags(&a->stepped[0], cudaEventDisableTiming)) != cudaSuccess ||
+      (e = cudaEventCreateWithFlags(&a->stepped[1], cudaEventDisableTiming)) != cudaSuccess ||
+      (e = cudaEventCreateWithFlags(&a->reduced[0], cudaEventDisableTiming)) != cudaSuccess ||
+      (e = cudaEventCreateWithFlags(&a->reduced[1], cudaEventDisableTiming)) != cudaSuccess) {
     const int r = afail(a, LM_ERR_CUDA, "adjoint tape: %s", cudaGetErrorString(e));
     lm_adjoint_destroy(a);
     return r;
@@ -157,12 +189,19 @@ int lm_adjoint_destroy(lm_adjoint* a) {
   if (!a) return LM_OK;
   cudaSetDevice(a->device);
   if (a->ctx) cudaStreamSynchronize(ctx_stream(a->ctx));
+  if (a->red_st) {
+    cudaStreamSynchronize(a->red_st);
+    cudaStreamDestroy(a->red_st);
+  }
+  for (int k = 0; k < 2; ++k) {
+    if (a->stepped[k]) cudaEventDestroy(a->stepped[k]);
+    if (a->reduced[k]) cudaEventDestroy(a->reduced[k]);
+  }
   release(a->uv);
   release(a->table);
   release(a->x), release(a->y), release(a->ck_x), release(a->ck_y), release(a->seg_x), release(a->seg_y);
   release(a->lx), release(a->ly), release(a->fin_x), release(a->fin_y), release(a->csum), release(a->st), release(a->ck_st), release(a->seg_st);
-  release(a->rec), release(a->key), release(a->k1), release(a->k2), release(a->v1), release(a->v2);
-  release(a->hist), release(a->hscan), release(a->bsum), release(a->cst), release(a->cen), release(a->mkey);
+  release(a->rec), release(a->cell), release(a->ent), release(a->count), release(a->place), release(a->list);
   if (a->err_d) cudaFree(a->err_d);
   if (a->err_h) cudaFreeHost(a->err_h);
   delete a;
@@ -183,6 +222,7 @@ int lm_adjoint_forward(lm_adjoint* a, const float* u, const float* v, int nt, in
                        float* lat_out) {
   if (!a) return LM_ERR_ARG;
   a->done = false;
+  a->seg_held = -1;
   if (!lon || !lat || !t_sec) return afail(a, LM_ERR_ARG, "NULL axis");
   if (nt < 2 || ny < 2 || nx < 2) return afail(a, LM_ERR_ARG, "field needs nt, ny, nx >= 2 (got %d, %d, %d)", nt, ny, nx);
   if (n < 0 || 4 * n >= (int64_t)0xffffffffu) return afail(a, LM_ERR_ARG, "n = %lld out of range", (long long)n);
@@ -209,7 +249,7 @@ int lm_adjoint_forward(lm_adjoint* a, const float* u, const float* v, int nt, in
   const size_t fe = (size_t)nt * ny * nx;
   const uint32_t N = (uint32_t)n;
   const int n_ck = (n_steps + checkpoint_every - 1) / checkpoint_every;
-  const size_t M = (size_t)4 * N;
+  const int B = batch_steps(N, cells, std::min(checkpoint_every, n_steps));
   const int prec = a->prec_next;
   const size_t es = adj_state_bytes(prec);  // lx, ly need no more (adj_lambda_bytes)
   int r;
@@ -219,13 +259,10 @@ int lm_adjoint_forward(lm_adjoint* a, const float* u, const float* v, int nt, in
       (r = grow(a, a->seg_x, es * checkpoint_every * N)) || (r = grow(a, a->seg_y, es * checkpoint_every * N)) ||
       (r = grow(a, a->seg_st, (size_t)checkpoint_every * N)) || (r = grow(a, a->lx, es * N)) ||
       (r = grow(a, a->ly, es * N)) || (r = grow(a, a->fin_x, es * N)) || (r = grow(a, a->fin_y, es * N)) ||
-      (r = grow(a, a->rec, M)) || (r = grow(a, a->key, M)) || (r = grow(a, a->mkey, N)) ||
-      (r = grow(a, a->mcode, N)) || (r = grow(a, a->scode, N)) || (r = grow(a, a->mark, cells + 1)) ||
-      (r = grow(a, a->tlist, cells)) || (r = grow(a, a->tcnt, (size_t)n_steps)) ||
-      (r = grow(a, a->k1, M)) || (r = grow(a, a->k2, M)) || (r = grow(a, a->v1, M)) || (r = grow(a, a->v2, M)) ||
-      (r = grow(a, a->hist, adj_sort_hist_len((uint32_t)M))) || (r = grow(a, a->hscan, adj_sort_hist_len((uint32_t)M))) ||
-      (r = grow(a, a->bsum, SCAN_BLOCKS)) || (r = grow(a, a->cst, 4 * cells + 1, true)) ||
-      (r = grow(a, a->cen, 4 * cells + 1, true)) || (r = grow(a, a->csum, cells * 24)))
+      (r = grow(a, a->rec, 2 * (size_t)4 * B * N)) || (r = grow(a, a->cell, 2 * (size_t)B * N)) ||
+      (r = grow(a, a->ent, 2 * (size_t)4 * B * N)) || (r = grow(a, a->count, 2 * B * (2 * cells + 2))) ||
+      (r = grow(a, a->place, 2 * B * cells)) || (r = grow(a, a->list, 2 * B * adj_items(N, cells))) ||
+      (r = grow(a, a->csum, 2 * B * cells * 24)))
     return r;
   launch_interleave(u, v, a->uv.p, fe, st);
   fill_field_view(a->fv, a->uv.p, nt, ny, nx, lon, lat, t_sec, dx, dy, dT);
@@ -236,6 +273,7 @@ int lm_adjoint_forward(lm_adjoint* a, const float* u, const float* v, int nt, in
   a->n_steps = n_steps;
   a->K = checkpoint_every;
   a->n_ck = n_ck;
+  a->batch = B;
   a->prec = prec;
   a->dt = dt_sec;
   ACK(cudaMemsetAsync(a->err_d, 0, sizeof(uint32_t), st));
@@ -253,8 +291,12 @@ int lm_adjoint_forward(lm_adjoint* a, const float* u, const float* v, int nt, in
       ACK(cudaMemcpyAsync(a->ck_y.p + es * s * N, a->y.p, es * N, cudaMemcpyDeviceToDevice, st));
       ACK(cudaMemcpyAsync(a->ck_st.p + (size_t)s * N, a->st.p, N, cudaMemcpyDeviceToDevice, st));
     }
-    launch_adj_forward(a->fv, prec, a->table.p, m0, m1, a->dt, N, a->x.p, a->y.p, a->st.p, nullptr, nullptr, nullptr,
+    // the last segment is the first to be reversed: its states are stored as they are computed
+    const bool keep = s == n_ck - 1;
+    launch_adj_forward(a->fv, prec, a->table.p, m0, m1, a->dt, N, a->x.p, a->y.p, a->st.p,
+                       keep ? a->seg_x.p : nullptr, keep ? a->seg_y.p : nullptr, keep ? a->seg_st.p : nullptr,
                        a->err_d, st);
+    if (keep) a->seg_held = s;
   }
   launch_adj_final(a->fv, prec, N, a->x.p, a->y.p, lon_out, lat_out, st);
   if (N) {
@@ -282,66 +324,43 @@ int lm_adjoint_backward(lm_adjoint* a, const float* g_lon, const float* g_lat, f
   cudaStream_t st = ctx_stream(a->ctx);
   const size_t fe = (size_t)a->nt * a->ny * a->nx;
   const uint32_t cells = (uint32_t)(a->nx - 1) * (uint32_t)(a->ny - 1);
-  const uint32_t sent = 4u * cells;
-  const int kb = key_bits_for(sent);
-  const uint32_t M = 4u * N;
   const size_t es = adj_state_bytes(a->prec);
-  const uint32_t cw = (uint32_t)(a->nx - 1), ch = (uint32_t)(a->ny - 1);
-  const int kbm = key_bits_for(2u * cells);
-  int r;
-  // Gather form first (microbes sorted by the cell where each step starts, records gathered from
-  // the 3 x 3 cells around every cell); if a stage left that neighbourhood anywhere, the whole
-  // sweep is redone with the records themselves sorted by cell.
-  for (int form = 0; form < 2; ++form) {
-    const bool gather = form == 0;
-    ACK(cudaMemsetAsync(g_u, 0, fe * sizeof(float), st));
-    ACK(cudaMemsetAsync(g_v, 0, fe * sizeof(float), st));
-    ACK(cudaMemsetAsync(a->err_d, 0, sizeof(uint32_t), st));
-    if (gather) {  // target lists start empty, stamps at 0 (step m stamps m + 1)
-      ACK(cudaMemsetAsync(a->mark.p, 0, sizeof(uint32_t) * (cells + 1), st));
-      ACK(cudaMemsetAsync(a->tcnt.p, 0, sizeof(uint32_t) * a->n_steps, st));
-    } else {  // the record form needs every segment bound at zero
-      ACK(cudaMemsetAsync(a->cst.p, 0, sizeof(uint32_t) * (4 * (size_t)cells + 1), st));
-      ACK(cudaMemsetAsync(a->cen.p, 0, sizeof(uint32_t) * (4 * (size_t)cells + 1), st));
-    }
-    if (N) launch_adj_seed(a->prec, N, g_lon, g_lat, a->lx.p, a->ly.p, st);
-    const AdjSortBufs sb{gather ? a->mkey.p : a->key.p, a->k1.p, a->k2.p, a->v1.p, a->v2.p,
-                         a->hist.p, a->hscan.p, a->bsum.p};
-    for (int s = a->n_ck - 1; s >= 0 && N; --s) {
-      const int m0 = s * a->K, m1 = std::min(m0 + a->K, a->n_steps);
+  ACK(cudaMemsetAsync(g_u, 0, fe * sizeof(float), st));
+  ACK(cudaMemsetAsync(g_v, 0, fe * sizeof(float), st));
+  ACK(cudaMemsetAsync(a->err_d, 0, sizeof(uint32_t), st));
+  if (N) launch_adj_seed(a->prec, N, g_lon, g_lat, a->lx.p, a->ly.p, st);
+  // the gradient's zeros are written on st before the first `stepped`, so before any reduction adds to it
+  int set = 0;
+  bool fresh[2] = {true, true};
+  for (int s = a->n_ck - 1; s >= 0 && N; --s) {
+    const int m0 = s * a->K, m1 = std::min(m0 + a->K, a->n_steps);
+    if (a->seg_held != s) {
       ACK(cudaMemcpyAsync(a->x.p, a->ck_x.p + es * s * N, es * N, cudaMemcpyDeviceToDevice, st));
       ACK(cudaMemcpyAsync(a->y.p, a->ck_y.p + es * s * N, es * N, cudaMemcpyDeviceToDevice, st));
       ACK(cudaMemcpyAsync(a->st.p, a->ck_st.p + (size_t)s * N, N, cudaMemcpyDeviceToDevice, st));
-      launch_adj_forward(a->fv, a->prec, a->table.p, m0, m1, a->dt, N, a->x.p, a->y.p, a->st.p, a->seg_x.p,
-                         a->seg_y.p, a->seg_st.p, a->err_d, st);
-      for (int m = m1 - 1; m >= m0; --m) {
-        const size_t o = (size_t)(m - m0) * N;
-        const AdjStep& sg = a->table_h[m];
-        launch_adj_step(a->fv, a->prec, sg, a->dt, N, a->seg_x.p + es * o, a->seg_y.p + es * o, a->seg_st.p + o,
-                        a->lx.p, a->ly.p, a->rec.p, a->key.p, sent, gather ? a->mkey.p : nullptr, a->mcode.p,
-                        2u * cells, a->err_d, st);
-        const uint32_t *skey, *sval;
-        const uint32_t stamp = (uint32_t)m + 1u;
-        if (gather) {
-          ACK(cudaMemsetAsync(a->cen.p, 0, sizeof(uint32_t) * 2 * cells, st));
-          adj_sort(sb, N, kbm, st, &skey, &sval);
-          launch_adj_cells(skey, sval, N, cw, ch, a->mcode.p, a->scode.p, a->cst.p, a->cen.p, a->mark.p, stamp,
-                           a->tlist.p, a->tcnt.p + m, st);
-          launch_adj_gather(cw, ch, a->tcnt.p + m, a->tlist.p, a->cst.p, a->cen.p, a->scode.p, sval, a->rec.p,
-                            a->csum.p, a->sms, st);
-        } else {
-          adj_sort(sb, M, kb, st, &skey, &sval);
-          launch_adj_bounds(skey, M, sent, a->cst.p, a->cen.p, st);
-          launch_adj_reduce(cells, a->cst.p, a->cen.p, sval, a->rec.p, a->csum.p, a->sms, st);
-        }
-        launch_adj_nodes(a->nx, a->ny, sg, a->csum.p, gather ? a->mark.p : nullptr, stamp, g_u, g_v, st);
-      }
+      launch_adj_forward(a->fv, a->prec, a->table.p, m0, m1, a->dt, N, a->x.p, a->y.p, a->st.p, a->seg_x.p, a->seg_y.p,
+                         a->seg_st.p, a->err_d, st);
+      a->seg_held = s;
     }
-    ACK(cudaGetLastError());
-    uint32_t err = 0;
-    if ((r = read_err(a, st, &err))) return r;
-    if (!(gather && (err & ADJ_WIDE))) break;
+    for (int m = m1 - 1; m >= m0; m -= a->batch) {
+      const AdjBatch b = batch_buffers(a, cells, set, std::min(a->batch, m - m0 + 1));
+      if (!fresh[set]) ACK(cudaStreamWaitEvent(st, a->reduced[set], 0));  // its last reduction is done
+      fresh[set] = false;
+      ACK(cudaMemsetAsync(b.count, 0, (size_t)b.steps * (2 * (size_t)cells + 2) * sizeof(uint32_t), st));
+      const size_t o = (size_t)(m - m0) * N;
+      launch_adj_step(a->fv, a->prec, a->table.p, m, a->dt, b, a->seg_x.p + es * o, a->seg_y.p + es * o,
+                      a->seg_st.p + o, a->lx.p, a->ly.p, st);
+      ACK(cudaEventRecord(a->stepped[set], st));
+      ACK(cudaStreamWaitEvent(a->red_st, a->stepped[set], 0));
+      launch_adj_reduce(a->nx, a->ny, a->table.p, m, b, g_u, g_v, a->sms, a->red_st);
+      ACK(cudaEventRecord(a->reduced[set], a->red_st));
+      set ^= 1;
+    }
   }
+  // what the caller's stream does next comes after the last reductions
+  for (int k = 0; k < 2; ++k)
+    if (!fresh[k]) ACK(cudaStreamWaitEvent(st, a->reduced[k], 0));
+  ACK(cudaGetLastError());
   if (N) launch_adj_unseed(a->prec, N, a->lx.p, a->ly.p, g_lon0, g_lat0, st);
   ACK(cudaGetLastError());
   ACK(cudaStreamSynchronize(st));

@@ -1597,5 +1597,13 @@ void fill_field_view(FieldView& f, float2* uv, int nt, int ny, int nx, const dou
   f.gy0d = lat[0] - org_lat;
   f.inv_dxd = 1.0 / dx;
   f.inv_dyd = 1.0 / dy;
+  auto two = [](double d) {
+    const float h = (float)d;
+    return make_float2(h, (float)(d - (double)h));
+  };
+  f.ds_mgx0 = two(-f.gx0d);
+  f.ds_mgy0 = two(-f.gy0d);
+  f.ds_inv_dx = two(f.inv_dxd);
+  f.ds_inv_dy = two(f.inv_dyd);
 }
 }  // namespace lm

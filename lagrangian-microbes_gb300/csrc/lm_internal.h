@@ -169,6 +169,8 @@ struct FieldView {
   double t0, dT;      // frame 0 time and frame spacing (seconds)
   // the same geometry in float64 (the adjoint's FP64-trajectory mode)
   double gx0d, gy0d, inv_dxd, inv_dyd;
+  // and as unevaluated float32 sums hi + lo (its double-float mode): -gx0, -gy0, 1/dx, 1/dy
+  float2 ds_mgx0, ds_mgy0, ds_inv_dx, ds_inv_dy;
 };
 
 struct PairParams {
@@ -322,9 +324,6 @@ void launch_sweep_long(const Bufs& b, const PairParams& pp, const StepArgs& a, C
 void launch_pair_counts(const Bufs& b, uint32_t n_valid, uint32_t n_long, uint32_t* cnt, int sms, cudaStream_t st);
 void launch_pair_rows(const Bufs& b, uint32_t n_valid, uint32_t n_long, const uint32_t* off, int32_t* pi, int32_t* pj,
                       int sms, cudaStream_t st);
-// Exclusive scan of n values (bsum: SCAN_BLOCKS words of working memory).
-void launch_scan(const uint32_t* in, uint32_t* out, size_t n, uint32_t* bsum, cudaStream_t st);
-
 // K4/K5 interaction dataflow (cooperative persistent kernel).
 // Grid of the cooperative launch with `threads` (512 or 1,024) per block; *block receives the block size.
 int rounds_grid(int device, int threads, int* block);
@@ -333,6 +332,24 @@ void launch_census(const Bufs& b, Ctrl* ctrl, cudaStream_t st);
 const void* lm_census_kernel();  // one kernel of the library, for attribute queries
 void launch_unpad(const float* src, float* dst, const int32_t* map, uint32_t nslots, cudaStream_t st);
 void launch_unpad8(const int8_t* src, int8_t* dst, const int32_t* map, uint32_t nslots, cudaStream_t st);
+
+// ---- stable radix sort (k_sort.cu) ----
+constexpr int RS_BITS_MAX = 10;                      // digit width of one pass
+constexpr uint32_t RS_RADIX_MAX = 1u << RS_BITS_MAX;
+
+struct SortBufs {
+  const uint32_t* key;      // input keys (m)
+  uint32_t *k1, *k2;        // ping-pong keys (m)
+  uint32_t *v1, *v2;        // ping-pong input indices (m)
+  uint32_t *hist, *hscan;   // radix_sort_hist_len(m)
+  uint32_t* bsum;           // SCAN_BLOCKS
+};
+size_t radix_sort_hist_len(uint32_t m);
+// Stable sort of m keys of key_bits bits; returns the sorted keys and their input indices.
+void radix_sort(const SortBufs& sb, uint32_t m, int key_bits, cudaStream_t st, const uint32_t** skey,
+                const uint32_t** sval);
+// Exclusive scan of n values (bsum: SCAN_BLOCKS words of working memory).
+void launch_scan(const uint32_t* in, uint32_t* out, size_t n, uint32_t* bsum, cudaStream_t st);
 
 // ---- K6/K7 adjoint of the advection (k_adjoint.cu) ----
 // Stage brackets of one step: frames k[g] and weights w[g] of the stage times t, t + dt/2, t + dt.
@@ -347,16 +364,28 @@ enum AdjPrecision { ADJ_F32 = 0, ADJ_F64 = 1, ADJ_DS = 2 };
 // Bytes of one position coordinate / one adjoint coordinate in each precision.
 inline size_t adj_state_bytes(int prec) { return prec == ADJ_F32 ? 4 : 8; }
 inline size_t adj_lambda_bytes(int prec) { return prec == ADJ_F64 ? 8 : 4; }
-constexpr int RS_BITS_MAX = 10;                      // digit width of one radix pass
-constexpr uint32_t RS_RADIX_MAX = 1u << RS_BITS_MAX;
-
-struct AdjSortBufs {
-  const uint32_t* key;      // input keys (m)
-  uint32_t *k1, *k2;        // ping-pong keys (m)
-  uint32_t *v1, *v2;        // ping-pong record ids (m)
-  uint32_t *hist, *hscan;   // adj_sort_hist_len(m)
-  uint32_t* bsum;           // SCAN_BLOCKS
+// Several consecutive backward steps whose records are reduced together: step q of the batch is step
+// m_last - q of the run.
+struct AdjBatch {
+  uint32_t n, cells;  // microbes, field cells
+  int steps;
+  float4* rec;      // [steps][n][4]   (a, b, dL/dU, dL/dV) of each stage
+  uint4* cell;      // [steps][n]      field cells of the four stages (NONE: the step was frozen)
+  uint32_t* count;  // [steps][cells]  entries of a cell (zero before the batch)
+  uint32_t* top;    // [steps][cells]  float bits of its largest |dL/dU|, |dL/dV| (zero before the batch)
+  uint32_t* total;  // [steps][2]      entries reserved, items listed (zero before the batch)
+  uint32_t* place;  // [steps][cells]  where a cell's entries go
+  uint4* list;      // [steps][adj_items] items: (cell, first entry, entries, entries of the cell)
+  uint2* ent;       // [steps][4 n]    (microbe, stage bits), a cell's entries together
+  long long* csum;  // [steps][cells][24] corner sums per stage time, scaled by the cell's `top`
 };
+// Entries of an item: what one warp adds up for a cell.
+constexpr uint32_t ADJ_ITEM = 128;
+// Items of a step at most: one per occupied cell and one per full item.
+inline size_t adj_items(uint32_t n, size_t cells) {
+  const size_t e = (size_t)4 * n;
+  return (cells < e ? cells : e) + e / ADJ_ITEM;
+}
 
 void launch_adj_stages(const FieldView& f, double t_start, double dt, int n_steps, AdjStep* table, uint32_t* err,
                        cudaStream_t st);
@@ -374,36 +403,14 @@ void launch_adj_unseed(int prec, uint32_t n, const void* lx, const void* ly, flo
 void launch_adj_forward(const FieldView& f, int prec, const AdjStep* table, int m0, int m1, double dt, uint32_t n,
                         void* x, void* y, uint8_t* status, void* rec_x, void* rec_y, uint8_t* rec_st, uint32_t* err,
                         cudaStream_t st);
-// mkey (or nullptr): gather form of the reduction. Per microbe, in mcode, 4 bits a stage: the slot
-// (dj + 1) * 3 + (di + 1) of the stage's cell around the cell b where the step starts, and in mkey
-// 2b + (1 when a stage leaves b), msent when frozen; a stage outside those 3 x 3 cells sets
-// ADJ_WIDE. Without mkey the step writes the four record keys (cell * 4 + stage time, or `sent`).
-constexpr uint32_t ADJ_WIDE = 1u << 8;
-void launch_adj_step(const FieldView& f, int prec, const AdjStep& s, double dt, uint32_t n, const void* x,
-                     const void* y, const uint8_t* status, void* lx, void* ly, float4* rec, uint32_t* key, uint32_t sent,
-                     uint32_t* mkey, uint32_t* mcode, uint32_t msent, uint32_t* err, cudaStream_t st);
-// After the sort of mkey: cell bounds, stage codes in sorted order, target cells listed once a step.
-void launch_adj_cells(const uint32_t* skey, const uint32_t* sval, uint32_t m, uint32_t cw, uint32_t ch,
-                      const uint32_t* mcode, uint32_t* scode, uint32_t* cst, uint32_t* cen, uint32_t* mark,
-                      uint32_t stamp, uint32_t* tlist, uint32_t* tcnt, cudaStream_t st);
-void launch_adj_gather(uint32_t cw, uint32_t ch, const uint32_t* tcnt, const uint32_t* tlist, const uint32_t* cst,
-                       const uint32_t* cen, const uint32_t* scode, const uint32_t* sval, const float4* rec,
-                       float* csum, int sms, cudaStream_t st);
+void launch_adj_step(const FieldView& f, int prec, const AdjStep* table, int m_last, double dt, const AdjBatch& b,
+                     const void* x, const void* y, const uint8_t* status, void* lx, void* ly, cudaStream_t st);
+// The records of a batch onto the gradient of the field.
+void launch_adj_reduce(int nx, int ny, const AdjStep* table, int m_last, const AdjBatch& b, float* gu, float* gv,
+                       int sms, cudaStream_t st);
 void launch_adj_signature(const FieldView& f, int prec, const AdjStep* table, int n_steps, double dt, uint32_t n,
                           const void* x, const void* y, const uint8_t* status, unsigned long long* sig,
                           cudaStream_t st);
-size_t adj_sort_hist_len(uint32_t m);
-// Stable sort of m keys of key_bits bits; returns the sorted keys and the record ids (input index).
-void adj_sort(const AdjSortBufs& sb, uint32_t m, int key_bits, cudaStream_t st, const uint32_t** skey,
-              const uint32_t** sval);
-void launch_adj_bounds(const uint32_t* skey, uint32_t m, uint32_t sent, uint32_t* cst, uint32_t* cen,
-                       cudaStream_t st);
-void launch_adj_reduce(uint32_t ncells, uint32_t* cst, uint32_t* cen, const uint32_t* sval, const float4* rec,
-                       float* csum, int sms, cudaStream_t st);
-// mark (or nullptr): only cells with mark[c] == stamp hold sums (the gather form's target list).
-void launch_adj_nodes(int nx, int ny, const AdjStep& s, const float* csum, const uint32_t* mark, uint32_t stamp,
-                      float* gu, float* gv, cudaStream_t st);
-
 // Field geometry from uniform axes (shared by lm_field_upload_batch and the adjoint tape).
 bool uniform_axis(const double* a, int n, double* d);
 void fill_field_view(FieldView& f, float2* uv, int nt, int ny, int nx, const double* lon, const double* lat,

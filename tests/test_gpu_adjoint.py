@@ -247,3 +247,75 @@ def test_adjoint_steps_longer_than_a_cell_fall_back_to_the_record_form(lm, orc):
     again = _gpu_grads(f, lon, lat, tlon, tlat, t0, dt, n_steps, 3)
     for a, b in zip(again[3], g):
         np.testing.assert_array_equal(a, b)
+
+
+def _tape_backward(f, lon, lat, g, n_steps, k, precision, dt=3600.0):
+    from lagrangian_microbes_gb300.adjoint import AdjointTape
+    dev = torch.device("cuda:0")
+    tape = AdjointTape(precision=precision)
+    tape.forward(torch.from_numpy(lon).to(dev), torch.from_numpy(lat).to(dev), torch.from_numpy(f.u).to(dev),
+                 torch.from_numpy(f.v).to(dev), f.lon, f.lat, f.times, float(f.times[0]), dt, n_steps, k)
+    out = [[t.cpu().numpy() for t in tape.backward(torch.from_numpy(g[0]).to(dev), torch.from_numpy(g[1]).to(dev))]
+           for _ in range(2)]
+    tape.close()
+    tape.ctx.close()
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
+    return out[0]
+
+
+@pytest.mark.parametrize("precision", ["f32", "ds", "f64"])
+@pytest.mark.parametrize("n", [1, 31, 127, 128, 129, 257, 5000])
+def test_adjoint_field_gradient_does_not_depend_on_the_order_of_the_microbes(small_field, n, precision):
+    """All microbes in one field cell (one item of its sums, several, a ragged last one) beside
+    scattered ones, adjoints over twelve decades: the field's gradient is bit-identical for shuffled
+    microbes (the sums are integers), and so are the microbes' own gradients."""
+    f = small_field
+    rng = np.random.default_rng(60 + n)
+    lon = np.concatenate([200.05 + 0.15 * rng.random(n), 199 + 3 * rng.random(300)]).astype(np.float32)
+    lat = np.concatenate([25.05 + 0.15 * rng.random(n), 24 + 3 * rng.random(300)]).astype(np.float32)
+    g = (rng.standard_normal((2, lon.size)) * 10.0 ** rng.uniform(-6, 6, lon.size)).astype(np.float32)
+    ref = _tape_backward(f, lon, lat, g, 7, 3, precision)
+    p = rng.permutation(lon.size)
+    got = _tape_backward(f, lon[p], lat[p], np.ascontiguousarray(g[:, p]), 7, 7, precision)
+    for a, b in zip(got[:2], ref[:2]):
+        np.testing.assert_array_equal(a, b[p])
+    for a, b in zip(got[2:], ref[2:]):
+        np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("n", [40, 400])
+def test_adjoint_dense_cells_match_fp64_autograd(lm, orc, small_field, n):
+    """n microbes per field cell of a 3 x 3 patch, against the FP64 autograd on the same cell paths
+    (float32 terms, so the bound of the scattered cases)."""
+    f = small_field
+    lon, lat, tlon, tlat = _case(f, 9 * n, 61, box=(200.0, 200.75, 25.0, 25.75))
+    t0, dt, n_steps = float(f.times[0]), 3600.0, 10
+    sig = _gpu_grads(f, lon, lat, tlon, tlat, t0, dt, n_steps, 4)[4]
+    same = sig == _fp64_signature(orc, f, lon, lat, t0, dt, n_steps)
+    assert same.mean() >= 0.97
+    g = _gpu_grads(f, lon, lat, tlon, tlat, t0, dt, n_steps, 4, weight=same)[3]
+    _, g64 = _fp64_grads(f, lon, lat, tlon, tlat, t0, dt, n_steps, weight=same)
+    errs = [_rel(a, b) for a, b in zip(g, g64)]
+    assert max(errs) < 1e-4, errs
+
+
+@pytest.mark.parametrize("bad", [np.inf, np.nan])
+def test_adjoint_non_finite_gradients_stay_in_their_cells(small_field, bad):
+    f = small_field
+    rng = np.random.default_rng(62)
+    lon = np.concatenate([200.05 + 0.15 * rng.random(300), [202.6]]).astype(np.float32)
+    lat = np.concatenate([25.05 + 0.15 * rng.random(300), [26.6]]).astype(np.float32)
+    g = rng.standard_normal((2, lon.size)).astype(np.float32)
+    clean = _tape_backward(f, lon[:-1], lat[:-1], np.ascontiguousarray(g[:, :-1]), 4, 4, "f32")
+    g[:, -1] = bad
+    got = _tape_backward(f, lon, lat, g, 4, 4, "f32")
+    assert not np.isfinite(got[0][-1]) and np.isfinite(got[0][:-1]).all()
+    for a, b in zip(got[2:], clean[2:]):
+        touched = ~np.isfinite(a)
+        assert touched.any() and not b[touched].any()  # the nodes around the one microbe alone
+        np.testing.assert_array_equal(a[~touched], b[~touched])
+    few = int((~np.isfinite(got[2])).sum())
+    g[:, 5] = bad  # and in a cell of several items
+    got = _tape_backward(f, lon, lat, g, 4, 4, "f32")
+    assert int((~np.isfinite(got[2])).sum()) > few
