@@ -221,6 +221,7 @@ __device__ __forceinline__ void step_begin_body(const Bufs& b, const FieldView& 
     ctrl->n_dir = 0;
     ctrl->n_long = 0;
     ctrl->ovf_used = 0;
+    ctrl->ev_taken = 0;
     ctrl->census[0] = ctrl->census[1] = ctrl->census[2] = ctrl->census[3] = 0;
     if (bracket) {  // float64 time arithmetic once per step, not once per advection block
       const uint32_t step = a.use_ctrl_step ? ctrl->step : a.step0;

@@ -750,7 +750,7 @@ __global__ void __launch_bounds__(LONG_WARPS * 32) k_sweep_long(Bufs b, PairPara
   bool too_many = false;
   for (uint32_t i = lane; i < count; i += 32) {
     const uint32_t d = b.deg[b.longv[gw + i * nw]];
-    sum += d;
+    sum += d + 1u;  // the list and its end mark
     too_many |= d > MAX_DEGREE;
   }
   for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
@@ -773,12 +773,13 @@ __global__ void __launch_bounds__(LONG_WARPS * 32) k_sweep_long(Bufs b, PairPara
     const bool mine = ib + lane < count;
     const uint32_t s_l = mine ? b.longv[gw + (ib + lane) * nw] : 0u;
     const uint32_t d_l = mine ? b.deg[s_l] : 0u;
-    unsigned long long incl = d_l;
+    const uint32_t room_l = mine ? d_l + 1u : 0u;
+    unsigned long long incl = room_l;
     for (int o = 1; o < 32; o <<= 1) {
       const unsigned long long y = __shfl_up_sync(0xffffffffu, incl, o);
       if (lane >= (uint32_t)o) incl += y;
     }
-    const unsigned long long o_l = run + incl - d_l;
+    const unsigned long long o_l = run + incl - room_l;
     run += __shfl_sync(0xffffffffu, incl, 31);
     uint32_t r0[6], r1[6], la_l = 0, base_l = 0, k0_l = 0, k1_l = 0, e_l = 0;
     int sp_l = 0;
@@ -912,6 +913,7 @@ __global__ void __launch_bounds__(LONG_WARPS * 32) k_sweep_long(Bufs b, PairPara
         first = b.ovf[o];
       }
       if (lane == 0) {
+        b.ovf[o + d] = NONE;
         b.slab[(size_t)s * SLAB] = (uint32_t)o;  // a long list's overflow offset, in its unused slab row
         b.wstate[s] = pack_state(first, 0u, sp);  // entry 0 of the list
       }

@@ -33,8 +33,8 @@
 // In pair-log runs each applied pair also gets a level = 1 + max(level of the previous pair at
 // either endpoint): pairs of one level share no microbe, and (level, i, j) is a deterministic
 // sequential order equal in effect to the priority order. The step's "rounds" is the max level.
-#include "lm_internal.h"
 #include "lm_philox.cuh"
+#include "lm_rounds.cuh"
 
 namespace lm {
 
@@ -47,27 +47,6 @@ namespace lm {
 // per SM) a block's range has a shorter edge for its area, so fewer pairs hand off through global
 // memory.
 constexpr int RD_THREADS_DEFAULT = 1024;
-constexpr unsigned long long ROUNDS_TIMEOUT_NS = 2000000000ull;  // 2 s
-
-__device__ __forceinline__ unsigned long long globaltimer() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-
-// Vertex state words are read and written with relaxed .gpu operations: each word is the only
-// shared state a pair needs, and a word changes only through the applier of its vertex's current
-// pair, so coherence of the single word is all the ordering required.
-__device__ __forceinline__ unsigned long long ld_relaxed(const unsigned long long* p) {
-  unsigned long long v;
-  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-  return v;
-}
-
-__device__ __forceinline__ void st_relaxed(unsigned long long* p, unsigned long long v) {
-  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
-
 __device__ __forceinline__ bool beats(int x, int y) {
   // rock(1) > scissors(3), paper(2) > rock(1), scissors(3) > paper(2)
   return (x == 1 && y == 3) || (x == 2 && y == 1) || (x == 3 && y == 2);
@@ -272,63 +251,18 @@ __device__ void tl_group(const Bufs& b, uint32_t step, Ctrl* ctrl, unsigned long
   }
 }
 
-// Groups of whole ensembles (consecutive in cell order) whose vertices fit the blocks' shared
-// memory, run one after another by every block. No barrier separates the groups: pairs never join
-// two ensembles, and a block that is still in group g while another has moved to g + 1 only
-// delays the handoffs of g + 1 that cross into it, whose words it loads from global memory when it
-// gets there (the same rule that covers blocks starting at different times).
-constexpr int TL_GROUPS_MAX = 64;
-
 // Returns false (nothing done) when the step does not fit the tile path (grid-uniform).
 template <int RD_THREADS>
 __device__ bool rounds_tiled(const Bufs& b, uint32_t step, Ctrl* ctrl, unsigned long long t0, uint32_t n_valid) {
   if (b.plog) return false;
-  const uint32_t cap = gridDim.x * TL_VMAX;
-  __shared__ uint32_t gb[TL_GROUPS_MAX + 1];
-  __shared__ int ng;
-  if (n_valid <= cap) {
-    if (threadIdx.x == 0) {
-      gb[0] = 0;
-      gb[1] = n_valid;
-      ng = 1;
-    }
-  } else {
-    // the k-th ensemble in key order, e = eord[k], holds the vertices from cstart[cell_base_e] to
-    // the next one's start; greedy groups of whole ensembles consecutive in that order, each at
-    // most `cap` vertices (none when one ensemble alone is larger)
-    extern __shared__ unsigned long long tl_raw[];
-    uint32_t* es = reinterpret_cast<uint32_t*>(tl_raw);
-    const uint32_t E = b.n_ens;
-    const bool fits = E + 1 <= (uint32_t)(TL_SMEM / sizeof(uint32_t));
-    if (fits) {
-      for (uint32_t e = threadIdx.x; e < E; e += blockDim.x) es[e] = b.cstart[b.grids[b.eord[e]].cell_base];
-      if (threadIdx.x == 0) es[E] = n_valid;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      bool ok = fits;
-      int g = 0;  // the open group starts at gb[g]
-      if (ok) gb[0] = es[0];
-      for (uint32_t e = 1; e <= E && ok; ++e) {
-        if (es[e] - gb[g] <= cap) continue;  // ensemble e - 1 fits the open group
-        if (es[e - 1] != gb[g]) {            // close the group before ensemble e - 1
-          if (g + 1 >= TL_GROUPS_MAX) {
-            ok = false;
-            break;
-          }
-          gb[++g] = es[e - 1];
-        }
-        ok = es[e] - gb[g] <= cap;  // else ensemble e - 1 alone is larger than the blocks hold
-      }
-      if (ok) gb[g + 1] = n_valid;
-      ng = ok ? g + 1 : 0;  // groups [gb[k], gb[k + 1]), k < ng
-    }
-  }
-  __syncthreads();
-  const int groups = ng;
+  extern __shared__ unsigned long long tl_raw[];
+  __shared__ TileGroups tg;
+  make_groups(b, n_valid, gridDim.x * TL_VMAX, reinterpret_cast<uint32_t*>(tl_raw), (uint32_t)(TL_SMEM / sizeof(uint32_t)),
+              tg);
+  const int groups = tg.n;
   if (groups <= 0) return false;
   for (int g = 0; g < groups; ++g) {
-    tl_group<RD_THREADS>(b, step, ctrl, t0, gb[g], gb[g + 1]);
+    tl_group<RD_THREADS>(b, step, ctrl, t0, tg.lo[g], tg.lo[g + 1]);
     __syncthreads();  // the block's shared lists are reused by the next group
   }
   return true;
@@ -342,7 +276,7 @@ __global__ void __launch_bounds__(RD_THREADS, 2) k_rounds(Bufs b, StepArgs a, Ct
   // one L2 slice and delayed the start of the pairs by 4-10 us
   __shared__ uint32_t cw[4];
   if (threadIdx.x == 0) {
-    cw[0] = ((volatile uint32_t*)&ctrl->halt)[0];
+    cw[0] = ((volatile uint32_t*)&ctrl->halt)[0] | ((volatile uint32_t*)&ctrl->ev_taken)[0];
     cw[1] = ((volatile uint32_t*)&ctrl->act_n)[0];
     cw[2] = ((volatile uint32_t*)&ctrl->n_valid)[0];
     cw[3] = a.use_ctrl_step ? ((volatile uint32_t*)&ctrl->step)[0] : a.step0;

@@ -126,7 +126,7 @@ struct lm_ctx {
   float *rec_lon = nullptr, *rec_lat = nullptr;
   int8_t* rec_sp = nullptr;
 
-  int rgrid = 0, rblock = 0;
+  int rgrid = 0, rblock = 0, egrid = 0;
   // tuning knobs (lm_set_tuning): block sizes and grid shapes that change speed, never results
   int tune_rounds_threads = 1024;  // interaction blocks: 1,024 threads x 2 vertices or 512 x 4
   int tune_long_per_sm = 6;        // long-list blocks per SM
@@ -510,7 +510,10 @@ cudaError_t enqueue_interaction(lm_ctx* c, const StepArgs& a, uint32_t flags, bo
   PROF(c, P_SWEEP_LONG, launch_sweep_long(b, c->pp, a, c->ctrl, c->sms, c->tune_long_per_sm, st));
   if (flags & LM_STEP_INTERACT) {
     cudaEvent_t pa = prof_begin(c);
-    cudaError_t e = launch_rounds(b, a, c->ctrl, c->rgrid, c->rblock, st);
+    cudaError_t e = cudaSuccess;
+    // dense batches (the kernel decides); other contexts save the launch
+    if (c->n_ens > 1 && c->nslots >= EV_SLOTS && c->egrid > 0 && !b.plog) e = launch_events(b, a, c->ctrl, c->egrid, st);
+    if (e == cudaSuccess) e = launch_rounds(b, a, c->ctrl, c->rgrid, c->rblock, st);
     prof_end(c, P_ROUNDS, pa);
     if (e != cudaSuccess) return e;
   }
@@ -824,6 +827,7 @@ int lm_ctx_create(int device, lm_ctx** out) {
       (e = cudaStreamSynchronize(c->st)) != cudaSuccess)
     return bail(fail(c, LM_ERR_CUDA, "ctrl init: %s", cudaGetErrorString(e)));
   c->rgrid = rounds_grid(device, c->tune_rounds_threads, &c->rblock);
+  c->egrid = events_grid(device);
   set_pair_params(c, 0.0, LM_NORM_L2);
   *out = c;
   return LM_OK;

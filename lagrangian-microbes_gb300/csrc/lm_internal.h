@@ -15,7 +15,7 @@
 //              uint32 sid[S], skey[S], sens[S]; float2 spos[S]  (particles in cell order)
 //              uint32 deg[S], slab[S][SLAB]     (neighbour lists up to SLAB, sorted by priority;
 //                                                a longer list's overflow offset in slot 0)
-//              uint32 ovf[cap]; uint64 oprio[cap]  (longer lists, allocated per step)
+//              uint32 ovf[cap]; uint64 oprio[cap]  (longer lists, allocated per step, NONE behind each)
 //              uint64 wstate[S] = species << 56 | list position << 32 | partner;
 //              uint32 level[S] (pair-log runs only), act[S]   (interaction dataflow)
 #pragma once
@@ -89,6 +89,7 @@ struct Ctrl {
   int stage_k[3];               // frame brackets of this step's stage times t, t+dt/2, t+dt
   float stage_w[3];
   int stage_ok;                 // 0 when a stage time left the field's time axis
+  uint32_t ev_taken;            // k_rounds_events applied the step's pairs
   uint32_t never;               // a flag nothing sets: the injected failure of the tests waits on it
 };
 
@@ -328,6 +329,10 @@ void launch_pair_rows(const Bufs& b, uint32_t n_valid, uint32_t n_long, const ui
 // Grid of the cooperative launch with `threads` (512 or 1,024) per block; *block receives the block size.
 int rounds_grid(int device, int threads, int* block);
 cudaError_t launch_rounds(const Bufs& b, const StepArgs& a, Ctrl* ctrl, int grid, int block, cudaStream_t st);
+// The same for dense batches of ensembles, launched before it (k_events.cu): grid, and the launch.
+constexpr uint32_t EV_SLOTS = 1u << 17;  // from this many slots
+int events_grid(int device);
+cudaError_t launch_events(const Bufs& b, const StepArgs& a, Ctrl* ctrl, int grid, cudaStream_t st);
 void launch_census(const Bufs& b, Ctrl* ctrl, cudaStream_t st);
 const void* lm_census_kernel();  // one kernel of the library, for attribute queries
 void launch_unpad(const float* src, float* dst, const int32_t* map, uint32_t nslots, cudaStream_t st);

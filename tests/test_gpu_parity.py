@@ -453,3 +453,40 @@ def test_gpu_cell_factor_does_not_change_results(engine, lm, orc):
         sim.close()
     np.testing.assert_array_equal(out[0], out[1])
     np.testing.assert_array_equal(out[0], out[2])
+
+
+@pytest.mark.parametrize("sizes, degree", [
+    ((70001, 61100, 33), 40),            # a few dense ensembles, one of a single warp's size
+    ((131072, 5, 1, 2000), 18),          # just over the rule's size, lists around its length
+    ((20000,) * 9, 120),                 # long chains, most pairs across blocks
+    ((330000, 330000, 40000), 20),       # two groups of ensembles
+])
+def test_dense_batches_worked_off_by_events_equal_the_ensembles_alone(engine, lm, sizes, degree):
+    """Batches that k_rounds_events takes (at least 2^17 slots, long lists of 16 entries and more on
+    average), species values outside 1..3 among them: every species as when each ensemble runs alone
+    in a context, where k_rounds applies the pairs."""
+    rng = np.random.default_rng(len(sizes) + degree)
+    f = lm.synthetic_psi_field(195.0, 215.0, 20.0, 35.0, 0.25, n_frames=4, frame_seconds=3600.0, seed=9)
+    members = []
+    for n in sizes:
+        side = np.sqrt(n * np.pi * 1e-4 / degree)
+        members.append((199 + 8 * rng.random() + side * rng.random(n), 24 + 4 * rng.random() + side * rng.random(n),
+                        rng.integers(0, 5, n).astype(np.int8)))
+    seeds = [int(s) for s in rng.integers(0, 2 ** 60, len(sizes))]
+    p = dict(p_rs=0.7, p_pr=0.55, p_sp=0.9)
+    batch = engine.EnsembleSimulation([f], members, radius=0.01, seeds=seeds, **p)
+    t0 = float(f.times[0])
+    batch.step(t0, 3600.0, 2)
+    st = batch.stats()
+    assert sum(sizes) >= 1 << 17 and 2 * st["pairs"] > 12 * sum(sizes)
+    plain = batch.species()
+    batch.upload_ensembles(members)
+    batch.capture(t0, 3600.0, 2, step0=0)
+    batch.run_graph(1)
+    np.testing.assert_array_equal(batch.species(), plain)
+    for (lon, lat, sp), seed, got in zip(members, seeds, batch.split(plain)):
+        one = engine.Simulation(f, lon, lat, sp, radius=0.01, seed=seed, **p)
+        one.step(t0, 3600.0, 2)
+        np.testing.assert_array_equal(one.species(), got)
+        one.close()
+    batch.close()
