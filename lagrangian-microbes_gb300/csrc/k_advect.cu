@@ -224,6 +224,7 @@ __device__ __forceinline__ void step_begin_body(const Bufs& b, const FieldView& 
     ctrl->ev_taken = 0;
     ctrl->census[0] = ctrl->census[1] = ctrl->census[2] = ctrl->census[3] = 0;
     if (bracket) {  // float64 time arithmetic once per step, not once per advection block
+      if (!a.use_ctrl_step) ctrl->step = a.step0;  // plain steps bring their index: no copy before them
       const uint32_t step = a.use_ctrl_step ? ctrl->step : a.step0;
       const double t0 = a.t_start + (double)(int)(step - a.step0) * a.dt;
       const double ts[3] = {t0, t0 + 0.5 * a.dt, t0 + a.dt};
@@ -281,6 +282,58 @@ void launch_step_turn(const Bufs& b, const FieldView* f, const StepArgs& an, Ctr
   FieldView fv{};
   if (f) fv = *f;
   launch_dep(k_step_end, dim3(bookkeeping_grid(b)), dim3(256), st, b, fv, an, f ? 1 : 0, ctrl, interact ? 1 : 0, 1);
+}
+
+// The state in caller order, packed as lon | lat | species | status of n microbes each (map NULL: slot k is microbe k).
+__global__ void k_pack_state(const float* __restrict__ xo, const float* __restrict__ yo,
+                             const int8_t* __restrict__ species, const uint8_t* __restrict__ status,
+                             const int32_t* __restrict__ map, uint32_t n, uint32_t S, int abs, float ox, float oy,
+                             unsigned char* __restrict__ out) {
+  const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= S) return;
+  const int32_t q = map ? map[p] : (p < n ? (int32_t)p : -1);
+  if (q < 0) return;
+  const float x = xo[p], y = yo[p];
+  float* f = reinterpret_cast<float*>(out);
+  f[q] = abs ? __fadd_rn(ox, x) : x;
+  f[(size_t)n + q] = abs ? __fadd_rn(oy, y) : y;
+  out[8 * (size_t)n + q] = (unsigned char)species[p];
+  out[9 * (size_t)n + q] = status[p];
+}
+
+void launch_pack_state(const float* xo, const float* yo, const int8_t* species, const uint8_t* status,
+                       const int32_t* map, uint32_t n, uint32_t S, int abs, float ox, float oy, unsigned char* out,
+                       cudaStream_t st) {
+  if (S) k_pack_state<<<(S + 255) / 256, 256, 0, st>>>(xo, yo, species, status, map, n, S, abs, ox, oy, out);
+}
+
+// A snapshot back into the state, four slots a thread, and the step counter with it: one launch for four copies, a
+// write of the counter and a synchronisation (a rewind of 10,000 microbes 41 -> 22 us, of 2,000,000 61 -> 26).
+__global__ void k_restore(const float* __restrict__ sx, const float* __restrict__ sy, const int8_t* __restrict__ ss,
+                          const uint8_t* __restrict__ sst, float* __restrict__ x, float* __restrict__ y,
+                          int8_t* __restrict__ sp, uint8_t* __restrict__ st, uint32_t S, uint32_t step, Ctrl* ctrl) {
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t == 0) ctrl->step = step;
+  const uint32_t p = 4 * t;
+  if (p + 3 < S) {
+    *reinterpret_cast<float4*>(x + p) = *reinterpret_cast<const float4*>(sx + p);
+    *reinterpret_cast<float4*>(y + p) = *reinterpret_cast<const float4*>(sy + p);
+    *reinterpret_cast<uint32_t*>(sp + p) = *reinterpret_cast<const uint32_t*>(ss + p);
+    *reinterpret_cast<uint32_t*>(st + p) = *reinterpret_cast<const uint32_t*>(sst + p);
+  } else {
+    for (uint32_t k = p; k < S; ++k) {
+      x[k] = sx[k];
+      y[k] = sy[k];
+      sp[k] = ss[k];
+      st[k] = sst[k];
+    }
+  }
+}
+
+void launch_restore(const float* sx, const float* sy, const int8_t* ss, const uint8_t* sst, float* x, float* y,
+                    int8_t* sp, uint8_t* st, uint32_t S, uint32_t step, Ctrl* ctrl, cudaStream_t stream) {
+  const uint32_t grid = S / 1024 + 1;  // (at least one thread sets the step)
+  k_restore<<<grid, 256, 0, stream>>>(sx, sy, ss, sst, x, y, sp, st, S, step, ctrl);
 }
 
 // Gathers from the padded slot layout into caller order (map[slot] = caller index or -1).

@@ -293,6 +293,11 @@ void launch_interleave(const float* u, const float* v, float2* uv, size_t n, cud
 void launch_particles_in(const double* lon, const double* lat, const int8_t* sp, const int32_t* map, uint32_t S,
                          double org_lon, double org_lat, float* xo, float* yo, int8_t* species, uint8_t* status,
                          cudaStream_t st);
+void launch_pack_state(const float* xo, const float* yo, const int8_t* species, const uint8_t* status,
+                       const int32_t* map, uint32_t n, uint32_t S, int abs, float ox, float oy, unsigned char* out,
+                       cudaStream_t st);
+void launch_restore(const float* sx, const float* sy, const int8_t* ss, const uint8_t* sst, float* x, float* y,
+                    int8_t* sp, uint8_t* st, uint32_t S, uint32_t step, Ctrl* ctrl, cudaStream_t stream);
 // step_begin also brackets the stage times of the step in the field's frames when `f` is given.
 void launch_step_begin(const Bufs& b, const FieldView* f, const StepArgs& a, Ctrl* ctrl, cudaStream_t st);
 void launch_step_end(Ctrl* ctrl, bool interact, cudaStream_t st);

@@ -196,3 +196,42 @@ def test_particles_from_page_locked_arrays_equal_host_conversion(lm, orc, small_
     for a, b in zip(*states):
         for k in ("xo", "yo", "species", "status"):
             np.testing.assert_array_equal(a[k], b[k], err_msg=k)
+
+
+@pytest.mark.parametrize("counts", [(1,), (3,), (26214,), (26215,), (26215 * 2 + 1,), (5, 1, 300), (20000, 6214), (40001, 0, 257)])
+def test_state_reads_and_rewinds_hold_every_microbe_in_its_place(lm, orc, small_field, counts):
+    """State reads on both sides of the staged size, of one and several ensembles, and a rewind of ragged sizes:
+    the uploaded values (float64 minus the field origin, rounded once; plus it, rounded once) in caller order."""
+    from lagrangian_microbes_gb300 import engine
+    rng = np.random.default_rng(sum(counts))
+    parts = [(rng.uniform(200.0, 201.0, k), rng.uniform(25.0, 26.0, k), rng.integers(1, 4, k).astype(np.int8)) for k in counts]
+    if len(counts) == 1:
+        sim = lm.Simulation(small_field, *parts[0], radius=0.01, seed=5)
+    else:
+        sim = engine.EnsembleSimulation(small_field, parts, radius=0.01, seeds=list(range(len(parts))))
+    lons, lats, sp = (np.concatenate([p[k] for p in parts]) for k in range(3))
+    ox, oy = np.float32(small_field.lon[0]), np.float32(small_field.lat[0])
+    xo, yo = (lons - np.float64(ox)).astype(np.float32), (lats - np.float64(oy)).astype(np.float32)
+
+    def check(step):
+        lon, lat, got, status = sim.state()
+        np.testing.assert_array_equal(lon, ox + xo)
+        np.testing.assert_array_equal(lat, oy + yo)
+        np.testing.assert_array_equal(got, sp)
+        assert not status.any()
+        np.testing.assert_array_equal(sim.species(), sp)
+        ck = sim.export_state()
+        np.testing.assert_array_equal(ck["xo"], xo)
+        np.testing.assert_array_equal(ck["yo"], yo)
+        np.testing.assert_array_equal(ck["species"], sp)
+        assert ck["step"] == step and not ck["status"].any()
+
+    sim.ctx.call("lm_set_step", 7)
+    sim.snapshot()
+    check(7)
+    sim.step(float(small_field.times[0]), 3600.0, 2, step0=11)
+    assert sim.stats()["step"] == 13
+    sim.restore()
+    assert sim.step_index == 7
+    check(7)
+    sim.close()
