@@ -157,7 +157,7 @@ int lm_set_cell_factor(lm_ctx* ctx, double factor);
 /* Launch shapes of the step kernels, chosen by an autotuner (Simulation.autotune): no knob changes
  * any result, only the speed. LM_TUNE_ROUNDS_THREADS: interaction blocks of 1024 threads owning two
  * vertices each (default) or 512 owning four; LM_TUNE_LONG_BLOCKS_PER_SM: blocks per SM of the
- * long-neighbour-list kernel (1..32, default 6); LM_TUNE_ADVECT_THREADS: advection threads per
+ * long-neighbour-list kernel (1..32, default 8); LM_TUNE_ADVECT_THREADS: advection threads per
  * block, 128 or 256 (default). Setting a knob forgets the captured graph (capture again). No
  * counterpart in the reference (its parallelism is joblib tiles, particle_advecter.py:143-148). */
 #define LM_TUNE_ROUNDS_THREADS 1

@@ -51,6 +51,20 @@ __device__ __forceinline__ bool within(const PairParams& pp, float2 a, float2 b)
   }
 }
 
+// The float32 side of within() without branches: the distance in the norm's terms, with the bounds below which it is
+// inside the radius (lo) and above which it is outside (hi); in between within() decides.
+struct Band {
+  float lo, hi;
+};
+__device__ __forceinline__ Band band_of(const PairParams& pp) {
+  return pp.norm == 2 ? Band{pp.r2f_lo, pp.r2f_hi} : Band{pp.rf_lo, pp.rf_hi};
+}
+__device__ __forceinline__ float norm_dist(int norm, float2 a, float2 b) {
+  const float dx = a.x - b.x, dy = a.y - b.y;
+  const float d2 = __fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy));
+  return norm == 2 ? d2 : norm == 1 ? fabsf(dx) + fabsf(dy) : fmaxf(fabsf(dx), fabsf(dy));
+}
+
 __device__ __forceinline__ unsigned long long pair_prio(uint32_t i, uint32_t j, uint32_t step, uint32_t k0,
                                                         uint32_t k1) {
   return order_hash(i, j, step, ((unsigned long long)k1 << 32) | k0);
@@ -659,41 +673,75 @@ __device__ void sort_segment(unsigned long long* __restrict__ pr, uint32_t* __re
   }
 }
 
-// Long lists (more than SLAB neighbours): one warp per vertex. The warp reserves the overflow space
-// of all its vertices with one atomic; for each batch of 32 vertices lane k loads vertex k's cell,
-// position, key runs and ensemble constants, so the dependent loads happen once per batch. For
-// each vertex the warp then walks its six key runs as one candidate range, 64 candidates a pass
-// (position and id loaded together), and gathers the neighbours with ballots into shared memory.
-// The order (priority descending, partner's local id ascending) comes from:
-//   - up to 32 entries: a rank sort in registers, one entry per lane;
-//   - up to LONG_SMEM_MAX: a bucket sort. The priorities are uniform 64-bit hashes, so 256 buckets
-//     on their top 8 bits (descending) hold about d / 256 entries each, and an insertion sort
-//     inside each bucket by the exact order finishes it;
-//   - beyond: a sort in global memory by one lane.
-// Only the sorted partners are kept (the priorities were needed for the order only).
+// Long lists (more than SLAB neighbours). A warp takes batches of up to 32 of them, consecutive in cell
+// order; lane k loads vertex k's cell, position, key runs and ensemble constants, so the dependent loads
+// happen once per batch, and one atomic reserves the overflow space of all its batches. Then:
+//   - the members of the batch that share a cell share its candidates: the 3x3 cells are read once into
+//     shared memory, and each member tests them from there, 32 a pass, and gathers its neighbours with
+//     ballots;
+//   - the lists of several members fill one area of LONG_AREA entries, and priorities, outcome draws and
+//     the order run over the area, an entry a lane, whatever the lengths of its lists. Only the entries
+//     whose endpoint applies the pair (half of them) are queued for a draw;
+//   - each entry's place is the number of larger keys in its list, the key being the upper 24 bits of the
+//     64-bit priority over the entry's index in its list (so keys differ). An area where two entries of a
+//     list agree in those 24 bits is ranked again by the whole priorities.
+// Members with more than LONG_FEW neighbours or LONG_CAND candidates are done one at a time (long_alone):
+// candidates from global memory, 64 a pass, and up to LONG_SMEM_MAX entries a bucket sort: the priorities
+// are uniform hashes, so 256 buckets on their top 8 bits (descending) hold about d / 256 entries each, and
+// an insertion sort inside each bucket by the exact order finishes it; beyond, a sort in global memory by
+// one lane. Only the sorted partners are kept (the priorities were needed for the order only).
+// Bound by instruction issue (73 % of the slots, 670 instructions a list of 34). A warp per list before
+// took 530 us for the 447,000 lists of 32 ensembles, 245 for the 338,000 of 2,000,000 mixed microbes and 66
+// for the 81,000 of 490,000; this takes 376, 146 and 43. At 6 blocks an SM (9 KB a warp) it took 438, 194, 54.
 constexpr int LONG_WARPS = 4;
 constexpr uint32_t LONG_SMEM_MAX = 512;
 constexpr uint32_t LONG_BUCKETS = 256;
 
-struct LongSmem {
-  unsigned long long p[LONG_SMEM_MAX];  // pair priority of entry i (gather order)
+struct LongSmem {  // (the priorities stay in the list's part of oprio)
   uint32_t t[LONG_SMEM_MAX];            // list entry (partner's cell-order index + outcome bits)
   uint16_t ord[LONG_SMEM_MAX];          // entries in list order
   uint32_t start[LONG_BUCKETS], cur[LONG_BUCKETS];
 };
 
+// What a warp keeps of a batch: its members, the candidates of the cell at hand and the area of lists.
+constexpr uint32_t LONG_FEW = 96;    // neighbours (keys keep 7 bits for the index)
+constexpr uint32_t LONG_CAND = 192;  // candidates
+constexpr uint32_t LONG_AREA = 224;  // entries (with these sizes 8 blocks of 4 warps fit an SM)
+struct LongArea {
+  uint32_t key[LONG_AREA];  // 16-byte aligned: four keys a load
+  uint32_t t[LONG_AREA];    // list entry (partner's cell-order index + outcome bits)
+  uint32_t lb[LONG_AREA];   // partner's local id; then the keys in list order
+  uint16_t queue[LONG_AREA];
+  uint8_t own[LONG_AREA];   // member of the batch the entry belongs to (0xff: a gap)
+  float2 cpos[LONG_CAND];
+  uint32_t ct[LONG_CAND];
+  // the members: the part of the priority's hash that its pairs share, position, index, local id, ensemble, list
+  // offset in ovf, length, place in the area, species
+  unsigned long long hash[32];
+  float2 ps[32];
+  uint32_t s[32], la[32], e[32], o[32];
+  uint16_t d[32], st[32];
+  int8_t sp[32];
+};
+union LongShared {
+  LongSmem one;
+  LongArea many;
+};
+
 // Does entry x come before entry y? Ties of the 64-bit priority (rare) go by the partner's local id.
-__device__ __forceinline__ bool long_before(const Bufs& b, const LongSmem& sh, uint32_t base, uint32_t x, uint32_t y) {
-  const unsigned long long px = sh.p[x], py = sh.p[y];
+__device__ __forceinline__ bool long_before(const Bufs& b, const LongSmem& sh, const unsigned long long* p, uint32_t base,
+                                            uint32_t x, uint32_t y) {
+  const unsigned long long px = p[x], py = p[y];
   if (px != py) return px > py;
   return b.sid[entry_id(sh.t[x])] - base < b.sid[entry_id(sh.t[y])] - base;
 }
 
 // The bucket sort of entries [0, d) of sh into sh.ord (one warp).
-__device__ __forceinline__ void long_sort(const Bufs& b, LongSmem& sh, uint32_t base, uint32_t d, uint32_t lane) {
+__device__ __forceinline__ void long_sort(const Bufs& b, LongSmem& sh, const unsigned long long* p, uint32_t base, uint32_t d,
+                                          uint32_t lane) {
   for (uint32_t i = lane; i < LONG_BUCKETS; i += 32) sh.cur[i] = 0;
   __syncwarp();
-  for (uint32_t i = lane; i < d; i += 32) atomicAdd(&sh.cur[255u - (uint32_t)(sh.p[i] >> 56)], 1u);
+  for (uint32_t i = lane; i < d; i += 32) atomicAdd(&sh.cur[255u - (uint32_t)(p[i] >> 56)], 1u);
   __syncwarp();
   // exclusive scan of the bucket counts: lane holds buckets 8 lane .. 8 lane + 7
   uint32_t c[8], tot = 0;
@@ -716,14 +764,14 @@ __device__ __forceinline__ void long_sort(const Bufs& b, LongSmem& sh, uint32_t 
   }
   __syncwarp();
   for (uint32_t i = lane; i < d; i += 32)
-    sh.ord[atomicAdd(&sh.cur[255u - (uint32_t)(sh.p[i] >> 56)], 1u)] = (uint16_t)i;
+    sh.ord[atomicAdd(&sh.cur[255u - (uint32_t)(p[i] >> 56)], 1u)] = (uint16_t)i;
   __syncwarp();
   for (uint32_t k = lane; k < LONG_BUCKETS; k += 32) {
     const uint32_t lo = sh.start[k], hi = sh.cur[k];
     for (uint32_t x = lo + 1; x < hi; ++x) {
       const uint16_t e = sh.ord[x];
       uint32_t y = x;
-      while (y > lo && long_before(b, sh, base, e, sh.ord[y - 1])) {
+      while (y > lo && long_before(b, sh, p, base, e, sh.ord[y - 1])) {
         sh.ord[y] = sh.ord[y - 1];
         --y;
       }
@@ -733,29 +781,202 @@ __device__ __forceinline__ void long_sort(const Bufs& b, LongSmem& sh, uint32_t 
   __syncwarp();
 }
 
-__global__ void __launch_bounds__(LONG_WARPS * 32) k_sweep_long(Bufs b, PairParams pp, StepArgs a, Ctrl* ctrl) {
+// One list by the whole warp, candidates from global memory.
+__device__ __noinline__ void long_alone(const Bufs& b, const PairParams& pp, uint32_t step, LongSmem& sh, uint32_t s,
+                                        uint32_t d, unsigned long long o) {
+  const uint32_t lane = threadIdx.x & 31u;
+  const Vertex v = load_vertex(b, s);
+  const EnsInfo& info = b.ens[v.e];
+  const uint32_t id0 = b.sid[s], la = id0 - v.base, base = v.base, k0 = info.seed_lo, k1 = info.seed_hi;
+  const int sp = b.species[id0];
+  const float2 ps = v.ps;
+  uint32_t t0[6], t1[6], c[7];
+  neighbour_runs(b, v, t0, t1);
+  // the six runs as one candidate range: candidate i is in the run q with c[q] <= i < c[q + 1]
+  c[0] = 0;
+#pragma unroll
+  for (int q = 0; q < 6; ++q) c[q + 1] = c[q] + (t1[q] - t0[q]);
+  const bool in_smem = d <= LONG_SMEM_MAX;
+  uint32_t m = 0;
+  // two slices of 32 candidates per pass, each candidate's position and id loaded together
+  for (uint32_t tb = 0; tb < c[6]; tb += 64) {
+    uint32_t t[2], id[2];
+    float2 pt[2];
+    bool in[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const uint32_t i = tb + 32u * h + lane;
+      uint32_t x = t0[0] + i;
+#pragma unroll
+      for (int q = 1; q < 6; ++q)
+        if (i >= c[q]) x = t0[q] + (i - c[q]);  // the last run starting at or before i (empty runs never win)
+      t[h] = x;
+      in[h] = i < c[6] && x != s;
+      pt[h] = in[h] ? b.spos[x] : ps;
+      id[h] = in[h] ? b.sid[x] : 0u;
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const bool ok = in[h] && within(pp, ps, pt[h]);
+      const uint32_t mask = __ballot_sync(0xffffffffu, ok);
+      if (ok) {
+        const uint32_t pos = m + __popc(mask & lanemask_lt_p());
+        if (pos < d) {  // the partner and its local id; priority and draw follow below
+          if (in_smem)
+            sh.t[pos] = t[h];
+          else
+            b.ovf[o + pos] = t[h];
+          b.oprio[o + pos] = id[h] - base;
+        }
+      }
+      m += __popc(mask);
+    }
+  }
+  // priorities and outcome draws of the d entries, one entry per lane (in the gather only the
+  // lanes that found a neighbour would work, about a third of them)
+  __syncwarp();
+  for (uint32_t i = lane; i < d; i += 32) {
+    const uint32_t tt = in_smem ? sh.t[i] : b.ovf[o + i];
+    const uint32_t lb = (uint32_t)b.oprio[o + i];
+    const unsigned long long p = pair_prio(min(la, lb), max(la, lb), step, k0, k1);
+    const uint32_t e = tt > s ? tt | win_bits(info, la, lb, step) : tt;
+    if (in_smem)
+      sh.t[i] = e;
+    else
+      b.ovf[o + i] = e;
+    b.oprio[o + i] = p;
+  }
+  uint32_t first;
+  if (in_smem) {
+    __syncwarp();
+    long_sort(b, sh, b.oprio + o, base, d, lane);
+    for (uint32_t i = lane; i < d; i += 32) b.ovf[o + i] = sh.t[sh.ord[i]];
+    first = sh.t[sh.ord[0]];
+    __syncwarp();  // the next vertex reuses the shared list
+  } else {
+    __syncwarp();
+    if (lane == 0) sort_segment(b.oprio + o, b.ovf + o, b.sid, d);
+    __syncwarp();
+    first = b.ovf[o];
+  }
+  if (lane == 0) {
+    b.ovf[o + d] = NONE;
+    b.slab[(size_t)s * SLAB] = (uint32_t)o;  // a long list's overflow offset, in its unused slab row
+    b.wstate[s] = pack_state(first, 0u, sp);  // entry 0 of the list
+  }
+}
+
+// Entry i of the area at place k of its list; the first one also makes its member ready.
+__device__ __forceinline__ void long_out(const Bufs& b, const LongArea& sh, uint32_t i, uint32_t v, uint32_t k) {
+  const uint32_t o = sh.o[v], t = sh.t[i];
+  b.ovf[(size_t)o + k] = t;
+  if (k == 0) {
+    const uint32_t s = sh.s[v];
+    b.ovf[(size_t)o + sh.d[v]] = NONE;
+    b.slab[(size_t)s * SLAB] = o;               // a long list's overflow offset, in its unused slab row
+    b.wstate[s] = pack_state(t, 0u, sh.sp[v]);  // entry 0 of the list
+  }
+}
+
+// The n entries of the area once more, placed by their whole priorities.
+__device__ __noinline__ void long_exact(const Bufs& b, const LongArea& sh, uint32_t n) {
+  for (uint32_t i = threadIdx.x & 31u; i < n; i += 32) {
+    const uint32_t v = sh.own[i];
+    if (v == 0xffu) continue;
+    const uint32_t st = sh.st[v], end = st + sh.d[v], la = sh.la[v];
+    const uint32_t base = b.ens[sh.e[v]].base, lb = b.sid[entry_id(sh.t[i])] - base;
+    const unsigned long long h = sh.hash[v], p = order_hash_from(h, min(la, lb), max(la, lb));
+    uint32_t k = 0;
+    for (uint32_t j = st; j < end; ++j) {
+      const uint32_t lj = b.sid[entry_id(sh.t[j])] - base;
+      k += before(order_hash_from(h, min(la, lj), max(la, lj)), lj, p, lb) ? 1u : 0u;
+    }
+    long_out(b, sh, i, v, k);
+  }
+}
+
+// Priorities, draws, order and output of the n entries of the area. (Not inlined, its loops not unrolled: with four
+// copies of an unrolled form the warps waited on instruction fetches, 7.9 of the 14 cycles between two instructions.)
+__device__ __noinline__ void long_flush(const Bufs& b, uint32_t step, LongArea& sh, uint32_t n) {
+  const uint32_t lane = threadIdx.x & 31u;
+  __syncwarp();
+  uint32_t queued = 0;
+#pragma unroll 1
+  for (uint32_t i0 = 0; i0 < n; i0 += 32) {
+    const uint32_t i = i0 + lane;
+    const uint32_t v = i < n ? sh.own[i] : 0xffu;
+    uint32_t key = 0;  // gaps between the lists stay below every entry
+    bool draw = false;
+    if (v != 0xffu) {
+      const uint32_t t = sh.t[i], la = sh.la[v], lb = b.sid[t] - b.ens[sh.e[v]].base;
+      const unsigned long long p = order_hash_from(sh.hash[v], min(la, lb), max(la, lb));
+      key = ((uint32_t)(p >> 33) & ~127u) | (127u - (i - sh.st[v]));
+      draw = t > sh.s[v];
+      sh.lb[i] = lb;
+    }
+    if (i < n) sh.key[i] = key;
+    const uint32_t mask = __ballot_sync(0xffffffffu, draw);
+    if (draw) sh.queue[queued + __popc(mask & lanemask_lt_p())] = (uint16_t)i;
+    queued += __popc(mask);
+  }
+  __syncwarp();
+#pragma unroll 1
+  for (uint32_t q = lane; q < queued; q += 32) {
+    const uint32_t i = sh.queue[q], v = sh.own[i];
+    sh.t[i] |= win_bits(b.ens[sh.e[v]], sh.la[v], sh.lb[i], step);
+  }
+  __syncwarp();
+#pragma unroll 1
+  for (uint32_t i = lane; i < n; i += 32) {
+    const uint32_t v = sh.own[i];
+    if (v == 0xffu) continue;
+    const uint32_t st = sh.st[v], end = st + sh.d[v], key = sh.key[i];
+    uint32_t k = 0;
+#pragma unroll 1
+    for (uint32_t j = st; j < end; j += 4) {  // keys have 31 bits: the difference is negative where the other is larger
+      const uint4 x = *reinterpret_cast<const uint4*>(&sh.key[j]);
+      k += ((key - x.x) >> 31) + ((key - x.y) >> 31) + ((key - x.z) >> 31) + ((key - x.w) >> 31);
+    }
+    sh.lb[st + k] = key;
+    long_out(b, sh, i, v, k);
+  }
+  __syncwarp();
+  bool tie = false;
+#pragma unroll 1
+  for (uint32_t i = lane; i + 1 < n; i += 32) {
+    const uint32_t v = sh.own[i];
+    tie |= v != 0xffu && v == sh.own[i + 1] && (sh.lb[i] ^ sh.lb[i + 1]) < 128u;
+  }
+  if (__any_sync(0xffffffffu, tie)) long_exact(b, sh, n);  // (about one list of 4,000 at 96 entries)
+  __syncwarp();
+}
+
+__global__ void __launch_bounds__(LONG_WARPS * 32, 8) k_sweep_long(Bufs b, PairParams pp, StepArgs a, Ctrl* ctrl) {
   pdl_wait();
   if (ctrl->halt) return;
-  __shared__ LongSmem sh_all[LONG_WARPS];
+  __shared__ __align__(16) LongShared sh_all[LONG_WARPS];
   const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
-  LongSmem& sh = sh_all[w];
+  LongArea& sh = sh_all[w].many;
   const uint32_t n_long = ctrl->n_long;
   const uint32_t step = a.use_ctrl_step ? ctrl->step : a.step0;
   const unsigned long long cap = ctrl->ovf_cap;
+  const Band band = band_of(pp);
   const uint32_t gw = blockIdx.x * LONG_WARPS + w, nw = gridDim.x * LONG_WARPS;
-  // this warp's vertices: gw, gw + nw, gw + 2 nw, ...; one atomic reserves the space of all of them
-  const uint32_t count = gw < n_long ? (n_long - gw + nw - 1) / nw : 0u;
-  if (count == 0) return;
+  // batches of `per` vertices, the same number for every warp as nearly as can be: this warp's are gw, gw + nw, ...
+  if (n_long == 0) return;
+  const uint32_t turns = (n_long + 32u * nw - 1) / (32u * nw), per = (n_long + turns * nw - 1) / (turns * nw);
   unsigned long long sum = 0;
   bool too_many = false;
-  for (uint32_t i = lane; i < count; i += 32) {
-    const uint32_t d = b.deg[b.longv[gw + i * nw]];
+  for (uint32_t q = gw * per; q < n_long; q += nw * per) {
+    if (lane >= per || q + lane >= n_long) continue;
+    const uint32_t d = b.deg[b.longv[q + lane]];
     sum += d + 1u;  // the list and its end mark
     too_many |= d > MAX_DEGREE;
   }
   for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
   too_many = __any_sync(0xffffffffu, too_many);
   unsigned long long run = 0;
+  if (sum == 0) return;
   if (lane == 0) run = atomicAdd(&ctrl->ovf_used, sum);
   run = __shfl_sync(0xffffffffu, run, 0);
   if (too_many || run + sum > cap) {  // positions would not fit the state word / the area is full
@@ -766,12 +987,11 @@ __global__ void __launch_bounds__(LONG_WARPS * 32) k_sweep_long(Bufs b, PairPara
     }
     return;
   }
-  for (uint32_t ib = 0; ib < count; ib += 32) {
-    // lane k holds vertex ib + k of this warp's list, and loads its cell, position, key runs and
-    // ensemble constants, for all 32 vertices at once (a chain of dependent loads per batch
-    // instead of one per vertex)
-    const bool mine = ib + lane < count;
-    const uint32_t s_l = mine ? b.longv[gw + (ib + lane) * nw] : 0u;
+  for (uint32_t q = gw * per; q < n_long; q += nw * per) {
+    // lane k loads member k's cell, position, key runs and ensemble constants: a chain of dependent loads per batch
+    const uint32_t nk = min(per, n_long - q);
+    const bool mine = lane < nk;
+    const uint32_t s_l = mine ? b.longv[q + lane] : 0u;
     const uint32_t d_l = mine ? b.deg[s_l] : 0u;
     const uint32_t room_l = mine ? d_l + 1u : 0u;
     unsigned long long incl = room_l;
@@ -781,143 +1001,90 @@ __global__ void __launch_bounds__(LONG_WARPS * 32) k_sweep_long(Bufs b, PairPara
     }
     const unsigned long long o_l = run + incl - room_l;
     run += __shfl_sync(0xffffffffu, incl, 31);
-    uint32_t r0[6], r1[6], la_l = 0, base_l = 0, k0_l = 0, k1_l = 0, e_l = 0;
-    int sp_l = 0;
-    float px_l = 0.f, py_l = 0.f;
+    uint32_t r0[6], len[6], key_l = 0;
 #pragma unroll
-    for (int q = 0; q < 6; ++q) r0[q] = r1[q] = 0u;
+    for (int r = 0; r < 6; ++r) r0[r] = len[r] = 0u;
     if (mine) {
       const Vertex v = load_vertex(b, s_l);
-      neighbour_runs(b, v, r0, r1);
-      const EnsInfo& info = b.ens[v.e];
-      k0_l = info.seed_lo;
-      k1_l = info.seed_hi;
-      e_l = v.e;
-      base_l = v.base;
-      const uint32_t id = b.sid[s_l];
-      la_l = id - v.base;
-      sp_l = b.species[id];
-      px_l = v.ps.x;
-      py_l = v.ps.y;
+      neighbour_runs(b, v, r0, len);
+#pragma unroll
+      for (int r = 0; r < 6; ++r) len[r] -= r0[r];
+      key_l = b.skey[s_l];
     }
-    const uint32_t nk = min(32u, count - ib);
-    for (uint32_t k = 0; k < nk; ++k) {
-      const uint32_t s = __shfl_sync(0xffffffffu, s_l, k);
-      const uint32_t d = __shfl_sync(0xffffffffu, d_l, k);
-      const unsigned long long o = __shfl_sync(0xffffffffu, o_l, k);
-      const uint32_t la = __shfl_sync(0xffffffffu, la_l, k), base = __shfl_sync(0xffffffffu, base_l, k);
-      const uint32_t k0 = __shfl_sync(0xffffffffu, k0_l, k), k1 = __shfl_sync(0xffffffffu, k1_l, k);
-      const float2 ps = make_float2(__shfl_sync(0xffffffffu, px_l, k), __shfl_sync(0xffffffffu, py_l, k));
-      const int sp = __shfl_sync(0xffffffffu, sp_l, k);
-      const EnsInfo& info = b.ens[__shfl_sync(0xffffffffu, e_l, k)];
-      // the six runs as one candidate range: candidate i is in the run q with c[q] <= i < c[q + 1]
+    uint32_t cand = 0;
+#pragma unroll
+    for (int r = 0; r < 6; ++r) cand += len[r];
+    const uint32_t large = __ballot_sync(0xffffffffu, d_l > LONG_FEW || cand > LONG_CAND);
+    for (uint32_t m = large; m; m &= m - 1) {  // one at a time, in the same shared memory
+      const int k = __ffs(m) - 1;
+      long_alone(b, pp, step, sh_all[w].one, __shfl_sync(0xffffffffu, s_l, k), __shfl_sync(0xffffffffu, d_l, k),
+                 __shfl_sync(0xffffffffu, o_l, k));
+    }
+    if (mine) {
+      const uint32_t id = b.sid[s_l], e = b.sens[s_l];
+      const EnsInfo& info = b.ens[e];
+      sh.hash[lane] = order_hash_base(step, ((unsigned long long)info.seed_hi << 32) | info.seed_lo);
+      sh.ps[lane] = b.spos[s_l];
+      sh.s[lane] = s_l;
+      sh.la[lane] = id - info.base;
+      sh.e[lane] = e;
+      sh.o[lane] = (uint32_t)o_l;
+      sh.d[lane] = (uint16_t)d_l;  // (read for the small ones only)
+      sh.sp[lane] = b.species[id];
+    }
+    uint32_t used = 0;  // entries in the area
+    for (uint32_t rest = (nk == 32u ? 0xffffffffu : (1u << nk) - 1u) & ~large; rest;) {
+      const int lead = __ffs(rest) - 1;
+      const uint32_t lead_key = __shfl_sync(0xffffffffu, key_l, lead);
+      uint32_t m = __ballot_sync(0xffffffffu, mine && key_l == lead_key) & rest;
+      rest &= ~m;
+      // the six runs as one candidate range: candidate i is in the run r with c[r] <= i < c[r + 1]
       uint32_t t0[6], c[7];
       c[0] = 0;
 #pragma unroll
-      for (int q = 0; q < 6; ++q) {
-        t0[q] = __shfl_sync(0xffffffffu, r0[q], k);
-        c[q + 1] = c[q] + (__shfl_sync(0xffffffffu, r1[q], k) - t0[q]);
+      for (int r = 0; r < 6; ++r) {
+        t0[r] = __shfl_sync(0xffffffffu, r0[r], lead);
+        c[r + 1] = c[r] + __shfl_sync(0xffffffffu, len[r], lead);
       }
-      const bool in_smem = d <= LONG_SMEM_MAX;
-      uint32_t m = 0;
-      // two slices of 32 candidates per pass, each candidate's position and id loaded together
-      for (uint32_t tb = 0; tb < c[6]; tb += 64) {
-        uint32_t t[2], id[2];
-        float2 pt[2];
-        bool in[2];
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const uint32_t i = tb + 32u * h + lane;
-          uint32_t x = t0[0] + i;
-#pragma unroll
-          for (int q = 1; q < 6; ++q)
-            if (i >= c[q]) x = t0[q] + (i - c[q]);  // the last run starting at or before i (empty runs never win)
-          t[h] = x;
-          in[h] = i < c[6] && x != s;
-          pt[h] = in[h] ? b.spos[x] : ps;
-          id[h] = in[h] ? b.sid[x] : 0u;
-        }
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const bool ok = in[h] && within(pp, ps, pt[h]);
-          const uint32_t mask = __ballot_sync(0xffffffffu, ok);
-          if (ok) {
-            const uint32_t pos = m + __popc(mask & lanemask_lt_p());
-            if (pos < d) {  // the partner and its local id; priority and draw follow below
-              if (in_smem) {
-                sh.p[pos] = id[h] - base;
-                sh.t[pos] = t[h];
-              } else {
-                b.ovf[o + pos] = t[h];
-                b.oprio[o + pos] = id[h] - base;
-              }
-            }
-          }
-          m += __popc(mask);
-        }
-      }
-      // priorities and outcome draws of the d entries, one entry per lane (in the gather only the
-      // lanes that found a neighbour would work, about a third of them)
       __syncwarp();
-      for (uint32_t i = lane; i < d; i += 32) {
-        const uint32_t tt = in_smem ? sh.t[i] : b.ovf[o + i];
-        const uint32_t lb = (uint32_t)(in_smem ? sh.p[i] : b.oprio[o + i]);
-        const unsigned long long p = pair_prio(min(la, lb), max(la, lb), step, k0, k1);
-        const uint32_t e = tt > s ? tt | win_bits(info, la, lb, step) : tt;
-        if (in_smem) {
-          sh.p[i] = p;
-          sh.t[i] = e;
-        } else {
-          b.ovf[o + i] = e;
-          b.oprio[o + i] = p;
-        }
+      for (uint32_t i = lane; i < c[6]; i += 32) {
+        uint32_t x = t0[0] + i;
+#pragma unroll
+        for (int r = 1; r < 6; ++r)
+          if (i >= c[r]) x = t0[r] + (i - c[r]);  // the last run starting at or before i (empty runs never win)
+        sh.cpos[i] = b.spos[x];
+        sh.ct[i] = x;
       }
-      uint32_t first;
-      if (d <= 32) {
-        // one entry per lane, ranked by counting the entries that come before it
-        __syncwarp();
-        const bool has = lane < d;
-        const unsigned long long pi = has ? sh.p[lane] : 0ull;
-        const uint32_t ti = has ? sh.t[lane] : 0u;
-        uint32_t rank = 0;
-        bool tie = false;
-        for (uint32_t j = 0; j < d; ++j) {
-          const unsigned long long pj = __shfl_sync(0xffffffffu, pi, j);
-          rank += pj > pi ? 1u : 0u;
-          tie |= pj == pi && j != lane;
+      const uint32_t nc = c[6];
+      __syncwarp();
+      for (; m; m &= m - 1) {
+        const int k = __ffs(m) - 1;
+        const uint32_t s = sh.s[k], d = sh.d[k], room = (d + 3u) & ~3u;
+        const float2 ps = sh.ps[k];
+        if (used + room > LONG_AREA) {
+          long_flush(b, step, sh, used);
+          used = 0;
         }
-        if (__any_sync(0xffffffffu, has && tie)) {
-          // equal priorities go by the partner's local id (the order hash is a bijection of the
-          // pair, so this is not expected within one list)
-          const uint32_t li = has ? b.sid[entry_id(ti)] - base : 0u;
-          for (uint32_t j = 0; j < d; ++j) {
-            const unsigned long long pj = __shfl_sync(0xffffffffu, pi, j);
-            const uint32_t lj = __shfl_sync(0xffffffffu, li, j);
-            rank += (pj == pi && j != lane && lj < li) ? 1u : 0u;
-          }
+        if (lane == 0) sh.st[k] = (uint16_t)used;
+        uint32_t found = 0;
+        for (uint32_t i0 = 0; i0 < nc; i0 += 32) {
+          const uint32_t i = i0 + lane;
+          const uint32_t t = i < nc ? sh.ct[i] : s;
+          const float2 pt = sh.cpos[i];
+          const float dist = norm_dist(pp.norm, ps, pt);
+          bool ok = t != s && dist < band.lo;
+          const bool unsure = t != s && !(dist < band.lo) && !(dist > band.hi);
+          if (__any_sync(0xffffffffu, unsure) && unsure) ok = within(pp, ps, pt);
+          const uint32_t mask = __ballot_sync(0xffffffffu, ok);
+          const uint32_t at = found + __popc(mask & lanemask_lt_p());
+          if (ok && at < d) sh.t[used + at] = t;
+          found += __popc(mask);
         }
-        if (has) b.ovf[o + rank] = ti;
-        const uint32_t r0m = __ballot_sync(0xffffffffu, has && rank == 0u);
-        first = __shfl_sync(0xffffffffu, ti, __ffs(r0m) - 1);
-        __syncwarp();  // the next vertex reuses the shared list
-      } else if (in_smem) {
-        __syncwarp();
-        long_sort(b, sh, base, d, lane);
-        for (uint32_t i = lane; i < d; i += 32) b.ovf[o + i] = sh.t[sh.ord[i]];
-        first = sh.t[sh.ord[0]];
-        __syncwarp();  // the next vertex reuses the shared list
-      } else {
-        __syncwarp();
-        if (lane == 0) sort_segment(b.oprio + o, b.ovf + o, b.sid, d);
-        __syncwarp();
-        first = b.ovf[o];
-      }
-      if (lane == 0) {
-        b.ovf[o + d] = NONE;
-        b.slab[(size_t)s * SLAB] = (uint32_t)o;  // a long list's overflow offset, in its unused slab row
-        b.wstate[s] = pack_state(first, 0u, sp);  // entry 0 of the list
+        for (uint32_t i = lane; i < room; i += 32) sh.own[used + i] = i < d ? (uint8_t)k : (uint8_t)0xff;
+        used += room;
       }
     }
+    if (used) long_flush(b, step, sh, used);
     // every vertex of the batch is active (it has > SLAB pairs): one atomic per batch
     uint32_t at = 0;
     if (lane == 0) at = atomicAdd(&ctrl->act_n, nk);
@@ -928,7 +1095,7 @@ __global__ void __launch_bounds__(LONG_WARPS * 32) k_sweep_long(Bufs b, PairPara
 
 void launch_sweep_long(const Bufs& b, const PairParams& pp, const StepArgs& a, Ctrl* ctrl, int sms,
                        int blocks_per_sm, cudaStream_t st) {
-  // at most 6 blocks of 36 KB fit an SM's shared memory; more queue behind them
+  // at most 8 blocks of 27 KB fit an SM's shared memory; more queue behind them
   launch_dep(k_sweep_long, dim3(sms * blocks_per_sm), dim3(LONG_WARPS * 32), st, b, pp, a, ctrl);
 }
 

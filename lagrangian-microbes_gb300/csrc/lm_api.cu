@@ -129,7 +129,7 @@ struct lm_ctx {
   int rgrid = 0, rblock = 0, egrid = 0;
   // tuning knobs (lm_set_tuning): block sizes and grid shapes that change speed, never results
   int tune_rounds_threads = 1024;  // interaction blocks: 1,024 threads x 2 vertices or 512 x 4
-  int tune_long_per_sm = 6;        // long-list blocks per SM
+  int tune_long_per_sm = 8;        // long-list blocks per SM
   int tune_advect_threads = 256;   // advection threads per block (128 or 256)
 
   // graph

@@ -53,13 +53,19 @@ __host__ __device__ __forceinline__ PairDraw pair_draw(uint32_t i, uint32_t j, u
 // Flood, "Fast splittable pseudorandom number generators", OOPSLA 2014) applied to the pair index
 // offset by Weyl multiples of seed and step. A bijection of its 64-bit input, so pairs of one step
 // never collide; cheap enough to evaluate for every neighbour-list entry.
-__host__ __device__ __forceinline__ unsigned long long order_hash(uint32_t i, uint32_t j, uint32_t step,
-                                                                  unsigned long long seed) {
-  unsigned long long z = (((unsigned long long)i << 32) | j) + seed * 0x9E3779B97F4A7C15ull +
-                         (unsigned long long)step * 0xD1B54A32D192ED03ull;
+// order_hash_base holds what the pairs of one seed and step share.
+__host__ __device__ __forceinline__ unsigned long long order_hash_base(uint32_t step, unsigned long long seed) {
+  return seed * 0x9E3779B97F4A7C15ull + (unsigned long long)step * 0xD1B54A32D192ED03ull;
+}
+__host__ __device__ __forceinline__ unsigned long long order_hash_from(unsigned long long base, uint32_t i, uint32_t j) {
+  unsigned long long z = (((unsigned long long)i << 32) | j) + base;
   z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
   z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
   return z ^ (z >> 31);
+}
+__host__ __device__ __forceinline__ unsigned long long order_hash(uint32_t i, uint32_t j, uint32_t step,
+                                                                  unsigned long long seed) {
+  return order_hash_from(order_hash_base(step, seed), i, j);
 }
 
 // Two uniforms in (-1, 1) for the diffusion kick of particle `p` at step `step`

@@ -161,7 +161,7 @@ class Simulation:
         return best, times
 
     TUNING_KNOBS = {"rounds_threads": (_lib.TUNE_ROUNDS_THREADS, (1024, 512)),
-                    "long_blocks_per_sm": (_lib.TUNE_LONG_BLOCKS_PER_SM, (6, 3, 12)),
+                    "long_blocks_per_sm": (_lib.TUNE_LONG_BLOCKS_PER_SM, (8, 4, 12)),
                     "advect_threads": (_lib.TUNE_ADVECT_THREADS, (256, 128))}
 
     def set_tuning(self, knob: str, value: int) -> None:

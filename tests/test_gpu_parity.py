@@ -154,6 +154,60 @@ def test_gpu_interaction_dense_lists_match_oracle(engine, orc):
     np.testing.assert_array_equal(got, want)
 
 
+def _clumps(rng, sizes, spread, pitch=0.05):
+    """Clumps of the given sizes on a grid of `pitch` degrees, each `spread` across, anywhere against the cells."""
+    lon, lat = [], []
+    for k, m in enumerate(sizes):
+        x, y = 200.0 + pitch * (k % 64) + 0.02 * rng.random(), 25.0 + pitch * (k // 64) + 0.02 * rng.random()
+        lon.append(x + spread * rng.random(m))
+        lat.append(y + spread * rng.random(m))
+    return np.concatenate(lon).astype(np.float32), np.concatenate(lat).astype(np.float32)
+
+
+@pytest.mark.parametrize("p, spread", [(2, 0.007), (1, 0.0049), (np.inf, 0.0099)])
+def test_gpu_long_lists_of_every_form_match_oracle(engine, orc, p, spread):
+    """Lists on both sides of every limit of the long-list kernel: clumps whose members are all one another's
+    neighbours, of 10 to 515 microbes (one pass, several, the shared lists' 96 neighbours and 192 candidates, the
+    shared bucket sort's 512), and short lists beside a crowd just out of reach (few neighbours, many candidates).
+    The species depend on the order of every list."""
+    rng = np.random.default_rng(int(1000 * spread))
+    sizes = [10, 17, 32, 33, 34, 64, 65, 95, 96, 97, 98, 99, 128, 192, 193, 194, 511, 512, 513, 514, 515] + [10, 12, 20, 40] * 20
+    lon, lat = _clumps(rng, sizes, spread)
+    for k, crowd in enumerate((150, 181, 182, 183, 400)):  # 11 microbes, and a crowd in the next cell out of reach
+        x, y = 200.0 + 0.02 * rng.random(), 26.0 + 0.05 * k
+        lon = np.concatenate([lon, (x + 0.0005 * rng.random(11)), (x + 0.0107 + 0.0005 * rng.random(crowd))]).astype(np.float32)
+        lat = np.concatenate([lat, (y + 0.0005 * rng.random(11)), (y + 0.0005 * rng.random(crowd))]).astype(np.float32)
+    sp = rng.integers(0, 5, lon.size).astype(np.int8)
+    probs = (0.6, 0.7, 0.55)
+    got, _, stats = _interact(engine, lon, lat, sp, 0.01, p, probs, 99, 4, log=False)
+    want, m = orc.interact_step(lon, lat, sp, 0.01, p, *probs, 99, 4)
+    assert stats["pairs"] == m >= sum(k * (k - 1) // 2 for k in sizes)
+    np.testing.assert_array_equal(got, want)
+
+
+def test_gpu_long_lists_whose_leading_priority_bits_agree(engine, orc):
+    """400 clumps of 97: lists of 96 pairs, some with two priorities equal in their upper 24 bits (the
+    long-list kernel ranks by those first)."""
+    rng = np.random.default_rng(8)
+    lon, lat = _clumps(rng, [97] * 400, 0.007)
+    sp = rng.integers(1, 4, lon.size).astype(np.int8)
+    seed, step, probs = 4242, 6, (0.6, 0.7, 0.55)
+    ids = np.arange(lon.size).reshape(400, 97)
+    i, j = np.minimum(ids[:, :, None], ids[:, None, :]), np.maximum(ids[:, :, None], ids[:, None, :])
+    u = np.uint64
+    with np.errstate(over="ignore"):
+        z = (i.astype(u) << u(32) | j.astype(u)) + u(seed) * u(0x9E3779B97F4A7C15) + u(step) * u(0xD1B54A32D192ED03)
+        z = (z ^ z >> u(30)) * u(0xBF58476D1CE4E5B9)
+        z = (z ^ z >> u(27)) * u(0x94D049BB133111EB)
+        z ^= z >> u(31)
+    top = np.sort((z >> u(40))[:, ~np.eye(97, dtype=bool)].reshape(400, 97, 96), axis=-1)
+    assert np.any(top[..., 1:] == top[..., :-1])
+    got, _, stats = _interact(engine, lon, lat, sp, 0.01, 2, probs, seed, step, log=False)
+    want, m = orc.interact_step(lon, lat, sp, 0.01, 2, *probs, seed, step)
+    assert stats["pairs"] == m == 400 * 97 * 96 // 2
+    np.testing.assert_array_equal(got, want)
+
+
 def test_gpu_interaction_other_species_values_unchanged(engine, orc):
     rng = np.random.default_rng(3)
     n = 2000
