@@ -624,55 +624,6 @@ void launch_count_pairs(const Bufs& b, const PairParams& pp, Ctrl* ctrl, int sms
   launch_dep(k_count_pairs, dim3(blocks), dim3(COUNT_THREADS), st, b, pp, ctrl);
 }
 
-// In-place sort of one long list (priorities pr, list entries nb) into `before` order.
-__device__ void sort_segment(unsigned long long* __restrict__ pr, uint32_t* __restrict__ nb,
-                             const uint32_t* __restrict__ sid, uint32_t d) {
-  if (d <= 64) {
-    for (uint32_t x = 1; x < d; ++x) {
-      const unsigned long long p = pr[x];
-      const uint32_t t = nb[x], it = sid[entry_id(t)];
-      uint32_t y = x;
-      while (y > 0) {
-        const unsigned long long q = pr[y - 1];
-        const uint32_t u = nb[y - 1];
-        if (!before(p, it, q, sid[entry_id(u)])) break;
-        pr[y] = q;
-        nb[y] = u;
-        --y;
-      }
-      pr[y] = p;
-      nb[y] = t;
-    }
-    return;
-  }
-  // heap sort for long lists: the heap's root is the element that comes last
-  auto sift = [&](uint32_t root, uint32_t len) {
-    while (true) {
-      uint32_t c = 2 * root + 1;
-      if (c >= len) break;
-      if (c + 1 < len && before(pr[c], sid[entry_id(nb[c])], pr[c + 1], sid[entry_id(nb[c + 1])])) ++c;
-      if (!before(pr[root], sid[entry_id(nb[root])], pr[c], sid[entry_id(nb[c])])) break;
-      const unsigned long long tp = pr[root];
-      pr[root] = pr[c];
-      pr[c] = tp;
-      const uint32_t tn = nb[root];
-      nb[root] = nb[c];
-      nb[c] = tn;
-      root = c;
-    }
-  };
-  for (uint32_t r = d / 2; r-- > 0;) sift(r, d);
-  for (uint32_t end = d - 1; end > 0; --end) {
-    const unsigned long long tp = pr[0];
-    pr[0] = pr[end];
-    pr[end] = tp;
-    const uint32_t tn = nb[0];
-    nb[0] = nb[end];
-    nb[end] = tn;
-    sift(0, end);
-  }
-}
-
 // Long lists (more than SLAB neighbours). A warp takes batches of up to 32 of them, consecutive in cell
 // order; lane k loads vertex k's cell, position, key runs and ensemble constants, so the dependent loads
 // happen once per batch, and one atomic reserves the overflow space of all its batches. Then:
@@ -688,19 +639,23 @@ __device__ void sort_segment(unsigned long long* __restrict__ pr, uint32_t* __re
 // Members with more than LONG_FEW neighbours or LONG_CAND candidates are done one at a time (long_alone):
 // candidates from global memory, 64 a pass, and up to LONG_SMEM_MAX entries a bucket sort: the priorities
 // are uniform hashes, so 256 buckets on their top 8 bits (descending) hold about d / 256 entries each, and
-// an insertion sort inside each bucket by the exact order finishes it; beyond, a sort in global memory by
-// one lane. Only the sorted partners are kept (the priorities were needed for the order only).
+// an insertion sort inside each bucket by the exact order finishes it; beyond, buckets in global memory.
+// Only the sorted partners are kept (the priorities were needed for the order only).
 // Bound by instruction issue (73 % of the slots, 670 instructions a list of 34). A warp per list before
 // took 530 us for the 447,000 lists of 32 ensembles, 245 for the 338,000 of 2,000,000 mixed microbes and 66
-// for the 81,000 of 490,000; this takes 376, 146 and 43. At 6 blocks an SM (9 KB a warp) it took 438, 194, 54.
+// for the 81,000 of 490,000; this takes 368, 144 and 42. At 6 blocks an SM (9 KB a warp) it took 438,
+// 194 and 54. Lists done alone: 1,100 neighbours each 21.4 -> 1.4 ms for 10,000 microbes (one lane sorted them
+// before); 210 each 0.15 -> 0.21 for 30,000, of 2.1 ms a step.
 constexpr int LONG_WARPS = 4;
 constexpr uint32_t LONG_SMEM_MAX = 512;
 constexpr uint32_t LONG_BUCKETS = 256;
 
-struct LongSmem {  // (the priorities stay in the list's part of oprio)
-  uint32_t t[LONG_SMEM_MAX];            // list entry (partner's cell-order index + outcome bits)
-  uint16_t ord[LONG_SMEM_MAX];          // entries in list order
-  uint32_t start[LONG_BUCKETS], cur[LONG_BUCKETS];
+struct LongSmem {
+  uint32_t key[LONG_SMEM_MAX];  // partner's local id, then the upper half of the pair's priority (gather order)
+  uint32_t t[LONG_SMEM_MAX];    // list entry (partner's cell-order index + outcome bits)
+  uint32_t cur[LONG_BUCKETS];
+  uint16_t ord[LONG_SMEM_MAX];  // entries in list order
+  uint16_t start[LONG_BUCKETS];
 };
 
 // What a warp keeps of a batch: its members, the candidates of the cell at hand and the area of lists.
@@ -728,26 +683,28 @@ union LongShared {
   LongArea many;
 };
 
-// Does entry x come before entry y? Ties of the 64-bit priority (rare) go by the partner's local id.
-__device__ __forceinline__ bool long_before(const Bufs& b, const LongSmem& sh, const unsigned long long* p, uint32_t base,
-                                            uint32_t x, uint32_t y) {
-  const unsigned long long px = p[x], py = p[y];
-  if (px != py) return px > py;
-  return b.sid[entry_id(sh.t[x])] - base < b.sid[entry_id(sh.t[y])] - base;
+// A list that is done alone: what its pairs' priorities need.
+struct LongHead {
+  unsigned long long hash;  // order_hash_base
+  uint32_t la, base;
+};
+
+// Does the pair with upper priority half x and entry ex come before (y, ey)? Equal halves go by the whole priority.
+__device__ __forceinline__ bool long_before(const Bufs& b, const LongHead& h, uint32_t x, uint32_t ex, uint32_t y,
+                                            uint32_t ey) {
+  if (x != y) return x > y;
+  const uint32_t lx = b.sid[entry_id(ex)] - h.base, ly = b.sid[entry_id(ey)] - h.base;
+  return before(order_hash_from(h.hash, min(h.la, lx), max(h.la, lx)), lx,
+                order_hash_from(h.hash, min(h.la, ly), max(h.la, ly)), ly);
 }
 
-// The bucket sort of entries [0, d) of sh into sh.ord (one warp).
-__device__ __forceinline__ void long_sort(const Bufs& b, LongSmem& sh, const unsigned long long* p, uint32_t base, uint32_t d,
-                                          uint32_t lane) {
-  for (uint32_t i = lane; i < LONG_BUCKETS; i += 32) sh.cur[i] = 0;
-  __syncwarp();
-  for (uint32_t i = lane; i < d; i += 32) atomicAdd(&sh.cur[255u - (uint32_t)(p[i] >> 56)], 1u);
-  __syncwarp();
-  // exclusive scan of the bucket counts: lane holds buckets 8 lane .. 8 lane + 7
-  uint32_t c[8], tot = 0;
+// Exclusive scan of the counts in cur; start gets the result as well.
+template <class T>
+__device__ __forceinline__ void long_scan(uint32_t* cur, T* start, uint32_t lane) {
+  uint32_t c[8], tot = 0;  // lane holds buckets 8 lane .. 8 lane + 7
 #pragma unroll
   for (int r = 0; r < 8; ++r) {
-    c[r] = sh.cur[8 * lane + r];
+    c[r] = cur[8 * lane + r];
     tot += c[r];
   }
   uint32_t incl = tot;
@@ -758,20 +715,28 @@ __device__ __forceinline__ void long_sort(const Bufs& b, LongSmem& sh, const uns
   uint32_t run = incl - tot;
 #pragma unroll
   for (int r = 0; r < 8; ++r) {
-    sh.start[8 * lane + r] = run;
-    sh.cur[8 * lane + r] = run;
+    start[8 * lane + r] = (T)run;
+    cur[8 * lane + r] = run;
     run += c[r];
   }
+}
+
+// The bucket sort of entries [0, d) of sh into sh.ord (one warp).
+__device__ __forceinline__ void long_sort(const Bufs& b, LongSmem& sh, const LongHead& h, uint32_t d, uint32_t lane) {
+  for (uint32_t i = lane; i < LONG_BUCKETS; i += 32) sh.cur[i] = 0;
   __syncwarp();
-  for (uint32_t i = lane; i < d; i += 32)
-    sh.ord[atomicAdd(&sh.cur[255u - (uint32_t)(p[i] >> 56)], 1u)] = (uint16_t)i;
+  for (uint32_t i = lane; i < d; i += 32) atomicAdd(&sh.cur[255u - (sh.key[i] >> 24)], 1u);
+  __syncwarp();
+  long_scan(sh.cur, sh.start, lane);
+  __syncwarp();
+  for (uint32_t i = lane; i < d; i += 32) sh.ord[atomicAdd(&sh.cur[255u - (sh.key[i] >> 24)], 1u)] = (uint16_t)i;
   __syncwarp();
   for (uint32_t k = lane; k < LONG_BUCKETS; k += 32) {
     const uint32_t lo = sh.start[k], hi = sh.cur[k];
     for (uint32_t x = lo + 1; x < hi; ++x) {
       const uint16_t e = sh.ord[x];
       uint32_t y = x;
-      while (y > lo && long_before(b, sh, p, base, e, sh.ord[y - 1])) {
+      while (y > lo && long_before(b, h, sh.key[e], sh.t[e], sh.key[sh.ord[y - 1]], sh.t[sh.ord[y - 1]])) {
         sh.ord[y] = sh.ord[y - 1];
         --y;
       }
@@ -781,89 +746,142 @@ __device__ __forceinline__ void long_sort(const Bufs& b, LongSmem& sh, const uns
   __syncwarp();
 }
 
-// One list by the whole warp, candidates from global memory.
+// The same in global memory for the d words w = upper priority half << 32 | entry; the entries in order go to nb. Each
+// entry's place in its bucket is the number of members before it. nb first holds the words' indices by bucket (20
+// bits) with those places above them; the upper halves of w, free by then, take the entries at their places. Lists
+// that this does not hold (2^20 entries, or 4,096 in a bucket) are put in order by one lane's heap instead.
+__device__ __forceinline__ void long_sort_global(const Bufs& b, LongSmem& sh, const LongHead& h, unsigned long long* w,
+                                                 uint32_t* nb, uint32_t d, uint32_t lane) {
+  constexpr uint32_t IDX_BITS = 20, IDX = (1u << IDX_BITS) - 1u, MOST = (1u << (32 - IDX_BITS)) - 1u;
+  uint32_t* start = sh.key;
+  auto first = [&](uint32_t i, uint32_t j) {  // word i before word j?
+    const unsigned long long x = w[i], y = w[j];
+    return long_before(b, h, (uint32_t)(x >> 32), (uint32_t)x, (uint32_t)(y >> 32), (uint32_t)y);
+  };
+  for (uint32_t i = lane; i < LONG_BUCKETS; i += 32) sh.cur[i] = 0;
+  __syncwarp();
+  for (uint32_t i = lane; i < d; i += 32) atomicAdd(&sh.cur[255u - (uint32_t)(w[i] >> 56)], 1u);
+  __syncwarp();
+  long_scan(sh.cur, start, lane);
+  __syncwarp();
+  for (uint32_t i = lane; i < d; i += 32) nb[atomicAdd(&sh.cur[255u - (uint32_t)(w[i] >> 56)], 1u)] = i;
+  __syncwarp();
+  bool large = d > IDX;
+  for (uint32_t k = lane; k < LONG_BUCKETS; k += 32) large |= sh.cur[k] - start[k] > MOST;
+  if (__any_sync(0xffffffffu, large)) {
+    if (lane == 0) {  // heap sort of the indices: the root comes last
+      auto sift = [&](uint32_t root, uint32_t len) {
+        for (uint32_t c = 2 * root + 1; c < len; c = 2 * root + 1) {
+          if (c + 1 < len && first(nb[c], nb[c + 1])) ++c;
+          if (!first(nb[root], nb[c])) break;
+          const uint32_t x = nb[root];
+          nb[root] = nb[c];
+          nb[c] = x;
+          root = c;
+        }
+      };
+      for (uint32_t r = d / 2; r-- > 0;) sift(r, d);
+      for (uint32_t end = d - 1; end > 0; --end) {
+        const uint32_t x = nb[0];
+        nb[0] = nb[end];
+        nb[end] = x;
+        sift(0, end);
+      }
+    }
+    __syncwarp();
+    for (uint32_t i = lane; i < d; i += 32) nb[i] = (uint32_t)w[nb[i]];
+    __syncwarp();
+    return;
+  }
+  for (uint32_t x = lane; x < d; x += 32) {
+    const uint32_t i = nb[x] & IDX, k = 255u - (uint32_t)(w[i] >> 56);
+    uint32_t place = 0;
+    for (uint32_t y = start[k]; y < sh.cur[k]; ++y) {
+      const uint32_t j = ((volatile uint32_t*)nb)[y] & IDX;  // (another lane may be adding its place)
+      place += j != i && first(j, i) ? 1u : 0u;
+    }
+    ((volatile uint32_t*)nb)[x] = i | place << IDX_BITS;
+  }
+  __syncwarp();
+  for (uint32_t k = 0, x = lane; x < d; x += 32) {
+    const uint32_t i = nb[x] & IDX;
+    while (sh.cur[k] <= x) ++k;  // the bucket of place x (its words' upper halves may be overwritten by now)
+    reinterpret_cast<uint32_t*>(w + start[k] + (nb[x] >> IDX_BITS))[1] = reinterpret_cast<const uint32_t*>(w + i)[0];
+  }
+  __syncwarp();
+  for (uint32_t i = lane; i < d; i += 32) nb[i] = reinterpret_cast<const uint32_t*>(w + i)[1];
+  __syncwarp();
+}
+
+// One list by the whole warp, candidates from global memory: candidate i is in the run q with c[q] <= i < c[q + 1],
+// which starts at t0[q].
 __device__ __noinline__ void long_alone(const Bufs& b, const PairParams& pp, uint32_t step, LongSmem& sh, uint32_t s,
-                                        uint32_t d, unsigned long long o) {
+                                        uint32_t d, unsigned long long o, const uint32_t* t0, const uint32_t* c) {
   const uint32_t lane = threadIdx.x & 31u;
-  const Vertex v = load_vertex(b, s);
-  const EnsInfo& info = b.ens[v.e];
-  const uint32_t id0 = b.sid[s], la = id0 - v.base, base = v.base, k0 = info.seed_lo, k1 = info.seed_hi;
+  const uint32_t id0 = b.sid[s];
+  const EnsInfo& info = b.ens[b.sens[s]];
+  const LongHead h = {order_hash_base(step, ((unsigned long long)info.seed_hi << 32) | info.seed_lo), id0 - info.base,
+                      info.base};
   const int sp = b.species[id0];
-  const float2 ps = v.ps;
-  uint32_t t0[6], t1[6], c[7];
-  neighbour_runs(b, v, t0, t1);
-  // the six runs as one candidate range: candidate i is in the run q with c[q] <= i < c[q + 1]
-  c[0] = 0;
-#pragma unroll
-  for (int q = 0; q < 6; ++q) c[q + 1] = c[q] + (t1[q] - t0[q]);
+  const float2 ps = b.spos[s];
   const bool in_smem = d <= LONG_SMEM_MAX;
   uint32_t m = 0;
-  // two slices of 32 candidates per pass, each candidate's position and id loaded together
+  // two slices of 32 candidates per pass
   for (uint32_t tb = 0; tb < c[6]; tb += 64) {
-    uint32_t t[2], id[2];
+    uint32_t t[2];
     float2 pt[2];
     bool in[2];
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const uint32_t i = tb + 32u * h + lane;
+    for (int r = 0; r < 2; ++r) {
+      const uint32_t i = tb + 32u * r + lane;
       uint32_t x = t0[0] + i;
 #pragma unroll
       for (int q = 1; q < 6; ++q)
         if (i >= c[q]) x = t0[q] + (i - c[q]);  // the last run starting at or before i (empty runs never win)
-      t[h] = x;
-      in[h] = i < c[6] && x != s;
-      pt[h] = in[h] ? b.spos[x] : ps;
-      id[h] = in[h] ? b.sid[x] : 0u;
+      t[r] = x;
+      in[r] = i < c[6] && x != s;
+      pt[r] = in[r] ? b.spos[x] : ps;
     }
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const bool ok = in[h] && within(pp, ps, pt[h]);
+    for (int r = 0; r < 2; ++r) {
+      const bool ok = in[r] && within(pp, ps, pt[r]);
       const uint32_t mask = __ballot_sync(0xffffffffu, ok);
-      if (ok) {
-        const uint32_t pos = m + __popc(mask & lanemask_lt_p());
-        if (pos < d) {  // the partner and its local id; priority and draw follow below
-          if (in_smem)
-            sh.t[pos] = t[h];
-          else
-            b.ovf[o + pos] = t[h];
-          b.oprio[o + pos] = id[h] - base;
-        }
+      const uint32_t pos = m + __popc(mask & lanemask_lt_p());
+      if (ok && pos < d) {
+        if (in_smem)
+          sh.t[pos] = t[r];
+        else
+          b.ovf[o + pos] = t[r];
       }
       m += __popc(mask);
     }
   }
-  // priorities and outcome draws of the d entries, one entry per lane (in the gather only the
-  // lanes that found a neighbour would work, about a third of them)
   __syncwarp();
+  // priorities and outcome draws of the d entries, one entry per lane
   for (uint32_t i = lane; i < d; i += 32) {
-    const uint32_t tt = in_smem ? sh.t[i] : b.ovf[o + i];
-    const uint32_t lb = (uint32_t)b.oprio[o + i];
-    const unsigned long long p = pair_prio(min(la, lb), max(la, lb), step, k0, k1);
-    const uint32_t e = tt > s ? tt | win_bits(info, la, lb, step) : tt;
-    if (in_smem)
+    const uint32_t t = in_smem ? sh.t[i] : b.ovf[o + i], lb = b.sid[t] - h.base;
+    const uint32_t hi = (uint32_t)(order_hash_from(h.hash, min(h.la, lb), max(h.la, lb)) >> 32);
+    const uint32_t e = t > s ? t | win_bits(info, h.la, lb, step) : t;
+    if (in_smem) {
+      sh.key[i] = hi;
       sh.t[i] = e;
-    else
-      b.ovf[o + i] = e;
-    b.oprio[o + i] = p;
+    } else {
+      b.oprio[o + i] = (unsigned long long)hi << 32 | e;
+    }
   }
-  uint32_t first;
+  __syncwarp();
   if (in_smem) {
-    __syncwarp();
-    long_sort(b, sh, b.oprio + o, base, d, lane);
+    long_sort(b, sh, h, d, lane);
     for (uint32_t i = lane; i < d; i += 32) b.ovf[o + i] = sh.t[sh.ord[i]];
-    first = sh.t[sh.ord[0]];
-    __syncwarp();  // the next vertex reuses the shared list
   } else {
-    __syncwarp();
-    if (lane == 0) sort_segment(b.oprio + o, b.ovf + o, b.sid, d);
-    __syncwarp();
-    first = b.ovf[o];
+    long_sort_global(b, sh, h, b.oprio + o, b.ovf + o, d, lane);
   }
   if (lane == 0) {
     b.ovf[o + d] = NONE;
     b.slab[(size_t)s * SLAB] = (uint32_t)o;  // a long list's overflow offset, in its unused slab row
-    b.wstate[s] = pack_state(first, 0u, sp);  // entry 0 of the list
+    b.wstate[s] = pack_state(in_smem ? sh.t[sh.ord[0]] : b.ovf[o], 0u, sp);  // entry 0 of the list
   }
+  __syncwarp();  // the next list reuses the shared memory
 }
 
 // Entry i of the area at place k of its list; the first one also makes its member ready.
@@ -965,11 +983,15 @@ __global__ void __launch_bounds__(LONG_WARPS * 32, 8) k_sweep_long(Bufs b, PairP
   // batches of `per` vertices, the same number for every warp as nearly as can be: this warp's are gw, gw + nw, ...
   if (n_long == 0) return;
   const uint32_t turns = (n_long + 32u * nw - 1) / (32u * nw), per = (n_long + turns * nw - 1) / (turns * nw);
+  // where most lists are done one at a time, a warp's are spread over all of them instead: the longest lie together
+  // (10,000 microbes with 1,100 neighbours each, ordered by one lane: 29 ms a step in order, 22 spread)
+  const bool spread = ctrl->n_dir > (unsigned long long)LONG_FEW * n_long;
+  const uint32_t first = spread ? gw : gw * per, next = spread ? nw : 1u, turn = nw * per;
   unsigned long long sum = 0;
   bool too_many = false;
-  for (uint32_t q = gw * per; q < n_long; q += nw * per) {
-    if (lane >= per || q + lane >= n_long) continue;
-    const uint32_t d = b.deg[b.longv[q + lane]];
+  for (uint32_t q = first; q < n_long; q += turn) {
+    if (lane >= per || q + lane * next >= n_long) continue;
+    const uint32_t d = b.deg[b.longv[q + lane * next]];
     sum += d + 1u;  // the list and its end mark
     too_many |= d > MAX_DEGREE;
   }
@@ -987,11 +1009,11 @@ __global__ void __launch_bounds__(LONG_WARPS * 32, 8) k_sweep_long(Bufs b, PairP
     }
     return;
   }
-  for (uint32_t q = gw * per; q < n_long; q += nw * per) {
+  for (uint32_t q = first; q < n_long; q += turn) {
     // lane k loads member k's cell, position, key runs and ensemble constants: a chain of dependent loads per batch
-    const uint32_t nk = min(per, n_long - q);
-    const bool mine = lane < nk;
-    const uint32_t s_l = mine ? b.longv[q + lane] : 0u;
+    const bool mine = lane < per && q + lane * next < n_long;
+    const uint32_t nk = __popc(__ballot_sync(0xffffffffu, mine));  // (the first nk lanes)
+    const uint32_t s_l = mine ? b.longv[q + lane * next] : 0u;
     const uint32_t d_l = mine ? b.deg[s_l] : 0u;
     const uint32_t room_l = mine ? d_l + 1u : 0u;
     unsigned long long incl = room_l;
@@ -1017,8 +1039,15 @@ __global__ void __launch_bounds__(LONG_WARPS * 32, 8) k_sweep_long(Bufs b, PairP
     const uint32_t large = __ballot_sync(0xffffffffu, d_l > LONG_FEW || cand > LONG_CAND);
     for (uint32_t m = large; m; m &= m - 1) {  // one at a time, in the same shared memory
       const int k = __ffs(m) - 1;
+      uint32_t t0[6], c[7];
+      c[0] = 0;
+#pragma unroll
+      for (int r = 0; r < 6; ++r) {
+        t0[r] = __shfl_sync(0xffffffffu, r0[r], k);
+        c[r + 1] = c[r] + __shfl_sync(0xffffffffu, len[r], k);
+      }
       long_alone(b, pp, step, sh_all[w].one, __shfl_sync(0xffffffffu, s_l, k), __shfl_sync(0xffffffffu, d_l, k),
-                 __shfl_sync(0xffffffffu, o_l, k));
+                 __shfl_sync(0xffffffffu, o_l, k), t0, c);
     }
     if (mine) {
       const uint32_t id = b.sid[s_l], e = b.sens[s_l];
