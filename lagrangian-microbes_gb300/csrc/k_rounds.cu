@@ -26,9 +26,10 @@
 // always ready, so the loop always progresses; every wait is still bounded (error flag + return
 // after a timeout).
 //
-// When every block can own its share of the vertices in shared memory (up to 2,048 each), the
-// pairs are applied by the tile-local path (rounds_tiled): handshakes between vertices of one
-// block go through shared memory and only pairs crossing blocks through global memory.
+// When every block can own its share of the vertices in shared memory (up to 2,048 each with their
+// lists, up to 12,288 with their state words only), the pairs are applied by the tile-local path
+// (rounds_tiled): handshakes between vertices of one block go through shared memory and only pairs
+// crossing blocks through global memory.
 //
 // In pair-log runs each applied pair also gets a level = 1 + max(level of the previous pair at
 // either endpoint): pairs of one level share no microbe, and (level, i, j) is a deterministic
@@ -251,7 +252,86 @@ __device__ void tl_group(const Bufs& b, uint32_t step, Ctrl* ctrl, unsigned long
   }
 }
 
-// Returns false (nothing done) when the step does not fit the tile path (grid-uniform).
+// The same for groups of up to WIDE_VMAX vertices per block: only the state words fit in shared memory, the lists
+// stay in global memory (L2 holds those of 2,000,000 microbes) and a thread polls up to 12 of its vertices in turn.
+// Taken when an ensemble does not fit tl_group's blocks (some 622,000 microbes) and fits these (3,700,000). Bound by
+// the polls' latency. Against the form on global words: 650,000 mixed microbes 204 -> 120 us, 2,000,000 439 -> 262,
+// 3,000,000 722 -> 403, a lattice of 1,200,000 129 -> 120. Keeping each vertex's next entry beside its word too (12
+// bytes a vertex) took 309 us at 2,000,000, staying on a vertex after a pair 264.
+constexpr uint32_t WIDE_VMAX = (uint32_t)(TL_SMEM / sizeof(unsigned long long));
+
+// Entry h > 0 of vertex s's list (NONE past the end); the length and the slab entry are loaded together.
+__device__ __forceinline__ uint32_t wide_entry(const Bufs& b, uint32_t s, uint32_t h) {
+  const uint32_t* row = b.slab + (size_t)s * SLAB;
+  const uint32_t d = b.deg[s], e = row[h & (SLAB - 1u)];
+  if (h >= d) return NONE;
+  return d <= SLAB ? e : b.ovf[(size_t)row[0] + h];
+}
+
+template <int RD_THREADS>
+__device__ void tl_wide(const Bufs& b, Ctrl* ctrl, unsigned long long t0, uint32_t g_lo, uint32_t g_hi) {
+  extern __shared__ unsigned long long tl_raw[];
+  static_assert(WIDE_VMAX / RD_THREADS <= 32u, "a thread's live vertices are the bits of a word");
+  const uint32_t n_g = g_hi - g_lo;
+  const uint32_t V = min(WIDE_VMAX, max(32u, (((n_g + gridDim.x - 1) / gridDim.x) + 31u) & ~31u));
+  const uint32_t lo = min(g_hi, g_lo + blockIdx.x * V);
+  const uint32_t hi = min(g_hi, lo + V);
+  const uint32_t nloc = hi - lo;
+  uint32_t live = 0;
+  for (uint32_t k = 0, l = threadIdx.x; l < nloc; ++k, l += RD_THREADS) {
+    const unsigned long long w = ld_relaxed(b.wstate + lo + l);
+    tl_raw[l] = w;
+    if (state_partner(w) != NONE) live |= 1u << k;
+  }
+  __syncthreads();
+  uint32_t polls = 0;
+  while (live) {
+    for (uint32_t m = live; m; m &= m - 1u) {
+      const uint32_t k = (uint32_t)__ffs(m) - 1u, l = threadIdx.x + k * RD_THREADS, s = lo + l;
+      const unsigned long long ws = ld_sh(tl_raw + l);
+      const uint32_t ue = state_partner(ws);
+      if (ue == NONE) {
+        live &= ~(1u << k);
+        continue;
+      }
+      const uint32_t u = entry_id(ue);
+      const bool u_local = u >= lo && u < hi;
+      if (s > u) {  // the owner of u applies (see tl_group)
+        if (!u_local) {
+          const unsigned long long g = ld_relaxed(b.wstate + s);
+          if (state_pos(g) > state_pos(ws)) st_sh(tl_raw + l, g);
+        }
+        continue;
+      }
+      const unsigned long long wu = u_local ? ld_sh(tl_raw + (u - lo)) : ld_relaxed(b.wstate + u);
+      if (state_partner(wu) != s) continue;
+      const uint32_t hs = state_pos(ws), hu = state_pos(wu);
+      const uint32_t ns = wide_entry(b, s, hs + 1u), nu = wide_entry(b, u, hu + 1u);
+      const int o = rps_outcome(state_species(ws), state_species(wu), ue);
+      const int new_s = o < 0 ? state_species(ws) : o, new_u = o < 0 ? state_species(wu) : o;
+      const unsigned long long nwu = pack_state(nu, hu + 1u, new_u), nws = pack_state(ns, hs + 1u, new_s);
+      const uint32_t nu_id = entry_id(nu), ns_id = entry_id(ns);
+      if (u_local) {
+        st_sh(tl_raw + (u - lo), nwu);
+        if (nu != NONE && (nu_id < lo || nu_id >= hi)) st_relaxed(b.wstate + u, nwu);
+      } else {
+        st_relaxed(b.wstate + u, nwu);
+      }
+      st_sh(tl_raw + l, nws);
+      if (ns != NONE && (ns_id < lo || ns_id >= hi)) st_relaxed(b.wstate + s, nws);
+    }
+    if (live && ((++polls & 63u) == 0u) && globaltimer() - t0 > ROUNDS_TIMEOUT_NS) {
+      atomicOr(&ctrl->err, (uint32_t)ERRB_TIMEOUT);
+      break;
+    }
+  }
+  for (uint32_t l = threadIdx.x; l < nloc; l += RD_THREADS) {
+    const unsigned long long w = ld_sh(tl_raw + l);
+    if (state_pos(w)) b.species[b.sid[lo + l]] = (int8_t)state_species(w);  // (it had pairs)
+  }
+}
+
+// Returns false (nothing done) when the step does not fit the tile paths (grid-uniform).
 template <int RD_THREADS>
 __device__ bool rounds_tiled(const Bufs& b, uint32_t step, Ctrl* ctrl, unsigned long long t0, uint32_t n_valid) {
   if (b.plog) return false;
@@ -259,8 +339,18 @@ __device__ bool rounds_tiled(const Bufs& b, uint32_t step, Ctrl* ctrl, unsigned 
   __shared__ TileGroups tg;
   make_groups(b, n_valid, gridDim.x * TL_VMAX, reinterpret_cast<uint32_t*>(tl_raw), (uint32_t)(TL_SMEM / sizeof(uint32_t)),
               tg);
-  const int groups = tg.n;
-  if (groups <= 0) return false;
+  int groups = tg.n;
+  if (groups <= 0) {  // an ensemble larger than the blocks' lists
+    __syncthreads();  // (every thread has read tg.n)
+    make_groups(b, n_valid, gridDim.x * WIDE_VMAX, reinterpret_cast<uint32_t*>(tl_raw), (uint32_t)(TL_SMEM / sizeof(uint32_t)),
+                tg);
+    groups = tg.n;
+    for (int g = 0; g < groups; ++g) {
+      tl_wide<RD_THREADS>(b, ctrl, t0, tg.lo[g], tg.lo[g + 1]);
+      __syncthreads();
+    }
+    return groups > 0;
+  }
   for (int g = 0; g < groups; ++g) {
     tl_group<RD_THREADS>(b, step, ctrl, t0, tg.lo[g], tg.lo[g + 1]);
     __syncthreads();  // the block's shared lists are reused by the next group

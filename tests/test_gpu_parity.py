@@ -208,6 +208,22 @@ def test_gpu_long_lists_whose_leading_priority_bits_agree(engine, orc):
     np.testing.assert_array_equal(got, want)
 
 
+@pytest.mark.parametrize("n, dense", [(640000, 0), (700001, 30000)])
+def test_gpu_interaction_beyond_the_blocks_lists_matches_oracle(engine, orc, n, dense):
+    """One ensemble larger than the lists that the blocks hold in shared memory (304 x 2,048 microbes): state words
+    there, lists in global memory; `dense` microbes have long lists. A logged run takes the form without blocks."""
+    rng = np.random.default_rng(n)
+    lon = np.concatenate([200 + rng.random(n - dense) * 4.0, 201 + rng.random(dense) * 0.3]).astype(np.float32)
+    lat = np.concatenate([25 + rng.random(n - dense) * 4.0, 26 + rng.random(dense) * 0.3]).astype(np.float32)
+    sp = rng.integers(0, 5, n).astype(np.int8)
+    probs = (0.6, 0.7, 0.55)
+    want, m = orc.interact_step(lon, lat, sp, 0.01, 2, *probs, 1234, 7)
+    for log in (False,) if dense else (False, True):  # (the pair log does not hold the dense one's pairs)
+        got, _, stats = _interact(engine, lon, lat, sp, 0.01, 2, probs, 1234, 7, log=log)
+        assert stats["pairs"] == m
+        np.testing.assert_array_equal(got, want)
+
+
 def test_gpu_interaction_other_species_values_unchanged(engine, orc):
     rng = np.random.default_rng(3)
     n = 2000
