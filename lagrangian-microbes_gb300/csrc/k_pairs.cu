@@ -11,9 +11,9 @@
 // One thread per particle (cell order) scans the three rows of its 3x3 cell neighbourhood; the
 // three cells of a row are consecutive keys, hence one contiguous run of the sorted array. Each
 // neighbour list is kept sorted by descending pair priority, the order in which the interaction
-// applies pairs: lists of up to SLAB entries are gathered in registers, sorted by a sorting network and stored in
-// the per-vertex slab; longer lists are rebuilt by a second kernel into a per-step overflow
-// area (allocated with an atomic cursor, regrown by the host on overflow) and sorted there.
+// applies pairs: lists of up to SLAB entries are gathered and ranked by k_sweep and stored in the
+// per-vertex slab; longer lists are rebuilt by a second kernel into a per-step overflow area
+// (allocated with an atomic cursor, regrown by the host on overflow) and put in order there.
 //
 // Pair priority: a 64-bit order hash of (seed, step, i, j) (the output function of SplitMix64, a
 // bijection of its input, so no two pairs of a step share a priority). Any fixed order is a valid
@@ -102,51 +102,25 @@ __device__ __forceinline__ Vertex load_vertex(const Bufs& b, uint32_t s) {
   return v;
 }
 
-// Calls f(t) for every cell-order index t != s within the radius of vertex v (in no particular
-// order). The key runs of the three rows (at most two each) are found first and all their cell
-// starts loaded together, so a microbe waits for one round of those loads instead of one per row.
-// (Walking the runs four candidates at a time as well needed 58 registers and was slower.)
-// The cell-order ranges [t0[k], t1[k]) of the (at most six) key runs of v's 3x3 neighbourhood,
-// all cell starts loaded together; missing runs are empty.
+// The cell-order ranges [t0[k], t1[k]) of the (at most six) key runs of v's 3x3 neighbourhood, all cell starts loaded
+// together, so a microbe waits for one round of those loads; missing runs are empty. A cell's key is a row's part
+// plus a column's part, so the columns (and whether they straddle a tile edge) are worked out once for the three rows.
 __device__ __forceinline__ void neighbour_runs(const Bufs& b, const Vertex& v, uint32_t* t0, uint32_t* t1) {
-  uint32_t klo[6], khi[6];
-  bool has[6];
+  const uint32_t sh = v.g.tshift, mask = (1u << sh) - 1u, ntx = tiles_x(v.g);
+  const uint32_t x0 = v.cx ? v.cx - 1u : 0u, x1 = min(v.cx + 1u, (uint32_t)v.g.ncx - 1u);
+  const bool two = (x0 >> sh) != (x1 >> sh);
+  const uint32_t lo = ((x0 >> sh) << (2u * sh)) + (x0 & mask), hi = ((x1 >> sh) << (2u * sh)) + (x1 & mask);
+  const uint32_t lo_end = two ? lo | mask : hi, hi_start = hi & ~mask;  // the edge lies between them
 #pragma unroll
-  for (int dy = -1; dy <= 1; ++dy) {
-    const int ry = (int)v.cy + dy;
+  for (int r = 0; r < 3; ++r) {
+    const int ry = (int)v.cy + r - 1;
     const bool row = ry >= 0 && ry < v.g.ncy;
-    const RowRuns rr = row_runs(v.g, max((int)v.cx - 1, 0), min((int)v.cx + 1, v.g.ncx - 1), row ? ry : (int)v.cy);
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      has[(dy + 1) * 2 + q] = row && q < rr.n;
-      klo[(dy + 1) * 2 + q] = rr.lo[q];
-      khi[(dy + 1) * 2 + q] = rr.hi[q];
-    }
-  }
-#pragma unroll
-  for (int k = 0; k < 6; ++k) {
-    t0[k] = has[k] ? b.cstart[klo[k]] : 0u;
-    t1[k] = has[k] ? b.cstart[khi[k] + 1] : 0u;
-  }
-}
-
-// The six runs are walked as one candidate range (candidate i lies in the run q with
-// c[q] <= i < c[q + 1]), so a warp's loop lasts as long as its longest total, not the sum of its
-// longest run of each row.
-template <class F>
-__device__ __forceinline__ void for_neighbours(const Bufs& b, const PairParams& pp, const Vertex& v, F&& f) {
-  uint32_t t0[6], t1[6];
-  neighbour_runs(b, v, t0, t1);
-  uint32_t c[7];
-  c[0] = 0;
-#pragma unroll
-  for (int q = 0; q < 6; ++q) c[q + 1] = c[q] + (t1[q] - t0[q]);
-  for (uint32_t i = 0; i < c[6]; ++i) {
-    uint32_t t = t0[0] + i;
-#pragma unroll
-    for (int q = 1; q < 6; ++q)
-      if (i >= c[q]) t = t0[q] + (i - c[q]);  // the last run starting at or before i (empty runs never win)
-    if (t != v.s && within(pp, v.ps, b.spos[t])) f(t);
+    const uint32_t y = (uint32_t)(row ? ry : (int)v.cy);
+    const uint32_t* c = b.cstart + v.g.cell_base + ((((y >> sh) * ntx) << (2u * sh)) + ((y & mask) << sh));
+    t0[2 * r] = row ? c[lo] : 0u;
+    t1[2 * r] = row ? c[lo_end + 1u] : 0u;
+    t0[2 * r + 1] = row && two ? c[hi_start] : 0u;
+    t1[2 * r + 1] = row && two ? c[hi + 1u] : 0u;
   }
 }
 
@@ -156,182 +130,180 @@ __device__ __forceinline__ uint32_t lanemask_lt_p() {
   return m;
 }
 
-__device__ __forceinline__ void append_active(const Bufs& b, Ctrl* ctrl, bool active, uint32_t s) {
-  const uint32_t mask = __ballot_sync(0xffffffffu, active);
-  if (mask) {
-    const int lane = threadIdx.x & 31;
-    const int leader = __ffs(mask) - 1;
-    uint32_t base = 0;
-    if (lane == leader) base = atomicAdd(&ctrl->act_n, (uint32_t)__popc(mask));
-    base = __shfl_sync(0xffffffffu, base, leader);
-    if (active) b.act[base + __popc(mask & lanemask_lt_p())] = s;
+// What a warp of k_sweep keeps: a column per lane (its neighbours, then their local ids, their outcome bits and at last
+// its list), the draws in queue order as lane * SLAB + slot, and each lane's local id and ensemble.
+struct SweepWarp {
+  uint32_t col[SLAB][32];
+  uint32_t la[32], ens[32];
+  uint16_t queue[32 * SLAB];
+};
+
+// The places of the m neighbours of column `lane` by their whole priorities, four bits each.
+__device__ __noinline__ uint32_t sweep_exact(const uint32_t* __restrict__ sid, const SweepWarp& sh, uint32_t lane,
+                                             uint32_t m, uint32_t la, uint32_t base, unsigned long long hash) {
+  uint32_t places = 0;
+  for (uint32_t i = 0; i < m; ++i) {
+    const uint32_t li = sid[sh.col[i][lane]] - base;
+    const unsigned long long p = order_hash_from(hash, min(la, li), max(la, li));
+    uint32_t k = 0;
+    for (uint32_t j = 0; j < m; ++j) {
+      const uint32_t lj = sid[sh.col[j][lane]] - base;
+      k += before(order_hash_from(hash, min(la, lj), max(la, lj)), lj, p, li) ? 1u : 0u;
+    }
+    places |= k << (4 * i);
   }
+  return places;
 }
 
-// The outcome draws of a warp's slab lists, spread evenly over its lanes: lane L needs the draws of
-// the entries in `mask` (bit k: entry k), pair (la, lb[k]) of ensemble `ens`. Drawn one slot per
-// lane in turn, at most 8 x 32 per warp, instead of each lane drawing its own (about half the slots
-// of a lattice list need a draw, and the lanes need them at different slots). The bits are merged
-// into e[k]. Every lane of the warp calls this.
-__device__ __forceinline__ void sweep_draws(const Bufs& b, uint32_t step, uint32_t mask, uint32_t la,
-                                            const uint32_t* lb, uint32_t ens, uint32_t* e) {
-  __shared__ uint32_t q_lb[SLOT_BLOCK / 32][32 * SLAB];    // local id of the partner, per draw
-  __shared__ uint16_t q_src[SLOT_BLOCK / 32][32 * SLAB];   // lane * SLAB + slot of the draw
-  __shared__ uint8_t q_bits[SLOT_BLOCK / 32][32 * SLAB];   // outcome bits, by lane * SLAB + slot
-  __shared__ uint32_t w_la[SLOT_BLOCK / 32][32], w_ens[SLOT_BLOCK / 32][32];
-  const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
-  const uint32_t cnt = __popc(mask);
+// Lists of up to SLAB neighbours, a microbe a thread. Bound by instruction issue and the latency of its loads, so:
+//   - the candidate loop does no more than the distance test and one store of the index into the lane's column, run
+//     by run (walking the six runs as one range took 5 selects a candidate: 47 us against 44 for 490,000 microbes on
+//     a lattice, two candidates at a time 46, the next position loaded ahead 45);
+//   - the order comes from the upper halves of the priorities: each pair of neighbours adds one to the place of the
+//     later one (packed four bits each). Equal halves send a microbe to sweep_exact;
+//   - the outcome draws of the warp are spread evenly over its lanes through a queue (about half the entries of a
+//     lattice list need a draw, and the lanes need them at different slots);
+//   - lists leave through the column as two 16-byte stores;
+//   - counters are added to once per block (below).
+// 53 -> 44 us for 490,000 microbes on a lattice, 64 -> 48 mixed, 211 -> 155 for 2,000,000 mixed, 142 -> 111 for 32
+// ensembles of 1,200,000 in all (a sorting network over 64-bit priorities, a shift register of neighbours and two
+// counters per warp before). Blocks of 128: 3-15 % slower with counters per warp; 5 blocks an SM 118 and 160 us on the
+// last two, 6 the figures above.
+__global__ void __launch_bounds__(SLOT_BLOCK, 6) k_sweep(Bufs b, PairParams pp, StepArgs a, Ctrl* ctrl) {
+  pdl_wait();
+  if (ctrl->halt) return;
+  __shared__ SweepWarp sh_all[SLOT_BLOCK / 32];
+  const uint32_t n_valid = ctrl->n_valid;
+  const uint32_t step = a.use_ctrl_step ? ctrl->step : a.step0;
+  const uint32_t s = blockIdx.x * SLOT_BLOCK + threadIdx.x, lane = threadIdx.x & 31u;
+  SweepWarp& sh = sh_all[threadIdx.x >> 5];
+  uint32_t m = 0, la = 0, base = 0, e = 0, id = 0;
+  unsigned long long hash = 0;
+  if (s < n_valid) {
+    const Vertex v = load_vertex(b, s);
+    const Band band = band_of(pp);
+    id = b.sid[s];
+    e = v.e;
+    base = v.base;
+    la = id - base;
+    hash = order_hash_base(step, ((unsigned long long)b.ens[e].seed_hi << 32) | b.ens[e].seed_lo);
+    uint32_t t0[6], t1[6];
+    neighbour_runs(b, v, t0, t1);
+#pragma unroll
+    for (int q = 0; q < 6; ++q) {
+      for (uint32_t t = t0[q]; t < t1[q]; ++t) {
+        const float2 pt = b.spos[t];
+        const float dist = norm_dist(pp.norm, v.ps, pt);
+        bool in = dist < band.lo;
+        if (!in && !(dist > band.hi)) in = within(pp, v.ps, pt);
+        if (in && t != s) {
+          if (m < SLAB) sh.col[m][lane] = t;
+          ++m;
+        }
+      }
+    }
+  }
+  const bool is_long = m > SLAB;
+  const uint32_t mk = is_long ? 0u : m;  // (longer lists are collected again by k_sweep_long)
+  uint32_t nb[SLAB], key[SLAB], need = 0, places = 0;
+  bool tie = false;
+#pragma unroll
+  for (int k = 0; k < (int)SLAB; ++k) {
+    key[k] = SLAB - 1u - k;  // empty slots last
+    nb[k] = 0;
+    if ((uint32_t)k < mk) {
+      const uint32_t t = sh.col[k][lane], lb = b.sid[t] - base;
+      key[k] = (uint32_t)(order_hash_from(hash, min(la, lb), max(la, lb)) >> 32);
+      tie |= key[k] < SLAB;
+      nb[k] = t;
+      need |= t > s ? 1u << k : 0u;  // the endpoint below in cell order applies the pair
+    }
+  }
+  if (mk > 1) {
+    // each of the first W slots against each: the one that loses moves back a place
+#define LM_PLACES(W)                                              \
+  _Pragma("unroll") for (int i = 0; i < W; ++i) {                 \
+    _Pragma("unroll") for (int j = i + 1; j < W; ++j) {           \
+      places += key[i] > key[j] ? 1u << (4 * j) : 1u << (4 * i);  \
+      tie |= key[i] == key[j];                                    \
+    }                                                             \
+  }
+    if (__all_sync(__activemask(), mk <= 4)) {
+      LM_PLACES(4)
+    } else {
+      LM_PLACES(8)
+    }
+#undef LM_PLACES
+    if (tie) places = sweep_exact(b.sid, sh, lane, mk, la, base, hash);
+  }
+  // the draws
+  const uint32_t cnt = __popc(need);
   uint32_t incl = cnt;
   for (int o = 1; o < 32; o <<= 1) {
     const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
     if (lane >= (uint32_t)o) incl += y;
   }
   const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
-  if (total == 0) return;
   uint32_t pos = incl - cnt;
 #pragma unroll
   for (int k = 0; k < (int)SLAB; ++k) {
-    if ((mask >> k) & 1u) {
-      q_lb[w][pos] = lb[k];
-      q_src[w][pos] = (uint16_t)(lane * SLAB + k);
-      ++pos;
+    if ((need >> k) & 1u) {
+      sh.col[k][lane] = b.sid[nb[k]] - base;
+      sh.queue[pos++] = (uint16_t)(lane * SLAB + k);
     }
   }
-  w_la[w][lane] = la;
-  w_ens[w][lane] = ens;
+  sh.la[lane] = la;
+  sh.ens[lane] = e;
   __syncwarp();
   for (uint32_t q = lane; q < total; q += 32) {
-    const uint32_t src = q_src[w][q], owner = src / SLAB;
-    const EnsInfo& info = b.ens[w_ens[w][owner]];
-    q_bits[w][src] = (uint8_t)(win_bits(info, w_la[w][owner], q_lb[w][q], step) >> ENTRY_WIN_SHIFT);
+    const uint32_t src = sh.queue[q], owner = src / SLAB;
+    uint32_t* slot = &sh.col[src % SLAB][owner];
+    *slot = win_bits(b.ens[sh.ens[owner]], sh.la[owner], *slot, step);
   }
   __syncwarp();
-#pragma unroll
-  for (int k = 0; k < (int)SLAB; ++k)
-    if ((mask >> k) & 1u) e[k] |= (uint32_t)q_bits[w][lane * SLAB + k] << ENTRY_WIN_SHIFT;
-}
-
-__global__ void __launch_bounds__(SLOT_BLOCK, 5) k_sweep(Bufs b, PairParams pp, StepArgs a, Ctrl* ctrl) {
-  pdl_wait();
-  if (ctrl->halt) return;
-  const uint32_t n_valid = ctrl->n_valid;
-  const uint32_t step = a.use_ctrl_step ? ctrl->step : a.step0;
-  const uint32_t s = blockIdx.x * SLOT_BLOCK + threadIdx.x;
-  bool active = false, is_long = false;
-  uint32_t m = 0;
-  // slab lists awaiting their outcome draws: entries, which ones need a draw, local ids, ensemble
-  uint32_t nbo[SLAB], draw_mask = 0, draw_la = 0, draw_lb[SLAB], draw_info = 0;
-#pragma unroll
-  for (int k = 0; k < (int)SLAB; ++k) nbo[k] = draw_lb[k] = 0;
   if (s < n_valid) {
-    const Vertex v = load_vertex(b, s);
-    const EnsInfo& info = b.ens[v.e];
-    const uint32_t k0 = info.seed_lo, k1 = info.seed_hi;
-    const uint32_t la = b.sid[s] - v.base;
-    unsigned long long pr[SLAB];
-    uint32_t nb[SLAB], pl[SLAB];
+    uint32_t first = NONE;
+    if (mk) {
+      uint32_t ent[SLAB];
 #pragma unroll
-    for (int k = 0; k < (int)SLAB; ++k) {
-      pr[k] = 0ull;
-      nb[k] = NONE;
-      pl[k] = NONE;
-    }
-    // phase 1: collect the neighbours (compile-time slots, predicated); the divergent candidate
-    // loop does no more than the distance test
-    for_neighbours(b, pp, v, [&](uint32_t t) {
-      // shift register: the newest neighbour in slot 0 (the slots are sorted below; entries past
-      // the eighth are collected again by the long-list kernel)
-#pragma unroll
-      for (int k = (int)SLAB - 1; k > 0; --k) nb[k] = nb[k - 1];
-      nb[0] = t;
-      ++m;
-    });
-    // phase 2: priorities over the slots, a loop whose trip count (the degree) is nearly the same
-    // across the warp
-    if (m <= SLAB) {
-#pragma unroll
-      for (int k = 0; k < (int)SLAB; ++k) {
-        if ((uint32_t)k < m) {
-          const uint32_t t = nb[k];
-          const uint32_t lb = b.sid[t] - v.base;
-          pr[k] = pair_prio(min(la, lb), max(la, lb), step, k0, k1);
-          pl[k] = lb;
-        }
-      }
-    }
-    // sorting network; empty slots (priority 0, partner NONE) sort last. When no list of the warp
-    // has more than 4 entries (most of a lattice), the 5-comparator network of 4 entries suffices.
-#define LM_CX(x, y)                                         \
-  if (before(pr[y], pl[y], pr[x], pl[x])) {                  \
-    const unsigned long long tp = pr[x]; pr[x] = pr[y]; pr[y] = tp; \
-    const uint32_t tn = nb[x]; nb[x] = nb[y]; nb[y] = tn;    \
-    const uint32_t tl = pl[x]; pl[x] = pl[y]; pl[y] = tl;    \
-  }
-    if (__all_sync(__activemask(), m <= 4)) {
-      if (m > 1) {
-        LM_CX(0, 1) LM_CX(2, 3) LM_CX(0, 2) LM_CX(1, 3) LM_CX(1, 2)
-      }
-    } else if (m > 1 && m <= SLAB) {
-      // 19-comparator network for 8 entries
-      LM_CX(0, 2) LM_CX(1, 3) LM_CX(4, 6) LM_CX(5, 7)
-      LM_CX(0, 4) LM_CX(1, 5) LM_CX(2, 6) LM_CX(3, 7)
-      LM_CX(0, 1) LM_CX(2, 3) LM_CX(4, 5) LM_CX(6, 7)
-      LM_CX(2, 4) LM_CX(3, 5) LM_CX(1, 4) LM_CX(3, 6)
-      LM_CX(1, 2) LM_CX(3, 4) LM_CX(5, 6)
-    }
-#undef LM_CX
-    b.deg[s] = m;
-    b.level[s] = 0;
-    if (m <= SLAB) {
-      // the outcomes of the pairs this vertex applies (partner above it in cell order), drawn by
-      // the whole warp (sweep_draws) and merged into the entries
-      uint32_t need = 0;
+      for (int k = 0; k < (int)SLAB; ++k) ent[k] = nb[k] | ((need >> k) & 1u ? sh.col[k][lane] : 0u);
 #pragma unroll
       for (int k = 0; k < (int)SLAB; ++k)
-        if ((uint32_t)k < m && nb[k] > s) need |= 1u << k;
-      draw_mask = need;
-      draw_la = la;
-#pragma unroll
-      for (int k = 0; k < (int)SLAB; ++k) {
-        draw_lb[k] = pl[k];
-        nbo[k] = nb[k];
-      }
-      draw_info = v.e;
-      active = m > 0;
-    } else {
-      is_long = true;
-      b.wstate[s] = pack_state(NONE, 0u, b.species[b.sid[s]]);  // set by k_sweep_long
+        if ((uint32_t)k < mk) sh.col[(places >> (4 * k)) & 7u][lane] = ent[k];
+      first = sh.col[0][lane];  // (entries past the list hold what is left there: never read)
+      uint4* row = reinterpret_cast<uint4*>(b.slab + (size_t)s * SLAB);
+      row[0] = make_uint4(first, sh.col[1][lane], sh.col[2][lane], sh.col[3][lane]);
+      if (mk > 4) row[1] = make_uint4(sh.col[4][lane], sh.col[5][lane], sh.col[6][lane], sh.col[7][lane]);
     }
+    b.deg[s] = m;
+    if (b.plog) b.level[s] = 0;
+    b.wstate[s] = pack_state(first, 0u, b.species[id]);  // entry 0 of the list; of long ones set by k_sweep_long
   }
-  sweep_draws(b, step, draw_mask, draw_la, draw_lb, draw_info, nbo);
-  if (s < n_valid && m <= SLAB) {
-#pragma unroll
-    for (int k = 0; k < (int)SLAB; ++k)
-      if ((uint32_t)k < m) b.slab[(size_t)s * SLAB + k] = nbo[k];
-    b.wstate[s] = pack_state(m ? nbo[0] : NONE, 0u, b.species[b.sid[s]]);  // entry 0 of the list
+  // The step's directed entries, and the list of the long ones (finished by k_sweep_long): one atomic each per block.
+  // With one per warp, and a list of all microbes with pairs besides, the warps waited for the counters' line (2,000,000
+  // microbes: 185 us against 168).
+  __shared__ uint32_t w_dir[SLOT_BLOCK / 32], w_long[SLOT_BLOCK / 32], long_at;
+  const uint32_t w = threadIdx.x >> 5, long_mask = __ballot_sync(0xffffffffu, is_long);
+  const uint32_t dir = __reduce_add_sync(0xffffffffu, m);
+  if (lane == 0) {
+    w_dir[w] = dir;
+    w_long[w] = __popc(long_mask);
   }
-  append_active(b, ctrl, active, s);
-  // long lists are finished by k_sweep_long
-  {
-    const uint32_t mask = __ballot_sync(0xffffffffu, is_long);
-    if (mask) {
-      const int lane = threadIdx.x & 31;
-      const int leader = __ffs(mask) - 1;
-      uint32_t base = 0;
-      if (lane == leader) base = atomicAdd(&ctrl->n_long, (uint32_t)__popc(mask));
-      base = __shfl_sync(0xffffffffu, base, leader);
-      if (is_long) b.longv[base + __popc(mask & lanemask_lt_p())] = s;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    unsigned long long entries = 0;
+    uint32_t longs = 0;
+    for (int k = 0; k < (int)(SLOT_BLOCK / 32); ++k) {
+      const uint32_t n = w_long[k];
+      w_long[k] = longs;
+      entries += w_dir[k];
+      longs += n;
     }
+    if (entries) atomicAdd(&ctrl->n_dir, entries);
+    if (longs) long_at = atomicAdd(&ctrl->n_long, longs);
   }
-  // directed entries of the step
-  __shared__ unsigned long long tot;
-  if (threadIdx.x == 0) tot = 0;
   __syncthreads();
-  unsigned long long mm = m;
-  for (int o = 16; o > 0; o >>= 1) mm += __shfl_xor_sync(0xffffffffu, mm, o);
-  if ((threadIdx.x & 31) == 0 && mm) atomicAdd(&tot, mm);
-  __syncthreads();
-  if (threadIdx.x == 0 && tot) atomicAdd(&ctrl->n_dir, tot);
+  if (is_long) b.longv[long_at + w_long[w] + __popc(long_mask & lanemask_lt_p())] = s;
 }
 
 void launch_sweep(const Bufs& b, const PairParams& pp, const StepArgs& a, Ctrl* ctrl, cudaStream_t st) {
@@ -1114,11 +1086,6 @@ __global__ void __launch_bounds__(LONG_WARPS * 32, 8) k_sweep_long(Bufs b, PairP
       }
     }
     if (used) long_flush(b, step, sh, used);
-    // every vertex of the batch is active (it has > SLAB pairs): one atomic per batch
-    uint32_t at = 0;
-    if (lane == 0) at = atomicAdd(&ctrl->act_n, nk);
-    at = __shfl_sync(0xffffffffu, at, 0);
-    if (lane < nk) b.act[at + lane] = s_l;
   }
 }
 

@@ -364,12 +364,11 @@ __global__ void __launch_bounds__(RD_THREADS, 2) k_rounds(Bufs b, StepArgs a, Ct
   // the control words, read by one thread per block: every thread of the 300-odd blocks loading
   // the same L2 line (the loads are volatile, so L1 does not merge them) queued ~10^4 requests on
   // one L2 slice and delayed the start of the pairs by 4-10 us
-  __shared__ uint32_t cw[4];
+  __shared__ uint32_t cw[3];
   if (threadIdx.x == 0) {
     cw[0] = ((volatile uint32_t*)&ctrl->halt)[0] | ((volatile uint32_t*)&ctrl->ev_taken)[0];
-    cw[1] = ((volatile uint32_t*)&ctrl->act_n)[0];
-    cw[2] = ((volatile uint32_t*)&ctrl->n_valid)[0];
-    cw[3] = a.use_ctrl_step ? ((volatile uint32_t*)&ctrl->step)[0] : a.step0;
+    cw[1] = ((volatile uint32_t*)&ctrl->n_valid)[0];
+    cw[2] = a.use_ctrl_step ? ((volatile uint32_t*)&ctrl->step)[0] : a.step0;
   }
   __syncthreads();
   if (cw[0]) return;
@@ -387,13 +386,13 @@ __global__ void __launch_bounds__(RD_THREADS, 2) k_rounds(Bufs b, StepArgs a, Ct
     }
     return;
   }
-  const uint32_t step = cw[3];
+  const uint32_t step = cw[2];
   const uint32_t cnt = cw[1];
   const uint32_t stride = gridDim.x * blockDim.x;
   const uint32_t first = blockIdx.x * blockDim.x + threadIdx.x;
   uint32_t max_level = 0;
   const unsigned long long t0 = globaltimer();
-  if (rounds_tiled<RD_THREADS>(b, step, ctrl, t0, cw[2])) return;  // levels are tracked only in pair-log runs
+  if (rounds_tiled<RD_THREADS>(b, step, ctrl, t0, cnt)) return;  // levels are tracked only in pair-log runs
   uint32_t polls = 0;
   if (cnt <= (uint32_t)POLL_BATCH * stride) {
     // every thread owns at most POLL_BATCH vertices: keep their ids in registers and stop polling
@@ -403,7 +402,7 @@ __global__ void __launch_bounds__(RD_THREADS, 2) k_rounds(Bufs b, StepArgs a, Ct
 #pragma unroll
     for (int k = 0; k < POLL_BATCH; ++k) {
       const uint32_t x = first + (uint32_t)k * stride;
-      sv[k] = x < cnt ? b.act[x] : NONE;
+      sv[k] = x < cnt ? x : NONE;
       if (sv[k] != NONE) live |= 1u << k;
     }
     while (live) {
@@ -439,7 +438,7 @@ __global__ void __launch_bounds__(RD_THREADS, 2) k_rounds(Bufs b, StepArgs a, Ct
 #pragma unroll
       for (int k = 0; k < POLL_BATCH; ++k) {
         const uint32_t x = x0 + (uint32_t)k * stride;
-        sv[k] = x < cnt ? b.act[x] : NONE;
+        sv[k] = x < cnt ? x : NONE;
         ws[k] = sv[k] != NONE ? ld_relaxed(b.wstate + sv[k]) : (unsigned long long)NONE;
       }
 #pragma unroll

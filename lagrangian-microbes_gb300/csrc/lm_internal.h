@@ -17,7 +17,7 @@
 //                                                a longer list's overflow offset in slot 0)
 //              uint32 ovf[cap]; uint64 oprio[cap]  (longer lists, allocated per step, NONE behind each)
 //              uint64 wstate[S] = species << 56 | list position << 32 | partner;
-//              uint32 level[S] (pair-log runs only), act[S]   (interaction dataflow)
+//              uint32 level[S] (pair-log runs only), act[S] (dense cells of a count-only step)
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -83,7 +83,7 @@ struct Ctrl {
   uint32_t rounds;              // longest dependency chain (levels) of the current step
   uint32_t max_rounds;          // max over steps since the last reset
   uint32_t plog_n;              // pair-log entries written this step
-  uint32_t act_n;               // active vertices (with at least one pair)
+  uint32_t act_n;               // dense cells listed for a count-only step
   uint32_t census[4];           // species counts after the step, all ensembles ([0] = other values)
   unsigned long long rounds_total;  // sum of per-step levels since the last reset
   int stage_k[3];               // frame brackets of this step's stage times t, t+dt/2, t+dt

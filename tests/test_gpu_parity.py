@@ -208,6 +208,42 @@ def test_gpu_long_lists_whose_leading_priority_bits_agree(engine, orc):
     np.testing.assert_array_equal(got, want)
 
 
+@pytest.mark.parametrize("seed, first, pair", [(6935, 353 * 9, (1, 0, 6)), (16514, 997 * 9, (5, 2, 7)), (16869, 31 * 9, (8, 2, 4))])
+def test_gpu_short_lists_whose_upper_priority_halves_agree(engine, orc, seed, first, pair):
+    """1,000 clumps of 9 under seeds for which one list holds two priorities equal in their upper 32 bits (the order
+    of lists of up to 8 goes by those first)."""
+    rng = np.random.default_rng(8)
+    lon, lat = _clumps(rng, [9] * 1000, 0.007)
+    sp = rng.integers(1, 4, lon.size).astype(np.int8)
+
+    def priority(i, j):
+        m = (1 << 64) - 1
+        z = ((first + min(i, j)) << 32 | (first + max(i, j))) + seed * 0x9E3779B97F4A7C15 + 6 * 0xD1B54A32D192ED03 & m
+        z = (z ^ z >> 30) * 0xBF58476D1CE4E5B9 & m
+        z = (z ^ z >> 27) * 0x94D049BB133111EB & m
+        return z ^ z >> 31
+
+    x, y = priority(pair[0], pair[1]), priority(pair[0], pair[2])
+    assert x >> 32 == y >> 32 and x != y
+    got, _, stats = _interact(engine, lon, lat, sp, 0.01, 2, (0.6, 0.7, 0.55), seed, 6, log=False)
+    want, m = orc.interact_step(lon, lat, sp, 0.01, 2, 0.6, 0.7, 0.55, seed, 6)
+    assert stats["pairs"] == m == 1000 * 36
+    np.testing.assert_array_equal(got, want)
+
+
+def test_gpu_short_lists_of_every_length_match_oracle(engine, orc):
+    """Clumps of 1 to 10 microbes (lists of 0 to 9: the packed places of 4 and of 8, the first long one), species
+    outside 1..3 among them, over several tile widths."""
+    rng = np.random.default_rng(18)
+    for repeat, norm in ((40, 2), (400, 1), (4, np.inf)):
+        lon, lat = _clumps(rng, list(range(1, 11)) * repeat, 0.0049)
+        sp = rng.integers(0, 5, lon.size).astype(np.int8)
+        got, _, stats = _interact(engine, lon, lat, sp, 0.01, norm, (0.6, 0.7, 0.55), 3, repeat, log=False)
+        want, m = orc.interact_step(lon, lat, sp, 0.01, norm, 0.6, 0.7, 0.55, 3, repeat)
+        assert stats["pairs"] == m == 165 * repeat
+        np.testing.assert_array_equal(got, want)
+
+
 @pytest.mark.parametrize("n, dense", [(640000, 0), (700001, 30000)])
 def test_gpu_interaction_beyond_the_blocks_lists_matches_oracle(engine, orc, n, dense):
     """One ensemble larger than the lists that the blocks hold in shared memory (304 x 2,048 microbes): state words
