@@ -67,6 +67,7 @@ struct lm_adjoint {
   // batch buffers, `stepped` (records written) and `reduced` (records read) per set
   cudaStream_t red_st = nullptr;
   cudaEvent_t stepped[2] = {}, reduced[2] = {};
+  cudaEvent_t given = nullptr;  // the default stream's work when a call begins
 };
 
 namespace {
@@ -158,6 +159,16 @@ int read_err(lm_adjoint* a, cudaStream_t st, uint32_t* out) {
   return LM_OK;
 }
 
+// On the context's own (non-blocking) stream nothing orders a call after the work that writes its arrays, or still reads
+// memory that it was given, on the default stream (torch's, unless the caller changed it): that stream's work up to
+// here comes first. Every call waits for its own work before it returns, so nothing is needed behind it.
+int after_default_stream(lm_adjoint* a) {
+  if (!ctx_on_own_stream(a->ctx)) return LM_OK;
+  ACK(cudaEventRecord(a->given, cudaStreamLegacy));
+  ACK(cudaStreamWaitEvent(ctx_stream(a->ctx), a->given, 0));
+  return LM_OK;
+}
+
 }  // namespace
 
 extern "C" {
@@ -173,6 +184,7 @@ int lm_adjoint_create(lm_ctx* ctx, lm_adjoint** out) {
   if ((e = cudaSetDevice(a->device)) != cudaSuccess || (e = cudaMalloc((void**)&a->err_d, sizeof(uint32_t))) != cudaSuccess ||
       (e = cudaMallocHost((void**)&a->err_h, sizeof(uint32_t))) != cudaSuccess ||
       (e = cudaStreamCreateWithFlags(&a->red_st, cudaStreamNonBlocking)) != cudaSuccess ||
+      (e = cudaEventCreateWithFlags(&a->given, cudaEventDisableTiming)) != cudaSuccess ||
       (e = cudaEventCreateWithFlags(&a->stepped[0], cudaEventDisableTiming)) != cudaSuccess ||
       (e = cudaEventCreateWithFlags(&a->stepped[1], cudaEventDisableTiming)) != cudaSuccess ||
       (e = cudaEventCreateWithFlags(&a->reduced[0], cudaEventDisableTiming)) != cudaSuccess ||
@@ -197,6 +209,7 @@ int lm_adjoint_destroy(lm_adjoint* a) {
     if (a->stepped[k]) cudaEventDestroy(a->stepped[k]);
     if (a->reduced[k]) cudaEventDestroy(a->reduced[k]);
   }
+  if (a->given) cudaEventDestroy(a->given);
   release(a->uv);
   release(a->table);
   release(a->x), release(a->y), release(a->ck_x), release(a->ck_y), release(a->seg_x), release(a->seg_y);
@@ -246,6 +259,7 @@ int lm_adjoint_forward(lm_adjoint* a, const float* u, const float* v, int nt, in
   }
   ACK(cudaSetDevice(a->device));
   cudaStream_t st = ctx_stream(a->ctx);
+  if (const int waited = after_default_stream(a)) return waited;
   const size_t fe = (size_t)nt * ny * nx;
   const uint32_t N = (uint32_t)n;
   const int n_ck = (n_steps + checkpoint_every - 1) / checkpoint_every;
@@ -322,6 +336,7 @@ int lm_adjoint_backward(lm_adjoint* a, const float* g_lon, const float* g_lat, f
   if (!on_device(g_u) || !on_device(g_v)) return afail(a, LM_ERR_ARG, "g_u and g_v must be device pointers");
   ACK(cudaSetDevice(a->device));
   cudaStream_t st = ctx_stream(a->ctx);
+  if (const int waited = after_default_stream(a)) return waited;
   const size_t fe = (size_t)a->nt * a->ny * a->nx;
   const uint32_t cells = (uint32_t)(a->nx - 1) * (uint32_t)(a->ny - 1);
   const size_t es = adj_state_bytes(a->prec);
@@ -373,6 +388,7 @@ int lm_adjoint_final_positions(lm_adjoint* a, double* lon, double* lat) {
   if (a->n && (!on_device(lon) || !on_device(lat))) return afail(a, LM_ERR_ARG, "lon and lat must be device pointers");
   ACK(cudaSetDevice(a->device));
   cudaStream_t st = ctx_stream(a->ctx);
+  if (const int waited = after_default_stream(a)) return waited;
   launch_adj_final64(a->fv, a->prec, a->n, a->fin_x.p, a->fin_y.p, lon, lat, st);
   ACK(cudaGetLastError());
   ACK(cudaStreamSynchronize(st));
@@ -385,6 +401,7 @@ int lm_adjoint_cell_signature(lm_adjoint* a, unsigned long long* sig) {
   if (a->n && !on_device(sig)) return afail(a, LM_ERR_ARG, "sig must be a device pointer");
   ACK(cudaSetDevice(a->device));
   cudaStream_t st = ctx_stream(a->ctx);
+  if (const int waited = after_default_stream(a)) return waited;
   launch_adj_signature(a->fv, a->prec, a->table.p, a->n_steps, a->dt, a->n, a->ck_x.p, a->ck_y.p, a->ck_st.p, sig,
                        st);
   ACK(cudaGetLastError());

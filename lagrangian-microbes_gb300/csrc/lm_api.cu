@@ -1560,6 +1560,7 @@ bool pdl_enabled() {
 int ctx_device(const lm_ctx* c) { return c->device; }
 int ctx_sms(const lm_ctx* c) { return c->sms; }
 cudaStream_t ctx_stream(const lm_ctx* c) { return c->st; }
+bool ctx_on_own_stream(const lm_ctx* c) { return c->st == c->own; }
 void ctx_set_error(lm_ctx* c, const char* msg) { c->err = msg ? msg : ""; }
 int ctx_scratch(lm_ctx* c, size_t bytes, void** p) {
   if (bytes > c->scratch_n) {

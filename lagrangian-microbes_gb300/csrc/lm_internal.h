@@ -432,6 +432,7 @@ void set_thread_error(const char* msg);
 int ctx_device(const lm_ctx* c);
 int ctx_sms(const lm_ctx* c);
 cudaStream_t ctx_stream(const lm_ctx* c);
+bool ctx_on_own_stream(const lm_ctx* c);  // no external stream set
 void ctx_set_error(lm_ctx* c, const char* msg);
 // A device buffer of at least `bytes` owned by the context (grown, never shrunk, freed with it), for
 // the working arrays of one synchronous call; its contents do not outlive the call.

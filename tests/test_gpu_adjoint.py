@@ -319,3 +319,31 @@ def test_adjoint_non_finite_gradients_stay_in_their_cells(small_field, bad):
     g[:, 5] = bad  # and in a cell of several items
     got = _tape_backward(f, lon, lat, g, 4, 4, "f32")
     assert int((~np.isfinite(got[2])).sum()) > few
+
+
+def test_tape_waits_for_the_default_streams_work(lm, small_field):
+    """Inputs still being written on the default stream when the call is made (a pause of some milliseconds before
+    them), forward and backward: the results of finished inputs."""
+    from lagrangian_microbes_gb300.adjoint import AdjointTape
+    lon, lat, _, _ = _case(small_field, 4000, 5)
+    dev = torch.device("cuda:0")
+    ready = [torch.from_numpy(np.ascontiguousarray(a, np.float32)).to(dev) for a in (lon, lat, small_field.u, small_field.v)]
+    weights = [torch.linspace(-1, 1, 4000, device=dev), torch.linspace(2, -1, 4000, device=dev)]
+    axes = (small_field.lon, small_field.lat, small_field.times)
+    t0 = float(small_field.times[0])
+    tape = AdjointTape(precision="ds")
+    want = tape.forward(*ready, *axes, t0, 3600.0, 6), None
+    want = want[0], tape.backward(*weights)
+    late = [torch.zeros_like(t) for t in ready + weights]
+    late[0].fill_(200.5), late[1].fill_(25.5)
+    torch.cuda.synchronize()
+    torch.cuda._sleep(20_000_000)
+    for a, b in zip(late[:4], ready):
+        a.copy_(b)
+    got = tape.forward(*late[:4], *axes, t0, 3600.0, 6)
+    torch.cuda._sleep(20_000_000)
+    for a, b in zip(late[4:], weights):
+        a.copy_(b)
+    for a, b in zip((*got, *tape.backward(*late[4:])), (*want[0], *want[1])):
+        assert torch.equal(a, b)
+    tape.close()
