@@ -312,6 +312,16 @@ int lm_distance_histogram(lm_ctx* ctx, const float* lat, const float* lon, int64
 int lm_species_histogram(lm_ctx* ctx, const float* lat, const float* lon, const int8_t* species, int64_t n, int bins,
                          double radius_m, uint64_t* counts);
 
+/* Mean squared great-circle distance (m^2, sphere of 6371.228 km, haversine in float64) between n >= 1 positions and
+ * their targets, all device arrays; no counterpart in the reference. lon, lat: float64; tlon, tlat: float64 or float32
+ * (targets_f64 0). loss: one float64. g (NULL: no derivatives): float64 [2][n], the derivatives by lon and by lat; the
+ * targets are then copied to targets, float64 [2][n]. work: LM_LOSS_PARTS float64. Enqueued on `stream` of `device`
+ * without waiting, so a stream under capture is accepted; needs no context. */
+#define LM_LOSS_PARTS 1216
+int lm_mean_squared_distance(int device, uintptr_t stream, int64_t n, const double* lon, const double* lat,
+                             const void* tlon, const void* tlat, int targets_f64, double* loss, double* g,
+                             double* targets, double* work);
+
 #ifdef __cplusplus
 }
 #endif

@@ -86,6 +86,8 @@ class Stats(ctypes.Structure):
         return d
 
 
+LOSS_PARTS = 1216  # LM_LOSS_PARTS
+
 _lock = threading.Lock()
 _lib = None
 
@@ -146,6 +148,7 @@ SIGNATURES = {
     "lm_adjoint_final_positions": [P, P, P],
     "lm_distance_histogram": [P, P, P, I64, P, I32, I32, F64, P],
     "lm_species_histogram": [P, P, P, P, I64, I32, F64, P],
+    "lm_mean_squared_distance": [I32, ctypes.c_size_t, I64, P, P, P, P, I32, P, P, P, P],
     "lm_debug_inject_wait": [P, F64],
 }
 

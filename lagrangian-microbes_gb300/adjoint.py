@@ -158,7 +158,73 @@ def great_circle_m(lon1, lat1, lon2, lat2):
     return 2 * EARTH_RADIUS_M * torch.asin(torch.sqrt(h.clamp(max=1.0)))
 
 
-def mean_squared_distance(lon, lat, target_lon, target_lat):
-    """Loss of the differentiation benchmark: mean squared great-circle distance (m^2), float64."""
+def _squared_distance_mean(lon, lat, target_lon, target_lat):
     d = great_circle_m(lon.double(), lat.double(), target_lon.double(), target_lat.double())
     return (d * d).mean()
+
+
+class _MeanSquaredDistance(torch.autograd.Function):
+    """The loss and its derivatives in one kernel (k_loss.cu). lon and lat are float64 tensors that only this node holds,
+    and the targets are copied, so that the caller may overwrite its own before the backward."""
+
+    @staticmethod
+    def forward(ctx, lon, lat, target_lon, target_lat):
+        n, dev = lon.numel(), lon.device
+        grad = any(ctx.needs_input_grad)
+        work = torch.empty(_lib.LOSS_PARTS + (4 * n if grad else 0), dtype=torch.float64, device=dev)
+        loss = torch.empty((), dtype=torch.float64, device=dev)
+        g = t = None
+        if grad:
+            g, t = work[_lib.LOSS_PARTS:].view((2, 2) + lon.shape).unbind(0)
+        rc = _lib.load().lm_mean_squared_distance(
+            dev.index, torch.cuda.current_stream(dev).cuda_stream, n, lon.data_ptr(), lat.data_ptr(),
+            target_lon.data_ptr(), target_lat.data_ptr(), int(target_lon.dtype == torch.float64), loss.data_ptr(),
+            g.data_ptr() if grad else None, t.data_ptr() if grad else None, work.data_ptr())
+        if rc != _lib.LM_OK:
+            raise _lib.LMError(rc, "the loss kernel could not be launched")
+        if grad:
+            ctx.save_for_backward(lon, lat, g, t)
+        return loss
+
+    @staticmethod
+    def backward(ctx, g_loss):
+        lon, lat, g, t = ctx.saved_tensors
+        if torch.is_grad_enabled():  # create_graph: the derivatives as differentiable operations
+            wanted = [x for x, need in zip((lon, lat), ctx.needs_input_grad) if need]
+            grads = iter(torch.autograd.grad(_squared_distance_mean(lon, lat, t[0], t[1]), wanted, g_loss,
+                                             create_graph=True))
+            return tuple(next(grads) if need else None for need in ctx.needs_input_grad[:2]) + (None, None)
+        g_lon, g_lat = (g_loss * g).unbind(0)
+        return g_lon, g_lat, None, None
+
+
+def _one_kernel(tensors) -> bool:
+    """Plain CUDA tensors of one shape on one device, targets without gradients, and nothing that looks into single
+    operations (tracing, compilation, functorch transforms, forward mode, dispatch and function modes)."""
+    first = tensors[0]
+    for t in tensors:
+        if (type(t) not in (torch.Tensor, torch.nn.Parameter) or not t.is_cuda or t.device != first.device
+                or t.layout is not torch.strided or t.shape != first.shape or not t.is_floating_point()
+                or t.is_neg() or t._is_zerotensor()):
+            return False
+    return (first.numel() > 0 and not tensors[2].requires_grad and not tensors[3].requires_grad
+            and not torch.jit.is_tracing() and not torch.compiler.is_compiling()
+            and torch._C._len_torch_dispatch_stack() == 0 and torch._C._len_torch_function_stack() == 0
+            and torch._C._functorch.peek_interpreter_stack() is None
+            and torch.autograd.forward_ad._current_level < 0)
+
+
+def mean_squared_distance(lon, lat, target_lon, target_lat):
+    """Loss of the differentiation benchmark: mean squared great-circle distance (m^2), float64."""
+    if not _one_kernel((lon, lat, target_lon, target_lat)):
+        return _squared_distance_mean(lon, lat, target_lon, target_lat)
+
+    def own(x):  # float64, contiguous, and not the caller's where the node keeps it
+        if x.dtype != torch.float64:
+            return x.double().contiguous()
+        return x.clone(memory_format=torch.contiguous_format) if keep else x.contiguous()
+
+    keep = torch.is_grad_enabled() and (lon.requires_grad or lat.requires_grad)
+    if target_lon.dtype != target_lat.dtype or target_lon.dtype not in (torch.float32, torch.float64):
+        target_lon, target_lat = target_lon.double(), target_lat.double()
+    return _MeanSquaredDistance.apply(own(lon), own(lat), target_lon.contiguous(), target_lat.contiguous())

@@ -347,3 +347,86 @@ def test_tape_waits_for_the_default_streams_work(lm, small_field):
     for a, b in zip((*got, *tape.backward(*late[4:])), (*want[0], *want[1])):
         assert torch.equal(a, b)
     tape.close()
+
+
+@pytest.mark.parametrize("n, dtype, target_dtype", [(1, "float32", "float32"), (255, "float64", "float32"), (257, "float32", "float64"),
+                                                    (4099, "float16", "float64"), (152 * 8 * 256 + 1, "float64", "float64")])
+def test_squared_distance_kernel_equals_the_tensor_operations(lm, n, dtype, target_dtype):
+    """k_loss against the same loss as torch operations. Each side rounds some 20 times on the way to a derivative, and
+    1 - q^2 >= 0.02 amplifies by at most 50: 20 x 51 x 2^-53 = 1.1e-13 a side, relative to the terms that are added."""
+    import torch
+    from lagrangian_microbes_gb300 import adjoint
+    gen = torch.Generator().manual_seed(n)
+    u = lambda lo, hi: (lo + (hi - lo) * torch.rand(n, generator=gen, dtype=torch.float64))
+    lon, lat = (t.to(getattr(torch, dtype)).cuda().requires_grad_() for t in (u(-180, 180), u(-89, 89)))
+    if n > 300:  # near and far targets (great circles up to 160 degrees)
+        tl, ta = lon.detach().cpu().double() + u(-0.5, 0.5), (lat.detach().cpu().double() + u(-0.5, 0.5)).clamp(-89, 89)
+    else:
+        tl, ta = lon.detach().cpu().double() + u(-100, 100), u(-40, 40)
+    tl, ta = (t.to(getattr(torch, target_dtype)).cuda() for t in (tl, ta))
+    assert adjoint._one_kernel((lon, lat, tl, ta))
+    want = adjoint._squared_distance_mean(lon, lat, tl, ta)
+    w_lon, w_lat = torch.autograd.grad(want, (lon, lat))
+    kept = tl.clone(), ta.clone()
+    got = adjoint.mean_squared_distance(lon, lat, tl, ta)
+    assert got.dtype == torch.float64 and got.shape == () and got.requires_grad
+    with torch.no_grad():
+        np.testing.assert_allclose(adjoint.mean_squared_distance(lon, lat, tl, ta).item(), want.item(), rtol=5e-13)
+        tl.zero_(), ta.zero_()  # the caller's buffers may be filled again before the backward
+    g_lon, g_lat = torch.autograd.grad(got, (lon, lat))
+    tl.copy_(kept[0]), ta.copy_(kept[1])
+    np.testing.assert_allclose(got.item(), want.item(), rtol=5e-13)
+    p1, p2 = lat.detach().double() * np.pi / 180, ta.double() * np.pi / 180
+    dl = (tl.double() - lon.detach().double()) * np.pi / 360
+    a, c = torch.sin((p2 - p1) / 2), torch.sin(dl)
+    terms = (a * torch.cos((p2 - p1) / 2)).abs() + (torch.sin(p1) * torch.cos(p2) * c * c).abs()
+    net = (a * torch.cos((p2 - p1) / 2) + torch.sin(p1) * torch.cos(p2) * c * c).abs()
+    eps = {"float16": 2.0 ** -10, "float32": 2.0 ** -23}.get(dtype, 0.0)  # the result's own rounding
+    for g, w, t in ((g_lon, w_lon, torch.ones_like(terms)), (g_lat, w_lat, terms / net.clamp(min=1e-300))):
+        assert g.dtype == lon.dtype
+        bound = w.double().abs() * (5e-13 * t + eps) + (6e-8 if dtype == "float16" else 1e-44)
+        assert bool(((g == w) | ((g.double() - w.double()).abs() <= bound)).all())  # (float16 overflows alike)
+
+
+def test_squared_distance_beyond_the_plain_call(lm):
+    """What the loss kernel does not take goes through the tensor operations, with their results: functorch transforms,
+    forward mode, derivatives by the targets, broadcast shapes, the CPU; and what it takes: second derivatives,
+    batched gradients, capture, another stream, a microbe on its target (its derivative is undefined there)."""
+    import torch
+    from lagrangian_microbes_gb300 import adjoint
+    f = adjoint.mean_squared_distance
+    gen = torch.Generator().manual_seed(3)
+    lon, lat, tl, ta = (torch.rand(2, 33, generator=gen, dtype=torch.float64).cuda() + k for k in (10, 20, 10.2, 20.1))
+    ref = adjoint._squared_distance_mean
+    close = lambda a, b: torch.testing.assert_close(a, b, rtol=1e-11, atol=0, equal_nan=True)
+    close(torch.func.vmap(f)(lon, lat, tl, ta), torch.func.vmap(ref)(lon, lat, tl, ta))
+    close(torch.func.grad(f)(lon, lat, tl, ta), torch.func.grad(ref)(lon, lat, tl, ta))
+    close(torch.func.jvp(f, (lon, lat, tl, ta), (lon, lat, tl, ta))[1], torch.func.jvp(ref, (lon, lat, tl, ta), (lon, lat, tl, ta))[1])
+    close(f(lon, lat[0], tl, ta[:, :1]), ref(lon, lat[0], tl, ta[:, :1]))
+    close(f(*(t.cpu() for t in (lon, lat, tl, ta))).cuda(), ref(lon, lat, tl, ta))
+    assert torch.isnan(f(lon[:, :0], lat[:, :0], tl[:, :0], ta[:, :0]))
+    x, y, tx = (t.clone().requires_grad_() for t in (lon, lat, tl))
+    for a, b in zip(torch.autograd.grad(f(x, y, tx, ta), (x, y, tx)), torch.autograd.grad(ref(x, y, tx, ta), (x, y, tx))):
+        close(a, b)
+    second = []
+    for g in (f, ref):
+        gx, gy = torch.autograd.grad(g(x, y, tl, ta), (x, y), create_graph=True)
+        second.append(torch.autograd.grad((gx * gx).sum() + (gx * gy).sum(), (x, y)))
+    for a, b in zip(*second):
+        torch.testing.assert_close(a, b, rtol=1e-9, atol=1e-3)
+    weights = torch.tensor([1.0, -2.0, 0.5], dtype=torch.float64).cuda()
+    (rows,) = torch.autograd.grad(f(x.t(), y.t(), tl.t(), ta.t()), x, weights, is_grads_batched=True)
+    close(rows, weights[:, None, None] * torch.autograd.grad(ref(x, y, tl, ta), x)[0])
+    (g,) = torch.autograd.grad(f(x, y, torch.cat([lon[:1], tl[1:]]), torch.cat([lat[:1], ta[1:]])), x)
+    assert torch.isnan(g[0]).all() and torch.isfinite(g[1]).all()
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        f(lon, lat, tl, ta)
+    torch.cuda.current_stream().wait_stream(side)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = f(lon, lat, tl, ta)
+    lon.add_(0.25)
+    graph.replay()
+    close(out, ref(lon, lat, tl, ta))
