@@ -248,8 +248,8 @@ __global__ void k_step_begin(Bufs b, FieldView f, StepArgs a, int bracket, Ctrl*
 }
 
 // End of a step; with `chain`, also the start of the next one (`an` its arguments).
-__global__ void k_step_end(Bufs b, FieldView f, StepArgs an, int bracket, Ctrl* ctrl, int interact, int chain) {
-  pdl_wait();
+__device__ __forceinline__ void step_end_body(const Bufs& b, const FieldView& f, const StepArgs& an, int bracket,
+                                              Ctrl* ctrl, int interact, int chain) {
   if (ctrl->halt) return;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     if (interact) {
@@ -260,6 +260,11 @@ __global__ void k_step_end(Bufs b, FieldView f, StepArgs an, int bracket, Ctrl* 
     ctrl->step += 1;
   }
   if (chain) step_begin_body(b, f, an, bracket, ctrl);
+}
+
+__global__ void k_step_end(Bufs b, FieldView f, StepArgs an, int bracket, Ctrl* ctrl, int interact, int chain) {
+  pdl_wait();
+  step_end_body(b, f, an, bracket, ctrl, interact, chain);
 }
 
 static int bookkeeping_grid(const Bufs& b) {
@@ -336,20 +341,29 @@ void launch_restore(const float* sx, const float* sy, const int8_t* ss, const ui
   k_restore<<<grid, 256, 0, stream>>>(sx, sy, ss, sst, x, y, sp, st, S, step, ctrl);
 }
 
-// Gathers from the padded slot layout into caller order (map[slot] = caller index or -1).
-template <class T>
-__global__ void k_unpad(const T* __restrict__ src, T* __restrict__ dst, const int32_t* __restrict__ map, uint32_t n) {
-  const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= n) return;
-  const int32_t q = map[p];
-  if (q >= 0) dst[q] = src[p];
+// One step's record into a ring slot in caller order, lon | lat | species of n microbes (NULL parts are left out; map
+// NULL: slot k is microbe k), and the end of the step (k_step_end's arguments): one launch for three copies or gathers
+// and the bookkeeping. 24 steps of 202,000 microbes without interaction: 658 us with those five launches, 438 with two,
+// 404 with this one.
+__global__ void __launch_bounds__(SLOT_BLOCK) k_record(Bufs b, const int32_t* __restrict__ map, uint32_t n,
+                                                       float* __restrict__ lon, float* __restrict__ lat,
+                                                       int8_t* __restrict__ species, FieldView f, StepArgs an,
+                                                       Ctrl* ctrl, int interact, int chain) {
+  pdl_wait();
+  step_end_body(b, f, an, 1, ctrl, interact, chain);
+  const uint32_t p = blockIdx.x * SLOT_BLOCK + threadIdx.x;
+  if (p >= b.nslots) return;
+  const int32_t q = map ? map[p] : (p < n ? (int32_t)p : -1);
+  if (q < 0) return;
+  if (lon) lon[q] = b.plon[p];
+  if (lat) lat[q] = b.plat[p];
+  if (species) species[q] = b.species[p];
 }
 
-void launch_unpad(const float* src, float* dst, const int32_t* map, uint32_t nslots, cudaStream_t st) {
-  if (nslots) k_unpad<float><<<(nslots + 255) / 256, 256, 0, st>>>(src, dst, map, nslots);
-}
-void launch_unpad8(const int8_t* src, int8_t* dst, const int32_t* map, uint32_t nslots, cudaStream_t st) {
-  if (nslots) k_unpad<int8_t><<<(nslots + 255) / 256, 256, 0, st>>>(src, dst, map, nslots);
+void launch_record(const Bufs& b, const int32_t* map, uint32_t n, float* lon, float* lat, int8_t* species,
+                   const FieldView& f, const StepArgs* next, Ctrl* ctrl, bool interact, cudaStream_t st) {
+  launch_dep(k_record, dim3((b.nslots + SLOT_BLOCK - 1) / SLOT_BLOCK), dim3(SLOT_BLOCK), st, b, map, n, lon, lat, species,
+             f, next ? *next : StepArgs{}, ctrl, interact ? 1 : 0, next ? 1 : 0);
 }
 
 }  // namespace lm

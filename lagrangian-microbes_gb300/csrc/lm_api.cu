@@ -113,16 +113,23 @@ struct lm_ctx {
   uint32_t* plog = nullptr;
   uint32_t plog_cap = 0;
 
-  // step records of lm_step (rec_lon / rec_lat / rec_species): every step's record is packed into
-  // one slot of a device ring (caller order), and copied to the caller's arrays on the copy stream
-  // rec_st REC_SLOTS - 1 steps later, so the copies of step k overlap the kernels of the next steps
-  // instead of holding up the compute stream.
-  static constexpr int REC_SLOTS = 3;
+  // step records of lm_step (rec_lon / rec_lat / rec_species): the records of rec_batch steps are packed
+  // into one slot of a device ring (caller order), and copied to the caller's arrays, where they follow
+  // one another, on the copy stream rec_st after REC_SLOTS - 1 more batches are under way, so the copies
+  // overlap the kernels of later steps instead of holding up the compute stream.
+  struct RecBatch {
+    int64_t first;  // its first step
+    int steps, slot;
+  };
+  static constexpr int REC_SLOTS = 3, REC_STEPS = 8;
+  static constexpr size_t REC_BYTES = 4 << 20;
   cudaStream_t rec_st = nullptr;
   unsigned char* rec_ring = nullptr;
-  size_t rec_slot = 0;  // bytes per slot: lon [n] float, lat [n] float, species [n] int8
+  size_t rec_slot = 0;  // bytes per slot: lon [rec_batch][n] float, lat float, species int8
+  int rec_batch = 1, rec_next = 0;
   cudaEvent_t rec_done[REC_SLOTS] = {}, rec_copied[REC_SLOTS] = {};
-  std::vector<int64_t> rec_pending;  // steps whose records wait in the ring, oldest first
+  RecBatch rec_open = {0, 0, 0};
+  std::vector<RecBatch> rec_pending;  // full batches that wait in the ring, oldest first
   float *rec_lon = nullptr, *rec_lat = nullptr;
   int8_t* rec_sp = nullptr;
 
@@ -530,9 +537,9 @@ cudaError_t enqueue_interaction(lm_ctx* c, const StepArgs& a, uint32_t flags, bo
 
 // One fused step; `advect` false re-runs only the interaction part of an advected step. `begun`:
 // the previous step's end already started this one; `next` (the next step of the same call, which
-// advects): this step's end also starts that one.
+// advects): this step's end also starts that one. `end` false: the step's record ends it (record_step).
 cudaError_t enqueue_step(lm_ctx* c, const StepArgs& a, uint32_t flags, bool advect, bool begun = false,
-                         const StepArgs* next = nullptr) {
+                         const StepArgs* next = nullptr, bool end = true) {
   const Bufs b = bufs(c, false);
   if (!begun) PROF(c, P_BOOKKEEPING, launch_step_begin(b, advect ? &c->fv : nullptr, a, c->ctrl, c->st));
   if (advect) PROF(c, P_ADVECT, launch_advect(c->fv, a, b, c->ctrl, c->tune_advect_threads, c->st));
@@ -542,6 +549,7 @@ cudaError_t enqueue_step(lm_ctx* c, const StepArgs& a, uint32_t flags, bool adve
   }
   if (flags & LM_STEP_CENSUS) PROF(c, P_CENSUS, launch_census(b, c->ctrl, c->st));
   const bool counted = (flags & (LM_STEP_INTERACT | LM_STEP_COUNT_PAIRS)) != 0;
+  if (!end) return cudaGetLastError();
   if (next)
     PROF(c, P_BOOKKEEPING, launch_step_turn(b, &c->fv, *next, c->ctrl, counted, c->st));
   else
@@ -608,10 +616,16 @@ int check_time(lm_ctx* c, double t, double dt, int64_t n_steps) {
 
 void set_pair_params(lm_ctx* c, double r, int norm) { c->pp = make_pair_params(r, norm, (float)c->cell_factor); }
 
-// The record ring: slots sized for the current particle count, the copy stream and the events.
+// The record ring: slots sized for the current particle count, the copy stream and the events. A slot takes as many
+// steps as fit REC_BYTES, so that small records do not cost three copies and two events each: with one step a slot, 24
+// steps of 202,000 microbes took 447 us; with two (3.6 MB) 404, with four 415. (658 with each record
+// packed by three copies as well.)
 int ensure_rec_ring(lm_ctx* c) {
   const size_t n = c->ntotal;
-  const size_t slot = (9 * n + 255) / 256 * 256;
+  c->rec_batch = (int)std::max<size_t>(1, std::min<size_t>(lm_ctx::REC_STEPS, lm_ctx::REC_BYTES / std::max<size_t>(9 * n, 1)));
+  c->rec_open.steps = 0;
+  c->rec_pending.clear();  // (a call that failed may have left some)
+  const size_t slot = (9 * n * c->rec_batch + 255) / 256 * 256;
   if (!c->rec_st) {
     CK(cudaStreamCreateWithFlags(&c->rec_st, cudaStreamNonBlocking));
     for (int q = 0; q < lm_ctx::REC_SLOTS; ++q) {
@@ -637,59 +651,67 @@ int ensure_rec_ring(lm_ctx* c) {
   return LM_OK;
 }
 
-// Copy the oldest pending record from its ring slot to the caller's arrays (copy stream, after the
-// step that packed it). Copies into pageable memory return once they are done; the compute stream
-// keeps running the steps queued behind that record meanwhile.
+// Copy the oldest pending batch from its ring slot to the caller's arrays (copy stream, after the
+// steps that packed it). Copies into pageable memory return once they are done; the compute stream
+// keeps running the steps queued behind meanwhile.
 int flush_record(lm_ctx* c) {
-  const int64_t k = c->rec_pending.front();
+  const lm_ctx::RecBatch r = c->rec_pending.front();
   c->rec_pending.erase(c->rec_pending.begin());
-  const int q = (int)(k % lm_ctx::REC_SLOTS);
-  const size_t n = c->ntotal;
-  unsigned char* slot = c->rec_ring + (size_t)q * c->rec_slot;
-  CK(cudaStreamWaitEvent(c->rec_st, c->rec_done[q], 0));
-  if (c->rec_lon) CK(cudaMemcpyAsync(c->rec_lon + k * n, slot, n * 4, cudaMemcpyDeviceToHost, c->rec_st));
-  if (c->rec_lat) CK(cudaMemcpyAsync(c->rec_lat + k * n, slot + n * 4, n * 4, cudaMemcpyDeviceToHost, c->rec_st));
-  if (c->rec_sp) CK(cudaMemcpyAsync(c->rec_sp + k * n, slot + n * 8, n, cudaMemcpyDeviceToHost, c->rec_st));
-  CK(cudaEventRecord(c->rec_copied[q], c->rec_st));
+  const size_t n = c->ntotal, at = (size_t)r.first * n, m = r.steps * n, all = c->rec_batch * n;
+  unsigned char* slot = c->rec_ring + (size_t)r.slot * c->rec_slot;
+  CK(cudaStreamWaitEvent(c->rec_st, c->rec_done[r.slot], 0));
+  if (c->rec_lon) CK(cudaMemcpyAsync(c->rec_lon + at, slot, m * 4, cudaMemcpyDeviceToHost, c->rec_st));
+  if (c->rec_lat) CK(cudaMemcpyAsync(c->rec_lat + at, slot + all * 4, m * 4, cudaMemcpyDeviceToHost, c->rec_st));
+  if (c->rec_sp) CK(cudaMemcpyAsync(c->rec_sp + at, slot + all * 8, m, cudaMemcpyDeviceToHost, c->rec_st));
+  CK(cudaEventRecord(c->rec_copied[r.slot], c->rec_st));
   return LM_OK;
 }
 
-// Every pending record in the caller's arrays.
+// The open batch is complete.
+int close_batch(lm_ctx* c) {
+  if (!c->rec_open.steps) return LM_OK;
+  CK(cudaEventRecord(c->rec_done[c->rec_open.slot], c->st));
+  c->rec_pending.push_back(c->rec_open);
+  c->rec_open.steps = 0;
+  return LM_OK;
+}
+
+// Every record so far in the caller's arrays.
 int flush_records(lm_ctx* c) {
   int r;
+  if ((r = close_batch(c))) return r;
   while (!c->rec_pending.empty())
     if ((r = flush_record(c))) return r;
   if (c->rec_st) CK(cudaStreamSynchronize(c->rec_st));
   return LM_OK;
 }
 
+bool recording(const lm_ctx* c) { return c->ntotal && (c->rec_lon || c->rec_lat || c->rec_sp); }
+
 // One step's record (positions before the kick, species after the step) into a ring slot in
-// caller order; its copy to the host follows REC_SLOTS - 1 steps later (flush_record).
-int record_step(lm_ctx* c, int64_t k) {
+// caller order; it also ends the step, and starts `next`.
+int record_step(lm_ctx* c, int64_t k, uint32_t flags, const StepArgs* next) {
   const uint32_t n = c->ntotal;
-  if (!n || !(c->rec_lon || c->rec_lat || c->rec_sp)) return LM_OK;
-  const int q = (int)(k % lm_ctx::REC_SLOTS);
-  unsigned char* slot = c->rec_ring + (size_t)q * c->rec_slot;
-  float* lon = reinterpret_cast<float*>(slot);
-  float* lat = reinterpret_cast<float*>(slot + (size_t)n * 4);
-  int8_t* sp = reinterpret_cast<int8_t*>(slot + (size_t)n * 8);
-  CK(cudaStreamWaitEvent(c->st, c->rec_copied[q], 0));  // the slot's previous copy has read it
-  const bool direct = (c->n_ens == 1);
-  if (c->rec_lon) {
-    if (direct) CK(cudaMemcpyAsync(lon, c->plon, n * 4, cudaMemcpyDeviceToDevice, c->st));
-    else launch_unpad(c->plon, lon, c->map_d, c->nslots, c->st);
-  }
-  if (c->rec_lat) {
-    if (direct) CK(cudaMemcpyAsync(lat, c->plat, n * 4, cudaMemcpyDeviceToDevice, c->st));
-    else launch_unpad(c->plat, lat, c->map_d, c->nslots, c->st);
-  }
-  if (c->rec_sp) {
-    if (direct) CK(cudaMemcpyAsync(sp, c->species, n, cudaMemcpyDeviceToDevice, c->st));
-    else launch_unpad8(c->species, sp, c->map_d, c->nslots, c->st);
-  }
-  CK(cudaEventRecord(c->rec_done[q], c->st));
-  c->rec_pending.push_back(k);
+  if (!recording(c)) return LM_OK;
+  lm_ctx::RecBatch& o = c->rec_open;
   int r;
+  if (!o.steps) {
+    while ((int)c->rec_pending.size() >= lm_ctx::REC_SLOTS)
+      if ((r = flush_record(c))) return r;
+    o.first = k;
+    o.slot = c->rec_next;
+    c->rec_next = (c->rec_next + 1) % lm_ctx::REC_SLOTS;
+    CK(cudaStreamWaitEvent(c->st, c->rec_copied[o.slot], 0));  // the slot's previous copies have read it
+  }
+  const size_t all = (size_t)c->rec_batch * n, at = (size_t)o.steps * n;
+  unsigned char* slot = c->rec_ring + (size_t)o.slot * c->rec_slot;
+  launch_record(bufs(c, false), c->n_ens == 1 ? nullptr : c->map_d, n,
+                c->rec_lon ? reinterpret_cast<float*>(slot) + at : nullptr,
+                c->rec_lat ? reinterpret_cast<float*>(slot + all * 4) + at : nullptr,
+                c->rec_sp ? reinterpret_cast<int8_t*>(slot + all * 8) + at : nullptr, c->fv, next, c->ctrl,
+                (flags & (LM_STEP_INTERACT | LM_STEP_COUNT_PAIRS)) != 0, c->st);
+  if (++o.steps < c->rec_batch) return LM_OK;
+  if ((r = close_batch(c))) return r;
   while ((int)c->rec_pending.size() >= lm_ctx::REC_SLOTS)
     if ((r = flush_record(c))) return r;
   return LM_OK;
@@ -718,9 +740,9 @@ int run_steps(lm_ctx* c, double t, double dt, int64_t n_steps, int64_t step0, ui
       // the last step keeps its counters for lm_stats; a per-step census read keeps them per step
       const bool chain = k + 1 < n_steps && !rec_census;
       const StepArgs an = step_args(t + dt * (k + 1), dt, step0 + k + 1, kh, false);
-      CK(enqueue_step(c, a, flags, !(redo && k == s), chained, chain ? &an : nullptr));
+      CK(enqueue_step(c, a, flags, !(redo && k == s), chained, chain ? &an : nullptr, !recording(c)));
       chained = chain;
-      if ((r = record_step(c, k))) return r;
+      if ((r = record_step(c, k, flags, chain ? &an : nullptr))) return r;
       if (rec_census)
         CK(cudaMemcpyAsync(c->hstage + 4 * k, c->ctrl->census, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost, c->st));
     }

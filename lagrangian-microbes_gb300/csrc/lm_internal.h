@@ -293,6 +293,9 @@ void launch_interleave(const float* u, const float* v, float2* uv, size_t n, cud
 void launch_particles_in(const double* lon, const double* lat, const int8_t* sp, const int32_t* map, uint32_t S,
                          double org_lon, double org_lat, float* xo, float* yo, int8_t* species, uint8_t* status,
                          cudaStream_t st);
+// A step's record and its end; `next`: the next step of the call, which it starts.
+void launch_record(const Bufs& b, const int32_t* map, uint32_t n, float* lon, float* lat, int8_t* species,
+                   const FieldView& f, const StepArgs* next, Ctrl* ctrl, bool interact, cudaStream_t st);
 void launch_pack_state(const float* xo, const float* yo, const int8_t* species, const uint8_t* status,
                        const int32_t* map, uint32_t n, uint32_t S, int abs, float ox, float oy, unsigned char* out,
                        cudaStream_t st);
@@ -340,8 +343,6 @@ int events_grid(int device);
 cudaError_t launch_events(const Bufs& b, const StepArgs& a, Ctrl* ctrl, int grid, cudaStream_t st);
 void launch_census(const Bufs& b, Ctrl* ctrl, cudaStream_t st);
 const void* lm_census_kernel();  // one kernel of the library, for attribute queries
-void launch_unpad(const float* src, float* dst, const int32_t* map, uint32_t nslots, cudaStream_t st);
-void launch_unpad8(const int8_t* src, int8_t* dst, const int32_t* map, uint32_t nslots, cudaStream_t st);
 
 // ---- stable radix sort (k_sort.cu) ----
 constexpr int RS_BITS_MAX = 10;                      // digit width of one pass

@@ -235,3 +235,25 @@ def test_state_reads_and_rewinds_hold_every_microbe_in_its_place(lm, orc, small_
     assert sim.step_index == 7
     check(7)
     sim.close()
+
+
+@pytest.mark.parametrize("n, steps, locked", [(1, 20, True), (30000, 17, False), (58254, 9, True), (58255, 9, False), (600000, 3, True)])
+def test_records_in_batches_equal_the_states_step_by_step(lm, orc, small_field, n, steps, locked):
+    """Records copied in batches (8 steps, fewer from 58,255 microbes on, one from 466,000) against the state read after
+    every step: positions without a kick are the recorded ones, the species those after the step."""
+    rng = np.random.default_rng(n)
+    lons, lats, sp = 200 + rng.random(n), 25 + rng.random(n), rng.integers(1, 4, n).astype(np.int8)
+    t0 = float(small_field.times[0])
+    sims = [lm.Simulation(small_field, lons, lats, sp, radius=0.002, p_rs=0.7, p_pr=0.6, p_sp=0.8, seed=5) for _ in range(2)]
+    out = sims[0].record_buffers(steps) if locked else None
+    rec = sims[0].step(t0, 600.0, steps, record=True, out=out)
+    for k in range(steps):
+        sims[1].step(t0 + 600.0 * k, 600.0, 1, step0=k)
+        lon, lat, species, _ = sims[1].state()
+        np.testing.assert_array_equal(rec["lon"][k], lon)
+        np.testing.assert_array_equal(rec["lat"][k], lat)
+        np.testing.assert_array_equal(rec["species"][k], species)
+    assert sims[0].stats()["step"] == steps == sims[1].stats()["step"]
+    assert sims[0].stats()["pairs_total"] == sims[1].stats()["pairs_total"]
+    for s in sims:
+        s.close()
