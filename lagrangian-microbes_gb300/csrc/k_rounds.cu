@@ -121,6 +121,10 @@ constexpr int POLL_BATCH = 2;  // vertices whose state words one thread loads be
 // vertex's word, so no fences are needed.
 static_assert(SLAB == 8, "the tile path copies a slab row as two 16-byte loads");
 constexpr uint32_t TL_VMAX = 2048;                     // vertices per block at most
+// and at least, while there are so many: in small ensembles most pairs would cross blocks, and a handoff through global
+// memory takes an L2 round trip. 10,000 microbes on a lattice: 32 us with 64 each on 157 blocks, 24 with 320 on 32, 25
+// with 512, 35 with 1,024; 3,000 mixed 47, 34, 36; 40,000 mixed 47, 43, 46. Beyond 97,000 the equal share is larger.
+constexpr uint32_t TL_VMIN = 320;
 constexpr size_t TL_SMEM = TL_VMAX * (8 + 4 + 4 + 4 * SLAB);  // words, slot ids, degrees, lists
 
 __device__ __forceinline__ unsigned long long ld_sh(const unsigned long long* p) {
@@ -145,9 +149,8 @@ __device__ __forceinline__ uint32_t tl_entry(const Bufs& b, const TileSmem& t, u
 }
 
 // The pairs among cell-order vertices [g_lo, g_hi) (a group of whole ensembles, so no pair leaves
-// it), at most TL_VMAX per block: each block owns an equal share, in whole warps. Every block of the
-// grid takes part (whole 1,024-vertex columns left 64 of the 304 blocks idle at 490k, and all but a
-// few idle for a small ensemble run alone).
+// it), at most TL_VMAX per block: each block owns an equal share, in whole warps (whole 1,024-vertex
+// columns left 64 of the 304 blocks idle at 490k).
 template <int RD_THREADS>
 __device__ void tl_group(const Bufs& b, uint32_t step, Ctrl* ctrl, unsigned long long t0, uint32_t g_lo,
                          uint32_t g_hi) {
@@ -159,9 +162,9 @@ __device__ void tl_group(const Bufs& b, uint32_t step, Ctrl* ctrl, unsigned long
   t.deg = t.sid + TL_VMAX;
   t.lst = t.deg + TL_VMAX;
   const uint32_t n_g = g_hi - g_lo;
-  // every block gets an equal share, rounded up to whole warps (at most TL_VMAX: the caller checked
-  // that the group fits the grid's shared memory)
-  const uint32_t V = min(TL_VMAX, max(32u, (((n_g + gridDim.x - 1) / gridDim.x) + 31u) & ~31u));
+  // every block gets an equal share of at least TL_VMIN, rounded up to whole warps (at most TL_VMAX: the caller
+  // checked that the group fits the grid's shared memory); the last blocks may have none
+  const uint32_t V = min(TL_VMAX, max(TL_VMIN, (((n_g + gridDim.x - 1) / gridDim.x) + 31u) & ~31u));
   const uint32_t lo = min(g_hi, g_lo + blockIdx.x * V);
   const uint32_t hi = min(g_hi, lo + V);
   const uint32_t nloc = hi - lo;

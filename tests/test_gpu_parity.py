@@ -260,6 +260,19 @@ def test_gpu_interaction_beyond_the_blocks_lists_matches_oracle(engine, orc, n, 
         np.testing.assert_array_equal(got, want)
 
 
+@pytest.mark.parametrize("n", [319, 320, 321, 641, 304 * 320, 304 * 320 + 1])
+def test_gpu_interaction_of_small_shares_matches_oracle(engine, orc, n):
+    """Ensembles around one block's least share, and around the size from which every block has more."""
+    rng = np.random.default_rng(n)
+    side = np.sqrt(n * np.pi * 1e-4 / 7)
+    lon, lat = (200 + side * rng.random(n)).astype(np.float32), (25 + side * rng.random(n)).astype(np.float32)
+    sp = rng.integers(0, 5, n).astype(np.int8)
+    got, _, stats = _interact(engine, lon, lat, sp, 0.01, 2, (0.6, 0.7, 0.55), 11, 2, log=False)
+    want, m = orc.interact_step(lon, lat, sp, 0.01, 2, 0.6, 0.7, 0.55, 11, 2)
+    assert stats["pairs"] == m
+    np.testing.assert_array_equal(got, want)
+
+
 def test_gpu_interaction_other_species_values_unchanged(engine, orc):
     rng = np.random.default_rng(3)
     n = 2000
