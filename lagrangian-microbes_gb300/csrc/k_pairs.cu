@@ -567,7 +567,8 @@ __global__ void __launch_bounds__(COUNT_THREADS) k_count_pairs(Bufs b, PairParam
   } else {
     for (uint32_t rest = __ballot_sync(0xffffffffu, valid); rest;) {  // the warp's cells in turn
       const int first = __ffs(rest) - 1;
-      const uint32_t grp = __ballot_sync(0xffffffffu, valid && key == __shfl_sync(0xffffffffu, key, first));
+      const uint32_t first_key = __shfl_sync(0xffffffffu, key, first);
+      const uint32_t grp = __ballot_sync(0xffffffffu, valid && key == first_key);
       uint32_t a[COUNT_RUNS], e[COUNT_RUNS];
 #pragma unroll
       for (int q = 0; q < COUNT_RUNS; ++q) {
