@@ -91,14 +91,16 @@ struct Vertex {
   float2 ps;
 };
 
+__device__ __forceinline__ uint32_t ens_of(const Bufs& b, uint32_t s) { return b.n_ens == 1 ? 0u : b.sens[s]; }
+
 __device__ __forceinline__ Vertex load_vertex(const Bufs& b, uint32_t s) {
   Vertex v;
   v.s = s;
-  v.e = b.sens[s];
+  v.e = ens_of(b, s);
+  v.ps = b.spos[s];
   v.g = b.grids[v.e];
   v.base = b.ens[v.e].base;
-  cell_coords(v.g, b.skey[s] - v.g.cell_base, &v.cx, &v.cy);
-  v.ps = b.spos[s];
+  cell_of(v.g, v.ps.x, v.ps.y, &v.cx, &v.cy);
   return v;
 }
 
@@ -383,7 +385,7 @@ __global__ void __launch_bounds__(ORDER_THREADS) k_count_order(Bufs b, Ctrl* ctr
   const uint32_t n = ctrl->act_n;
   for (uint32_t q = blockIdx.x; q < n; q += gridDim.x) {
     const uint32_t key = b.act[q], c0 = b.cstart[key], c1 = b.cstart[key + 1];
-    const EnsGrid g = b.grids[b.sens[c0]];
+    const EnsGrid g = b.grids[ens_of(b, c0)];
     uint32_t cx, cy;
     cell_coords(g, key - g.cell_base, &cx, &cy);
     const float ox = g.x0 + (float)cx * g.c, oy = g.y0 + (float)cy * g.c, scale = 32.f * g.inv_c;
@@ -555,7 +557,7 @@ __global__ void __launch_bounds__(COUNT_THREADS) k_count_pairs(Bufs b, PairParam
   uint32_t r0[COUNT_RUNS] = {0, 0, 0, 0}, r1[COUNT_RUNS] = {0, 0, 0, 0}, key = NONE;
   if (valid) {
     v = load_vertex(b, s);
-    key = b.skey[s];
+    key = v.g.cell_base + cell_index(v.g, v.cx, v.cy);
     count_runs(v, b, r0, r1);
   }
   uint32_t most = 0;
@@ -792,7 +794,7 @@ __device__ __noinline__ void long_alone(const Bufs& b, const PairParams& pp, uin
                                         uint32_t d, unsigned long long o, const uint32_t* t0, const uint32_t* c) {
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t id0 = b.sid[s];
-  const EnsInfo& info = b.ens[b.sens[s]];
+  const EnsInfo& info = b.ens[ens_of(b, s)];
   const LongHead h = {order_hash_base(step, ((unsigned long long)info.seed_hi << 32) | info.seed_lo), id0 - info.base,
                       info.base};
   const int sp = b.species[id0];
@@ -1004,7 +1006,7 @@ __global__ void __launch_bounds__(LONG_WARPS * 32, 8) k_sweep_long(Bufs b, PairP
       neighbour_runs(b, v, r0, len);
 #pragma unroll
       for (int r = 0; r < 6; ++r) len[r] -= r0[r];
-      key_l = b.skey[s_l];
+      key_l = v.g.cell_base + cell_index(v.g, v.cx, v.cy);
     }
     uint32_t cand = 0;
 #pragma unroll
@@ -1023,7 +1025,7 @@ __global__ void __launch_bounds__(LONG_WARPS * 32, 8) k_sweep_long(Bufs b, PairP
                  __shfl_sync(0xffffffffu, o_l, k), t0, c);
     }
     if (mine) {
-      const uint32_t id = b.sid[s_l], e = b.sens[s_l];
+      const uint32_t id = b.sid[s_l], e = ens_of(b, s_l);
       const EnsInfo& info = b.ens[e];
       sh.hash[lane] = order_hash_base(step, ((unsigned long long)info.seed_hi << 32) | info.seed_lo);
       sh.ps[lane] = b.spos[s_l];

@@ -63,7 +63,7 @@ struct lm_ctx {
   float *xo = nullptr, *yo = nullptr, *plon = nullptr, *plat = nullptr;
   int8_t* species = nullptr;
   uint8_t* status = nullptr;
-  uint32_t *key = nullptr, *rank = nullptr, *sid = nullptr, *skey = nullptr, *sens = nullptr, *deg = nullptr;
+  uint32_t *key = nullptr, *rank = nullptr, *sid = nullptr, *sens = nullptr, *deg = nullptr;
   uint32_t *slab = nullptr, *longv = nullptr, *level = nullptr;
   unsigned long long* wstate = nullptr;
   uint32_t* act = nullptr;
@@ -293,7 +293,7 @@ int ensure_slots(lm_ctx* c, uint32_t slots, uint32_t n_ens) {
     if ((r = dalloc(c, &c->xo, cap)) || (r = dalloc(c, &c->yo, cap)) || (r = dalloc(c, &c->plon, cap)) ||
         (r = dalloc(c, &c->plat, cap)) || (r = dalloc(c, &c->species, cap)) || (r = dalloc(c, &c->status, cap)) ||
         (r = dalloc(c, &c->key, cap)) || (r = dalloc(c, &c->rank, cap)) || (r = dalloc(c, &c->sid, cap)) ||
-        (r = dalloc(c, &c->skey, cap)) || (r = dalloc(c, &c->sens, cap)) || (r = dalloc(c, &c->deg, cap)) ||
+        (r = dalloc(c, &c->sens, cap)) || (r = dalloc(c, &c->deg, cap)) ||
         (r = dalloc(c, &c->slab, (size_t)cap * SLAB)) ||
         (r = dalloc(c, &c->longv, cap)) || (r = dalloc(c, &c->wstate, cap)) ||
         (r = dalloc(c, &c->level, cap)) || (r = dalloc(c, &c->act, cap)) || (r = dalloc(c, &c->spos, cap)) ||
@@ -410,7 +410,6 @@ Bufs bufs(const lm_ctx* c, bool log) {
   b.cstart = c->cstart;
   b.csum = c->csum;
   b.sid = c->sid;
-  b.skey = c->skey;
   b.sens = c->sens;
   b.spos = c->spos;
   b.deg = c->deg;
@@ -910,7 +909,7 @@ int lm_ctx_destroy(lm_ctx* c) {
   if (c->gexec) cudaGraphExecDestroy(c->gexec);
   if (c->graph) cudaGraphDestroy(c->graph);
   void* bufs_[] = {c->uv,     c->xo,    c->yo,     c->plon,   c->plat,   c->species, c->status, c->key,
-                   c->rank,   c->sid,   c->skey,   c->sens,   c->deg,    c->slab,    c->longv,
+                   c->rank,   c->sid,   c->sens,   c->deg,    c->slab,    c->longv,
                    c->wstate, c->level,  c->act,    c->spos,
                    c->map_d,  c->block_ens, c->ens_d, c->grids, c->eord, c->ebox, c->census,  c->ccount, c->cstart,
                    c->csum,   c->ovf,   c->oprio,  c->ctrl,   c->plog,  c->scratch, c->snap_xo, c->snap_yo, c->snap_sp,
