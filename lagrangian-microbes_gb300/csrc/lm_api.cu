@@ -1311,7 +1311,7 @@ int lm_query_pairs(lm_ctx* c, int64_t n, const float* lon, const float* lat, int
     }
     break;
   }
-  if ((r = clear_err_bits(c, ERRB_NAN))) return r;  // non-finite query points are never paired
+  if ((c->hctrl->err & ERRB_NAN) && (r = clear_err_bits(c, ERRB_NAN))) return r;  // non-finite query points are never paired
   const uint64_t m = c->hctrl->n_dir / 2;
   *n_pairs = (int64_t)m;
   if (!pi || !pj || m == 0) return LM_OK;  // count query
@@ -1360,7 +1360,7 @@ int lm_count_pairs(lm_ctx* c, int64_t n, const float* lon, const float* lat, int
   PROF(c, P_BOOKKEEPING, launch_step_begin(bufs(c, false), nullptr, a, c->ctrl, c->st));
   CK(enqueue_interaction(c, a, LM_STEP_COUNT_PAIRS, true, false));
   if ((r = read_ctrl(c))) return r;
-  if ((r = clear_err_bits(c, ERRB_NAN))) return r;  // non-finite query points are never paired
+  if ((c->hctrl->err & ERRB_NAN) && (r = clear_err_bits(c, ERRB_NAN))) return r;  // non-finite query points are never paired
   *n_pairs = (int64_t)(c->hctrl->n_dir / 2);
   return LM_OK;
 }
