@@ -212,6 +212,7 @@ __device__ __forceinline__ void step_begin_body(const Bufs& b, const FieldView& 
     b.ebox[4 * e + 2] = 0u;           // max: start at the smallest encoding
     b.ebox[4 * e + 3] = 0u;
     b.census[4 * e + 0] = b.census[4 * e + 1] = b.census[4 * e + 2] = b.census[4 * e + 3] = 0u;
+    if (b.edir) b.edir[2 * e] = b.edir[2 * e + 1] = 0ull;
   }
   if (t == 0) {
     ctrl->act_n = 0;

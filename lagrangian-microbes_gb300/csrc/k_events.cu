@@ -21,12 +21,8 @@
 // Bound by the dependency chains and by issue: a dependent pair waits for one pass of a worker warp (some
 // 250 instructions), one across blocks for two L2 round trips.
 //
-// The rule: batches of ensembles of at least EV_SLOTS microbes (other contexts never launch this kernel,
-// and save the launch), when most list entries are in long lists and those are EV_MEAN entries long on
-// average. Per launch, polled / by events: 32 ensembles of 1e3-2e5 microbes on 0.5-3 degrees 1,108 / 636
-// us; 8 x 60k at 48 neighbours 921 / 496, at 22 329 / 241, at 15 181 / 172, at 11 138 / 139, at 7 80 / 91;
-// 3 x 10k at 28 neighbours 197 / 230. Where lists are short, polling wins: a ready pair is found by its
-// owner within a pass of a few instructions, and the claims and queues cost more than the polls saved.
+// Batches of ensembles of at least EV_SLOTS microbes launch this kernel (other contexts save the launch), and it takes
+// the groups of TileGroups::taken. 32 ensembles of 1e3-2e5 microbes on 0.5-3 degrees: 1,108 us polled, 636 by events.
 #include "lm_rounds.cuh"
 
 namespace lm {
@@ -37,7 +33,6 @@ constexpr uint32_t EV_VMIN = 128;      // and at least, while there are that man
                                        // pairs across blocks
 constexpr size_t EV_SMEM = EV_VMAX * (8 + 4 * SLAB + 2 + 2);  // words, rows, two queues
 constexpr int EV_THREADS = 512;
-constexpr uint32_t EV_MEAN = 16;       // mean length of the long lists from which the kernel takes the step
 constexpr uint32_t EV_WATCHERS = 8;    // watcher warps of a block
 constexpr uint32_t PENDING = 0xfffffffeu;  // a global word's partner: the owner looks it up (no valid entry)
 constexpr uint32_t EV_CLAIM = 1u << 29, EV_LONG = 1u << 28, EV_POS = MAX_DEGREE;  // fields of the upper half
@@ -418,27 +413,26 @@ __device__ void ev_group(const Bufs& b, Ctrl* ctrl, unsigned long long t0, uint3
   }
 }
 
-// Takes the step (ev_taken, so that k_rounds leaves it alone) when the rule holds and its ensembles fit the
-// blocks; otherwise nothing is done.
+// The groups of the rule (ev_taken: k_rounds leaves them out), when the ensembles fit the blocks; else nothing.
 __global__ void __launch_bounds__(EV_THREADS, 2) k_rounds_events(Bufs b, StepArgs a, Ctrl* ctrl) {
   __shared__ uint32_t cw[2];
   __shared__ TileGroups tg;
   extern __shared__ unsigned long long ev_raw[];
   if (threadIdx.x == 0) {
-    const uint32_t n_long = ((volatile uint32_t*)&ctrl->n_long)[0];
-    const unsigned long long dir = ((volatile unsigned long long*)&ctrl->n_dir)[0];
-    const unsigned long long in_long = ((volatile unsigned long long*)&ctrl->ovf_used)[0] - n_long;  // less the end marks
-    cw[0] = ((volatile uint32_t*)&ctrl->halt)[0] == 0u && in_long >= (unsigned long long)EV_MEAN * n_long && 2 * in_long >= dir;
+    // where fewer than half of the entries are in long lists no group is worth the look (15 us at 7 neighbours)
+    const unsigned long long in_long = ((volatile unsigned long long*)&ctrl->ovf_used)[0];
+    cw[0] = ((volatile uint32_t*)&ctrl->halt)[0] || 2 * in_long < ((volatile unsigned long long*)&ctrl->n_dir)[0];
     cw[1] = ((volatile uint32_t*)&ctrl->n_valid)[0];
   }
   __syncthreads();
-  if (!cw[0] || cw[1] == 0u) return;
+  if (cw[0] || cw[1] == 0u) return;
   if (b.plog || a.test_wait_ns) return;  // logged steps and the injected failure are k_rounds' own
-  make_groups(b, cw[1], gridDim.x * EV_VMAX, reinterpret_cast<uint32_t*>(ev_raw), (uint32_t)(EV_SMEM / sizeof(uint32_t)), tg);
-  if (tg.n <= 0) return;
+  make_groups(b, cw[1], gridDim.x * EV_VMAX, reinterpret_cast<uint32_t*>(ev_raw), (uint32_t)(EV_SMEM / sizeof(uint32_t)), tg, true);
+  if (tg.n <= 0 || !tg.taken) return;
   if (blockIdx.x == 0 && threadIdx.x == 0) ctrl->ev_taken = 1u;
   const unsigned long long t0 = globaltimer();
   for (int g = 0; g < tg.n; ++g) {
+    if (!((tg.taken >> g) & 1ull)) continue;
     ev_group(b, ctrl, t0, tg.lo[g], tg.lo[g + 1]);
     __syncthreads();  // the shared memory is the next group's
   }

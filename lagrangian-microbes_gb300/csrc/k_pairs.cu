@@ -287,6 +287,19 @@ __global__ void __launch_bounds__(SLOT_BLOCK, 6) k_sweep(Bufs b, PairParams pp, 
   __shared__ uint32_t w_dir[SLOT_BLOCK / 32], w_long[SLOT_BLOCK / 32], long_at;
   const uint32_t w = threadIdx.x >> 5, long_mask = __ballot_sync(0xffffffffu, is_long);
   const uint32_t dir = __reduce_add_sync(0xffffffffu, m);
+  if (b.edir) {  // per ensemble (a warp of one ensemble, the rule in cell order, adds once), degrees of 1,023 at most
+    const uint32_t m2 = min(m, 1023u), lead = __shfl_sync(0xffffffffu, e, 0);
+    if (__all_sync(0xffffffffu, e == lead || m == 0u)) {
+      const uint32_t sq = __reduce_add_sync(0xffffffffu, m2 * m2);
+      if (lane == 0 && dir) {
+        atomicAdd(b.edir + 2 * lead, (unsigned long long)dir);
+        atomicAdd(b.edir + 2 * lead + 1, (unsigned long long)sq);
+      }
+    } else if (m) {
+      atomicAdd(b.edir + 2 * e, (unsigned long long)m);
+      atomicAdd(b.edir + 2 * e + 1, (unsigned long long)(m2 * m2));
+    }
+  }
   if (lane == 0) {
     w_dir[w] = dir;
     w_long[w] = __popc(long_mask);

@@ -72,6 +72,7 @@ struct lm_ctx {
   EnsGrid* grids = nullptr;
   uint32_t* eord = nullptr;
   uint32_t* ebox = nullptr;
+  unsigned long long* edir = nullptr;
   uint32_t* census = nullptr;
 
   // cells
@@ -308,7 +309,7 @@ int ensure_slots(lm_ctx* c, uint32_t slots, uint32_t n_ens) {
   if (n_ens > c->ens_cap || !c->ens_d) {
     const uint32_t cap = std::max<uint32_t>(n_ens, 1);
     if ((r = dalloc(c, &c->ens_d, cap)) || (r = dalloc(c, &c->grids, cap)) || (r = dalloc(c, &c->eord, cap)) ||
-        (r = dalloc(c, &c->ebox, (size_t)4 * cap)) ||
+        (r = dalloc(c, &c->ebox, (size_t)4 * cap)) || (r = dalloc(c, &c->edir, (size_t)2 * cap)) ||
         (r = dalloc(c, &c->census, (size_t)4 * cap)))
       return r;
     CK(cudaMemsetAsync(c->census, 0, sizeof(uint32_t) * 4 * cap, c->st));
@@ -388,6 +389,9 @@ int upload_ens(lm_ctx* c) {
   return LM_OK;
 }
 
+// Dense batches may go by events (their groups are k_rounds' own only when both grids hold as much).
+bool events_run(const lm_ctx* c) { return c->n_ens > 1 && c->nslots >= EV_SLOTS && c->egrid > 0 && c->egrid == c->rgrid; }
+
 Bufs bufs(const lm_ctx* c, bool log) {
   Bufs b;
   b.ens = c->ens_d;
@@ -402,6 +406,7 @@ Bufs bufs(const lm_ctx* c, bool log) {
   b.plon = c->plon;
   b.plat = c->plat;
   b.ebox = c->ebox;
+  b.edir = events_run(c) ? c->edir : nullptr;
   b.grids = c->grids;
   b.eord = c->eord;
   b.key = c->key;
@@ -526,7 +531,7 @@ cudaError_t enqueue_interaction(lm_ctx* c, const StepArgs& a, uint32_t flags, bo
     cudaEvent_t pa = prof_begin(c);
     cudaError_t e = cudaSuccess;
     // dense batches (the kernel decides); other contexts save the launch
-    if (c->n_ens > 1 && c->nslots >= EV_SLOTS && c->egrid > 0 && !b.plog) e = launch_events(b, a, c->ctrl, c->egrid, st);
+    if (b.edir && !b.plog) e = launch_events(b, a, c->ctrl, c->egrid, st);
     if (e == cudaSuccess) e = launch_rounds(b, a, c->ctrl, c->rgrid, c->rblock, st);
     prof_end(c, P_ROUNDS, pa);
     if (e != cudaSuccess) return e;
@@ -911,7 +916,7 @@ int lm_ctx_destroy(lm_ctx* c) {
   void* bufs_[] = {c->uv,     c->xo,    c->yo,     c->plon,   c->plat,   c->species, c->status, c->key,
                    c->rank,   c->sid,   c->sens,   c->deg,    c->slab,    c->longv,
                    c->wstate, c->level,  c->act,    c->spos,
-                   c->map_d,  c->block_ens, c->ens_d, c->grids, c->eord, c->ebox, c->census,  c->ccount, c->cstart,
+                   c->map_d,  c->block_ens, c->ens_d, c->grids, c->eord, c->ebox, c->edir, c->census,  c->ccount, c->cstart,
                    c->csum,   c->ovf,   c->oprio,  c->ctrl,   c->plog,  c->scratch, c->snap_xo, c->snap_yo, c->snap_sp,
                    c->snap_st};
   for (void* p : bufs_)

@@ -89,7 +89,7 @@ struct Ctrl {
   int stage_k[3];               // frame brackets of this step's stage times t, t+dt/2, t+dt
   float stage_w[3];
   int stage_ok;                 // 0 when a stage time left the field's time axis
-  uint32_t ev_taken;            // k_rounds_events applied the step's pairs
+  uint32_t ev_taken;            // k_rounds_events applied pairs of this step (TileGroups::taken)
   uint32_t never;               // a flag nothing sets: the injected failure of the tests waits on it
 };
 
@@ -239,6 +239,7 @@ struct Bufs {
   float* plon;
   float* plat;
   uint32_t* ebox;     // [E][4] ordered-int encoded min x, min y, max x, max y
+  unsigned long long* edir;  // [E][2] directed entries and sum of squared degrees (NULL: k_rounds_events does not run)
   EnsGrid* grids;     // [E]
   uint32_t* eord;     // [E] the ensembles in the order of their key ranges (cell order)
   uint32_t* key;

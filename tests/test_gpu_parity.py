@@ -579,15 +579,20 @@ def test_gpu_cell_factor_does_not_change_results(engine, lm, orc):
     ((131072, 5, 1, 2000), 18),          # just over the rule's size, lists around its length
     ((20000,) * 9, 120),                 # long chains, most pairs across blocks
     ((330000, 330000, 40000), 20),       # two groups of ensembles
+    ((131072, 5, 1, 2000), 27),          # around the least density of a group
+    ((20000,) * 9, 60),                  # and the greatest
+    ((330000, 330000, 40000), 32),       # two groups by events
+    ((300000, 300000, 300000, 100000), (180, 32, 6, 40)),  # one polled (its entries see 170), one by events (28)
 ])
 def test_dense_batches_worked_off_by_events_equal_the_ensembles_alone(engine, lm, sizes, degree):
-    """Batches that k_rounds_events takes (at least 2^17 slots, long lists of 16 entries and more on
-    average), species values outside 1..3 among them: every species as when each ensemble runs alone
-    in a context, where k_rounds applies the pairs."""
-    rng = np.random.default_rng(len(sizes) + degree)
+    """Batches of at least 2^17 slots, whose groups k_rounds_events takes (26 to 64 neighbours) or leaves, species
+    values outside 1..3 among them: every species as when each ensemble runs alone in a context, where k_rounds
+    applies the pairs."""
+    degrees = np.broadcast_to(degree, len(sizes))
+    rng = np.random.default_rng(len(sizes) + int(degrees[0]))
     f = lm.synthetic_psi_field(195.0, 215.0, 20.0, 35.0, 0.25, n_frames=4, frame_seconds=3600.0, seed=9)
     members = []
-    for n in sizes:
+    for n, degree in zip(sizes, degrees):
         side = np.sqrt(n * np.pi * 1e-4 / degree)
         members.append((199 + 8 * rng.random() + side * rng.random(n), 24 + 4 * rng.random() + side * rng.random(n),
                         rng.integers(0, 5, n).astype(np.int8)))
