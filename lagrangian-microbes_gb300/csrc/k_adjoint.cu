@@ -156,8 +156,10 @@ struct VelJac {
   T inv_mc;                              // d flon / d U = 1 / (M cos lat)
 };
 
-// Velocity and Jacobian in cell (i, j) at bilinear fractions (a, b); `lat` is the absolute latitude.
-template <class T>
+// Velocity and Jacobian in cell (i, j) at bilinear fractions (a, b); `lat` is the absolute latitude. JAC false: the
+// velocity alone (the compiler drops what feeds only the Jacobian, but not the sine that comes with the cosine in
+// float64: 3.70 ms a forward of 48 steps of 100,000 microbes with it, 3.46 without).
+template <bool JAC = true, class T>
 __device__ __forceinline__ void vel_jac_at(const FieldView& f, int k, T w, int i, int j, T a, T b, T lat, T inv_dx,
                                            T inv_dy, VelJac<T>& r) {
   const float2* p = f.uv + ((size_t)k * f.ny + j) * f.nx + i;
@@ -184,8 +186,11 @@ __device__ __forceinline__ void vel_jac_at(const FieldView& f, int k, T w, int i
   const T M = (T)M_PER_DEG;
   T c, tan_lat;
   if constexpr (sizeof(T) == 8) {  // one argument reduction, one division
-    T sn;
-    sincospi(lat * (T(1) / T(180)), &sn, &c);
+    T sn = 0;
+    if constexpr (JAC)
+      sincospi(lat * (T(1) / T(180)), &sn, &c);
+    else
+      c = cospi_t(lat * (T(1) / T(180)));
     r.inv_mc = T(1) / (M * c);
     r.flon = u * r.inv_mc;
     tan_lat = sn * M * r.inv_mc;
@@ -206,14 +211,14 @@ __device__ __forceinline__ void vel_jac_at(const FieldView& f, int k, T w, int i
   r.b = b;
 }
 
-template <class T>
+template <bool JAC = true, class T>
 __device__ __forceinline__ bool vel_jac(const FieldView& f, const Geo<T>& g, int k, T w, T xo, T yo, VelJac<T>& r) {
   const T fx = (xo - g.gx0) * g.inv_dx;
   const T fy = (yo - g.gy0) * g.inv_dy;
   if (!(fx >= T(0) && fx <= g.max_fx && fy >= T(0) && fy <= g.max_fy)) return false;
   const int i = min((int)fx, f.nx - 2);
   const int j = min((int)fy, f.ny - 2);
-  vel_jac_at<T>(f, k, w, i, j, fx - (T)i, fy - (T)j, g.org_lat + yo, g.inv_dx, g.inv_dy, r);
+  vel_jac_at<JAC>(f, k, w, i, j, fx - (T)i, fy - (T)j, g.org_lat + yo, g.inv_dx, g.inv_dy, r);
   return true;
 }
 
@@ -231,10 +236,10 @@ template <>
 __device__ __forceinline__ bool rk4_t<double>(const FieldView& f, const Geo<double>& g, const AdjStep& s, double dt,
                                               double x, double y, double& nx, double& ny) {
   VelJac<double> J1, J2, J3, J4;
-  bool ok = vel_jac(f, g, s.k[0], s.wd[0], x, y, J1);
-  ok = ok && vel_jac(f, g, s.k[1], s.wd[1], x + 0.5 * dt * J1.flon, y + 0.5 * dt * J1.flat, J2);
-  ok = ok && vel_jac(f, g, s.k[1], s.wd[1], x + 0.5 * dt * J2.flon, y + 0.5 * dt * J2.flat, J3);
-  ok = ok && vel_jac(f, g, s.k[2], s.wd[2], x + dt * J3.flon, y + dt * J3.flat, J4);
+  bool ok = vel_jac<false>(f, g, s.k[0], s.wd[0], x, y, J1);
+  ok = ok && vel_jac<false>(f, g, s.k[1], s.wd[1], x + 0.5 * dt * J1.flon, y + 0.5 * dt * J1.flat, J2);
+  ok = ok && vel_jac<false>(f, g, s.k[1], s.wd[1], x + 0.5 * dt * J2.flon, y + 0.5 * dt * J2.flat, J3);
+  ok = ok && vel_jac<false>(f, g, s.k[2], s.wd[2], x + dt * J3.flon, y + dt * J3.flat, J4);
   if (!ok) return false;
   nx = x + (J1.flon + 2.0 * J2.flon + 2.0 * J3.flon + J4.flon) * (dt * (1.0 / 6.0));
   ny = y + (J1.flat + 2.0 * J2.flat + 2.0 * J3.flat + J4.flat) * (dt * (1.0 / 6.0));
@@ -474,7 +479,7 @@ __device__ __forceinline__ bool vel_jac_ds(const FieldView& f, const GeoDS& g, i
   float a, b;
   if (!ds_cell(ds_mul(ds_add(xo, g.mgx0), g.inv_dx), g.max_fx, f.nx - 1, i, a)) return false;
   if (!ds_cell(ds_mul(ds_add(yo, g.mgy0), g.inv_dy), g.max_fy, f.ny - 1, j, b)) return false;
-  vel_jac_at<float>(f, k, w, i, j, a, b, __fadd_rn(g.org_lat, yo.hi), g.inv_dxf, g.inv_dyf, r);
+  vel_jac_at(f, k, w, i, j, a, b, __fadd_rn(g.org_lat, yo.hi), g.inv_dxf, g.inv_dyf, r);
   return true;
 }
 
@@ -662,7 +667,7 @@ __global__ void __launch_bounds__(256) k_adj_signature(FieldView f, const AdjSte
       VelJac<T> J;
       const T sx = q == 0 ? x : x + hs[q] * dt * kx[q - 1];
       const T sy = q == 0 ? y : y + hs[q] * dt * ky[q - 1];
-      ok = vel_jac(f, g, ks[q], ws[q], sx, sy, J);
+      ok = vel_jac<false>(f, g, ks[q], ws[q], sx, sy, J);
       if (ok) {
         h = (h ^ ((J.cell / cw) * nx + J.cell % cw)) * 0x100000001B3ull;
         kx[q] = J.flon;
