@@ -134,7 +134,7 @@ struct lm_ctx {
   float *rec_lon = nullptr, *rec_lat = nullptr;
   int8_t* rec_sp = nullptr;
 
-  int rgrid = 0, rblock = 0, egrid = 0;
+  int rgrid = 0, rblock = 0, egrid = -1;  // egrid: of k_rounds_events, asked for by the first layout that may use it
   // tuning knobs (lm_set_tuning): block sizes and grid shapes that change speed, never results
   int tune_rounds_threads = 1024;  // interaction blocks: 1,024 threads x 2 vertices or 512 x 4
   int tune_long_per_sm = 8;        // long-list blocks per SM
@@ -354,6 +354,7 @@ int layout(lm_ctx* c, uint32_t n_ens, const int64_t* counts) {
   }
   if (slot) CK(cudaMemcpyAsync(c->map_d, c->hmap.data(), slot * sizeof(int32_t), cudaMemcpyHostToDevice, c->st));
   CK(cudaMemcpyAsync(c->block_ens, bens.data(), bens.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, c->st));
+  if (n_ens > 1 && c->nslots >= EV_SLOTS && c->egrid < 0) c->egrid = events_grid(c->device);
   // key ranges in index order until the first k_grid (which may reorder them; one ensemble never is)
   std::vector<uint32_t> eord(n_ens);
   for (uint32_t e = 0; e < n_ens; ++e) eord[e] = e;
@@ -901,7 +902,6 @@ int lm_ctx_create(int device, lm_ctx** out) {
       (e = cudaStreamSynchronize(c->st)) != cudaSuccess)
     return bail(fail(c, LM_ERR_CUDA, "ctrl init: %s", cudaGetErrorString(e)));
   c->rgrid = rounds_grid(device, c->tune_rounds_threads, &c->rblock);
-  c->egrid = events_grid(device);
   set_pair_params(c, 0.0, LM_NORM_L2);
   *out = c;
   return LM_OK;
