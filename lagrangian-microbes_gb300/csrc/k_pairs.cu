@@ -670,6 +670,7 @@ union LongShared {
   LongSmem one;
   LongArea many;
 };
+static_assert(sizeof(LongShared) % 16 == 0, "every warp's keys are read 16 bytes at a time");
 
 // A list that is done alone: what its pairs' priorities need.
 struct LongHead {

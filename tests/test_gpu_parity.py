@@ -582,6 +582,7 @@ def test_gpu_cell_factor_does_not_change_results(engine, lm, orc):
     ((131072, 5, 1, 2000), 27),          # around the least density of a group
     ((20000,) * 9, 60),                  # and the greatest
     ((330000, 330000, 40000), 32),       # two groups by events
+    ((640000, 30000), 14),               # one ensemble larger than the blocks' lists: state words only, for all
     ((300000, 300000, 300000, 100000), (180, 32, 6, 40)),  # one polled (its entries see 170), one by events (28)
 ])
 def test_dense_batches_worked_off_by_events_equal_the_ensembles_alone(engine, lm, sizes, degree):
