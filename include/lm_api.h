@@ -250,7 +250,8 @@ int lm_count_pairs_noalloc(const float* d_lon, const float* d_lat, int64_t n, do
  * field and the state every `checkpoint_every` steps; the backward sweep recomputes each segment
  * from its checkpoint. The velocity gradient is a deterministic segmented reduction (bit-identical
  * from run to run, no float atomics). All arrays are DEVICE pointers (float32), on ctx's stream
- * (lm_ctx_set_stream); errors through lm_last_error(ctx). Destroy tapes before their context. */
+ * (lm_ctx_set_stream); on the context's own stream a call comes after the work of the legacy default
+ * stream so far. Errors through lm_last_error(ctx). Destroy tapes before their context. */
 typedef struct lm_adjoint lm_adjoint;
 int lm_adjoint_create(lm_ctx* ctx, lm_adjoint** out);
 int lm_adjoint_destroy(lm_adjoint* adj);
