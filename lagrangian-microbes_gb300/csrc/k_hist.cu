@@ -21,18 +21,22 @@
 //     one bin, its pairs are counted at once;
 //   * a leaf pair whose bounds straddle one bin boundary is evaluated by two lanes: 64 values of a (as
 //     the squared chord of unit vectors) against that boundary's threshold in a;
-//   * what is left (close, ragged and diagonal leaf pairs) is evaluated pair by pair (dh_pair_bin).
+//   * what is left (close, ragged and diagonal leaf pairs, and those within 0.9 degrees of a pole) is
+//     evaluated pair by pair (dh_pair_bin).
 //
 // The definition of a pair's bin stays the reference's float32 chain (dh_bin: haversine_distance32
 // operation by operation, divisions and products rounded as written, the lower index first, with
 // CUDA's sinpif / cospif / asinf / log10f; round half to even; bins at or past `bins` go to an
 // overflow count, where the reference indexes past its array). The chain's 10 log10 d is off the
 // true value by 1.6e-5 at most (log10f within 2 ulp of values up to 7.3, the product by ten rounded
-// once, asinf within 2 ulp, the rest below 2e-6), a comparison of a by less than 3e-6, and the
-// hardware log2 by 1.4e-5 more, so a route decides a pair only when its value lies farther than
-// DH_MARGIN_A = 5e-5 (a alone) or DH_MARGIN = 1e-4 (log2) from the boundary; the chain itself decides
-// every other pair. LM_HIST_EXACT=1 in the environment makes every pair take the
-// chain (the tests compare the two).
+// once, asinf within 2 ulp, the rest below 2e-6), a bound of a taken from the chain's own cosines by
+// less than 3e-6, a squared chord by less than 1.8e-5 (dh_two_bins), and the hardware log2 by 1.4e-5
+// more. The chain's cosine comes from latitude / 180 rounded to float32, 1.5e-8 at most, so it is off by
+// 4.7e-8 / cos relative; the unit vectors do not carry that, and the chord differs from the chain by
+// 2.1e-7 / cos for it: 1.4e-5 at cos >= DH_COS_VEC = 1/64, below which chords are not taken. So a route
+// decides a pair only when its value lies farther than DH_MARGIN_A = 5e-5 (a alone) or DH_MARGIN = 1e-4
+// (log2) from the boundary; the chain itself decides every other pair. LM_HIST_EXACT=1 in the
+// environment makes every pair take the chain (the tests compare the two).
 //
 // Bound by instruction issue. At 490k microbes on 5 x 5 degrees (three species, 4.0e10 pairs) a call
 // took 100.0 ms with every pair evaluated by itself; counted by groups it takes 8.1 ms: 19 % of the
@@ -276,6 +280,7 @@ __device__ __forceinline__ int dh_bin(float la1, float lo1, float c1, float la2,
 
 constexpr float DH_MARGIN = 1e-4f;      // routes through the hardware log2
 constexpr float DH_MARGIN_A = 5e-5f;    // routes that compare a with a threshold
+constexpr float DH_COS_VEC = 0.015625f;  // smallest cos(latitude) of the leaf pairs decided by chords
 constexpr float DH_PI_360 = 8.72664625997164788e-3f;  // pi / 360
 constexpr float DH_NEAR_DEG = 24.0f;  // |dlat|, |dlon| up to which dh_hav<true> holds
 
@@ -548,7 +553,8 @@ __device__ __forceinline__ void dh_leaf_pairs(DhShared& sh, uint32_t sj, bool di
     }
     if (span == 1)
       atomicAdd(mine + k * DH_COPIES, ma * mb);
-    else if (span == 2 && ma * mb == DH_LEAF * DH_LEAF && lo >= sh.a_vec)
+    else if (span == 2 && ma * mb == DH_LEAF * DH_LEAF && lo >= sh.a_vec &&
+             fminf(sh.leaf[0][a].c0, sh.leaf[sj][b].c0) >= DH_COS_VEC)
       sh.list[atomicAdd(&sh.n_two, 1u)] = a | (b << 5) | ((uint32_t)k << 10);
     else
       sh.list[DH_LEAVES * DH_LEAVES - 1u - atomicAdd(&sh.n_gen, 1u)] = a | (b << 5);

@@ -188,3 +188,19 @@ def test_species_of_any_type_select_the_same_points(pdh, dtype):
         want = pdh.pairwise_distance_histogram(lat[species == k], lon[species == k], 70)
         np.testing.assert_array_equal(got[k][0], want[0])
         assert got[k][1] == want[1]
+
+
+@pytest.mark.parametrize("band", [(89.99, 90.0), (89.8, 90.0), (88.0, 88.5), (-90.0, -89.9)])
+def test_points_around_a_pole_keep_the_reference_chain_bins(pdh, monkeypatch, band):
+    """The chain's cos(latitude) carries the float32 rounding of latitude / 180, which is a large part of the cosine near
+    a pole: pairs there must not be decided by coordinates that do not carry it (integers, so exactly)."""
+    rng = np.random.default_rng(18)
+    n = 16_000
+    lat = rng.uniform(*band, n).astype(np.float32)
+    lon = rng.uniform(-180, 180, n).astype(np.float32)
+    fast = pdh.pairwise_distance_histogram(lat, lon, 70)
+    monkeypatch.setenv("LM_HIST_EXACT", "1")
+    exact = pdh.pairwise_distance_histogram(lat, lon, 70)
+    monkeypatch.delenv("LM_HIST_EXACT")
+    np.testing.assert_array_equal(fast[0], exact[0])
+    assert fast[1] == exact[1]
