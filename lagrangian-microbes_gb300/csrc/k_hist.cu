@@ -501,7 +501,7 @@ __device__ __forceinline__ void dh_two_bins(DhShared& sh, uint32_t sj, const DhR
         }
       }
     }
-    const uint32_t m = (uint32_t)below;
+    const uint32_t m = __float2uint_rn(below);  // (a place just below 1 may leave the sum an ulp short)
     if (m) atomicAdd(mine + k * DH_COPIES, m);
     if (m != rows * DH_LEAF) atomicAdd(mine + (k + 1) * DH_COPIES, rows * DH_LEAF - m);
   }

@@ -478,7 +478,7 @@ __device__ __forceinline__ uint32_t count_tile(const PairParams& pp, float scale
     f1 += fa + fb;
     f2 = fmaf(fa, fa, fmaf(fb, fb, f2));
   }
-  uint32_t c = (uint32_t)f1;
+  uint32_t c = __float2uint_rn(f1);  // (a place just below 1 may leave the sum an ulp short)
   if (f1 != f2) {
     c = 0;
     for (int k = 0; k < 32; ++k) c += within(pp, me, tile[k]) ? 1u : 0u;

@@ -139,3 +139,19 @@ def test_query_rows_of_every_list_length_are_in_order(engine, orc, size):
     oi, oj = orc.pairs(lon, lat, 0.01, 2)
     np.testing.assert_array_equal(pi, oi)
     np.testing.assert_array_equal(pj, oj)
+
+
+def test_count_at_the_inner_edge_of_the_float32_band(engine):
+    """A radius and a distance whose place in the band around the radius comes out 5 units in the last place below 1, so
+    that the sum of the places of a tile falls short of the whole number it stands for."""
+    r, d = 0.007813882993826751, np.float32(0.007813866)
+    assert float(d) < r
+    far = np.array([0.999 * d] * 5 + [d] + [1.003 * d] * 26, np.float32)
+    lon = np.concatenate([np.zeros(2048, np.float32), np.tile(far, 16)])
+    lat = np.zeros(lon.size, np.float32)
+    inside = int((far <= r).sum()) * 16
+    among = lambda m: m * (m - 1) // 2  # each of the two groups spans less than the radius
+    want = among(2048) + 2048 * inside + among(16 * far.size)
+    q = engine.PairQuery(r, np.inf)
+    assert q.count(lon, lat) == want
+    q.ctx.close()
