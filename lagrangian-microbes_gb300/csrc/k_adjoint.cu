@@ -10,13 +10,14 @@
 // For every stage it emits a record (a, b, dL/dU_s, dL/dV_s) for the field cell it sampled: the
 // stage's bilinear fractions inside its cell and its adjoint in field units.
 //
-// K7, the deterministic reduction of the records onto the grid. Sums are taken in integers (scaled by
-// a power of two from the cell's largest adjoint, at least 38 bits below it), so they do not depend on
-// the order of the records and no sort is needed:
+// K7, the deterministic reduction of the records onto the grid. A cell has 24 sums (two components, three
+// stage times, four corners). The terms of a sum are split at fixed powers of two, 2^(22 k), and the
+// parts are added as integers, so a sum does not depend on the order of the records and no sort is
+// needed; three parts are kept from the largest term down, at least 43 bits below it (FixSum):
 //   k_adj_alloc    reserves room for the entries of every occupied cell (K6 counted them) and lists
 //                  the cells, in whatever order its blocks come;
 //   k_adj_scatter  puts an entry (microbe, which of its stages) into each cell a microbe sampled;
-//   k_adj_gather   one warp per listed cell: its records into the four corner sums of each stage time;
+//   k_adj_gather   a warp for every 128 entries of a cell: their sums, put together by the cell's last warp;
 //   k_adj_nodes    adds, for every grid node, the four cells around it in a fixed order and spreads the
 //                  three stage times onto the field's frames with the linear-in-time weights.
 // The gradient is bit-identical from run to run and for every checkpoint interval. A sort of the
@@ -24,7 +25,8 @@
 // took 13 launches a step; here several steps share one set of launches when their records fit L2
 // together (a microbe's steps only depend on its own adjoint), and a batch is reduced on a stream of its
 // own beside the next one's steps. Forward and backward with the benchmark's loss: 5,000 microbes x 24
-// steps in f64 5.96 -> 2.87 ms, 100k x 48 in f32 6.62 -> 2.30 ms, 1M x 24 in ds 7.02 -> 4.54 ms.
+// steps in f64 5.96 -> 2.21 ms, 100k x 48 in f32 6.62 -> 1.62 ms, 1M x 24 in ds 7.02 -> 4.10 ms (0.6, 0.7 and
+// 0.5 ms of it through the loss in one kernel, k_loss.cu).
 #include <algorithm>
 
 #include "lm_field.cuh"
@@ -290,10 +292,9 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_forward(FieldView f, const 
 }
 
 // The backward of one RK4 step of microbe p from its four stage Jacobians (every precision):
-// lambda_{m+1} -> lambda_m in gx, gy, plus its 4 records. Returns the float bits of the records' largest
-// |dL/dU|, |dL/dV| (NaN above infinity above every number).
+// lambda_{m+1} -> lambda_m in gx, gy, plus its 4 records.
 template <class T>
-__device__ __forceinline__ uint32_t adj_tail(const VelJac<T>* J, T dt, T& gx, T& gy, float4* __restrict__ rec) {
+__device__ __forceinline__ void adj_tail(const VelJac<T>* J, T dt, T& gx, T& gy, float4* __restrict__ rec) {
   const T h6 = dt * (T(1) / T(6)), h3 = dt * (T(1) / T(3)), h2 = T(0.5) * dt;
   // dL/dk4, then back through x3 = x + dt k3, x2 = x + dt/2 k2, x1 = x + dt/2 k1
   const T g4x = h6 * gx, g4y = h6 * gy;
@@ -308,18 +309,10 @@ __device__ __forceinline__ uint32_t adj_tail(const VelJac<T>* J, T dt, T& gx, T&
   gy = gy + ((x0y + x1y) + (x2y + x3y));
   // records: dL/dU_s = dL/dk_s,lon / (M cos lat_s), dL/dV_s = dL/dk_s,lat / M (float32 for the reduction)
   const T invM = T(1) / (T)M_PER_DEG;
-  const float4 r[4] = {
-      make_float4((float)J[0].a, (float)J[0].b, (float)(g1x * J[0].inv_mc), (float)(g1y * invM)),
-      make_float4((float)J[1].a, (float)J[1].b, (float)(g2x * J[1].inv_mc), (float)(g2y * invM)),
-      make_float4((float)J[2].a, (float)J[2].b, (float)(g3x * J[2].inv_mc), (float)(g3y * invM)),
-      make_float4((float)J[3].a, (float)J[3].b, (float)(g4x * J[3].inv_mc), (float)(g4y * invM))};
-  uint32_t top = 0;
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    rec[k] = r[k];
-    top = max(top, max(__float_as_uint(r[k].z) & 0x7fffffffu, __float_as_uint(r[k].w) & 0x7fffffffu));
-  }
-  return top;
+  rec[0] = make_float4((float)J[0].a, (float)J[0].b, (float)(g1x * J[0].inv_mc), (float)(g1y * invM));
+  rec[1] = make_float4((float)J[1].a, (float)J[1].b, (float)(g2x * J[1].inv_mc), (float)(g2y * invM));
+  rec[2] = make_float4((float)J[2].a, (float)J[2].b, (float)(g3x * J[2].inv_mc), (float)(g3y * invM));
+  rec[3] = make_float4((float)J[3].a, (float)J[3].b, (float)(g4x * J[3].inv_mc), (float)(g4y * invM));
 }
 
 // A microbe has one entry in every cell its stages sampled: the stages of that cell as bits. The cell
@@ -334,23 +327,14 @@ __device__ __forceinline__ void for_other_cells(const uint4& c, F&& f) {
   if (c.w != c.x && c.w != c.y && c.w != c.z) f(c.w, 8u);
 }
 
-// Count the entries of one microbe's step and raise its cells' largest adjoint to `top` (every lane of the
-// warp calls this; `ok` false: no entries). Lanes with the same first cell, the usual case, share the
-// atomics.
-__device__ __forceinline__ void count_entries(const AdjBatch& b, int q, bool ok, const uint4& c, uint32_t top) {
+// Count the entries of one microbe's step (every lane of the warp calls this; `ok` false: no entries). Lanes
+// with the same first cell, the usual case, share the atomic.
+__device__ __forceinline__ void count_entries(const AdjBatch& b, int q, bool ok, const uint4& c) {
   uint32_t* count = b.count + (size_t)q * b.cells;
-  uint32_t* most = b.top + (size_t)q * b.cells;
   const uint32_t peers = __match_any_sync(0xffffffffu, ok ? c.x : NONE);
-  const uint32_t t = __reduce_max_sync(peers, top);
   if (!ok) return;
-  if ((threadIdx.x & 31u) == (uint32_t)(__ffs(peers) - 1)) {
-    atomicAdd(count + c.x, (uint32_t)__popc(peers));
-    atomicMax(most + c.x, t);
-  }
-  for_other_cells(c, [&](uint32_t cell, uint32_t) {
-    atomicAdd(count + cell, 1u);
-    atomicMax(most + cell, top);
-  });
+  if ((threadIdx.x & 31u) == (uint32_t)(__ffs(peers) - 1)) atomicAdd(count + c.x, (uint32_t)__popc(peers));
+  for_other_cells(c, [&](uint32_t cell, uint32_t) { atomicAdd(count + cell, 1u); });
 }
 
 // Steps m_last, m_last - 1, ... (`steps` of them) of every microbe: lambda_{m+1} -> lambda_m, plus 4
@@ -373,7 +357,6 @@ __global__ void __launch_bounds__(ADJ_THREADS, sizeof(T) == 8 ? 1 : 7) k_adj_ste
     VelJac<T> J[4];
     bool ok = live && sts[o] == STATUS_OK;
     uint4 c = make_uint4(NONE, NONE, NONE, NONE);
-    uint32_t top = 0;
     if (ok) {
       const T x = xs[o], y = ys[o];
       ok = ok && vel_jac(f, g, s.k[0], w0, x, y, J[0]);
@@ -386,12 +369,12 @@ __global__ void __launch_bounds__(ADJ_THREADS, sizeof(T) == 8 ? 1 : 7) k_adj_ste
         ok = isfinite(nx) && isfinite(ny);
       }
       if (ok) {
-        top = adj_tail<T>(J, dt, gx, gy, b.rec + 4 * ((size_t)q * b.n + p));
+        adj_tail<T>(J, dt, gx, gy, b.rec + 4 * ((size_t)q * b.n + p));
         c = make_uint4(J[0].cell, J[1].cell, J[2].cell, J[3].cell);
       }
     }
     if (live) b.cell[(size_t)q * b.n + p] = c;
-    count_entries(b, q, ok, c, top);
+    count_entries(b, q, ok, c);
   }
   if (live) {
     lx[p] = gx;
@@ -590,17 +573,16 @@ __global__ void __launch_bounds__(ADJ_THREADS, 7) k_adj_step_ds(FieldView f, con
     VelJac<float> J[4];
     bool ok = live && sts[o] == STATUS_OK;
     uint4 c = make_uint4(NONE, NONE, NONE, NONE);
-    uint32_t top = 0;
     if (ok) {
       DS nx, ny;
       ok = rk4_ds(f, g, s, dt, xs[o], ys[o], J, nx, ny) && ds_finite(nx) && ds_finite(ny);
       if (ok) {
-        top = adj_tail<float>(J, dt, gx, gy, b.rec + 4 * ((size_t)q * b.n + p));
+        adj_tail<float>(J, dt, gx, gy, b.rec + 4 * ((size_t)q * b.n + p));
         c = make_uint4(J[0].cell, J[1].cell, J[2].cell, J[3].cell);
       }
     }
     if (live) b.cell[(size_t)q * b.n + p] = c;
-    count_entries(b, q, ok, c, top);
+    count_entries(b, q, ok, c);
   }
   if (live) {
     lx[p] = gx;
@@ -686,48 +668,47 @@ __global__ void __launch_bounds__(256) k_adj_signature(FieldView f, const AdjSte
 
 // ---------------------------------------------------------------- K7: reduction onto the grid
 
-// Room for the entries of every occupied cell of step blockIdx.y (consecutive from place[c]) and the
-// list of items, one per ADJ_ITEM entries of a cell: one reservation of each per block.
+// Room for the entries of every occupied cell of step blockIdx.y (consecutive from place[c]), the list of
+// items, one per ADJ_ITEM entries of a cell, and room for the parts of cells of several items: one
+// reservation of each per block.
 constexpr int ALLOC_THREADS = 512;
-__global__ void __launch_bounds__(ALLOC_THREADS) k_adj_alloc(AdjBatch b, uint32_t items_cap) {
+__global__ void __launch_bounds__(ALLOC_THREADS) k_adj_alloc(AdjBatch b) {
   pdl_wait();
-  __shared__ uint32_t we[ALLOC_THREADS / 32], wl[ALLOC_THREADS / 32], base[2];
+  __shared__ uint32_t ws[3][ALLOC_THREADS / 32], base[3];
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const uint32_t c = blockIdx.x * ALLOC_THREADS + threadIdx.x;
   const size_t o = (size_t)blockIdx.y * b.cells;
   const uint32_t m = c < b.cells ? b.count[o + c] : 0u, items = (m + ADJ_ITEM - 1) / ADJ_ITEM;
-  uint32_t se = m, sl = items;  // inclusive sums over the warp
+  const uint32_t parts = items > 1 ? items : 0u;
+  uint32_t sum[3] = {m, items, parts};  // inclusive sums over the warp
   for (int d = 1; d < 32; d <<= 1) {
-    const uint32_t x = __shfl_up_sync(0xffffffffu, se, d), y = __shfl_up_sync(0xffffffffu, sl, d);
-    if (lane >= (uint32_t)d) {
-      se += x;
-      sl += y;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const uint32_t x = __shfl_up_sync(0xffffffffu, sum[k], d);
+      if (lane >= (uint32_t)d) sum[k] += x;
     }
   }
-  if (lane == 31) {
-    we[warp] = se;
-    wl[warp] = sl;
-  }
+  if (lane == 31)
+    for (int k = 0; k < 3; ++k) ws[k][warp] = sum[k];
   __syncthreads();
-  if (threadIdx.x < 2) {
-    uint32_t* w = threadIdx.x ? wl : we;
+  if (threadIdx.x < 3) {
+    uint32_t* w = ws[threadIdx.x];
     uint32_t t = 0;
     for (int k = 0; k < ALLOC_THREADS / 32; ++k) {
       const uint32_t x = w[k];
       w[k] = t;
       t += x;
     }
-    base[threadIdx.x] = t ? atomicAdd(b.total + 2 * blockIdx.y + threadIdx.x, t) : 0u;
+    base[threadIdx.x] = t ? atomicAdd(b.total + 4 * blockIdx.y + threadIdx.x, t) : 0u;
   }
   __syncthreads();
   if (!m) return;
-  const uint32_t at = base[0] + we[warp] + se - m;
+  const uint32_t at = base[0] + ws[0][warp] + sum[0] - m;
+  const uint32_t part = base[2] + ws[2][warp] + sum[2] - parts;
   b.place[o + c] = at;
-  uint4* list = b.list + (size_t)blockIdx.y * items_cap + base[1] + wl[warp] + sl - items;
-  for (uint32_t k = 0; k < items; ++k) list[k] = make_uint4(c, at + k * ADJ_ITEM, min(ADJ_ITEM, m - k * ADJ_ITEM), m);
-  if (items > 1) {  // several warps add to the cell's sums
-    for (int k = 0; k < 24; ++k) b.csum[(o + c) * 24 + k] = 0ll;
-  }
+  uint4* list = b.list + (size_t)blockIdx.y * adj_items(b.n, b.cells) + base[1] + ws[1][warp] + sum[1] - items;
+  for (uint32_t k = 0; k < items; ++k)
+    list[k] = make_uint4(c, at + k * ADJ_ITEM, min(ADJ_ITEM, m - k * ADJ_ITEM), parts ? part + k : NONE);
 }
 
 // Entries of the microbes' steps into their cells, in whatever order they come.
@@ -748,141 +729,236 @@ __global__ void __launch_bounds__(256) k_adj_scatter(AdjBatch b) {
   for_other_cells(c, [&](uint32_t cell, uint32_t mask) { ent[atomicAdd(place + cell, 1u)] = make_uint2(p, mask); });
 }
 
-// Integer sum of products v scaled into [-2^21, 2^21]: hi takes the nearest integer, lo the remainder
-// in 2^-20. Adding 1.5 * 2^23 leaves the integer in a float's low bits; the sums run on the raw bits
-// (the constant is taken out at the end), so a term is four FMA-pipe operations and two adds.
-constexpr float FIX_MAGIC = 12582912.0f;  // 1.5 * 2^23
+// Sum of float32 terms as three integers. A term is split at the fixed powers of two 2^(22 k): its part in
+// units of 2^(22 k) is the rest of the parts above, rounded to the nearest integer, so in any unit above it
+// a term is 0 and its parts do not depend on where the splitting starts. The sum keeps three units, from
+// the first in which the largest term has at most 21 bits (`top`) down: 43 bits below that term at least,
+// where the term itself was rounded 24 below. (One scale for the 24 sums of a cell, two parts below the
+// largest adjoint of all, lost the small terms of a corner beside a large adjoint elsewhere in the cell:
+// 1e-2 of the sum at a ratio of 1e-10.) Adding 1.5 * 2^23 leaves the integer in a float's low bits, and
+// the sums run on the raw bits (the constant is taken out at the end).
+constexpr float FIX_MAGIC = 12582912.0f, FIX_UNIT = 4194304.0f;  // 1.5 * 2^23, 2^22
 struct FixSum {
-  uint32_t hi, lo;
+  uint32_t a, b, c;
 };
-__device__ __forceinline__ void fix_add(FixSum& a, float v, float scale) {
+__device__ __forceinline__ void fix_add(FixSum& s, float v, float scale) {
   const float t = fmaf(v, scale, FIX_MAGIC);
-  const float rest = fmaf(v, scale, FIX_MAGIC - t);  // exact, in [-1/2, 1/2]
-  a.hi += __float_as_uint(t);
-  a.lo += __float_as_uint(fmaf(rest, 1048576.0f, FIX_MAGIC));
+  const float r = fmaf(v, scale, FIX_MAGIC - t);  // exact, in [-1/2, 1/2]
+  const float t1 = fmaf(r, FIX_UNIT, FIX_MAGIC);
+  const float r1 = fmaf(r, FIX_UNIT, FIX_MAGIC - t1);  // exact
+  s.a += __float_as_uint(t);
+  s.b += __float_as_uint(t1);
+  s.c += __float_as_uint(fmaf(r1, FIX_UNIT, FIX_MAGIC));
+}
+// The first unit of terms up to the one of float bits `most` is 2^(22 (top - 6)): 1 <= top <= 11 (from 1, the
+// last unit lies below the smallest float). Its reciprocal.
+__device__ __forceinline__ uint32_t fix_top(uint32_t most) { return max(((most >> 23) + 6u) / 22u, 1u); }
+__device__ __forceinline__ float fix_scale(uint32_t top) { return __uint_as_float((259u - 22u * top) << 23); }
+
+// A sum that is infinite or undefined: `top` is FIX_SPECIAL, and a says which of the terms were there.
+constexpr uint32_t FIX_SPECIAL = 15u, FIX_NAN = 1u, FIX_PLUS = 2u, FIX_MINUS = 4u;
+__device__ __forceinline__ uint32_t fix_flags(float v) {
+  return isfinite(v) ? 0u : isnan(v) ? FIX_NAN : v > 0.f ? FIX_PLUS : FIX_MINUS;
 }
 
-// v[i] summed over the warp, for i = lane & 15 (12 values, zeros above): every step but the last
-// halves the values a lane keeps, 16 exchanges in all.
-__device__ __forceinline__ uint32_t sum_by_lane(const uint32_t (&in)[12]) {
+// (a 2^44 + b 2^22 + c) units of the last place of `top`, rounded once.
+__device__ __forceinline__ float fix_value(uint32_t top, long long a, long long b, long long c) {
+  if (top == FIX_SPECIAL)
+    return ((uint32_t)a & FIX_NAN) || (a & (FIX_PLUS | FIX_MINUS)) == (FIX_PLUS | FIX_MINUS) ? NAN
+           : a & FIX_PLUS                                                                   ? INFINITY
+                                                                                            : -INFINITY;
+  b += c >> 22;
+  a += b >> 22;
+  const long long low = (b & 0x3fffffll) << 22 | (c & 0x3fffffll);  // in [0, 2^44)
+  const long long mag = a < 0 ? -a : a;
+  int e = 22 * ((int)top - 6) - 44;
+  long long x;  // at least 41 bits, or all of them; what is cut off leaves its mark in the last bit
+  if (mag < 1ll << 18) {
+    x = (a << 44) + low;
+  } else if (mag < 1ll << 32) {
+    x = ((a << 29) + (low >> 15)) | (low & 0x7fffll ? 1ll : 0ll);
+    e += 15;
+  } else {
+    x = ((a << 8) + (low >> 36)) | (low & 0xfffffffffll ? 1ll : 0ll);
+    e += 36;
+  }
+  return ldexpf(__ll2float_rn(x), e);
+}
+
+// Eight values of every lane combined over the lanes of the same last two bits: lane l gets value
+// (l >> 4 & 1) * 4 + (l >> 3 & 1) * 2 + (l >> 2 & 1). Every step halves what a lane keeps. Lanes of last
+// bits 1 and 2 (the two stages at t + dt/2) then get each other's too.
+template <class F>
+__device__ __forceinline__ uint32_t by_stage(const uint32_t (&in)[8], F&& op) {
   const uint32_t lane = threadIdx.x & 31u;
   uint32_t v[8];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const uint32_t up = i + 8 < 12 ? in[i + 8 < 12 ? i + 8 : 0] : 0u;
-    const uint32_t send = lane & 8u ? in[i] : up, keep = lane & 8u ? up : in[i];
-    v[i] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
-  }
+  for (int i = 0; i < 8; ++i) v[i] = in[i];
 #pragma unroll
   for (int h = 4; h > 0; h >>= 1) {
+    const bool upper = (lane & (4u * h)) != 0u;
 #pragma unroll
     for (int i = 0; i < h; ++i) {
-      const uint32_t send = lane & (uint32_t)h ? v[i] : v[i + h], keep = lane & (uint32_t)h ? v[i + h] : v[i];
-      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, h);
+      const uint32_t send = upper ? v[i] : v[i + h], keep = upper ? v[i + h] : v[i];
+      v[i] = op(keep, __shfl_xor_sync(0xffffffffu, send, 4 * h));
     }
   }
-  return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 16);
+  const uint32_t other = __shfl_xor_sync(0xffffffffu, v[0], 3), s = lane & 3u;
+  return s == 1u || s == 2u ? op(v[0], other) : v[0];
 }
 
-// The stages `mask` of one entry's records into one component's sums, the four corners (00, 01, 10, 11)
-// of each stage time: stage 1 at t (group 0), stages 2 and 3 at t + dt/2 (group 1), stage 4 at t + dt
-// (group 2).
-template <int G>
-__device__ __forceinline__ void gather_add(const float4& r, bool V, float scale, FixSum (&acc)[12]) {
-  const float a = r.x, b = r.y, g = V ? r.w : r.z;
+// The terms of a record: corners (00, 01, 10, 11) of dL/dU, then of dL/dV.
+template <class F>
+__device__ __forceinline__ void for_terms(const float4& r, F&& f) {
+  const float a = r.x, b = r.y;
   const float w[4] = {(1.f - a) * (1.f - b), a * (1.f - b), (1.f - a) * b, a * b};
 #pragma unroll
-  for (int q = 0; q < 4; ++q) fix_add(acc[4 * G + q], w[q] * g, scale);
+  for (int q = 0; q < 4; ++q) {
+    f(q, w[q] * r.z);
+    f(4 + q, w[q] * r.w);
+  }
 }
 
-__device__ __forceinline__ uint32_t adjoint_bits(const float4& r) {
-  return max(__float_as_uint(r.z) & 0x7fffffffu, __float_as_uint(r.w) & 0x7fffffffu);
-}
+// A sum in parts of its own `top`, and another one added to it: the parts below the larger top's last unit
+// are dropped from either (there they are the same integers whatever the sum's other terms).
+struct FixTotal {
+  uint32_t top = 0u;
+  long long a = 0, b = 0, c = 0;
+  __device__ __forceinline__ void join(uint32_t t, int xa, int xb, int xc) {
+    if (t == FIX_SPECIAL || top == FIX_SPECIAL) {
+      a = (top == FIX_SPECIAL ? a : 0ll) | (t == FIX_SPECIAL ? (long long)xa : 0ll);
+      top = FIX_SPECIAL;
+      return;
+    }
+    const uint32_t up = t > top ? t - top : 0u, down = t < top ? top - t : 0u;
+    if (up) {
+      c = up == 1u ? b : up == 2u ? a : 0ll;
+      b = up == 1u ? a : 0ll;
+      a = 0ll;
+      top = t;
+    }
+    a += down == 0u ? xa : 0;
+    b += down == 0u ? xb : down == 1u ? xa : 0;
+    c += down == 0u ? xc : down == 1u ? xb : down == 2u ? xa : 0;
+  }
+  __device__ __forceinline__ float value() const { return fix_value(top, a, b, c); }
+};
 
-// A cell's scale is 2^adj_scale_bits: 2^(21 - e) for 2^e above its largest |dL/dU|, |dL/dV|, so a term
-// is kept to 2^(e - 42), where its own float32 rounding is 2^-25 of it (coarser by the factor that
-// keeps the 64-bit sums of more than 2^20 entries in range). m: entries of the cell.
-__device__ __forceinline__ int adj_scale_bits(uint32_t top, uint32_t m) {
-  const int big = m > (1u << 20) ? 12 - __clz(m) : 0;  // log2(m) - 20, rounded up
-  return 21 - big - (max((int)(top >> 23), 20) - 126);
-}
-constexpr uint32_t ADJ_NOT_FINITE = 0x7f800000u;  // `top` from here: some adjoint is infinite or NaN
-
-// Two warps per item, one for dL/dU and one for dL/dV, one entry per lane at a time. Cells of several
-// items add up with integer atomics. Sums that are not finite are formed in float by the first item.
-__global__ void __launch_bounds__(256, 4) k_adj_gather(AdjBatch b, uint32_t items_cap) {
+// A warp per item: four lanes take an entry, one each of its stages (stage 1 at t, 2 and 3 at t + dt/2, 4 at
+// t + dt), so a warp reads the records of eight entries at a time and holds those of ADJ_CHUNK in
+// registers: the largest terms first, then the sums. The items of a cell of several leave their sums in
+// `part`, and the warp that finishes the last one puts them together (in integers, whichever it is).
+// Bound by instruction issue (64 % of the slots; the rest is latency of the records' loads): 47 us a step for
+// 1M microbes, where two parts a term, scaled by the cell's largest adjoint, took 35 and kept too few bits
+// (the counting of the largest by k_adj_step took 18 us more there: 66 -> 48). Forward and backward of 24
+// such steps: chunks of 32 entries at four blocks an SM 4.13 ms, at three 4.20, at five (spills) 4.28, chunks
+// of 64 at three 4.21; items of 64 4.22, of 256 4.38; the records read twice (69 us) 4.69.
+constexpr int GATHER_THREADS = 256, GATHER_BLOCKS = 4;  // threads a block, blocks an SM
+constexpr uint32_t ADJ_ROUNDS = 4, ADJ_CHUNK = 8 * ADJ_ROUNDS;
+__global__ void __launch_bounds__(GATHER_THREADS, GATHER_BLOCKS) k_adj_gather(AdjBatch b) {
   pdl_wait();
-  const uint32_t lane = threadIdx.x & 31u, q = blockIdx.y;
-  const uint32_t nt = b.total[2 * q + 1];
+  const uint32_t lane = threadIdx.x & 31u, s = lane & 3u, q = blockIdx.y;
+  const uint32_t nt = b.total[4 * q + 1];
   const size_t oc = (size_t)q * b.cells;
-  const uint4* list = b.list + (size_t)q * items_cap;
+  const uint4* list = b.list + (size_t)q * adj_items(b.n, b.cells);
   const uint2* ent = b.ent + (size_t)q * 4 * b.n;
   const float4* rec = b.rec + (size_t)q * 4 * b.n;
-  const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, stride = (gridDim.x * blockDim.x) >> 6;
-  const bool V = warp & 1u;
-  const uint32_t one = __float_as_uint(FIX_MAGIC);
-  uint4 next = (warp >> 1) < nt ? list[warp >> 1] : make_uint4(0u, 0u, 0u, 0u);
-  for (uint32_t t = warp >> 1; t < nt; t += stride) {
-    const uint32_t c = next.x, lo = next.y, m = next.z, all = next.w;
-    const uint32_t top = b.top[oc + c];
-    next = t + stride < nt ? list[t + stride] : make_uint4(0u, 0u, 0u, 0u);
-    long long* out = b.csum + (oc + c) * 24;  // per stage time: the corners of dL/dU, then of dL/dV
-    if (top >= ADJ_NOT_FINITE) {
-      const bool first = all <= ADJ_ITEM || lo + all - 1u == b.place[oc + c] - 1u;  // place: one past the cell
-      if (!V && first && lane < 24) {
-        float s = 0.f;
-        for (uint32_t i = 0; i < all; ++i) {
-          const uint2 x = ent[lo + i];
-          for (uint32_t k = 0; k < 4; ++k) {
-            if (!((x.y >> k) & 1u) || (k + 1) / 2 != lane / 8) continue;
-            const float4 z = rec[4 * (size_t)x.x + k];
-            s += (lane & 1u ? z.x : 1.f - z.x) * (lane & 2u ? z.y : 1.f - z.y) * (lane & 4u ? z.w : z.z);
-          }
-        }
-        out[lane] = (long long)__float_as_uint(s);
+  int4* part = b.part + (size_t)q * adj_parts(b.n) * 24;
+  // where this lane's sum goes: stage time, then by_stage's value (lanes of last bits 2 hold the same as those of 1)
+  const uint32_t at = (s == 0u ? 0u : s == 3u ? 16u : 8u) + ((lane >> 4 & 1u) * 4u + (lane >> 3 & 1u) * 2u + (lane >> 2 & 1u));
+  const uint32_t stride = gridDim.x * (GATHER_THREADS / 32);
+  uint32_t t = blockIdx.x * (GATHER_THREADS / 32) + (threadIdx.x >> 5);
+  uint4 next = t < nt ? list[t] : make_uint4(0u, 0u, 0u, 0u);
+  for (; t < nt; t += stride) {
+    const uint4 item = next;
+    next = t + stride < nt ? list[t + stride] : item;
+    const uint32_t c = item.x, lo = item.y, m = item.z;
+    FixTotal total;
+    for (uint32_t k0 = 0; k0 < m; k0 += ADJ_CHUNK) {
+      uint2 e[ADJ_ROUNDS];
+      float4 r[ADJ_ROUNDS];
+#pragma unroll
+      for (uint32_t k = 0; k < ADJ_ROUNDS; ++k) {
+        const uint32_t i = k0 + 8u * k + (lane >> 2);
+        e[k] = i < m ? ent[lo + i] : make_uint2(0u, 0u);
       }
+      uint32_t bits = 0u;  // of the largest adjoint (NaN above infinity above every number)
+#pragma unroll
+      for (uint32_t k = 0; k < ADJ_ROUNDS; ++k) {
+        r[k] = (e[k].y >> s) & 1u ? rec[4 * (size_t)e[k].x + s] : make_float4(0.f, 0.f, 0.f, 0.f);
+        bits = max(bits, max(__float_as_uint(r[k].z) & 0x7fffffffu, __float_as_uint(r[k].w) & 0x7fffffffu));
+      }
+      const uint32_t rounds = (m - k0 + 7u) / 8u;  // with entries; the records of the others add zeros
+      uint32_t v[8];
+      float most[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) most[k] = 0.f;
+#pragma unroll
+      for (uint32_t k = 0; k < ADJ_ROUNDS; k += 2) {
+        if (k >= rounds) break;
+        for_terms(r[k], [&](int i, float x) { most[i] = fmaxf(most[i], fabsf(x)); });
+        for_terms(r[k + 1], [&](int i, float x) { most[i] = fmaxf(most[i], fabsf(x)); });
+      }
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[k] = __float_as_uint(most[k]);
+      const uint32_t top = fix_top(by_stage(v, [](uint32_t x, uint32_t y) { return max(x, y); }));
+      uint32_t flags = 0u;
+      if (__any_sync(0xffffffffu, bits >= 0x7f800000u)) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[k] = 0u;
+#pragma unroll
+        for (uint32_t k = 0; k < ADJ_ROUNDS; ++k) for_terms(r[k], [&](int i, float x) { v[i] |= fix_flags(x); });
+        flags = by_stage(v, [](uint32_t x, uint32_t y) { return x | y; });
+      }
+      const float own = fix_scale(top);
+      float scale[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        scale[k] = __shfl_sync(0xffffffffu, own, (k & 4) << 2 | (k & 2) << 2 | (k & 1) << 2 | (int)s);
+      FixSum sum[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) sum[k].a = sum[k].b = sum[k].c = 0u;
+#pragma unroll
+      for (uint32_t k = 0; k < ADJ_ROUNDS; k += 2) {
+        if (k >= rounds) break;
+        for_terms(r[k], [&](int i, float x) { fix_add(sum[i], x, scale[i]); });
+        for_terms(r[k + 1], [&](int i, float x) { fix_add(sum[i], x, scale[i]); });
+      }
+      const uint32_t magic = min((rounds + 1u) & ~1u, ADJ_ROUNDS) * __float_as_uint(FIX_MAGIC);
+      auto add = [](uint32_t x, uint32_t y) { return x + y; };
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[k] = sum[k].a - magic;
+      const uint32_t sa = by_stage(v, add);  // at most 2 * ADJ_CHUNK terms of 2^21
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[k] = sum[k].b - magic;
+      const uint32_t sb = by_stage(v, add);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[k] = sum[k].c - magic;
+      const uint32_t sc = by_stage(v, add);
+      total.join(flags ? FIX_SPECIAL : top, (int)(flags ? flags : sa), (int)sb, (int)sc);
+    }
+    float* out = b.csum + (oc + c) * 24 + at;
+    if (item.w == NONE) {
+      if (s != 2u) *out = total.value();
       continue;
     }
-    const float scale = __uint_as_float((uint32_t)(adj_scale_bits(top, all) + 127) << 23);
-    FixSum acc[12];
-#pragma unroll
-    for (int k = 0; k < 12; ++k) acc[k].hi = acc[k].lo = 0u;
-    uint32_t n0 = 0, n1 = 0, n2 = 0;  // terms a group's sums took
-    uint2 ents[ADJ_ITEM / 32];
-#pragma unroll
-    for (uint32_t k = 0; k < ADJ_ITEM / 32; ++k)
-      ents[k] = lane + 32 * k < m ? ent[lo + lane + 32 * k] : make_uint2(0u, 0u);
-#pragma unroll
-    for (uint32_t k4 = 0; k4 < ADJ_ITEM / 32; ++k4) {
-      if (32 * k4 >= m) break;  // warp-uniform
-      const uint2 e = ents[k4];
-      const float4* rp = rec + 4 * (size_t)e.x;
-      float4 r[4];
-#pragma unroll
-      for (int k = 0; k < 4; ++k)
-        if ((e.y >> k) & 1u) r[k] = rp[k];
-      if (e.y & 1u) gather_add<0>(r[0], V, scale, acc);
-      if (e.y & 2u) gather_add<1>(r[1], V, scale, acc);
-      if (e.y & 4u) gather_add<1>(r[2], V, scale, acc);
-      if (e.y & 8u) gather_add<2>(r[3], V, scale, acc);
-      n0 += e.y & 1u;
-      n1 += __popc(e.y & 6u);
-      n2 += (e.y >> 3) & 1u;
+    if (s != 2u) part[(size_t)item.w * 24 + at] = make_int4((int)total.top, (int)total.a, (int)total.b, (int)total.c);
+    __threadfence();
+    __syncwarp();
+    const uint32_t all = b.count[oc + c], items = (all + ADJ_ITEM - 1) / ADJ_ITEM;
+    uint32_t before = 0;
+    if (lane == 0) before = atomicAdd(b.done + oc + c, 1u);
+    if (__shfl_sync(0xffffffffu, before, 0) != items - 1u) continue;
+    __threadfence();
+    const uint32_t index = (lo - (b.place[oc + c] - all)) / ADJ_ITEM;  // of this item (place: past the cell's last entry)
+    const int4* p = part + (size_t)(item.w - index) * 24 + at;
+    total = FixTotal();
+#pragma unroll 4
+    for (uint32_t k = 0; k < items; ++k) {
+      const int4 x = __ldcg(p + (size_t)k * 24);
+      total.join((uint32_t)x.x, x.y, x.z, x.w);
     }
-    uint32_t v[12];
-#pragma unroll
-    for (int k = 0; k < 12; ++k) v[k] = acc[k].hi - one * (k < 4 ? n0 : k < 8 ? n1 : n2);
-    const int hi = (int)sum_by_lane(v);  // at most 2 * ADJ_ITEM terms of 2^21
-#pragma unroll
-    for (int k = 0; k < 12; ++k) v[k] = acc[k].lo - one * (k < 4 ? n0 : k < 8 ? n1 : n2);
-    const long long sum = (long long)hi * 1048576ll + (int)sum_by_lane(v);
-    if (lane < 12) {
-      long long* at = out + (lane >> 2) * 8 + (lane & 3u) + (V ? 4 : 0);
-      if (all <= ADJ_ITEM)
-        *at = sum;
-      else
-        atomicAdd(reinterpret_cast<unsigned long long*>(at), (unsigned long long)sum);
-    }
+    if (s != 2u) *out = total.value();
   }
 }
 
@@ -918,15 +994,11 @@ __global__ void __launch_bounds__(32 * NODE_STEPS) k_adj_nodes(int nx, int ny, c
 #pragma unroll
       for (int t = 0; t < 4; ++t) {
         if (m[t] == 0u) continue;  // only cells with entries were summed
-        const size_t cell = (size_t)q * b.cells + (size_t)cj_[t] * cw + ci_[t];
-        const uint32_t top = b.top[cell];
-        const int bits = adj_scale_bits(top, m[t]) + 20;
-        const long long* cs = b.csum + cell * 24 + corner[t];
+        const float* cs = b.csum + ((size_t)q * b.cells + (size_t)cj_[t] * cw + ci_[t]) * 24 + corner[t];
 #pragma unroll
         for (int g = 0; g < 3; ++g) {
-          const long long u = cs[g * 8], v = cs[g * 8 + 4];
-          U[g] += top < ADJ_NOT_FINITE ? ldexpf(__ll2float_rn(u), -bits) : __uint_as_float((uint32_t)u);
-          V[g] += top < ADJ_NOT_FINITE ? ldexpf(__ll2float_rn(v), -bits) : __uint_as_float((uint32_t)v);
+          U[g] += cs[g * 8];
+          V[g] += cs[g * 8 + 4];
         }
       }
     }
@@ -1081,12 +1153,12 @@ void launch_adj_reduce(int nx, int ny, const AdjStep* table, int m_last, const A
                        int sms, cudaStream_t st) {
   if (!b.n) return;
   const unsigned steps = (unsigned)b.steps;
-  const uint32_t items = (uint32_t)adj_items(b.n, b.cells);
-  launch_dep(k_adj_alloc, dim3(grid_for(b.cells, ALLOC_THREADS), steps), dim3(ALLOC_THREADS), st, b, items);
+  launch_dep(k_adj_alloc, dim3(grid_for(b.cells, ALLOC_THREADS), steps), dim3(ALLOC_THREADS), st, b);
   launch_dep(k_adj_scatter, dim3(grid_for(b.n, 256), steps), dim3(256), st, b);
-  // two warps per item, at most eight blocks an SM over all steps
-  const unsigned cap = std::max(1u, (unsigned)(sms > 0 ? sms : 152) * 8u / steps);
-  launch_dep(k_adj_gather, dim3(std::min(grid_for((size_t)items * 64, 256), cap), steps), dim3(256), st, b, items);
+  // a warp per item, at most GATHER_BLOCKS blocks an SM over all steps
+  const unsigned cap = std::max(1u, (unsigned)(sms > 0 ? sms : 152) * GATHER_BLOCKS / steps);
+  const unsigned want = grid_for(adj_items(b.n, b.cells) * 32, GATHER_THREADS);
+  launch_dep(k_adj_gather, dim3(std::min(want, cap), steps), dim3(GATHER_THREADS), st, b);
   launch_dep(k_adj_nodes, dim3(grid_for((size_t)nx * ny, 32)), dim3(32, std::min(b.steps, NODE_STEPS)), st, nx, ny, table, m_last, b, gu, gv);
 }
 

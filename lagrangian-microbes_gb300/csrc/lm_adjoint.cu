@@ -8,8 +8,8 @@
 //   ck_*    T, T, uint8 [ceil(S/K)][n]     state at steps 0, K, 2K, ... (T = float or double)
 //   seg_*   T, T, uint8 [K][n]             state before every step of the segment being reversed
 //   lx, ly  T [n]                          the adjoint dL/dx_m
-//   rec, cell, count, place, list, ent, csum, total   the backward steps whose records are reduced
-//                                          together (AdjBatch), B at a time
+//   rec, cell, count, place, list, ent, part, csum   the backward steps whose records are reduced together
+//                                          (AdjBatch), B at a time
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -54,13 +54,14 @@ struct lm_adjoint {
   DBuf<unsigned char> x, y, ck_x, ck_y, seg_x, seg_y, lx, ly, fin_x, fin_y;
   int batch = 1;     // backward steps reduced together
   int seg_held = -1;  // segment whose states seg_* hold
-  DBuf<long long> csum;
+  DBuf<float> csum;
+  DBuf<int4> part;
   DBuf<uint8_t> st, ck_st, seg_st;
   DBuf<float4> rec;
   DBuf<uint4> cell;
   DBuf<uint2> ent;
   DBuf<uint4> list;
-  DBuf<uint32_t> count, place;  // count: [B][cells], top [B][cells] and the totals [B][2], zeroed together
+  DBuf<uint32_t> count, place;  // count: [B][cells], done [B][cells] and the totals [B][4], zeroed together
   uint32_t* err_d = nullptr;
   uint32_t* err_h = nullptr;
   // the reduction of a batch runs on a stream of its own beside the next batch's steps: two sets of
@@ -129,7 +130,7 @@ bool on_device(const void* p) {
 // launches of a batch cost about 25 us however little they do: at 100k microbes eight steps share them,
 // at 1M the records of one step fill L2.
 int batch_steps(uint32_t n, uint64_t cells, int K) {
-  const double fit = std::min(96e6 / (110.0 * n + 1.0), 1e9 / (2.0 * 220.0 * cells));
+  const double fit = std::min(96e6 / (110.0 * n + 1.0), 1e9 / (2.0 * 125.0 * cells));
   return std::max(1, std::min({16, K, (int)std::min(fit, 16.0)}));
 }
 
@@ -142,12 +143,13 @@ AdjBatch batch_buffers(const lm_adjoint* a, uint32_t cells, int set, int steps) 
   b.steps = steps;
   b.rec = a->rec.p + 4 * k * a->n;
   b.cell = a->cell.p + k * a->n;
-  b.count = a->count.p + k * (2 * (size_t)cells + 2);
-  b.top = b.count + (size_t)steps * cells;
-  b.total = b.top + (size_t)steps * cells;
+  b.count = a->count.p + k * (2 * (size_t)cells + 4);
+  b.done = b.count + (size_t)steps * cells;
+  b.total = b.done + (size_t)steps * cells;
   b.place = a->place.p + k * cells;
   b.list = a->list.p + k * adj_items(a->n, cells);
   b.ent = a->ent.p + 4 * k * a->n;
+  b.part = a->part.p + k * adj_parts(a->n) * 24;
   b.csum = a->csum.p + k * cells * 24;
   return b;
 }
@@ -213,7 +215,7 @@ int lm_adjoint_destroy(lm_adjoint* a) {
   release(a->uv);
   release(a->table);
   release(a->x), release(a->y), release(a->ck_x), release(a->ck_y), release(a->seg_x), release(a->seg_y);
-  release(a->lx), release(a->ly), release(a->fin_x), release(a->fin_y), release(a->csum), release(a->st), release(a->ck_st), release(a->seg_st);
+  release(a->lx), release(a->ly), release(a->fin_x), release(a->fin_y), release(a->csum), release(a->part), release(a->st), release(a->ck_st), release(a->seg_st);
   release(a->rec), release(a->cell), release(a->ent), release(a->count), release(a->place), release(a->list);
   if (a->err_d) cudaFree(a->err_d);
   if (a->err_h) cudaFreeHost(a->err_h);
@@ -274,9 +276,9 @@ int lm_adjoint_forward(lm_adjoint* a, const float* u, const float* v, int nt, in
       (r = grow(a, a->seg_st, (size_t)checkpoint_every * N)) || (r = grow(a, a->lx, es * N)) ||
       (r = grow(a, a->ly, es * N)) || (r = grow(a, a->fin_x, es * N)) || (r = grow(a, a->fin_y, es * N)) ||
       (r = grow(a, a->rec, 2 * (size_t)4 * B * N)) || (r = grow(a, a->cell, 2 * (size_t)B * N)) ||
-      (r = grow(a, a->ent, 2 * (size_t)4 * B * N)) || (r = grow(a, a->count, 2 * B * (2 * cells + 2))) ||
+      (r = grow(a, a->ent, 2 * (size_t)4 * B * N)) || (r = grow(a, a->count, 2 * B * (2 * cells + 4))) ||
       (r = grow(a, a->place, 2 * B * cells)) || (r = grow(a, a->list, 2 * B * adj_items(N, cells))) ||
-      (r = grow(a, a->csum, 2 * B * cells * 24)))
+      (r = grow(a, a->part, 2 * B * adj_parts(N) * 24)) || (r = grow(a, a->csum, 2 * B * cells * 24)))
     return r;
   launch_interleave(u, v, a->uv.p, fe, st);
   fill_field_view(a->fv, a->uv.p, nt, ny, nx, lon, lat, t_sec, dx, dy, dT);
@@ -361,7 +363,7 @@ int lm_adjoint_backward(lm_adjoint* a, const float* g_lon, const float* g_lat, f
       const AdjBatch b = batch_buffers(a, cells, set, std::min(a->batch, m - m0 + 1));
       if (!fresh[set]) ACK(cudaStreamWaitEvent(st, a->reduced[set], 0));  // its last reduction is done
       fresh[set] = false;
-      ACK(cudaMemsetAsync(b.count, 0, (size_t)b.steps * (2 * (size_t)cells + 2) * sizeof(uint32_t), st));
+      ACK(cudaMemsetAsync(b.count, 0, (size_t)b.steps * (2 * (size_t)cells + 4) * sizeof(uint32_t), st));
       const size_t o = (size_t)(m - m0) * N;
       launch_adj_step(a->fv, a->prec, a->table.p, m, a->dt, b, a->seg_x.p + es * o, a->seg_y.p + es * o,
                       a->seg_st.p + o, a->lx.p, a->ly.p, st);

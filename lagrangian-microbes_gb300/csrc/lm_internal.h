@@ -390,20 +390,23 @@ struct AdjBatch {
   float4* rec;      // [steps][n][4]   (a, b, dL/dU, dL/dV) of each stage
   uint4* cell;      // [steps][n]      field cells of the four stages (NONE: the step was frozen)
   uint32_t* count;  // [steps][cells]  entries of a cell (zero before the batch)
-  uint32_t* top;    // [steps][cells]  float bits of its largest |dL/dU|, |dL/dV| (zero before the batch)
-  uint32_t* total;  // [steps][2]      entries reserved, items listed (zero before the batch)
+  uint32_t* done;   // [steps][cells]  its items that are summed, of cells of several (zero before the batch)
+  uint32_t* total;  // [steps][4]      entries and parts reserved, items listed (zero before the batch)
   uint32_t* place;  // [steps][cells]  where a cell's entries go
-  uint4* list;      // [steps][adj_items] items: (cell, first entry, entries, entries of the cell)
+  uint4* list;      // [steps][adj_items] items: (cell, first entry, entries, place of its parts or NONE)
   uint2* ent;       // [steps][4 n]    (microbe, stage bits), a cell's entries together
-  long long* csum;  // [steps][cells][24] corner sums per stage time, scaled by the cell's `top`
+  int4* part;       // [steps][adj_parts][24] sums of an item of a cell of several
+  float* csum;      // [steps][cells][24] corner sums per stage time: of dL/dU, then of dL/dV
 };
 // Entries of an item: what one warp adds up for a cell.
 constexpr uint32_t ADJ_ITEM = 128;
 // Items of a step at most: one per occupied cell and one per full item.
-inline size_t adj_items(uint32_t n, size_t cells) {
+__host__ __device__ inline size_t adj_items(uint32_t n, size_t cells) {
   const size_t e = (size_t)4 * n;
   return (cells < e ? cells : e) + e / ADJ_ITEM;
 }
+// Items of cells of several at most: fewer than two for each ADJ_ITEM entries.
+__host__ __device__ inline size_t adj_parts(uint32_t n) { return (size_t)8 * n / ADJ_ITEM; }
 
 void launch_adj_stages(const FieldView& f, double t_start, double dt, int n_steps, AdjStep* table, uint32_t* err,
                        cudaStream_t st);

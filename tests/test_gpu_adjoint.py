@@ -284,6 +284,80 @@ def test_adjoint_field_gradient_does_not_depend_on_the_order_of_the_microbes(sma
         np.testing.assert_array_equal(a, b)
 
 
+def _still_field(lm, n_frames=3):
+    axis = 0.125 * np.arange(17)
+    zero = np.zeros((n_frames, 17, 17), np.float32)
+    return lm.VelocityField(200.0 + axis, 25.0 + axis, 3600.0 * np.arange(n_frames), zero, zero)
+
+
+def _still_gradient(f, lon, lat, g, share, magnitude=False):
+    """dL/dU, dL/dV per frame of one step in a field at rest, in float64: a microbe stays where it is, so a node gets its
+    bilinear weight times its adjoint times the frame's share of the step, in field units. Positions are multiples of
+    1/4 of a cell here, exact in every precision."""
+    out = np.zeros((2, len(share), 17, 17))
+    x, y = (lon.astype(np.float64) - 200.0) * 8.0, (lat.astype(np.float64) - 25.0) * 8.0
+    i, j = np.minimum(x.astype(int), 15), np.minimum(y.astype(int), 15)
+    a, b = x - i, y - j
+    m = 1852.0 * 60.0
+    per = np.stack([g[0] / (m * np.cos(np.deg2rad(lat.astype(np.float64)))), g[1] / m])
+    if magnitude:
+        per = np.abs(per)
+    for dj, di, w in ((0, 0, (1 - a) * (1 - b)), (0, 1, a * (1 - b)), (1, 0, (1 - a) * b), (1, 1, a * b)):
+        for k in range(2):
+            for fr, s in enumerate(share):
+                np.add.at(out[k, fr], (j + dj, i + di), w * per[k].astype(np.float64) * s)
+    return out
+
+
+@pytest.mark.parametrize("precision", ["f32", "ds", "f64"])
+@pytest.mark.parametrize("n, large", [(3, 1e8), (3, 1e12), (200, 1e10), (700, 1e14), (0, 0)])
+def test_adjoint_small_terms_beside_large_ones_keep_their_digits(lm, n, large, precision):
+    """A node's sum of small terms is as accurate as its own terms, whatever adjoints the field cell holds elsewhere: one
+    large adjoint on a cell's corner beside n ordinary ones (no term of it at the other nodes, none in dL/dV), and
+    adjoints over fourteen decades on the edges and inside of 36 cells. Bound: some 20 roundings of 2^-24 and a float32
+    cosine within 2 ulp on the way from a term to the gradient, 24 x 2^-24 = 1.43e-6 of the terms' magnitude."""
+    f = _still_field(lm)
+    rng = np.random.default_rng(63 + n)
+    if large:
+        q = rng.integers(1, 4, (2, n))  # inside the cell
+        lon = np.concatenate([[200.5], 200.5 + 0.03125 * q[0]]).astype(np.float32)
+        lat = np.concatenate([[25.25], 25.25 + 0.03125 * q[1]]).astype(np.float32)
+        g = rng.uniform(0.5, 2.0, (2, n + 1)).astype(np.float32)
+        g[0, 0] = large
+    else:
+        lon = (200.5 + 0.03125 * rng.integers(0, 24, 500)).astype(np.float32)
+        lat = (25.5 + 0.03125 * rng.integers(0, 24, 500)).astype(np.float32)
+        g = (rng.standard_normal((2, 500)) * 10.0 ** rng.uniform(-7, 7, 500)).astype(np.float32)
+    got = _tape_backward(f, lon, lat, g, 1, 1, precision)
+    share = (1800.0, 1800.0, 0.0)  # of 3,600 s: stage 1 at frame 0, stages 2 and 3 between the frames, stage 4 at frame 1
+    want, size = (_still_gradient(f, lon, lat, g, share, m) for m in (False, True))
+    for k in range(2):
+        err = np.abs(got[2 + k].astype(np.float64) - want[k])
+        assert (err <= 1.5e-6 * size[k]).all(), (k, (err / np.maximum(size[k], 1e-300)).max())
+
+
+@pytest.mark.parametrize("n", [30, 500])
+def test_adjoint_finite_sums_of_a_cell_with_an_infinite_adjoint_are_exact(lm, n):
+    """One infinite longitude adjoint makes its cell's sums of dL/dU infinite or undefined; dL/dV at the last stage's
+    frame has finite terms only and stays what it is, for shuffled microbes bit by bit."""
+    f = _still_field(lm)
+    rng = np.random.default_rng(64 + n)
+    lon = (200.5 + 0.03125 * rng.integers(0, 4, n)).astype(np.float32)
+    lat = (25.5 + 0.03125 * rng.integers(0, 4, n)).astype(np.float32)
+    g = (rng.standard_normal((2, n)) * 10.0 ** rng.uniform(-3, 3, n)).astype(np.float32)
+    g[0, n // 2] = np.inf
+    got = _tape_backward(f, lon, lat, g, 1, 1, "f32", dt=7200.0)  # the stages at frames 0, 1, 1 and 2
+    share = (0.0, 0.0, 1200.0)
+    want, size = (_still_gradient(f, lon, lat, np.where(np.isfinite(g), g, 0), share, m)[1, 2] for m in (False, True))
+    assert (np.abs(got[3][2].astype(np.float64) - want) <= 1.5e-6 * size).all()
+    assert not np.isfinite(got[2][2, 4:6, 4:6]).any() and (got[2][2] == 0).sum() >= 17 * 17 - 9
+    for _ in range(3):
+        p = rng.permutation(n)
+        again = _tape_backward(f, lon[p], lat[p], np.ascontiguousarray(g[:, p]), 1, 1, "f32", dt=7200.0)
+        for a, b in zip(again[2:], got[2:]):
+            np.testing.assert_array_equal(a, b)
+
+
 @pytest.mark.parametrize("n", [40, 400])
 def test_adjoint_dense_cells_match_fp64_autograd(lm, orc, small_field, n):
     """n microbes per field cell of a 3 x 3 patch, against the FP64 autograd on the same cell paths
