@@ -336,6 +336,42 @@ def test_adjoint_small_terms_beside_large_ones_keep_their_digits(lm, n, large, p
         assert (err <= 1.5e-6 * size[k]).all(), (k, (err / np.maximum(size[k], 1e-300)).max())
 
 
+@pytest.mark.parametrize("precision", ["f64", "ds", "f32"])
+def test_adjoint_takes_the_stages_that_the_forward_took_at_the_domain_edge(lm, precision):
+    """A steady zonal flow towards the domain's edge: the longest step whose last stage the forward still finds inside has
+    a gradient in the backward, and the next longer one, which the forward freezes, has none. The two agree only if
+    their stage positions do, to the last bit."""
+    from lagrangian_microbes_gb300.adjoint import AdjointTape
+    axis = 0.125 * np.arange(17)
+    lats = np.linspace(25.03, 26.96, 48).astype(np.float32)
+    dev = torch.device("cuda:0")
+    u = torch.full((2, 17, 17), 0.731, device=dev)
+    args = (u, torch.zeros_like(u), 200.0 + axis, 25.0 + axis, np.array([0.0, 20000.0]), 0.0)
+    tape = AdjointTape(precision=precision)
+
+    def ends(lat, dt):  # is the step taken?
+        lon0, lat0 = torch.full((len(lat),), 201.9375, device=dev), torch.from_numpy(lat).to(dev)
+        lon, _ = tape.forward(lon0, lat0, *args, dt, 1, 1, True)
+        return (lon.double() != lon0.double()).cpu().numpy()
+
+    one = torch.ones(1, device=dev)
+    step = np.float32 if precision != "f64" else np.float64  # the kernels' type of dt
+    for lat in lats:
+        lo, hi = step(5000.0), step(15000.0)
+        assert ends(lat[None], float(lo))[0] and not ends(lat[None], float(hi))[0]
+        while np.nextafter(lo, hi) < hi:
+            mid = step((float(lo) + float(hi)) / 2)
+            if ends(lat[None], float(mid))[0]:
+                lo = mid
+            else:
+                hi = mid
+        for dt, taken in ((lo, True), (hi, False)):
+            assert ends(lat[None], float(dt))[0] == taken
+            assert tape.backward(one, 0 * one)[2].any().item() == taken, (lat, dt)
+    tape.close()
+    tape.ctx.close()
+
+
 @pytest.mark.parametrize("n", [30, 500])
 def test_adjoint_finite_sums_of_a_cell_with_an_infinite_adjoint_are_exact(lm, n):
     """One infinite longitude adjoint makes its cell's sums of dL/dU infinite or undefined; dL/dV at the last stage's
