@@ -201,6 +201,8 @@ class _MeanSquaredDistance(torch.autograd.Function):
 def _one_kernel(tensors) -> bool:
     """Plain CUDA tensors of one shape on one device, targets without gradients, and nothing that looks into single
     operations (tracing, compilation, functorch transforms, forward mode, dispatch and function modes)."""
+    if torch.compiler.is_compiling() or torch.jit.is_tracing():  # first: the checks below do not compile
+        return False
     first = tensors[0]
     for t in tensors:
         if (type(t) not in (torch.Tensor, torch.nn.Parameter) or not t.is_cuda or t.device != first.device
@@ -208,7 +210,6 @@ def _one_kernel(tensors) -> bool:
                 or t.is_neg() or t._is_zerotensor()):
             return False
     return (first.numel() > 0 and not tensors[2].requires_grad and not tensors[3].requires_grad
-            and not torch.jit.is_tracing() and not torch.compiler.is_compiling()
             and torch._C._len_torch_dispatch_stack() == 0 and torch._C._len_torch_function_stack() == 0
             and torch._C._functorch.peek_interpreter_stack() is None
             and torch.autograd.forward_ad._current_level < 0)

@@ -540,3 +540,20 @@ def test_squared_distance_beyond_the_plain_call(lm):
     lon.add_(0.25)
     graph.replay()
     close(out, ref(lon, lat, tl, ta))
+
+
+def test_squared_distance_compiles_and_traces_as_one_graph(lm):
+    """Under torch.compile without graph breaks, and under torch.jit.trace, the loss is its tensor operations."""
+    from lagrangian_microbes_gb300 import adjoint
+    f = adjoint.mean_squared_distance
+    gen = torch.Generator().manual_seed(4)
+    lon, lat, tl, ta = (torch.rand(65, generator=gen, dtype=torch.float64).cuda() + k for k in (10, 20, 10.2, 20.1))
+    close = lambda a, b: torch.testing.assert_close(a, b, rtol=1e-11, atol=0)
+    want = adjoint._squared_distance_mean(lon, lat, tl, ta)
+    close(torch.compile(f, fullgraph=True, backend="eager")(lon, lat, tl, ta), want)
+    x = lon.clone().requires_grad_()
+    (g,) = torch.autograd.grad(torch.compile(f, fullgraph=True, backend="eager")(x, lat, tl, ta), x)
+    (w,) = torch.autograd.grad(adjoint._squared_distance_mean(x, lat, tl, ta), x)
+    close(g, w)
+    traced = torch.jit.trace(f, (lon, lat, tl, ta))
+    close(traced(lon + 0.5, lat, tl, ta), adjoint._squared_distance_mean(lon + 0.5, lat, tl, ta))
