@@ -767,6 +767,7 @@ int dh_run(lm_ctx* c, const float* lat, const float* lon, const int8_t* species,
   const int mb = std::min(DH_CURVE_BITS, 32 - seg_bits) & ~1;
   const size_t hl = radix_sort_hist_len(n);
   const size_t out_n = nb * n_seg;
+  const ScratchCall scratch(c);
   DhArena ar;
   float *dlat = nullptr, *dlon = nullptr;
   int8_t* dsp = nullptr;

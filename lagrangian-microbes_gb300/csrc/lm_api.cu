@@ -1339,6 +1339,7 @@ int lm_query_pairs(lm_ctx* c, int64_t n, const float* lon, const float* lat, int
   // the pairs i < j in (i, j) order, written on the device: counts per i, their prefix sums, the rows
   const size_t nn = ((size_t)n + 63) / 64 * 64, mm = ((size_t)m + 63) / 64 * 64;
   void* mem = nullptr;
+  const ScratchCall scratch(c);
   if ((r = ctx_scratch(c, (2 * nn + SCAN_BLOCKS + 2 * mm) * sizeof(uint32_t), &mem))) return r;
   uint32_t* cnt = static_cast<uint32_t*>(mem);
   uint32_t* off = cnt + nn;
@@ -1618,6 +1619,12 @@ int ctx_scratch(lm_ctx* c, size_t bytes, void** p) {
   }
   *p = c->scratch;
   return LM_OK;
+}
+void ctx_scratch_done(lm_ctx* c) {
+  if (c->scratch_n <= SCRATCH_KEEP) return;
+  cudaFree(c->scratch);  // (after whatever still runs on it)
+  c->scratch = nullptr;
+  c->scratch_n = 0;
 }
 
 bool uniform_axis(const double* a, int n, double* d) {

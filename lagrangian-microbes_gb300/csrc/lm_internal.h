@@ -445,9 +445,17 @@ int ctx_sms(const lm_ctx* c);
 cudaStream_t ctx_stream(const lm_ctx* c);
 bool ctx_on_own_stream(const lm_ctx* c);  // no external stream set
 void ctx_set_error(lm_ctx* c, const char* msg);
-// A device buffer of at least `bytes` owned by the context (grown, never shrunk, freed with it), for
-// the working arrays of one synchronous call; its contents do not outlive the call.
+// A device buffer of at least `bytes` owned by the context for the working arrays of one synchronous call; its contents
+// do not outlive the call. Up to SCRATCH_KEEP bytes stay for the next call (an allocation and its release cost as much as
+// a small query), more goes back when the call's ScratchCall ends.
+constexpr size_t SCRATCH_KEEP = 64 << 20;
 int ctx_scratch(lm_ctx* c, size_t bytes, void** p);
+void ctx_scratch_done(lm_ctx* c);
+struct ScratchCall {
+  lm_ctx* c;
+  explicit ScratchCall(lm_ctx* ctx) : c(ctx) {}
+  ~ScratchCall() { ctx_scratch_done(c); }
+};
 
 // Ordered-int encoding of floats for atomicMin/atomicMax.
 __host__ __device__ inline uint32_t enc_f(float f) {

@@ -204,3 +204,18 @@ def test_points_around_a_pole_keep_the_reference_chain_bins(pdh, monkeypatch, ba
     monkeypatch.delenv("LM_HIST_EXACT")
     np.testing.assert_array_equal(fast[0], exact[0])
     assert fast[1] == exact[1]
+
+
+def test_a_large_calls_working_memory_goes_back(pdh, lm):
+    """8 million points without a species (no pairs) need some 550 MB of working arrays; the context keeps 64 MB at most
+    for its next call."""
+    torch = pytest.importorskip("torch")
+    n = 8_000_000
+    zeros = np.zeros(n, np.float32)
+    ctx = lm._lib.Context()
+    pdh.species_distance_histograms(zeros[:8], zeros[:8], np.zeros(8, np.int8), 70, ctx=ctx)
+    before = torch.cuda.mem_get_info()[0]
+    got = pdh.species_distance_histograms(zeros, zeros, np.zeros(n, np.int8), 70, ctx=ctx)
+    assert all(c.sum() == 0 and o == 0 for c, o in got.values())
+    assert before - torch.cuda.mem_get_info()[0] <= 96 << 20  # (allocations come in blocks)
+    ctx.close()
