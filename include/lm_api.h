@@ -36,7 +36,8 @@ extern "C" {
 #define LM_ERR_STATE 4          /* call out of order (no field / no particles / no parameters) */
 #define LM_ERR_OUT_OF_BOUNDS 5  /* particles left the field domain (they are frozen and excluded) */
 #define LM_ERR_NAN 6            /* non-finite positions */
-#define LM_ERR_ROUND_CAP 7      /* a microbe has more than 2^24 - 1 neighbours in one step */
+#define LM_ERR_ROUND_CAP 7      /* a microbe has more than 2^24 - 1 neighbours in one step, or the
+                                   lists of those with more than 8 exceed 2^32 - 16 entries */
 #define LM_ERR_TIMEOUT 8        /* a bounded device wait gave up; the context stays usable */
 #define LM_ERR_TIME 9           /* a stage time fell outside the field's time axis */
 #define LM_ERR_GRID 10          /* field axes are not uniformly spaced / ascending */

@@ -275,9 +275,14 @@ int set_cells_capacity(lm_ctx* c, uint32_t cap) {
   return LM_OK;
 }
 
+// Entries of the long lists at most. With the slab rows of the others (8 entries, of MAX_SLOTS microbes at most) a step
+// has fewer than 2^33 list entries, two a pair: fewer than 2^32 pairs, so their prefix sums fit 32 bits.
+constexpr size_t OVF_MAX = 0xfffffff0ull;
+static_assert((OVF_MAX + (unsigned long long)SLAB * MAX_SLOTS) / 2 < 0xffffffffull, "pairs are indexed with 32 bits");
+
 int set_ovf_capacity(lm_ctx* c, size_t cap) {
   int r;
-  cap = std::min<size_t>(cap, 0xfffffff0ull);
+  cap = std::min(cap, OVF_MAX);
   if ((r = dalloc(c, &c->ovf, cap)) || (r = dalloc(c, &c->oprio, cap))) return r;
   c->ovf_cap = cap;
   unsigned long long cv = cap;
@@ -489,6 +494,11 @@ int regrow(lm_ctx* c) {
   if (h.err & ERRB_ROUNDCAP) {
     write_err(c, 0u, 0u);
     return fail(c, LM_ERR_ROUND_CAP, "a microbe has more than %u neighbours", MAX_DEGREE);
+  }
+  if (h.ovf_used > OVF_MAX) {  // (offsets have 32 bits; a larger area would halt the step again and again)
+    const unsigned long long used = h.ovf_used;
+    write_err(c, 0u, 0u);
+    return fail(c, LM_ERR_ROUND_CAP, "neighbour lists of %llu entries (at most %zu)", used, OVF_MAX);
   }
   if (h.ovf_used > c->ovf_cap) {
     size_t need = (size_t)h.ovf_used;
@@ -1335,7 +1345,6 @@ int lm_query_pairs(lm_ctx* c, int64_t n, const float* lon, const float* lat, int
   if (!pi || !pj || m == 0) return LM_OK;  // count query
   if ((int64_t)m > cap)
     return fail(c, LM_ERR_CAPACITY, "pair buffer holds %lld pairs, %llu needed", (long long)cap, (unsigned long long)m);
-  if (m > 0xffffffffull) return fail(c, LM_ERR_OOM, "too many pairs for one query (%llu)", (unsigned long long)m);
   // the pairs i < j in (i, j) order, written on the device: counts per i, their prefix sums, the rows
   const size_t nn = ((size_t)n + 63) / 64 * 64, mm = ((size_t)m + 63) / 64 * 64;
   void* mem = nullptr;

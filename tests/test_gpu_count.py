@@ -155,3 +155,18 @@ def test_count_at_the_inner_edge_of_the_float32_band(engine):
     q = engine.PairQuery(r, np.inf)
     assert q.count(lon, lat) == want
     q.ctx.close()
+
+
+def test_lists_beyond_32_bit_offsets_are_refused_and_the_context_stays_usable(engine, lm):
+    """70,000 microbes in one place have 4.9e9 list entries, more than the area of long lists can ever hold: an error, where
+    the area would be enlarged and the search repeated for ever. They can still be counted."""
+    n = 70_000
+    lon, lat = np.full(n, 200.5, np.float32), np.full(n, 25.5, np.float32)
+    q = engine.PairQuery(0.01, 2)
+    with pytest.raises(lm.LMError) as failed:
+        q.pairs(lon, lat)
+    assert failed.value.code == lm._lib.LM_ERR_ROUND_CAP
+    assert q.count(lon, lat) == n * (n - 1) // 2
+    pi, pj = q.pairs(lon[:300], lat[:300])
+    assert pi.size == 300 * 299 // 2 and (pi < pj).all()
+    q.ctx.close()
