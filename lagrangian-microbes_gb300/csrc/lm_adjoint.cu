@@ -53,6 +53,7 @@ struct lm_adjoint {
   // positions of adj_state_bytes(prec) per element; adjoint state lx, ly of adj_lambda_bytes(prec)
   DBuf<unsigned char> x, y, ck_x, ck_y, seg_x, seg_y, lx, ly, fin_x, fin_y;
   int batch = 1;     // backward steps reduced together
+  int sets = 2;      // of batch buffers
   int seg_held = -1;  // segment whose states seg_* hold
   DBuf<float> csum;
   DBuf<int4> part;
@@ -132,6 +133,25 @@ bool on_device(const void* p) {
 int batch_steps(uint32_t n, uint64_t cells, int K) {
   const double fit = std::min(96e6 / (110.0 * n + 1.0), 1e9 / (2.0 * 125.0 * cells));
   return std::max(1, std::min({16, K, (int)std::min(fit, 16.0)}));
+}
+
+// The batch buffers for B steps, `sets` times. (At most 137 bytes a microbe and 124 a field cell for one step.)
+int batch_alloc(lm_adjoint* a, uint32_t n, uint64_t cells, int B, int sets) {
+  const size_t k = (size_t)sets * B;
+  int r;
+  if ((r = grow(a, a->rec, 4 * k * n)) || (r = grow(a, a->cell, k * n)) || (r = grow(a, a->ent, 4 * k * n)) ||
+      (r = grow(a, a->count, k * (2 * cells + 4))) || (r = grow(a, a->place, k * cells)) ||
+      (r = grow(a, a->list, k * adj_items(n, cells))) || (r = grow(a, a->part, k * adj_parts(n) * 24)) ||
+      (r = grow(a, a->csum, k * cells * 24)))
+    return r;
+  a->batch = B;
+  a->sets = sets;
+  return LM_OK;
+}
+
+void batch_release(lm_adjoint* a) {
+  release(a->rec), release(a->cell), release(a->ent), release(a->count), release(a->place), release(a->list);
+  release(a->part), release(a->csum);
 }
 
 // Set `set` of the batch buffers, for `steps` steps.
@@ -215,8 +235,8 @@ int lm_adjoint_destroy(lm_adjoint* a) {
   release(a->uv);
   release(a->table);
   release(a->x), release(a->y), release(a->ck_x), release(a->ck_y), release(a->seg_x), release(a->seg_y);
-  release(a->lx), release(a->ly), release(a->fin_x), release(a->fin_y), release(a->csum), release(a->part), release(a->st), release(a->ck_st), release(a->seg_st);
-  release(a->rec), release(a->cell), release(a->ent), release(a->count), release(a->place), release(a->list);
+  release(a->lx), release(a->ly), release(a->fin_x), release(a->fin_y), release(a->st), release(a->ck_st), release(a->seg_st);
+  batch_release(a);
   if (a->err_d) cudaFree(a->err_d);
   if (a->err_h) cudaFreeHost(a->err_h);
   delete a;
@@ -265,7 +285,6 @@ int lm_adjoint_forward(lm_adjoint* a, const float* u, const float* v, int nt, in
   const size_t fe = (size_t)nt * ny * nx;
   const uint32_t N = (uint32_t)n;
   const int n_ck = (n_steps + checkpoint_every - 1) / checkpoint_every;
-  const int B = batch_steps(N, cells, std::min(checkpoint_every, n_steps));
   const int prec = a->prec_next;
   const size_t es = adj_state_bytes(prec);  // lx, ly need no more (adj_lambda_bytes)
   int r;
@@ -274,12 +293,18 @@ int lm_adjoint_forward(lm_adjoint* a, const float* u, const float* v, int nt, in
       (r = grow(a, a->ck_y, es * n_ck * N)) || (r = grow(a, a->ck_st, (size_t)n_ck * N)) ||
       (r = grow(a, a->seg_x, es * checkpoint_every * N)) || (r = grow(a, a->seg_y, es * checkpoint_every * N)) ||
       (r = grow(a, a->seg_st, (size_t)checkpoint_every * N)) || (r = grow(a, a->lx, es * N)) ||
-      (r = grow(a, a->ly, es * N)) || (r = grow(a, a->fin_x, es * N)) || (r = grow(a, a->fin_y, es * N)) ||
-      (r = grow(a, a->rec, 2 * (size_t)4 * B * N)) || (r = grow(a, a->cell, 2 * (size_t)B * N)) ||
-      (r = grow(a, a->ent, 2 * (size_t)4 * B * N)) || (r = grow(a, a->count, 2 * B * (2 * cells + 4))) ||
-      (r = grow(a, a->place, 2 * B * cells)) || (r = grow(a, a->list, 2 * B * adj_items(N, cells))) ||
-      (r = grow(a, a->part, 2 * B * adj_parts(N) * 24)) || (r = grow(a, a->csum, 2 * B * cells * 24)))
+      (r = grow(a, a->ly, es * N)) || (r = grow(a, a->fin_x, es * N)) || (r = grow(a, a->fin_y, es * N)))
     return r;
+  // two sets, so that a batch is reduced beside the next one's steps, unless there is only one; where the memory does not
+  // hold them, smaller batches, at last one set of one step
+  const int K = std::min(checkpoint_every, n_steps);
+  int B = batch_steps(N, cells, K), sets = n_steps <= K && B >= n_steps ? 1 : 2;
+  while ((r = batch_alloc(a, N, cells, B, sets)) == LM_ERR_OOM && (B > 1 || sets > 1)) {
+    batch_release(a);
+    if (B > 1) B = (B + 1) / 2;
+    else sets = 1;
+  }
+  if (r) return r;
   launch_interleave(u, v, a->uv.p, fe, st);
   fill_field_view(a->fv, a->uv.p, nt, ny, nx, lon, lat, t_sec, dx, dy, dT);
   a->nt = nt;
@@ -289,7 +314,6 @@ int lm_adjoint_forward(lm_adjoint* a, const float* u, const float* v, int nt, in
   a->n_steps = n_steps;
   a->K = checkpoint_every;
   a->n_ck = n_ck;
-  a->batch = B;
   a->prec = prec;
   a->dt = dt_sec;
   ACK(cudaMemsetAsync(a->err_d, 0, sizeof(uint32_t), st));
@@ -371,7 +395,7 @@ int lm_adjoint_backward(lm_adjoint* a, const float* g_lon, const float* g_lat, f
       ACK(cudaStreamWaitEvent(a->red_st, a->stepped[set], 0));
       launch_adj_reduce(a->nx, a->ny, a->table.p, m, b, g_u, g_v, a->sms, a->red_st);
       ACK(cudaEventRecord(a->reduced[set], a->red_st));
-      set ^= 1;
+      set = (set + 1) % a->sets;
     }
   }
   // what the caller's stream does next comes after the last reductions

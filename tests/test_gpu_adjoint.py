@@ -431,6 +431,39 @@ def test_adjoint_non_finite_gradients_stay_in_their_cells(small_field, bad):
     assert int((~np.isfinite(got[2])).sum()) > few
 
 
+def test_adjoint_takes_smaller_batches_where_memory_is_short(lm, small_field):
+    """4,000,000 microbes with 1.4 GB left on the device: one set of batch buffers for one step fits (270 bytes a microbe
+    with the tape's own), two do not. The gradients are those of a run with the memory it likes."""
+    from lagrangian_microbes_gb300.adjoint import AdjointTape
+    f, n, dev = small_field, 4_000_000, torch.device("cuda:0")
+    gen = torch.Generator(device=dev).manual_seed(5)
+    lon, lat = (lo + 2.0 * torch.rand(n, device=dev, generator=gen) for lo in (199.5, 24.5))
+    g = [torch.randn(n, device=dev, generator=gen) for _ in range(2)]
+    u, v = torch.from_numpy(f.u).to(dev), torch.from_numpy(f.v).to(dev)
+
+    def run():
+        tape = AdjointTape(precision="ds")
+        out = tape.forward(lon, lat, u, v, f.lon, f.lat, f.times, float(f.times[0]), 3600.0, 4, 4)
+        out = [t.cpu() for t in (*out, *tape.backward(*g))]
+        tape.close()
+        tape.ctx.close()
+        return out
+
+    want = run()
+    torch.cuda.empty_cache()
+    left = torch.cuda.mem_get_info()[0] - 1400 * 10 ** 6
+    if left < 0:
+        pytest.skip("less than 1.4 GB free")
+    hog = torch.empty(left, dtype=torch.uint8, device=dev)
+    try:
+        got = run()
+    finally:
+        del hog
+        torch.cuda.empty_cache()
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
+
+
 def test_tape_waits_for_the_default_streams_work(lm, small_field):
     """Inputs still being written on the default stream when the call is made (a pause of some milliseconds before
     them), forward and backward: the results of finished inputs."""
