@@ -65,11 +65,6 @@ __device__ __forceinline__ float norm_dist(int norm, float2 a, float2 b) {
   return norm == 2 ? d2 : norm == 1 ? fabsf(dx) + fabsf(dy) : fmaxf(fabsf(dx), fabsf(dy));
 }
 
-__device__ __forceinline__ unsigned long long pair_prio(uint32_t i, uint32_t j, uint32_t step, uint32_t k0,
-                                                        uint32_t k1) {
-  return order_hash(i, j, step, ((unsigned long long)k1 << 32) | k0);
-}
-
 // The three rock-paper-scissors outcomes of pair (local ids la, lb) at `step`, as list-entry bits:
 // the pair's Philox uniform (interactions.py:20's np.random.rand(), keyed by the pair) against the
 // ensemble's forward-win threshold of each matchup (interactions.py:24-35), u53 < t exactly as

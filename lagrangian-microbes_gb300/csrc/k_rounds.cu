@@ -163,7 +163,7 @@ __device__ __forceinline__ uint32_t tl_entry(const Bufs& b, const TileSmem& t, u
 // it), at most TL_VMAX per block: each block owns an equal share, in whole warps (whole 1,024-vertex
 // columns left 64 of the 304 blocks idle at 490k).
 template <int RD_THREADS>
-__device__ void tl_group(const Bufs& b, uint32_t step, Ctrl* ctrl, unsigned long long t0, uint32_t g_lo,
+__device__ void tl_group(const Bufs& b, Ctrl* ctrl, unsigned long long t0, uint32_t g_lo,
                          uint32_t g_hi) {
   constexpr int TL_VPT = (int)TL_VMAX / RD_THREADS;  // vertices per thread at most
   extern __shared__ unsigned long long tl_raw[];
@@ -347,7 +347,7 @@ __device__ void tl_wide(const Bufs& b, Ctrl* ctrl, unsigned long long t0, uint32
 
 // Returns false (nothing done) when the step does not fit the tile paths (grid-uniform).
 template <int RD_THREADS>
-__device__ bool rounds_tiled(const Bufs& b, uint32_t step, Ctrl* ctrl, unsigned long long t0, uint32_t n_valid,
+__device__ bool rounds_tiled(const Bufs& b, Ctrl* ctrl, unsigned long long t0, uint32_t n_valid,
                              bool ev_taken) {
   if (b.plog) return false;
   extern __shared__ unsigned long long tl_raw[];
@@ -368,7 +368,7 @@ __device__ bool rounds_tiled(const Bufs& b, uint32_t step, Ctrl* ctrl, unsigned 
   }
   for (int g = 0; g < groups; ++g) {
     if (ev_taken && ((tg.taken >> g) & 1ull)) continue;
-    tl_group<RD_THREADS>(b, step, ctrl, t0, tg.lo[g], tg.lo[g + 1]);
+    tl_group<RD_THREADS>(b, ctrl, t0, tg.lo[g], tg.lo[g + 1]);
     __syncthreads();  // the block's shared lists are reused by the next group
   }
   return true;
@@ -380,12 +380,11 @@ __global__ void __launch_bounds__(RD_THREADS, 2) k_rounds(Bufs b, StepArgs a, Ct
   // the control words, read by one thread per block: every thread of the 300-odd blocks loading
   // the same L2 line (the loads are volatile, so L1 does not merge them) queued ~10^4 requests on
   // one L2 slice and delayed the start of the pairs by 4-10 us
-  __shared__ uint32_t cw[4];
+  __shared__ uint32_t cw[3];
   if (threadIdx.x == 0) {
     cw[0] = ((volatile uint32_t*)&ctrl->halt)[0];
-    cw[3] = ((volatile uint32_t*)&ctrl->ev_taken)[0];
+    cw[2] = ((volatile uint32_t*)&ctrl->ev_taken)[0];
     cw[1] = ((volatile uint32_t*)&ctrl->n_valid)[0];
-    cw[2] = a.use_ctrl_step ? ((volatile uint32_t*)&ctrl->step)[0] : a.step0;
   }
   __syncthreads();
   if (cw[0]) return;
@@ -403,13 +402,12 @@ __global__ void __launch_bounds__(RD_THREADS, 2) k_rounds(Bufs b, StepArgs a, Ct
     }
     return;
   }
-  const uint32_t step = cw[2];
   const uint32_t cnt = cw[1];
   const uint32_t stride = gridDim.x * blockDim.x;
   const uint32_t first = blockIdx.x * blockDim.x + threadIdx.x;
   uint32_t max_level = 0;
   const unsigned long long t0 = globaltimer();
-  if (rounds_tiled<RD_THREADS>(b, step, ctrl, t0, cnt, cw[3] != 0u)) return;  // levels are tracked only in pair-log runs
+  if (rounds_tiled<RD_THREADS>(b, ctrl, t0, cnt, cw[2] != 0u)) return;  // levels are tracked only in pair-log runs
   uint32_t polls = 0;
   if (cnt <= (uint32_t)POLL_BATCH * stride) {
     // every thread owns at most POLL_BATCH vertices: keep their ids in registers and stop polling

@@ -16,7 +16,6 @@
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
-#include <vector>
 
 #include "lm_api.h"
 #include "lm_internal.h"
@@ -49,7 +48,6 @@ struct lm_adjoint {
   int prec = ADJ_DS;  // working precision of the recorded run
   int prec_next = ADJ_DS;
   DBuf<AdjStep> table;
-  std::vector<AdjStep> table_h;
   // positions of adj_state_bytes(prec) per element; adjoint state lx, ly of adj_lambda_bytes(prec)
   DBuf<unsigned char> x, y, ck_x, ck_y, seg_x, seg_y, lx, ly, fin_x, fin_y;
   int batch = 1;     // backward steps reduced together
@@ -318,8 +316,6 @@ int lm_adjoint_forward(lm_adjoint* a, const float* u, const float* v, int nt, in
   a->dt = dt_sec;
   ACK(cudaMemsetAsync(a->err_d, 0, sizeof(uint32_t), st));
   launch_adj_stages(a->fv, t_start, dt_sec, n_steps, a->table.p, a->err_d, st);
-  a->table_h.resize(n_steps);
-  ACK(cudaMemcpyAsync(a->table_h.data(), a->table.p, sizeof(AdjStep) * n_steps, cudaMemcpyDeviceToHost, st));
   uint32_t err;
   if ((r = read_err(a, st, &err))) return r;
   if (err & ERRB_TIME) return afail(a, LM_ERR_TIME, "a stage time fell outside the field's time axis");

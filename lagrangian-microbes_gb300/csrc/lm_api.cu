@@ -749,7 +749,6 @@ int run_steps(lm_ctx* c, double t, double dt, int64_t n_steps, int64_t step0, ui
               float* rec_lon, float* rec_lat, int8_t* rec_species, int64_t* rec_census) {
   int r;
   if ((r = refuse_capture(c))) return r;
-  if (n_steps < 1 && (r = write_ctrl_step(c, step0))) return r;  // (a step sets the counter as it begins)
   if (rec_census && (r = ensure_hstage(c, (size_t)4 * n_steps))) return r;
   c->rec_lon = rec_lon;
   c->rec_lat = rec_lat;

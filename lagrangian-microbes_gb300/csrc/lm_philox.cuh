@@ -63,11 +63,6 @@ __host__ __device__ __forceinline__ unsigned long long order_hash_from(unsigned 
   z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
   return z ^ (z >> 31);
 }
-__host__ __device__ __forceinline__ unsigned long long order_hash(uint32_t i, uint32_t j, uint32_t step,
-                                                                  unsigned long long seed) {
-  return order_hash_from(order_hash_base(step, seed), i, j);
-}
-
 // Two uniforms in (-1, 1) for the diffusion kick of particle `p` at step `step`
 // (first for latitude, second for longitude, the reference's order).
 __host__ __device__ __forceinline__ void diffusion_draw(uint32_t p, uint32_t step, uint32_t k0, uint32_t k1,
