@@ -266,6 +266,9 @@ int lm_adjoint_destroy(lm_adjoint* adj);
 #define LM_ADJ_F64 1
 #define LM_ADJ_DS 2
 int lm_adjoint_set_precision(lm_adjoint* adj, int precision);
+/* Do the tape's next forwards store the states of their last checkpoint interval as they go (1, the default), which a
+ * backward begins with, or not (0: for runs without a backward; one may follow all the same and computes them)? */
+int lm_adjoint_keep_states(lm_adjoint* adj, int keep);
 /* u, v [nt][ny][nx] m/s and the axes as lm_field_upload (axes are host arrays); n microbes from
  * lon0/lat0 (absolute degrees) for n_steps steps of dt_sec from t_sec0; final positions into
  * lon_out/lat_out. Microbes leaving the domain are frozen (LM_ERR_OUT_OF_BOUNDS is returned, the tape is

@@ -59,8 +59,9 @@ class AdjointTape:
         self.ctx.call("lm_ctx_set_stream", torch.cuda.current_stream(dev).cuda_stream)
 
     def forward(self, lon0, lat0, u, v, lon_axis, lat_axis, t_axis, t0: float, dt: float, n_steps: int,
-                checkpoint_every: int = 32, allow_out_of_bounds: bool = False):
-        """Run and record; returns (lon, lat) float32 device tensors."""
+                checkpoint_every: int = 32, allow_out_of_bounds: bool = False, keep_states: bool = True):
+        """Run and record; returns (lon, lat) float32 device tensors. ``keep_states=False``, for runs that no backward
+        follows, does not store the last segment's states, which the first step of a backward computes again."""
         for name, t in (("lon0", lon0), ("lat0", lat0), ("u", u), ("v", v)):
             if not (t.is_cuda and t.dtype == torch.float32 and t.is_contiguous()):
                 raise ValueError(f"{name} must be a contiguous float32 CUDA tensor")
@@ -76,6 +77,7 @@ class AdjointTape:
         lon = torch.empty_like(lon0)
         lat = torch.empty_like(lat0)
         self._stream(lon0.device)
+        self.ctx.check(self._lib.lm_adjoint_keep_states(self._h, int(keep_states)))
         rc = self._lib.lm_adjoint_forward(self._h, u.data_ptr(), v.data_ptr(), nt, ny, nx, _lib.ptr(ax[0]),
                                           _lib.ptr(ax[1]), _lib.ptr(ax[2]), n, lon0.data_ptr(), lat0.data_ptr(),
                                           float(t0), float(dt), int(n_steps), int(checkpoint_every),
@@ -125,9 +127,10 @@ class AdjointTape:
 
 class _AdvectRK4(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, lon0, lat0, u, v, tape, axes, t0, dt, n_steps, checkpoint_every, allow_oob):
+    def forward(ctx, lon0, lat0, u, v, tape, axes, t0, dt, n_steps, checkpoint_every, allow_oob, keep_states):
         lon, lat = tape.forward(lon0.detach().contiguous(), lat0.detach().contiguous(), u.detach().contiguous(),
-                                v.detach().contiguous(), *axes, t0, dt, n_steps, checkpoint_every, allow_oob)
+                                v.detach().contiguous(), *axes, t0, dt, n_steps, checkpoint_every, allow_oob,
+                                keep_states)
         ctx.tape = tape
         return lon, lat
 
@@ -138,7 +141,7 @@ class _AdvectRK4(torch.autograd.Function):
         if g_lat is None:
             g_lat = torch.zeros(ctx.tape.n, dtype=torch.float32, device=g_lon.device)
         g_lon0, g_lat0, g_u, g_v = ctx.tape.backward(g_lon, g_lat)
-        return g_lon0, g_lat0, g_u, g_v, None, None, None, None, None, None, None
+        return (g_lon0, g_lat0, g_u, g_v) + (None,) * 8
 
 
 def advect_rk4(lon0, lat0, u, v, lon_axis, lat_axis, t_axis, t0: float, dt: float, n_steps: int,
@@ -147,7 +150,8 @@ def advect_rk4(lon0, lat0, u, v, lon_axis, lat_axis, t_axis, t0: float, dt: floa
     """Differentiable RK4 advection (float32 CUDA tensors in and out); see the module docstring."""
     tape = tape or AdjointTape(device=lon0.device.index or 0, precision=precision)
     return _AdvectRK4.apply(lon0, lat0, u, v, tape, (lon_axis, lat_axis, t_axis), float(t0), float(dt),
-                            int(n_steps), int(checkpoint_every), bool(allow_out_of_bounds))
+                            int(n_steps), int(checkpoint_every), bool(allow_out_of_bounds),
+                            torch.is_grad_enabled() and any(t.requires_grad for t in (lon0, lat0, u, v)))
 
 
 def great_circle_m(lon1, lat1, lon2, lat2):

@@ -53,6 +53,7 @@ struct lm_adjoint {
   int batch = 1;     // backward steps reduced together
   int sets = 2;      // of batch buffers
   int seg_held = -1;  // segment whose states seg_* hold
+  bool keep = true;   // the forward stores those of its last segment (lm_adjoint_keep_states)
   DBuf<float> csum;
   DBuf<int4> part;
   DBuf<uint8_t> st, ck_st, seg_st;
@@ -241,6 +242,12 @@ int lm_adjoint_destroy(lm_adjoint* a) {
   return LM_OK;
 }
 
+int lm_adjoint_keep_states(lm_adjoint* a, int keep) {
+  if (!a) return LM_ERR_ARG;
+  a->keep = keep != 0;
+  return LM_OK;
+}
+
 int lm_adjoint_set_precision(lm_adjoint* a, int precision) {
   if (!a) return LM_ERR_ARG;
   if (precision != LM_ADJ_F32 && precision != LM_ADJ_F64 && precision != LM_ADJ_DS)
@@ -328,7 +335,7 @@ int lm_adjoint_forward(lm_adjoint* a, const float* u, const float* v, int nt, in
       ACK(cudaMemcpyAsync(a->ck_st.p + (size_t)s * N, a->st.p, N, cudaMemcpyDeviceToDevice, st));
     }
     // the last segment is the first to be reversed: its states are stored as they are computed
-    const bool keep = s == n_ck - 1;
+    const bool keep = a->keep && s == n_ck - 1;
     launch_adj_forward(a->fv, prec, a->table.p, m0, m1, a->dt, N, a->x.p, a->y.p, a->st.p,
                        keep ? a->seg_x.p : nullptr, keep ? a->seg_y.p : nullptr, keep ? a->seg_st.p : nullptr,
                        a->err_d, st);

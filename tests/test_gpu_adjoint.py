@@ -431,6 +431,34 @@ def test_adjoint_non_finite_gradients_stay_in_their_cells(small_field, bad):
     assert int((~np.isfinite(got[2])).sum()) > few
 
 
+def test_forward_without_a_gradient_does_not_store_its_states(lm, small_field, monkeypatch):
+    """Only a run that autograd records stores the last segment's states; a backward finds the same gradient either way."""
+    from lagrangian_microbes_gb300 import adjoint
+    f, dev = small_field, torch.device("cuda:0")
+    lon, lat, _, _ = _case(f, 700, 6)
+    put = lambda a: torch.from_numpy(np.ascontiguousarray(a, np.float32)).to(dev)
+    args = [put(a) for a in (lon, lat, f.u, f.v)]
+    rest = (f.lon, f.lat, f.times, float(f.times[0]), 3600.0, 5)
+    asked, plain = [], adjoint.AdjointTape.forward
+    monkeypatch.setattr(adjoint.AdjointTape, "forward",
+                        lambda self, *a, **k: asked.append(k.get("keep_states", a[12] if len(a) > 12 else True)) or plain(self, *a, **k))
+    tape = adjoint.AdjointTape()
+    adjoint.advect_rk4(*args, *rest, tape=tape)
+    args[0].requires_grad_()
+    with torch.no_grad():
+        adjoint.advect_rk4(*args, *rest, tape=tape)
+    adjoint.advect_rk4(*args, *rest, tape=tape)
+    assert asked == [False, False, True]
+    one = torch.ones(700, device=dev)
+    got = []
+    for keep in (True, False):
+        plain(tape, *(t.detach() for t in args), *rest, checkpoint_every=2, keep_states=keep)
+        got.append(tape.backward(one, 2 * one))
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
+    tape.close()
+
+
 def test_adjoint_takes_smaller_batches_where_memory_is_short(lm, small_field):
     """4,000,000 microbes with 1.4 GB left on the device: one set of batch buffers for one step fits (270 bytes a microbe
     with the tape's own), two do not. The gradients are those of a run with the memory it likes."""
