@@ -626,9 +626,8 @@ void launch_count_pairs(const Bufs& b, const PairParams& pp, Ctrl* ctrl, int sms
 // Only the sorted partners are kept (the priorities were needed for the order only).
 // Bound by instruction issue (73 % of the slots, 670 instructions a list of 34). A warp per list before
 // took 530 us for the 447,000 lists of 32 ensembles, 245 for the 338,000 of 2,000,000 mixed microbes and 66
-// for the 81,000 of 490,000; this takes 368, 144 and 42. At 6 blocks an SM (9 KB a warp) it took 438,
-// 194 and 54. Lists done alone: 1,100 neighbours each 21.4 -> 1.4 ms for 10,000 microbes (one lane sorted them
-// before); 210 each 0.15 -> 0.21 for 30,000, of 2.1 ms a step.
+// for the 81,000 of 490,000; this takes 368, 133 and 40. At 6 blocks an SM (9 KB a warp) it took 438,
+// 194 and 54. 10,000 microbes with 1,100 neighbours each 21.4 -> 1.0 ms (one lane sorted such lists before).
 constexpr int LONG_WARPS = 4;
 constexpr uint32_t LONG_SMEM_MAX = 512;
 constexpr uint32_t LONG_BUCKETS = 256;
@@ -799,20 +798,26 @@ __device__ __forceinline__ void long_sort_global(const Bufs& b, LongSmem& sh, co
 
 // One list by the whole warp, candidates from global memory: candidate i is in the run q with c[q] <= i < c[q + 1],
 // which starts at t0[q].
-__device__ __noinline__ void long_alone(const Bufs& b, const PairParams& pp, uint32_t step, LongSmem& sh, uint32_t s,
-                                        uint32_t d, unsigned long long o, const uint32_t* t0, const uint32_t* c) {
+__device__ __forceinline__ void long_alone(const Bufs& b, const PairParams& pp, uint32_t step, LongSmem& sh, uint32_t s,
+                                           uint32_t d, unsigned long long o, const uint32_t (&t0)[6], const uint32_t (&c)[7]) {
   const uint32_t lane = threadIdx.x & 31u;
-  const uint32_t id0 = b.sid[s];
-  const EnsInfo& info = b.ens[ens_of(b, s)];
+  const float2* __restrict__ spos = b.spos;
+  const uint32_t* __restrict__ sid = b.sid;
+  uint32_t* const list = b.ovf + o;
+  unsigned long long* const prio = b.oprio + o;
+  const Band band = band_of(pp);
+  const int norm = pp.norm;
+  const uint32_t id0 = sid[s];
+  const EnsInfo info = b.ens[ens_of(b, s)];
   const LongHead h = {order_hash_base(step, ((unsigned long long)info.seed_hi << 32) | info.seed_lo), id0 - info.base,
                       info.base};
   const int sp = b.species[id0];
-  const float2 ps = b.spos[s];
+  const float2 ps = spos[s];
   const bool in_smem = d <= LONG_SMEM_MAX;
   uint32_t m = 0;
-  // two slices of 32 candidates per pass
+  // two slices of 32 candidates per pass, each candidate's position and id loaded together
   for (uint32_t tb = 0; tb < c[6]; tb += 64) {
-    uint32_t t[2];
+    uint32_t t[2], id[2];
     float2 pt[2];
     bool in[2];
 #pragma unroll
@@ -824,18 +829,25 @@ __device__ __noinline__ void long_alone(const Bufs& b, const PairParams& pp, uin
         if (i >= c[q]) x = t0[q] + (i - c[q]);  // the last run starting at or before i (empty runs never win)
       t[r] = x;
       in[r] = i < c[6] && x != s;
-      pt[r] = in[r] ? b.spos[x] : ps;
+      pt[r] = in[r] ? spos[x] : ps;
+      id[r] = in[r] ? sid[x] : 0u;
     }
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
-      const bool ok = in[r] && within(pp, ps, pt[r]);
+      const float dist = norm_dist(norm, ps, pt[r]);
+      bool ok = in[r] && dist < band.lo;
+      const bool unsure = in[r] && !(dist < band.lo) && !(dist > band.hi);
+      if (__any_sync(0xffffffffu, unsure) && unsure) ok = within(pp, ps, pt[r]);
       const uint32_t mask = __ballot_sync(0xffffffffu, ok);
       const uint32_t pos = m + __popc(mask & lanemask_lt_p());
-      if (ok && pos < d) {
-        if (in_smem)
+      if (ok && pos < d) {  // the partner and its local id; priority and draw follow below
+        if (in_smem) {
           sh.t[pos] = t[r];
-        else
-          b.ovf[o + pos] = t[r];
+          sh.key[pos] = id[r] - h.base;
+        } else {
+          list[pos] = t[r];
+          prio[pos] = id[r] - h.base;
+        }
       }
       m += __popc(mask);
     }
@@ -843,29 +855,99 @@ __device__ __noinline__ void long_alone(const Bufs& b, const PairParams& pp, uin
   __syncwarp();
   // priorities and outcome draws of the d entries, one entry per lane
   for (uint32_t i = lane; i < d; i += 32) {
-    const uint32_t t = in_smem ? sh.t[i] : b.ovf[o + i], lb = b.sid[t] - h.base;
+    const uint32_t t = in_smem ? sh.t[i] : list[i], lb = in_smem ? sh.key[i] : (uint32_t)prio[i];
     const uint32_t hi = (uint32_t)(order_hash_from(h.hash, min(h.la, lb), max(h.la, lb)) >> 32);
     const uint32_t e = t > s ? t | win_bits(info, h.la, lb, step) : t;
     if (in_smem) {
       sh.key[i] = hi;
       sh.t[i] = e;
     } else {
-      b.oprio[o + i] = (unsigned long long)hi << 32 | e;
+      prio[i] = (unsigned long long)hi << 32 | e;
     }
   }
   __syncwarp();
   if (in_smem) {
     long_sort(b, sh, h, d, lane);
-    for (uint32_t i = lane; i < d; i += 32) b.ovf[o + i] = sh.t[sh.ord[i]];
+    for (uint32_t i = lane; i < d; i += 32) list[i] = sh.t[sh.ord[i]];
   } else {
-    long_sort_global(b, sh, h, b.oprio + o, b.ovf + o, d, lane);
+    long_sort_global(b, sh, h, prio, list, d, lane);
   }
   if (lane == 0) {
-    b.ovf[o + d] = NONE;
+    list[d] = NONE;
     b.slab[(size_t)s * SLAB] = (uint32_t)o;  // a long list's overflow offset, in its unused slab row
-    b.wstate[s] = pack_state(in_smem ? sh.t[sh.ord[0]] : b.ovf[o], 0u, sp);  // entry 0 of the list
+    b.wstate[s] = pack_state(in_smem ? sh.t[sh.ord[0]] : list[0], 0u, sp);  // entry 0 of the list
   }
   __syncwarp();  // the next list reuses the shared memory
+}
+
+// A batch of up to `per` lists, lane k's the one at place q + k * next: its vertex, length, overflow offset, key runs (one
+// chain of dependent loads for all of them) and cell key. `run`: the offset of the batch's first list, moved behind its last.
+struct LongBatch {
+  bool mine;
+  uint32_t s, d, key, cand;
+  unsigned long long o;
+  uint32_t r0[6], len[6];
+  __device__ __forceinline__ LongBatch(const Bufs& b, uint32_t q, uint32_t next, uint32_t per, uint32_t n_long,
+                                       unsigned long long& run) {
+    const uint32_t lane = threadIdx.x & 31u;
+    mine = lane < per && q + lane * next < n_long;
+    s = mine ? b.longv[q + lane * next] : 0u;
+    d = mine ? b.deg[s] : 0u;
+    const uint32_t room = mine ? d + 1u : 0u;
+    unsigned long long incl = room;
+    for (int k = 1; k < 32; k <<= 1) {
+      const unsigned long long y = __shfl_up_sync(0xffffffffu, incl, k);
+      if (lane >= (uint32_t)k) incl += y;
+    }
+    o = run + incl - room;
+    run += __shfl_sync(0xffffffffu, incl, 31);
+    key = cand = 0u;
+#pragma unroll
+    for (int r = 0; r < 6; ++r) r0[r] = len[r] = 0u;
+    if (mine) {
+      const Vertex v = load_vertex(b, s);
+      neighbour_runs(b, v, r0, len);
+#pragma unroll
+      for (int r = 0; r < 6; ++r) len[r] -= r0[r];
+      key = v.g.cell_base + cell_index(v.g, v.cx, v.cy);
+    }
+#pragma unroll
+    for (int r = 0; r < 6; ++r) cand += len[r];
+  }
+  // The lists that are done one at a time.
+  __device__ __forceinline__ uint32_t alone() const {
+    return __ballot_sync(0xffffffffu, d > LONG_FEW || cand > LONG_CAND);
+  }
+  // Lane k's runs as one range, in every lane.
+  __device__ __forceinline__ void range(int k, uint32_t (&t0)[6], uint32_t (&c)[7]) const {
+    c[0] = 0;
+#pragma unroll
+    for (int r = 0; r < 6; ++r) {
+      t0[r] = __shfl_sync(0xffffffffu, r0[r], k);
+      c[r + 1] = c[r] + __shfl_sync(0xffffffffu, len[r], k);
+    }
+  }
+};
+
+// The lists of a warp's batches that are done one at a time, after the others and in the same shared memory. Its own walk
+// over the batches, so that neither side's registers weigh on the other. Called from the other's loop instead, with the
+// runs on the stack and the kernel's parameters behind references (which the stores between two uses made it load again),
+// and the ids read after the gather: 200,000 microbes with 218 neighbours each 1.33 ms, 490,000 3.23, 30,000 0.21; now 0.89,
+// 2.15 and 0.14 (0.94, 2.29 and 0.15 when a warp did every list of any length by itself).
+__device__ __forceinline__ void long_rest(const Bufs& b, const PairParams& pp, uint32_t step, LongSmem& sh, uint32_t first,
+                                          uint32_t next, uint32_t turn, uint32_t per, uint32_t n_long,
+                                          unsigned long long run) {
+  __syncwarp();  // (the shared memory has been the area's)
+  for (uint32_t q = first; q < n_long; q += turn) {
+    const LongBatch l(b, q, next, per, n_long, run);
+    for (uint32_t m = l.alone(); m; m &= m - 1) {
+      const int k = __ffs(m) - 1;
+      uint32_t t0[6], c[7];
+      l.range(k, t0, c);
+      long_alone(b, pp, step, sh, __shfl_sync(0xffffffffu, l.s, k), __shfl_sync(0xffffffffu, l.d, k),
+                 __shfl_sync(0xffffffffu, l.o, k), t0, c);
+    }
+  }
 }
 
 // Entry i of the area at place k of its list; the first one also makes its member ready.
@@ -993,46 +1075,14 @@ __global__ void __launch_bounds__(LONG_WARPS * 32, 8) k_sweep_long(Bufs b, PairP
     }
     return;
   }
+  const unsigned long long run0 = run;
+  bool rest = false;
   for (uint32_t q = first; q < n_long; q += turn) {
-    // lane k loads member k's cell, position, key runs and ensemble constants: a chain of dependent loads per batch
-    const bool mine = lane < per && q + lane * next < n_long;
-    const uint32_t nk = __popc(__ballot_sync(0xffffffffu, mine));  // (the first nk lanes)
-    const uint32_t s_l = mine ? b.longv[q + lane * next] : 0u;
-    const uint32_t d_l = mine ? b.deg[s_l] : 0u;
-    const uint32_t room_l = mine ? d_l + 1u : 0u;
-    unsigned long long incl = room_l;
-    for (int o = 1; o < 32; o <<= 1) {
-      const unsigned long long y = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= (uint32_t)o) incl += y;
-    }
-    const unsigned long long o_l = run + incl - room_l;
-    run += __shfl_sync(0xffffffffu, incl, 31);
-    uint32_t r0[6], len[6], key_l = 0;
-#pragma unroll
-    for (int r = 0; r < 6; ++r) r0[r] = len[r] = 0u;
-    if (mine) {
-      const Vertex v = load_vertex(b, s_l);
-      neighbour_runs(b, v, r0, len);
-#pragma unroll
-      for (int r = 0; r < 6; ++r) len[r] -= r0[r];
-      key_l = v.g.cell_base + cell_index(v.g, v.cx, v.cy);
-    }
-    uint32_t cand = 0;
-#pragma unroll
-    for (int r = 0; r < 6; ++r) cand += len[r];
-    const uint32_t large = __ballot_sync(0xffffffffu, d_l > LONG_FEW || cand > LONG_CAND);
-    for (uint32_t m = large; m; m &= m - 1) {  // one at a time, in the same shared memory
-      const int k = __ffs(m) - 1;
-      uint32_t t0[6], c[7];
-      c[0] = 0;
-#pragma unroll
-      for (int r = 0; r < 6; ++r) {
-        t0[r] = __shfl_sync(0xffffffffu, r0[r], k);
-        c[r + 1] = c[r] + __shfl_sync(0xffffffffu, len[r], k);
-      }
-      long_alone(b, pp, step, sh_all[w].one, __shfl_sync(0xffffffffu, s_l, k), __shfl_sync(0xffffffffu, d_l, k),
-                 __shfl_sync(0xffffffffu, o_l, k), t0, c);
-    }
+    const LongBatch l(b, q, next, per, n_long, run);
+    const bool mine = l.mine;
+    const uint32_t s_l = l.s, nk = __popc(__ballot_sync(0xffffffffu, mine));  // (the first nk lanes)
+    const uint32_t large = l.alone();
+    rest |= large != 0u;
     if (mine) {
       const uint32_t id = b.sid[s_l], e = ens_of(b, s_l);
       const EnsInfo& info = b.ens[e];
@@ -1041,24 +1091,19 @@ __global__ void __launch_bounds__(LONG_WARPS * 32, 8) k_sweep_long(Bufs b, PairP
       sh.s[lane] = s_l;
       sh.la[lane] = id - info.base;
       sh.e[lane] = e;
-      sh.o[lane] = (uint32_t)o_l;
-      sh.d[lane] = (uint16_t)d_l;  // (read for the small ones only)
+      sh.o[lane] = (uint32_t)l.o;
+      sh.d[lane] = (uint16_t)l.d;  // (read for the small ones only)
       sh.sp[lane] = b.species[id];
     }
     uint32_t used = 0;  // entries in the area
-    for (uint32_t rest = (nk == 32u ? 0xffffffffu : (1u << nk) - 1u) & ~large; rest;) {
-      const int lead = __ffs(rest) - 1;
-      const uint32_t lead_key = __shfl_sync(0xffffffffu, key_l, lead);
-      uint32_t m = __ballot_sync(0xffffffffu, mine && key_l == lead_key) & rest;
-      rest &= ~m;
+    for (uint32_t left = (nk == 32u ? 0xffffffffu : (1u << nk) - 1u) & ~large; left;) {
+      const int lead = __ffs(left) - 1;
+      const uint32_t lead_key = __shfl_sync(0xffffffffu, l.key, lead);
+      uint32_t m = __ballot_sync(0xffffffffu, mine && l.key == lead_key) & left;
+      left &= ~m;
       // the six runs as one candidate range: candidate i is in the run r with c[r] <= i < c[r + 1]
       uint32_t t0[6], c[7];
-      c[0] = 0;
-#pragma unroll
-      for (int r = 0; r < 6; ++r) {
-        t0[r] = __shfl_sync(0xffffffffu, r0[r], lead);
-        c[r + 1] = c[r] + __shfl_sync(0xffffffffu, len[r], lead);
-      }
+      l.range(lead, t0, c);
       __syncwarp();
       for (uint32_t i = lane; i < c[6]; i += 32) {
         uint32_t x = t0[0] + i;
@@ -1099,6 +1144,7 @@ __global__ void __launch_bounds__(LONG_WARPS * 32, 8) k_sweep_long(Bufs b, PairP
     }
     if (used) long_flush(b, step, sh, used);
   }
+  if (rest) long_rest(b, pp, step, sh_all[w].one, first, next, turn, per, n_long, run0);
 }
 
 void launch_sweep_long(const Bufs& b, const PairParams& pp, const StepArgs& a, Ctrl* ctrl, int sms,
