@@ -669,9 +669,13 @@ __global__ void __launch_bounds__(256) k_adj_signature(FieldView f, const AdjSte
 
 // ---------------------------------------------------------------- K7: reduction onto the grid
 
+// Entries of an item of a cell of m entries (a multiple of ADJ_ITEM).
+__device__ __forceinline__ uint32_t item_size(uint32_t m) {
+  return ADJ_ITEM * max(1u, m / (ADJ_ITEM * ADJ_SPLIT) + (m % (ADJ_ITEM * ADJ_SPLIT) ? 1u : 0u));
+}
+
 // Room for the entries of every occupied cell of step blockIdx.y (consecutive from place[c]), the list of
-// items, one per ADJ_ITEM entries of a cell, and room for the parts of cells of several items: one
-// reservation of each per block.
+// items and room for the parts of cells of several items: one reservation of each per block.
 constexpr int ALLOC_THREADS = 512;
 __global__ void __launch_bounds__(ALLOC_THREADS) k_adj_alloc(AdjBatch b) {
   pdl_wait();
@@ -679,7 +683,7 @@ __global__ void __launch_bounds__(ALLOC_THREADS) k_adj_alloc(AdjBatch b) {
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const uint32_t c = blockIdx.x * ALLOC_THREADS + threadIdx.x;
   const size_t o = (size_t)blockIdx.y * b.cells;
-  const uint32_t m = c < b.cells ? b.count[o + c] : 0u, items = (m + ADJ_ITEM - 1) / ADJ_ITEM;
+  const uint32_t m = c < b.cells ? b.count[o + c] : 0u, size = item_size(m), items = m / size + (m % size ? 1u : 0u);
   const uint32_t parts = items > 1 ? items : 0u;
   uint32_t sum[3] = {m, items, parts};  // inclusive sums over the warp
   for (int d = 1; d < 32; d <<= 1) {
@@ -709,7 +713,9 @@ __global__ void __launch_bounds__(ALLOC_THREADS) k_adj_alloc(AdjBatch b) {
   b.place[o + c] = at;
   uint4* list = b.list + (size_t)blockIdx.y * adj_items(b.n, b.cells) + base[1] + ws[1][warp] + sum[1] - items;
   for (uint32_t k = 0; k < items; ++k)
-    list[k] = make_uint4(c, at + k * ADJ_ITEM, min(ADJ_ITEM, m - k * ADJ_ITEM), parts ? part + k : NONE);
+    list[k] = make_uint4(c, at + k * size, min(size, m - k * size), parts ? part + k : NONE);
+  uint32_t* done = b.done + (size_t)blockIdx.y * adj_parts(b.n) + part;
+  for (uint32_t k = 0; k < parts; ++k) done[k] = 0u;
 }
 
 // Entries of the microbes' steps into their cells, in whatever order they come.
@@ -825,9 +831,9 @@ __device__ __forceinline__ void for_terms(const float4& r, F&& f) {
 struct FixTotal {
   uint32_t top = 0u;
   long long a = 0, b = 0, c = 0;
-  __device__ __forceinline__ void join(uint32_t t, int xa, int xb, int xc) {
+  __device__ __forceinline__ void join(uint32_t t, long long xa, long long xb, long long xc) {
     if (t == FIX_SPECIAL || top == FIX_SPECIAL) {
-      a = (top == FIX_SPECIAL ? a : 0ll) | (t == FIX_SPECIAL ? (long long)xa : 0ll);
+      a = (top == FIX_SPECIAL ? a : 0ll) | (t == FIX_SPECIAL ? xa : 0ll);
       top = FIX_SPECIAL;
       return;
     }
@@ -838,22 +844,60 @@ struct FixTotal {
       a = 0ll;
       top = t;
     }
-    a += down == 0u ? xa : 0;
-    b += down == 0u ? xb : down == 1u ? xa : 0;
-    c += down == 0u ? xc : down == 1u ? xb : down == 2u ? xa : 0;
+    a += down == 0u ? xa : 0ll;
+    b += down == 0u ? xb : down == 1u ? xa : 0ll;
+    c += down == 0u ? xc : down == 1u ? xb : down == 2u ? xa : 0ll;
   }
   __device__ __forceinline__ float value() const { return fix_value(top, a, b, c); }
 };
 
+// The sums of an item, or of several: [3][24], a lane's own at `part`.
+constexpr uint32_t PART_GROUP = 32;
+static_assert(ADJ_SPLIT <= PART_GROUP * PART_GROUP, "two levels put a cell's items together");
+__device__ __forceinline__ void part_store(long long* part, uint32_t slot, const FixTotal& t, bool on) {
+  long long* p = part + (size_t)slot * 72;
+  if (on) {
+    p[0] = t.a * 16 + t.top;  // (|a| < 2^54)
+    p[24] = t.b;
+    p[48] = t.c;
+  }
+  __threadfence();
+  __syncwarp();
+}
+// Is this the last of n warps to come here? (whole warp; the others' parts can be read then)
+__device__ __forceinline__ bool part_last(uint32_t* done, uint32_t n) {
+  uint32_t before = 0;
+  if ((threadIdx.x & 31u) == 0) before = atomicAdd(done, 1u);
+  const bool last = __shfl_sync(0xffffffffu, before, 0) == n - 1u;
+  if (last) __threadfence();
+  return last;
+}
+__device__ __noinline__ FixTotal part_merge(const long long* p, uint32_t stride, uint32_t n) {
+  FixTotal total;
+  for (uint32_t k0 = 0; k0 < n; k0 += 4) {
+    long long x[4][3];
+#pragma unroll
+    for (uint32_t k = 0; k < 4; ++k) {
+#pragma unroll
+      for (uint32_t j = 0; j < 3; ++j) x[k][j] = k0 + k < n ? __ldcg(p + (size_t)(k0 + k) * stride + 24 * j) : 0ll;
+    }
+#pragma unroll
+    for (uint32_t k = 0; k < 4; ++k) total.join((uint32_t)x[k][0] & 15u, x[k][0] >> 4, x[k][1], x[k][2]);
+  }
+  return total;
+}
+
 // A warp per item: four lanes take an entry, one each of its stages (stage 1 at t, 2 and 3 at t + dt/2, 4 at
 // t + dt), so a warp reads the records of eight entries at a time and holds those of ADJ_CHUNK in
 // registers: the largest terms first, then the sums. The items of a cell of several leave their sums in
-// `part`, and the warp that finishes the last one puts them together (in integers, whichever it is).
+// `part`, and the warps that finish last put them together (in integers, whichever they are).
 // Bound by instruction issue (64 % of the slots; the rest is latency of the records' loads): 47 us a step for
 // 1M microbes, where two parts a term, scaled by the cell's largest adjoint, took 35 and kept too few bits
 // (the counting of the largest by k_adj_step took 18 us more there: 66 -> 48). Forward and backward of 24
 // such steps: chunks of 32 entries at four blocks an SM 4.13 ms, at three 4.20, at five (spills) 4.28, chunks
-// of 64 at three 4.21; items of 64 4.22, of 256 4.38; the records read twice (69 us) 4.69.
+// of 64 at three 4.21; items of 64 4.22, of 256 4.38; the records read twice (69 us) 4.69. In crowded cells
+// the putting together counts: 8 steps of 1M microbes in 56 cells 2.98 ms, in one 23.2, by one warp for all
+// items of 128; 2.22 and 2.71 in two levels with at most 1,024 items (256 items: 2.22 and 3.92).
 constexpr int GATHER_THREADS = 256, GATHER_BLOCKS = 4;  // threads a block, blocks an SM
 constexpr uint32_t ADJ_ROUNDS = 4, ADJ_CHUNK = 8 * ADJ_ROUNDS;
 __global__ void __launch_bounds__(GATHER_THREADS, GATHER_BLOCKS) k_adj_gather(AdjBatch b) {
@@ -864,9 +908,9 @@ __global__ void __launch_bounds__(GATHER_THREADS, GATHER_BLOCKS) k_adj_gather(Ad
   const uint4* list = b.list + (size_t)q * adj_items(b.n, b.cells);
   const uint2* ent = b.ent + (size_t)q * 4 * b.n;
   const float4* rec = b.rec + (size_t)q * 4 * b.n;
-  int4* part = b.part + (size_t)q * adj_parts(b.n) * 24;
   // where this lane's sum goes: stage time, then by_stage's value (lanes of last bits 2 hold the same as those of 1)
   const uint32_t at = (s == 0u ? 0u : s == 3u ? 16u : 8u) + ((lane >> 4 & 1u) * 4u + (lane >> 3 & 1u) * 2u + (lane >> 2 & 1u));
+  long long* part = b.part + (size_t)q * adj_parts(b.n) * 72 + at;
   const uint32_t stride = gridDim.x * (GATHER_THREADS / 32);
   uint32_t t = blockIdx.x * (GATHER_THREADS / 32) + (threadIdx.x >> 5);
   uint4 next = t < nt ? list[t] : make_uint4(0u, 0u, 0u, 0u);
@@ -943,21 +987,19 @@ __global__ void __launch_bounds__(GATHER_THREADS, GATHER_BLOCKS) k_adj_gather(Ad
       if (s != 2u) *out = total.value();
       continue;
     }
-    if (s != 2u) part[(size_t)item.w * 24 + at] = make_int4((int)total.top, (int)total.a, (int)total.b, (int)total.c);
-    __threadfence();
-    __syncwarp();
-    const uint32_t all = b.count[oc + c], items = (all + ADJ_ITEM - 1) / ADJ_ITEM;
-    uint32_t before = 0;
-    if (lane == 0) before = atomicAdd(b.done + oc + c, 1u);
-    if (__shfl_sync(0xffffffffu, before, 0) != items - 1u) continue;
-    __threadfence();
-    const uint32_t index = (lo - (b.place[oc + c] - all)) / ADJ_ITEM;  // of this item (place: past the cell's last entry)
-    const int4* p = part + (size_t)(item.w - index) * 24 + at;
-    total = FixTotal();
-#pragma unroll 4
-    for (uint32_t k = 0; k < items; ++k) {
-      const int4 x = __ldcg(p + (size_t)k * 24);
-      total.join((uint32_t)x.x, x.y, x.z, x.w);
+    const uint32_t all = b.count[oc + c], size = item_size(all), items = all / size + (all % size ? 1u : 0u);
+    const uint32_t index = (lo - (b.place[oc + c] - all)) / size;  // of this item (place: past the cell's last entry)
+    // up to PART_GROUP items are put together by the last of them, and up to as many groups by the last group
+    const uint32_t first = item.w - index, head = first + index / PART_GROUP * PART_GROUP;
+    uint32_t* done = b.done + (size_t)q * adj_parts(b.n);
+    part_store(part, item.w, total, s != 2u);
+    if (!part_last(done + head, min(PART_GROUP, first + items - head))) continue;
+    total = part_merge(part + (size_t)head * 72, 72, min(PART_GROUP, first + items - head));
+    if (items > PART_GROUP) {
+      part_store(part, head, total, s != 2u);
+      const uint32_t groups = (items + PART_GROUP - 1) / PART_GROUP;
+      if (!part_last(done + first + 1, groups)) continue;  // (a place that no group counts in)
+      total = part_merge(part + (size_t)first * 72, 72 * PART_GROUP, groups);
     }
     if (s != 2u) *out = total.value();
   }

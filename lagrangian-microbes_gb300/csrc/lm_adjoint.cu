@@ -55,13 +55,13 @@ struct lm_adjoint {
   int seg_held = -1;  // segment whose states seg_* hold
   bool keep = true;   // the forward stores those of its last segment (lm_adjoint_keep_states)
   DBuf<float> csum;
-  DBuf<int4> part;
+  DBuf<long long> part;
   DBuf<uint8_t> st, ck_st, seg_st;
   DBuf<float4> rec;
   DBuf<uint4> cell;
   DBuf<uint2> ent;
   DBuf<uint4> list;
-  DBuf<uint32_t> count, place;  // count: [B][cells], done [B][cells] and the totals [B][4], zeroed together
+  DBuf<uint32_t> pdone, count, place;  // count: [B][cells] and the totals [B][4], zeroed together
   uint32_t* err_d = nullptr;
   uint32_t* err_h = nullptr;
   // the reduction of a batch runs on a stream of its own beside the next batch's steps: two sets of
@@ -134,13 +134,13 @@ int batch_steps(uint32_t n, uint64_t cells, int K) {
   return std::max(1, std::min({16, K, (int)std::min(fit, 16.0)}));
 }
 
-// The batch buffers for B steps, `sets` times. (At most 137 bytes a microbe and 124 a field cell for one step.)
+// The batch buffers for B steps, `sets` times. (At most 149 bytes a microbe and 120 a field cell for one step.)
 int batch_alloc(lm_adjoint* a, uint32_t n, uint64_t cells, int B, int sets) {
   const size_t k = (size_t)sets * B;
   int r;
   if ((r = grow(a, a->rec, 4 * k * n)) || (r = grow(a, a->cell, k * n)) || (r = grow(a, a->ent, 4 * k * n)) ||
-      (r = grow(a, a->count, k * (2 * cells + 4))) || (r = grow(a, a->place, k * cells)) ||
-      (r = grow(a, a->list, k * adj_items(n, cells))) || (r = grow(a, a->part, k * adj_parts(n) * 24)) ||
+      (r = grow(a, a->count, k * (cells + 4))) || (r = grow(a, a->place, k * cells)) ||
+      (r = grow(a, a->list, k * adj_items(n, cells))) || (r = grow(a, a->part, k * adj_parts(n) * 72)) || (r = grow(a, a->pdone, k * adj_parts(n))) ||
       (r = grow(a, a->csum, k * cells * 24)))
     return r;
   a->batch = B;
@@ -150,7 +150,7 @@ int batch_alloc(lm_adjoint* a, uint32_t n, uint64_t cells, int B, int sets) {
 
 void batch_release(lm_adjoint* a) {
   release(a->rec), release(a->cell), release(a->ent), release(a->count), release(a->place), release(a->list);
-  release(a->part), release(a->csum);
+  release(a->part), release(a->pdone), release(a->csum);
 }
 
 // Set `set` of the batch buffers, for `steps` steps.
@@ -162,13 +162,13 @@ AdjBatch batch_buffers(const lm_adjoint* a, uint32_t cells, int set, int steps) 
   b.steps = steps;
   b.rec = a->rec.p + 4 * k * a->n;
   b.cell = a->cell.p + k * a->n;
-  b.count = a->count.p + k * (2 * (size_t)cells + 4);
-  b.done = b.count + (size_t)steps * cells;
-  b.total = b.done + (size_t)steps * cells;
+  b.count = a->count.p + k * ((size_t)cells + 4);
+  b.total = b.count + (size_t)steps * cells;
   b.place = a->place.p + k * cells;
   b.list = a->list.p + k * adj_items(a->n, cells);
   b.ent = a->ent.p + 4 * k * a->n;
-  b.part = a->part.p + k * adj_parts(a->n) * 24;
+  b.done = a->pdone.p + k * adj_parts(a->n);
+  b.part = a->part.p + k * adj_parts(a->n) * 72;
   b.csum = a->csum.p + k * cells * 24;
   return b;
 }
@@ -390,7 +390,7 @@ int lm_adjoint_backward(lm_adjoint* a, const float* g_lon, const float* g_lat, f
       const AdjBatch b = batch_buffers(a, cells, set, std::min(a->batch, m - m0 + 1));
       if (!fresh[set]) ACK(cudaStreamWaitEvent(st, a->reduced[set], 0));  // its last reduction is done
       fresh[set] = false;
-      ACK(cudaMemsetAsync(b.count, 0, (size_t)b.steps * (2 * (size_t)cells + 4) * sizeof(uint32_t), st));
+      ACK(cudaMemsetAsync(b.count, 0, (size_t)b.steps * ((size_t)cells + 4) * sizeof(uint32_t), st));
       const size_t o = (size_t)(m - m0) * N;
       launch_adj_step(a->fv, a->prec, a->table.p, m, a->dt, b, a->seg_x.p + es * o, a->seg_y.p + es * o,
                       a->seg_st.p + o, a->lx.p, a->ly.p, st);

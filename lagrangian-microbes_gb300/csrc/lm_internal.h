@@ -390,16 +390,16 @@ struct AdjBatch {
   float4* rec;      // [steps][n][4]   (a, b, dL/dU, dL/dV) of each stage
   uint4* cell;      // [steps][n]      field cells of the four stages (NONE: the step was frozen)
   uint32_t* count;  // [steps][cells]  entries of a cell (zero before the batch)
-  uint32_t* done;   // [steps][cells]  its items that are summed, of cells of several (zero before the batch)
   uint32_t* total;  // [steps][4]      entries and parts reserved, items listed (zero before the batch)
   uint32_t* place;  // [steps][cells]  where a cell's entries go
   uint4* list;      // [steps][adj_items] items: (cell, first entry, entries, place of its parts or NONE)
   uint2* ent;       // [steps][4 n]    (microbe, stage bits), a cell's entries together
-  int4* part;       // [steps][adj_parts][24] sums of an item of a cell of several
+  long long* part;  // [steps][adj_parts][3][24] sums of an item of a cell of several
+  uint32_t* done;   // [steps][adj_parts] counters of items whose sums are there
   float* csum;      // [steps][cells][24] corner sums per stage time: of dL/dU, then of dL/dV
 };
-// Entries of an item: what one warp adds up for a cell.
-constexpr uint32_t ADJ_ITEM = 128;
+// Entries of an item, what one warp adds up for a cell: ADJ_ITEM, or the multiple of it that makes ADJ_SPLIT items.
+constexpr uint32_t ADJ_ITEM = 128, ADJ_SPLIT = 1024;
 // Items of a step at most: one per occupied cell and one per full item.
 __host__ __device__ inline size_t adj_items(uint32_t n, size_t cells) {
   const size_t e = (size_t)4 * n;

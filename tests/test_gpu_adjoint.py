@@ -310,7 +310,7 @@ def _still_gradient(f, lon, lat, g, share, magnitude=False):
 
 
 @pytest.mark.parametrize("precision", ["f32", "ds", "f64"])
-@pytest.mark.parametrize("n, large", [(3, 1e8), (3, 1e12), (200, 1e10), (700, 1e14), (0, 0)])
+@pytest.mark.parametrize("n, large", [(3, 1e8), (3, 1e12), (200, 1e10), (700, 1e14), (4500, 1e8), (140_000, 1e12), (0, 0)])
 def test_adjoint_small_terms_beside_large_ones_keep_their_digits(lm, n, large, precision):
     """A node's sum of small terms is as accurate as its own terms, whatever adjoints the field cell holds elsewhere: one
     large adjoint on a cell's corner beside n ordinary ones (no term of it at the other nodes, none in dL/dV), and
@@ -460,7 +460,7 @@ def test_forward_without_a_gradient_does_not_store_its_states(lm, small_field, m
 
 
 def test_adjoint_takes_smaller_batches_where_memory_is_short(lm, small_field):
-    """4,000,000 microbes with 1.4 GB left on the device: one set of batch buffers for one step fits (270 bytes a microbe
+    """4,000,000 microbes with 1.4 GB left on the device: one set of batch buffers for one step fits (283 bytes a microbe
     with the tape's own), two do not. The gradients are those of a run with the memory it likes."""
     from lagrangian_microbes_gb300.adjoint import AdjointTape
     f, n, dev = small_field, 4_000_000, torch.device("cuda:0")
