@@ -114,14 +114,16 @@ constexpr int POLL_BATCH = 2;  // vertices whose state words one thread loads be
 // Block b owns the vertices [b V, b V + V) (V <= TL_VMAX: an equal share in whole warps) and keeps their state words,
 // slot ids, degrees and list entries in shared memory. A pair whose two microbes the block owns
 // hands off through shared memory (tens of cycles instead of an L2 round trip); a pair that
-// crosses blocks goes through the global state words: the vertex's word is published there while
-// its current partner is outside the block, the owner of the lower endpoint applies the pair and
-// writes the other endpoint's global word, and that endpoint's owner pulls the change back into
-// shared memory. As in the global path, only the applier of a vertex's current pair writes the
-// vertex's word. A vertex has two words, though, and whoever writes both writes the global one first
-// (publish): as soon as the shared one shows the next pair, the vertex's owner may apply that pair with
-// the other block and publish a newer word, which a global store still on its way would take back (the
-// other block would wait for the pair after it until the time limit).
+// crosses blocks goes through the global state words: the owner of the lower endpoint applies the pair
+// and writes the other endpoint's global word, and that endpoint's owner pulls the change back into
+// shared memory. So a vertex's word is published there when another block is to apply its pair (its
+// partner is outside and below), and then only: nobody looks at the global word of the lower endpoint,
+// whose owner applies the pair itself. (Published for every crossing pair, that word could still be on
+// its way when the owner had applied the pair and published a newer one, which it then replaced; the
+// other block would wait until the time limit.) With that, whoever writes a vertex's global word has
+// seen the one before it: only the applier of a vertex's current pair writes the vertex's words, a
+// block's own appliers follow one another through the shared word, and another block's applier comes
+// in between only through the published word and is pulled back before the next. No fences are needed.
 static_assert(SLAB == 8, "the tile path copies a slab row as two 16-byte loads");
 constexpr uint32_t TL_VMAX = 2048;                     // vertices per block at most
 // and at least, while there are so many: in small ensembles most pairs would cross blocks, and a handoff through global
@@ -135,14 +137,6 @@ __device__ __forceinline__ unsigned long long ld_sh(const unsigned long long* p)
 }
 __device__ __forceinline__ void st_sh(unsigned long long* p, unsigned long long v) {
   *(volatile unsigned long long*)p = v;
-}
-
-// The global word of a vertex whose next pair crosses, before its shared word: after the stores that led to the words
-// read here (an earlier word of the vertex among them), and before the shared word's.
-__device__ __forceinline__ void publish(unsigned long long* p, unsigned long long v) {
-  __threadfence_block();
-  st_relaxed(p, v);
-  __threadfence_block();
 }
 
 struct TileSmem {
@@ -244,13 +238,13 @@ __device__ void tl_group(const Bufs& b, Ctrl* ctrl, unsigned long long t0, uint3
       const unsigned long long nwu = pack_state(nu, hu + 1u, new_u), nws = pack_state(ns, hs + 1u, new_s);
       const uint32_t nu_id = entry_id(nu), ns_id = entry_id(ns);
       if (u_local) {
-        if (nu != NONE && (nu_id < lo || nu_id >= hi)) publish(b.wstate + u, nwu);  // u's next pair crosses
         st_sh(t.w + (u - lo), nwu);
+        if (nu_id < lo) st_relaxed(b.wstate + u, nwu);  // another block applies u's next pair (NONE is above every id)
       } else {
         st_relaxed(b.wstate + u, nwu);  // u's owner pulls it
       }
-      if (ns != NONE && (ns_id < lo || ns_id >= hi)) publish(b.wstate + s, nws);  // s's next pair crosses
       st_sh(t.w + l, nws);
+      if (ns_id < lo) st_relaxed(b.wstate + s, nws);  // another block applies s's next pair
     }
     if (live && ((++polls & 63u) == 0u) && globaltimer() - t0 > ROUNDS_TIMEOUT_NS) {
       atomicOr(&ctrl->err, (uint32_t)ERRB_TIMEOUT);
@@ -326,13 +320,13 @@ __device__ void tl_wide(const Bufs& b, Ctrl* ctrl, unsigned long long t0, uint32
       const unsigned long long nwu = pack_state(nu, hu + 1u, new_u), nws = pack_state(ns, hs + 1u, new_s);
       const uint32_t nu_id = entry_id(nu), ns_id = entry_id(ns);
       if (u_local) {
-        if (nu != NONE && (nu_id < lo || nu_id >= hi)) publish(b.wstate + u, nwu);
         st_sh(tl_raw + (u - lo), nwu);
+        if (nu_id < lo) st_relaxed(b.wstate + u, nwu);
       } else {
         st_relaxed(b.wstate + u, nwu);
       }
-      if (ns != NONE && (ns_id < lo || ns_id >= hi)) publish(b.wstate + s, nws);
       st_sh(tl_raw + l, nws);
+      if (ns_id < lo) st_relaxed(b.wstate + s, nws);
     }
     if (live && ((++polls & 63u) == 0u) && globaltimer() - t0 > ROUNDS_TIMEOUT_NS) {
       atomicOr(&ctrl->err, (uint32_t)ERRB_TIMEOUT);

@@ -1,12 +1,14 @@
-"""Order of the two stores of an interaction handoff (k_rounds.cu, tl_group and tl_wide), on the CPU.
+"""Which handoffs of the interaction publish a vertex's word (k_rounds.cu, tl_group and tl_wide), on the CPU.
 
-A vertex of a block has a word in shared memory and one in global memory. Thread A applies the pair (s, u) inside the
-block and moves u on to a pair with another block; u's owner B may then apply that pair and move u on to the next, which
-the other block's thread R applies. Every interleaving of the three threads' loads and stores is followed: if each thread
-writes the global word before the shared one, u always gets through its list; the other way round an older global word
-can replace a newer one, and R waits for ever (the kernel: until its time limit). The sources are held to that order.
+A vertex u of a block has a word in shared memory and one in global memory. Its pairs, in order, are local ones (L: some
+thread of the block applies the pair and moves u's shared word on), pairs across blocks that u's owner applies (D: u is
+the lower endpoint) and pairs that another block applies (U: it looks at u's global word, writes it, and u's owner pulls
+the result into the shared word). Every interleaving of the threads' loads and stores is followed. Published only before
+a U, u always gets through its list; published before every pair across blocks, an older global word can replace a newer
+one, and the other block waits for ever (the kernel: until its time limit).
 """
 
+import itertools
 import os
 import re
 
@@ -15,51 +17,56 @@ import pytest
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "lagrangian-microbes_gb300", "csrc")
 
 
-def stuck(global_first):
-    """Does some interleaving end with u short of its last pair? Positions of u: 0 the pair (s, u), 1 a pair that B
-    applies across blocks, 2 one that R applies, 3 the end."""
-    order = ("G", "S") if global_first else ("S", "G")
-    # A and B: (position they write, stores left); R is one step
-    start = (0, 0, (1, order), None)  # shared word, global word, A's stores, B's stores
-    seen, todo, lost = set(), [start], False
+def stuck(pairs, publish):
+    """Does some interleaving end with u short of its last pair? `publish`: the kinds of next pair that are published."""
+    end = len(pairs)
+    kind = lambda p: pairs[p] if p < end else "-"
+    stores = lambda p: (("S", p),) + ((("G", p),) if kind(p) in publish else ())
+    # shared and global position, stores still to come of the owner and of the local appliers (one thread a pair)
+    todo, seen = [(0, 0, (), ())], set()
     while todo:
         state = todo.pop()
         if state in seen:
             continue
         seen.add(state)
-        S, G, a, b = state
+        S, G, owner, others = state
         after = []
-        for who, st in (("a", a), ("b", b)):
-            if not st:
-                continue
-            pos, left = st
-            S2, G2 = (pos, G) if left[0] == "S" else (S, pos)
-            rest = (pos, left[1:]) if left[1:] else None
-            after.append((S2, G2, rest, b) if who == "a" else (S2, G2, a, rest))
-        if b is None and S == 1:
-            after.append((S, G, a, (2, order)))  # B sees the pair and applies it
-        if b is None and S == 2 and G > S:
-            after.append((G, G, a, b))           # B pulls R's result
-        if G == 2:
-            after.append((S, 3, a, b))           # R sees itself named and applies
-        if not after and S != 3:
-            lost = True
+
+        def store(st, S=S, G=G):
+            return (st[1], G) if st[0] == "S" else (S, st[1])
+
+        if owner:
+            after.append((*store(owner[0]), owner[1:], others))
+        elif kind(S) == "D":
+            after.append((S, G, stores(S + 1), others))
+        elif kind(S) == "U" and G > S:
+            after.append((S, G, (("S", G),), others))
+        for k, thread in enumerate(others):
+            rest = tuple(t for t in others[:k] + (thread[1:],) + others[k + 1:] if t)
+            after.append((*store(thread[0]), owner, rest))
+        if kind(S) == "L" and not any(("S", S + 1) in t for t in others):
+            after.append((S, G, owner, tuple(sorted(others + (stores(S + 1),)))))
+        if kind(G) == "U":  # another block sees itself named (before any store of u's block, the lists' first pair)
+            after.append((S, G + 1, owner, others))
+        if not after and S != end:
+            return True
         todo += after
-    return lost
+    return False
 
 
-def test_a_handoff_gets_through_only_with_the_global_word_first():
-    assert stuck(global_first=False)
-    assert not stuck(global_first=True)
+@pytest.mark.parametrize("length", [1, 2, 3, 4, 5])
+def test_a_vertex_gets_through_every_sequence_of_pairs(length):
+    sequences = ["".join(p) for p in itertools.product("LDU", repeat=length)]
+    assert not [p for p in sequences if stuck(p, "U")]
+    lost = [p for p in sequences if stuck(p, "DU")]
+    assert all(re.search("LD.*U", p) for p in lost) and set(lost) >= {p for p in sequences if "LDU" in p}
 
 
-@pytest.mark.parametrize("word", ["u", "s"])
-def test_kernels_publish_before_the_shared_word_shows_the_pair(word):
+def test_kernels_publish_what_another_block_applies_and_nothing_else():
     with open(os.path.join(CSRC, "k_rounds.cu")) as f:
-        lines = f.read().split("\n")
-    published = [k for k, line in enumerate(lines) if re.search(rf"publish\(b\.wstate \+ {word}, nw{word}\)", line)]
-    assert len(published) == 2  # tl_group and tl_wide
-    for k in published:
-        assert re.search(rf"st_sh\(.*, nw{word}\);", lines[k + 1])
-    # the other stores of a global word are of vertices that the block does not own
-    assert len([line for line in lines if re.search(rf"st_relaxed\(b\.wstate \+ {word}, nw{word}\)", line)]) == (2 if word == "u" else 0)
+        source = f.read()
+    source = source[source.index("__device__ void tl_group("):source.index("__device__ bool rounds_tiled(")]
+    for word in "us":  # tl_group and tl_wide
+        assert len(re.findall(rf"if \(n{word}_id < lo\) st_relaxed\(b\.wstate \+ {word}, nw{word}\);", source)) == 2
+    assert len(re.findall(r"\} else \{\s*st_relaxed\(b\.wstate \+ u, nwu\);", source)) == 2  # u belongs to another block
+    assert source.count("st_relaxed(") == 6
