@@ -22,7 +22,7 @@
 // 250 instructions), one across blocks for two L2 round trips.
 //
 // Batches of ensembles of at least EV_SLOTS microbes launch this kernel (other contexts save the launch), and it takes
-// the groups of TileGroups::taken. 32 ensembles of 1e3-2e5 microbes on 0.5-3 degrees: 1,108 us polled, 648 shared out (of which 552 here).
+// the groups of TileGroups::taken. 32 ensembles of 1e3-2e5 microbes on 0.5-3 degrees: 1,108 us polled, 636 shared out (of which 548 here).
 #include "lm_rounds.cuh"
 
 namespace lm {

@@ -41,6 +41,8 @@ __device__ __forceinline__ void st_relaxed(unsigned long long* p, unsigned long 
 // ensembles of 1e3-2e5 microbes (16 groups), fresh lattices / after 9 days of flow, polled 6.37 / 7.39 ms; events from 14
 // to 64 neighbours 6.10 / 7.55, to 128 6.35 / 8.98, from 26 to 64 6.06 / 7.13, to 88 5.87 / 7.11 (but a step 16.97
 // ms against 16.46), from 34 to 88 5.87 / 7.41.
+// So the range is the uneven batch's: the mean cannot tell the two kinds apart, and even groups of 14 to 26 or 64 to
+// 128 neighbours are polled although events are faster there.
 constexpr int TL_GROUPS_MAX = 64;
 constexpr unsigned long long EV_MEAN_LO = 26, EV_MEAN_HI = 64;
 struct TileGroups {
