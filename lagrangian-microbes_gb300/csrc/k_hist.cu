@@ -31,12 +31,12 @@
 // true value by 1.6e-5 at most (log10f within 2 ulp of values up to 7.3, the product by ten rounded
 // once, asinf within 2 ulp, the rest below 2e-6), a bound of a taken from the chain's own cosines by
 // less than 3e-6, a squared chord by less than 1.8e-5 (dh_two_bins), and the hardware log2 by 1.4e-5
-// more. The chain's cosine comes from latitude / 180 rounded to float32, 1.5e-8 at most, so it is off by
-// 4.7e-8 / cos relative; the unit vectors do not carry that, and the chord differs from the chain by
-// 2.1e-7 / cos for it: 1.4e-5 at cos >= DH_COS_VEC = 1/64, below which chords are not taken. So a route
-// decides a pair only when its value lies farther than DH_MARGIN_A = 5e-5 (a alone) or DH_MARGIN = 1e-4
-// (log2) from the boundary; the chain itself decides every other pair. LM_HIST_EXACT=1 in the
-// environment makes every pair take the chain (the tests compare the two).
+// more. The chain's cosine comes from latitude / 180 rounded to float32, 1.5e-8 at most up to 90 degrees,
+// so it is off by 4.7e-8 / cos relative; the unit vectors do not carry that, and the chord differs from
+// the chain by 2.1e-7 / cos for it: 1.4e-5 at cos >= DH_COS_VEC = 1/64, below which (and past 90 degrees)
+// chords are not taken. So a route decides a pair only when its value lies farther than DH_MARGIN_A =
+// 5e-5 (a alone) or DH_MARGIN = 1e-4 (log2) from the boundary; the chain itself decides every other
+// pair. LM_HIST_EXACT=1 in the environment makes every pair take the chain (the tests compare the two).
 //
 // Bound by instruction issue. At 490k microbes on 5 x 5 degrees (three species, 4.0e10 pairs) a call
 // took 100.0 ms with every pair evaluated by itself; counted by groups it takes 8.1 ms: 19 % of the
@@ -576,7 +576,8 @@ __device__ __forceinline__ void dh_load_tile(const float4* __restrict__ pts, con
       const float4 p = pts[t];
       vec[t] = vecs[t];
       pt[t] = p;
-      b = DhBox{p.x, p.x, p.y, p.y, p.z, p.z};
+      // past 90 degrees (where latitude / 180 may round to anything) no box serves: as for a negative cosine
+      b = DhBox{p.x, p.x, p.y, p.y, fabsf(p.x) <= 90.f ? p.z : -1.f, p.z};
     }
     for (int o = 4; o > 0; o >>= 1) {
       const DhBox c{__shfl_xor_sync(0xffffffffu, b.la0, o), __shfl_xor_sync(0xffffffffu, b.la1, o),

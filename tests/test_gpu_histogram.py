@@ -190,10 +190,11 @@ def test_species_of_any_type_select_the_same_points(pdh, dtype):
         assert got[k][1] == want[1]
 
 
-@pytest.mark.parametrize("band", [(89.99, 90.0), (89.8, 90.0), (88.0, 88.5), (-90.0, -89.9)])
+@pytest.mark.parametrize("band", [(89.99, 90.0), (89.8, 90.0), (88.0, 88.5), (-90.0, -89.9), (36025.0, 36030.0)])
 def test_points_around_a_pole_keep_the_reference_chain_bins(pdh, monkeypatch, band):
     """The chain's cos(latitude) carries the float32 rounding of latitude / 180, which is a large part of the cosine near
-    a pole: pairs there must not be decided by coordinates that do not carry it (integers, so exactly)."""
+    a pole, and of large latitudes: pairs there must not be decided by coordinates that do not carry it (integers, so
+    exactly)."""
     rng = np.random.default_rng(18)
     n = 16_000
     lat = rng.uniform(*band, n).astype(np.float32)
