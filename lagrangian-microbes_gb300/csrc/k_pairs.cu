@@ -216,6 +216,7 @@ __global__ void __launch_bounds__(SLOT_BLOCK, 6) k_sweep(Bufs b, PairParams pp, 
       need |= t > s ? 1u << k : 0u;  // the endpoint below in cell order applies the pair
     }
   }
+  const bool few = __all_sync(0xffffffffu, mk <= 4);
   if (mk > 1) {
     // each of the first W slots against each: the one that loses moves back a place
 #define LM_PLACES(W)                                              \
@@ -225,7 +226,7 @@ __global__ void __launch_bounds__(SLOT_BLOCK, 6) k_sweep(Bufs b, PairParams pp, 
       tie |= key[i] == key[j];                                    \
     }                                                             \
   }
-    if (__all_sync(__activemask(), mk <= 4)) {
+    if (few) {
       LM_PLACES(4)
     } else {
       LM_PLACES(8)
