@@ -175,27 +175,6 @@ __global__ void k_dh_species_segs(DhCtl* ctl, DhSeg* segs) {
   ctl->n_items = items;
 }
 
-// Index of cell (x, y) of a 2^bits x 2^bits grid along Hilbert's curve (level by level from the coarsest:
-// the quadrant's place on the curve, then the coordinates turned into the quadrant's own frame).
-__device__ __forceinline__ uint32_t dh_hilbert(uint32_t x, uint32_t y, int bits) {
-  uint32_t d = 0;
-  for (int k = bits - 1; k >= 0; --k) {
-    const uint32_t rx = (x >> k) & 1u, ry = (y >> k) & 1u;
-    d = (d << 2) | ((3u * rx) ^ ry);
-    if (!ry) {
-      if (rx) {
-        const uint32_t m = (2u << k) - 1u;
-        x = ~x & m;
-        y = ~y & m;
-      }
-      const uint32_t t = x;
-      x = y;
-      y = t;
-    }
-  }
-  return d;
-}
-
 // Sort key: segment, then the point's place along Hilbert's curve over the common bounding box (mb
 // bits). Any order of the points gives the same counts; this one makes the leaves small (8 points of a
 // lattice's species span 0.032 degrees on average, 0.055 in Morton order).
@@ -214,7 +193,7 @@ __global__ void __launch_bounds__(256) k_dh_key(const float* __restrict__ lat, c
     // a zero extent or an overflowing one gives NaN or 0 here, which the clamp takes to cell 0
     const uint32_t qa = (uint32_t)fminf(fmaxf((lat[i] - a0) / wa * cells, 0.f), cells - 1.f);
     const uint32_t qo = (uint32_t)fminf(fmaxf((lon[i] - o0) / wo * cells, 0.f), cells - 1.f);
-    m = dh_hilbert(qa, qo, mb / 2);
+    m = hilbert_place(qa, qo, mb / 2);
   }
   key[i] = (s << mb) | m;
 }

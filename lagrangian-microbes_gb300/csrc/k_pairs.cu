@@ -365,22 +365,6 @@ __device__ __forceinline__ void count_runs(const Vertex& v, const Bufs& b, uint3
   }
 }
 
-// Place of sub-cell (x, y) of a 32 x 32 grid along Hilbert's curve.
-__device__ __forceinline__ uint32_t hilbert32(uint32_t x, uint32_t y) {
-  uint32_t d = 0;
-#pragma unroll
-  for (int k = 4; k >= 0; --k) {
-    const uint32_t rx = (x >> k) & 1u, ry = (y >> k) & 1u;
-    d = (d << 2) | ((3u * rx) ^ ry);
-    if (!ry) {  // into the quadrant's own frame: mirrored when it is the last one, and transposed
-      const uint32_t m = rx ? (2u << k) - 1u : 0u, t = x ^ m;
-      x = y ^ m;
-      y = t;
-    }
-  }
-  return d;
-}
-
 // The members of every dense cell (listed in act by k_scatter) in the order of their 32 x 32 sub-cells
 // along the curve: a counting sort through shared memory, one block per cell, by way of `tmp` (the
 // state words, unused here). Only the positions move: counting needs no ids.
@@ -401,7 +385,7 @@ __global__ void __launch_bounds__(ORDER_THREADS) k_count_order(Bufs b, Ctrl* ctr
     auto sub = [&](float2 p) {  // any assignment is valid, so the clamps only keep it in range
       const uint32_t x = (uint32_t)fminf(fmaxf((p.x - ox) * scale, 0.f), 31.f);
       const uint32_t y = (uint32_t)fminf(fmaxf((p.y - oy) * scale, 0.f), 31.f);
-      return hilbert32(x, y);
+      return hilbert_place(x, y, 5);
     };
     for (uint32_t i = threadIdx.x; i < ORDER_BINS; i += ORDER_THREADS) cnt[i] = 0;
     __syncthreads();
@@ -625,9 +609,9 @@ void launch_count_pairs(const Bufs& b, const PairParams& pp, Ctrl* ctrl, int sms
 // are uniform hashes, so 256 buckets on their top 8 bits (descending) hold about d / 256 entries each, and
 // an insertion sort inside each bucket by the exact order finishes it; beyond, buckets in global memory.
 // Only the sorted partners are kept (the priorities were needed for the order only).
-// Bound by instruction issue (73 % of the slots, 670 instructions a list of 34). A warp per list before
+// Bound by instruction issue (76 % of the slots, 645 instructions a list of 34). A warp per list before
 // took 530 us for the 447,000 lists of 32 ensembles, 245 for the 338,000 of 2,000,000 mixed microbes and 66
-// for the 81,000 of 490,000; this takes 368, 133 and 40. At 6 blocks an SM (9 KB a warp) it took 438,
+// for the 81,000 of 490,000; this takes 366, 132 and 40. At 6 blocks an SM (9 KB a warp) it took 438,
 // 194 and 54. 10,000 microbes with 1,100 neighbours each 21.4 -> 1.0 ms (one lane sorted such lists before).
 constexpr int LONG_WARPS = 4;
 constexpr uint32_t LONG_SMEM_MAX = 512;

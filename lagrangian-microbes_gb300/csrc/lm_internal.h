@@ -457,6 +457,22 @@ struct ScratchCall {
   ~ScratchCall() { ctx_scratch_done(c); }
 };
 
+// Place of cell (x, y) of a 2^bits x 2^bits grid along Hilbert's curve (level by level from the coarsest: the quadrant's
+// place on the curve, then the coordinates turned into the quadrant's own frame).
+__device__ __forceinline__ uint32_t hilbert_place(uint32_t x, uint32_t y, int bits) {
+  uint32_t d = 0;
+  for (int k = bits - 1; k >= 0; --k) {
+    const uint32_t rx = (x >> k) & 1u, ry = (y >> k) & 1u;
+    d = (d << 2) | ((3u * rx) ^ ry);
+    if (!ry) {  // mirrored in the last quadrant, and transposed
+      const uint32_t m = rx ? (2u << k) - 1u : 0u, t = x ^ m;
+      x = y ^ m;
+      y = t;
+    }
+  }
+  return d;
+}
+
 // Ordered-int encoding of floats for atomicMin/atomicMax.
 __host__ __device__ inline uint32_t enc_f(float f) {
   uint32_t u;
