@@ -1,6 +1,7 @@
 // K6 + K7: adjoint of the RK4 advection. The reference has no differentiation; the forward scheme
 // is the one of K1 (particle_advecter.py:177-187, 220-223), shared through lm_field.cuh so that
-// recomputed trajectories are bit-identical to lm_step's.
+// float32 trajectories are bit-identical to lm_step's; in every precision the backward recomputes its own
+// forward's.
 //
 // K6 k_adj_step: one thread per microbe takes x_m (recomputed from a checkpoint) and the adjoint
 // lambda_{m+1} = dL/dx_{m+1}, and returns lambda_m by running the four RK4 stages forward and
