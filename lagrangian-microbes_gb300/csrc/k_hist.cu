@@ -568,6 +568,9 @@ __device__ __forceinline__ void dh_load_tile(const float4* __restrict__ pts, con
   }
 }
 
+// SHARED_OUT: fewer items than blocks are shared out by parts, the groups of tile J in turn, so that all blocks have
+// work (one form for both took 0.5 % more at 490,000).
+template <bool SHARED_OUT>
 __global__ void __launch_bounds__(DH_THREADS, 8) k_dist_hist(const float4* __restrict__ pts,
                                                           const float4* __restrict__ vec,
                                                           const DhTile* __restrict__ tiles,
@@ -583,7 +586,9 @@ __global__ void __launch_bounds__(DH_THREADS, 8) k_dist_hist(const float4* __res
   for (int q = threadIdx.x; q < DH_WARPS * nb * DH_COPIES; q += DH_THREADS) hist[q] = 0;
   for (int q = threadIdx.x; q < rule.bins; q += DH_THREADS) thr[q] = rule.thr[q];
   uint32_t* mine = hist + (size_t)warp * nb * DH_COPIES + (lane & (DH_COPIES - 1));
-  const unsigned long long n_items = ctl->n_items;
+  uint32_t cut = 0;  // 2^cut parts an item
+  while (SHARED_OUT && cut < 3u && (ctl->n_items << (cut + 1u)) <= gridDim.x) ++cut;
+  const unsigned long long n_items = ctl->n_items << cut;
   // consecutive items share their tile J; a share small enough that the last blocks do not wait long
   const unsigned long long share = min(8ull, max(1ull, n_items / (8ull * gridDim.x)));
   int cur = -1;
@@ -598,7 +603,7 @@ __global__ void __launch_bounds__(DH_THREADS, 8) k_dist_hist(const float4* __res
     bool have_j = false;
     for (unsigned long long w = w0; w < w1; ++w) {
       int sg = cur < 0 ? 0 : cur;  // a block's items come in segment order
-      while (sg + 1 < (int)n_seg && w >= segs[sg + 1].item0) ++sg;
+      while (sg + 1 < (int)n_seg && (w >> cut) >= segs[sg + 1].item0) ++sg;
       if (sg != cur || since >= DH_FLUSH) {  // block-uniform
         if (cur >= 0) dh_flush(hist, nb, counts + (size_t)cur * nb);
         if (sg != cur) J = ~0ull;
@@ -608,13 +613,13 @@ __global__ void __launch_bounds__(DH_THREADS, 8) k_dist_hist(const float4* __res
       const DhSeg S = segs[sg];
       if (J == ~0ull) {
         // item t of the segment is tile pair (I, J) with J (J + 1) / 2 <= t < (J + 1) (J + 2) / 2
-        const unsigned long long t = w - S.item0;
+        const unsigned long long t = (w >> cut) - S.item0;
         J = (unsigned long long)((sqrtf(8.0f * (float)t + 1.0f) - 1.0f) * 0.5f);
         while (J * (J + 1) / 2 > t) --J;
         while ((J + 1) * (J + 2) / 2 <= t) ++J;
         I = t - J * (J + 1) / 2;
         have_j = false;
-      } else if (++I > J) {
+      } else if ((w & ((1u << cut) - 1u)) == 0u && ++I > J) {
         ++J;
         I = 0;
         have_j = false;
@@ -645,7 +650,7 @@ __global__ void __launch_bounds__(DH_THREADS, 8) k_dist_hist(const float4* __res
       // pairs of 32-point groups
       for (uint32_t g = threadIdx.x; g < gi * gj; g += DH_THREADS) {
         const uint32_t a = g % gi, b = g / gi;
-        if (diagonal && a > b) continue;
+        if ((diagonal && a > b) || ((b ^ (uint32_t)w) & ((1u << cut) - 1u))) continue;
         const DhBox u = dh_group_box(sh.leaf[0], a, lvi), v = dh_group_box(sh.leaf[sj], b, lvj);
         if (!dh_near(u, v)) sh.wide = 1u;
         float lo, hi;
@@ -815,11 +820,19 @@ int dh_run(lm_ctx* c, const float* lat, const float* lon, const int8_t* species,
   k_dh_gather<<<(unsigned)n_tiles, DH_TILE, 0, st>>>(dlat, dlon, sval, dseg, n_seg, pts, vec, tiles);
   const size_t smem = (size_t)DH_WARPS * nb * DH_COPIES * sizeof(uint32_t) + (size_t)bins * sizeof(float2);
   int per_sm = 0;
-  if ((r = dh_cuda(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_dist_hist, DH_THREADS, smem))))
+  if ((r = dh_cuda(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_dist_hist<false>, DH_THREADS, smem))))
     return r;
-  const unsigned long long most = species ? dh_items(n) + 3ull : hc.n_items;  // (a bound when the counts are on the device)
-  const unsigned blocks = (unsigned)std::min<unsigned long long>(most, (unsigned long long)std::max(per_sm, 1) * sms);
-  k_dist_hist<<<blocks, DH_THREADS, smem, st>>>(pts, vec, tiles, dseg, n_seg, dctl, rule, dcnt);
+  // bounds of the items when the counts are on the device (even thirds, one species). With at most half as many as
+  // blocks, whole items leave SMs idle: 3,000 points on the globe 368 us so and 207 shared out (357 pair by pair), at
+  // one place 470 and 200 (406), 300 on the globe 258 and 162; from 17,000 on, all blocks have items.
+  const unsigned long long least = species ? 3 * dh_items(n / 3) : hc.n_items, most = species ? dh_items(n) + 3 : hc.n_items;
+  const unsigned long long fit = (unsigned long long)std::max(per_sm, 1) * sms;
+  if (2 * least <= fit)
+    k_dist_hist<true><<<(unsigned)std::min(most * DH_GROUPS, fit), DH_THREADS, smem, st>>>(pts, vec, tiles, dseg, n_seg,
+                                                                                         dctl, rule, dcnt);
+  else
+    k_dist_hist<false><<<(unsigned)std::min(most, fit), DH_THREADS, smem, st>>>(pts, vec, tiles, dseg, n_seg, dctl, rule,
+                                                                                dcnt);
   if ((r = dh_cuda(c, cudaGetLastError()))) return r;
   std::vector<uint64_t> out(out_n);
   if ((r = dh_cuda(c, cudaMemcpyAsync(out.data(), dcnt, out_n * sizeof(uint64_t), cudaMemcpyDeviceToHost, st))) ||

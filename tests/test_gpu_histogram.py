@@ -207,6 +207,25 @@ def test_points_around_a_pole_keep_the_reference_chain_bins(pdh, monkeypatch, ba
     assert fast[1] == exact[1]
 
 
+@pytest.mark.parametrize("n", [4096, 4097, 6145, 8705])
+def test_few_tile_pairs_are_shared_out_by_their_groups(pdh, orc, n):
+    """Calls of up to 608 pairs of tiles split them among the blocks: by eight up to 152, by four up to 304, by two. The
+    sizes lie at those limits (17, 25 and 35 tiles are beyond them); the parts of a call per species differ from those of
+    each species alone."""
+    rng = np.random.default_rng(n)
+    lat, lon = rng.uniform(-80, 80, n).astype(np.float32), rng.uniform(-180, 180, n).astype(np.float32)
+    lat[: n // 3], lon[: n // 3] = _points(rng, n // 3, box=(25.0, 26.0, 200.0, 201.0))
+    counts, over = pdh.pairwise_distance_histogram(lat, lon, 70)
+    d, a = orc.distance_histogram(lat, lon, 70)
+    assert orc.histogram_consistent(_full(counts, over), d, a)
+    species = rng.choice([1, 2, 2, 3, 3, 3], n).astype(np.int8)
+    got = pdh.species_distance_histograms(lon, lat, species, 70)
+    for k in (1, 2, 3):
+        alone = pdh.pairwise_distance_histogram(lat[species == k], lon[species == k], 70)
+        np.testing.assert_array_equal(got[k][0], alone[0])
+        assert got[k][1] == alone[1]
+
+
 def test_a_large_calls_working_memory_goes_back(pdh, lm):
     """8 million points without a species (no pairs) need some 550 MB of working arrays; the context keeps 64 MB at most
     for its next call."""
