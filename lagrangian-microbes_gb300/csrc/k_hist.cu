@@ -14,7 +14,7 @@
 //
 //   * work items are the tiles (I, J), I <= J, of 256 x 256 sorted points of a segment; a block loads
 //     both tiles (latitude, longitude, cos(latitude), index) and the boxes of their 8-point leaves
-//     into shared memory;
+//     into shared memory (few of them are shared out by groups of J);
 //   * the haversine a = sin^2(dlat / 2) + cos cos sin^2(dlon / 2) of a pair of boxes is bounded from
 //     the extremes of dlat, dlon and cos(latitude), first for the 8 x 8 pairs of 32-point groups,
 //     then for the leaf pairs of the groups that are left. If every a of a pair of groups lies inside
